@@ -12,6 +12,6 @@ _DEFAULT = "/root/reference"
 
 
 def reference_root():
-    """The reference tree's root, or None when it is not present."""
+    """The reference tree's root, or None when it is not present (or empty)."""
     p = os.environ.get(ENV, _DEFAULT)
-    return p if p and os.path.isdir(p) else None
+    return p if p and os.path.isdir(p) and os.listdir(p) else None
