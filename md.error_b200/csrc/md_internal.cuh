@@ -116,6 +116,9 @@ struct md_system {
   // pinned host staging
   void* h_stage = nullptr;
   size_t h_stage_bytes = 0;
+  // device staging of the calls that copy to or from the host (sys_scratch)
+  void* d_stage = nullptr;
+  size_t d_stage_bytes = 0;
   // atom types (TypeType of the reference): by original id and by current
   // slot (refreshed by every cell sort); 0 for every atom unless given
   uint8_t* type_by_id = nullptr;
@@ -193,6 +196,18 @@ struct md_engine {
 };
 // per-atom correction values (by atom id) of an md_fcorr
 const double4a* fcorr_values(const md_fcorr* f);
+
+// Device workspace of one host-synchronising call on the system's stream:
+// *p holds `bytes` until the next sys_scratch of this system, or until
+// sys_scratch_done when *owned is set.  Up to SYS_SCRATCH_KEEP the system keeps
+// the buffer and frees it when it is destroyed: a stream-ordered allocation
+// per call had the pool return its memory at every synchronisation and map it
+// again, about 250 us of host time for 1.5 MB (frames of the 4,000-atom fluid
+// read after 50 steps: two such calls in 2.0 ms).  Larger requests are
+// allocated and freed with the call.
+constexpr size_t SYS_SCRATCH_KEEP = 64u << 20;
+int sys_scratch(md_system* s, size_t bytes, void** p, bool* owned);
+int sys_scratch_done(md_system* s, void* p, bool owned);
 
 // launch helper: direct launch or kernel-node recording ---------------------
 struct Recorder {

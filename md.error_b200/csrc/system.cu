@@ -242,6 +242,31 @@ static int ensure_stage(md_system* s, size_t bytes) {
   return MD_OK;
 }
 
+int sys_scratch(md_system* s, size_t bytes, void** p, bool* owned) {
+  *p = nullptr;
+  *owned = bytes > SYS_SCRATCH_KEEP;
+  if (*owned) {
+    MD_CUDA(cudaMallocAsync(p, bytes, s->stream));
+    return MD_OK;
+  }
+  if (s->d_stage_bytes < bytes) {
+    MD_CUDA(cudaSetDevice(s->device));
+    MD_CUDA(cudaStreamSynchronize(s->stream));  // the old buffer's last use
+    if (s->d_stage) cudaFree(s->d_stage);
+    s->d_stage = nullptr;
+    s->d_stage_bytes = 0;
+    MD_CUDA(cudaMalloc(&s->d_stage, bytes));
+    s->d_stage_bytes = bytes;
+  }
+  *p = s->d_stage;
+  return MD_OK;
+}
+
+int sys_scratch_done(md_system* s, void* p, bool owned) {
+  if (owned && p) MD_CUDA(cudaFreeAsync(p, s->stream));
+  return MD_OK;
+}
+
 __global__ void k_type_slot(int N, const int* __restrict__ id, const uint8_t* __restrict__ by_id,
                             uint8_t* __restrict__ by_slot, const DevState* st, int gate) {
   if (gate && !(st->flags & FLAG_REBUILD)) return;
@@ -376,7 +401,7 @@ extern "C" int md_system_destroy(md_system* s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   void* ptrs[] = {s->pos, s->vel, s->force, s->image, s->id, s->rcut, s->t_pos, s->t_vel,
                   s->t_force, s->t_image, s->t_id, s->t_rcut, s->st, s->partials, s->nb_rows, s->d_lattice,
-                  s->type_by_id, s->type};
+                  s->type_by_id, s->type, s->d_stage};
   for (void* p : ptrs) if (p) cudaFree(p);
   topo_destroy(s->topo);
   if (s->h_stage) cudaFreeHost(s->h_stage);
@@ -419,8 +444,10 @@ static int download(md_system* s, int what, double* out) {
   if (int r = check_sys(s)) return r;
   if (!out) return MD_ERR_BADARG;
   size_t bytes = sizeof(double) * 3 * (size_t)s->N;
-  double* d = nullptr;
-  MD_CUDA(cudaMallocAsync((void**)&d, bytes, s->stream));
+  void* buf;
+  bool owned;
+  if (int r = sys_scratch(s, bytes, &buf, &owned)) return r;
+  double* d = (double*)buf;
   int nb = ceil_div(s->N, 256);
   if (s->prec == MD_PREC_FP64)
     k_download<double><<<nb, 256, 0, s->stream>>>(s->N, what, (double4a*)s->pos, (double4a*)s->vel, s->force, s->image, s->id, s->st, d);
@@ -429,7 +456,7 @@ static int download(md_system* s, int what, double* out) {
   MD_CHECK_LAUNCH("download");
   if (int r = ensure_stage(s, bytes)) return r;
   MD_CUDA(cudaMemcpyAsync(s->h_stage, d, bytes, cudaMemcpyDeviceToHost, s->stream));
-  MD_CUDA(cudaFreeAsync(d, s->stream));
+  if (int r = sys_scratch_done(s, buf, owned)) return r;
   MD_CUDA(cudaStreamSynchronize(s->stream));
   memcpy(out, s->h_stage, bytes);
   return MD_OK;
@@ -444,8 +471,10 @@ static int upload_vec(md_system* s, int what, const double* in) {
   if (int r = ensure_stage(s, bytes)) return r;
   MD_CUDA(cudaStreamSynchronize(s->stream));
   memcpy(s->h_stage, in, bytes);
-  double* d = nullptr;
-  MD_CUDA(cudaMallocAsync((void**)&d, bytes, s->stream));
+  void* buf;
+  bool owned;
+  if (int r = sys_scratch(s, bytes, &buf, &owned)) return r;
+  double* d = (double*)buf;
   MD_CUDA(cudaMemcpyAsync(d, s->h_stage, bytes, cudaMemcpyHostToDevice, s->stream));
   int nb = ceil_div(s->N, 256);
   if (s->prec == MD_PREC_FP64)
@@ -453,7 +482,7 @@ static int upload_vec(md_system* s, int what, const double* in) {
   else
     k_set_vec<float><<<nb, 256, 0, s->stream>>>(s->N, what, d, s->id, (float4*)s->pos, (float4*)s->vel);
   MD_CHECK_LAUNCH("set vec");
-  MD_CUDA(cudaFreeAsync(d, s->stream));
+  if (int r = sys_scratch_done(s, buf, owned)) return r;
   MD_CUDA(cudaStreamSynchronize(s->stream));
   return MD_OK;
 }
@@ -477,8 +506,10 @@ static int charge_io(md_system* s, int dir, double* q, int what = 0) {
   const size_t bytes = sizeof(double) * (size_t)s->N;
   if (int r = ensure_stage(s, bytes)) return r;
   MD_CUDA(cudaStreamSynchronize(s->stream));
-  double* d = nullptr;
-  MD_CUDA(cudaMallocAsync((void**)&d, bytes, s->stream));
+  void* buf;
+  bool owned;
+  if (int r = sys_scratch(s, bytes, &buf, &owned)) return r;
+  double* d = (double*)buf;
   if (dir == 0) {
     memcpy(s->h_stage, q, bytes);
     MD_CUDA(cudaMemcpyAsync(d, s->h_stage, bytes, cudaMemcpyHostToDevice, s->stream));
@@ -496,7 +527,7 @@ static int charge_io(md_system* s, int dir, double* q, int what = 0) {
   }
   MD_CHECK_LAUNCH("charge / mass io");
   if (dir == 1) MD_CUDA(cudaMemcpyAsync(s->h_stage, d, bytes, cudaMemcpyDeviceToHost, s->stream));
-  MD_CUDA(cudaFreeAsync(d, s->stream));
+  if (int r = sys_scratch_done(s, buf, owned)) return r;
   MD_CUDA(cudaStreamSynchronize(s->stream));
   if (dir == 1) memcpy(q, s->h_stage, bytes);
   return MD_OK;
@@ -545,14 +576,16 @@ extern "C" int md_system_set_box(md_system* s, const double box[3]) {
 static int rcut_io(md_system* s, int dir, float* host) {
   if (int r = check_sys(s)) return r;
   if (!host) return MD_ERR_BADARG;
-  float* d = nullptr;
   size_t bytes = sizeof(float) * s->N;
-  MD_CUDA(cudaMallocAsync((void**)&d, bytes, s->stream));
+  void* buf;
+  bool owned;
+  if (int r = sys_scratch(s, bytes, &buf, &owned)) return r;
+  float* d = (float*)buf;
   if (dir == 0) MD_CUDA(cudaMemcpyAsync(d, host, bytes, cudaMemcpyHostToDevice, s->stream));
   k_rcut_io<<<ceil_div(s->N, 256), 256, 0, s->stream>>>(s->N, dir, s->rcut, s->id, d);
   MD_CHECK_LAUNCH("rcut io");
   if (dir == 1) MD_CUDA(cudaMemcpyAsync(host, d, bytes, cudaMemcpyDeviceToHost, s->stream));
-  MD_CUDA(cudaFreeAsync(d, s->stream));
+  if (int r = sys_scratch_done(s, buf, owned)) return r;
   MD_CUDA(cudaStreamSynchronize(s->stream));
   return MD_OK;
 }
