@@ -1,10 +1,9 @@
-// Smooth particle-mesh Ewald (reciprocal part) and the exact Ewald sum.
+// Smooth particle-mesh Ewald (reciprocal part).
 // Reference (RE = longRange.hetero/profile.test/template/tools/real.error):
 //   calQ spread                      RE/src/EleRecBSpline.cpp:541-619
 //   calB / calPsiFPhiF (ik)          RE/src/EleRecBSpline.cpp:729-877
 //   applyInteractionCalPotential ik  RE/src/EleRecBSpline.cpp:393-536
 //   analytic differentiation         RE/src/EleRecFBSpline.cpp:771-907, 1146-1195
-//   exact reciprocal sum (ES)        RE/src/EleRecES.cpp:49-144
 //
 // Chain of one force evaluation (each step one kernel):
 //   spread      charges into a shared-memory tile per block of 64 charges,
@@ -1140,82 +1139,6 @@ k_selfcorr_apply(int N, const typename V4<R>::T* __restrict__ pos, int K0, int K
   force[i] = F;
 }
 
-// ---------------------------------------------------------------- exact Ewald (FP64)
-// S(m) = sum_i q_i exp(2 pi i m.r_i) for every m of the |m_d| <= K_d/2 box
-// (EleRecES::calPotential), then E = sum_m e^{-pi^2 m^2/beta^2}/m^2 |S|^2 / (2 pi V)
-// and F_i = sum_m (2/V) e^{..}/m^2 (S_r q_i sin - S_i q_i cos) m (applyInteraction).
-__global__ void k_ewald_sk(int N, const double4a* __restrict__ pos, const float4* __restrict__ posf, int prec,
-                           int M0, int M1, int M2, const DevState* st, double2* __restrict__ S) {
-  const long nm = (long)(2 * M0 + 1) * (2 * M1 + 1) * (2 * M2 + 1);
-  const long mi = blockIdx.x;
-  if (mi >= nm) return;
-  const int m2 = (int)(mi % (2 * M2 + 1)) - M2, m1 = (int)((mi / (2 * M2 + 1)) % (2 * M1 + 1)) - M1,
-            m0 = (int)(mi / ((long)(2 * M2 + 1) * (2 * M1 + 1))) - M0;
-  const double m[3] = {m0 * st->Li[0], m1 * st->Li[1], m2 * st->Li[2]};
-  double sr = 0, si = 0;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    double x, y, z, q;
-    if (prec == MD_PREC_FP64) { const double4a p = pos[i]; x = p.x; y = p.y; z = p.z; q = p.w; }
-    else { const float4 p = posf[i]; x = p.x; y = p.y; z = p.z; q = p.w; }
-    double s, c;
-    sincospi(2.0 * (m[0] * x + m[1] * y + m[2] * z), &s, &c);
-    sr += q * c;
-    si += q * s;
-  }
-  double v[2] = {sr, si};
-  __shared__ double red[32][2];
-  for (int o = 16; o > 0; o >>= 1) {
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-    v[1] += __shfl_xor_sync(0xffffffffu, v[1], o);
-  }
-  if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5][0] = v[0]; red[threadIdx.x >> 5][1] = v[1]; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0, b = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { a += red[w][0]; b += red[w][1]; }
-    S[mi] = make_double2(a, b);
-  }
-}
-
-__global__ void k_ewald_force(int N, const double4a* __restrict__ pos, const float4* __restrict__ posf, int prec,
-                              int M0, int M1, int M2, double beta, const DevState* st, const double2* __restrict__ S,
-                              double4a* __restrict__ force, int add_forces, double* partials, unsigned* counter,
-                              double* energy) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const long nm = (long)(2 * M0 + 1) * (2 * M1 + 1) * (2 * M2 + 1);
-  const double V = st->L[0] * st->L[1] * st->L[2];
-  const double sc = M_PI * M_PI / (beta * beta);
-  double x = 0, y = 0, z = 0, q = 0;
-  if (i < N) {
-    if (prec == MD_PREC_FP64) { const double4a p = pos[i]; x = p.x; y = p.y; z = p.z; q = p.w; }
-    else { const float4 p = posf[i]; x = p.x; y = p.y; z = p.z; q = p.w; }
-  }
-  double fx = 0, fy = 0, fz = 0, e = 0;
-  for (long mi = 0; mi < nm; ++mi) {
-    const int m2 = (int)(mi % (2 * M2 + 1)) - M2, m1 = (int)((mi / (2 * M2 + 1)) % (2 * M1 + 1)) - M1,
-              m0 = (int)(mi / ((long)(2 * M2 + 1) * (2 * M1 + 1))) - M0;
-    if (!m0 && !m1 && !m2) continue;
-    const double m[3] = {m0 * st->Li[0], m1 * st->Li[1], m2 * st->Li[2]};
-    const double mm = m[0] * m[0] + m[1] * m[1] + m[2] * m[2];
-    const double ex = exp(-sc * mm) / mm;
-    const double2 s = S[mi];
-    if (i == 0) e += ex * (s.x * s.x + s.y * s.y);
-    if (i < N) {
-      double sn, cs;
-      sincospi(2.0 * (m[0] * x + m[1] * y + m[2] * z), &sn, &cs);
-      const double coeff = (s.x * q * sn - s.y * q * cs) * 2.0 / V * ex;
-      fx += coeff * m[0]; fy += coeff * m[1]; fz += coeff * m[2];
-    }
-  }
-  if (i < N && add_forces) {
-    double4a f = force[i];
-    f.x += fx; f.y += fy; f.z += fz;
-    force[i] = f;
-  }
-  if (i == 0) *energy = e / (2.0 * M_PI * V);
-  (void)partials; (void)counter;
-}
-
 // ---------------------------------------------------------------- host
 template <class R, int LOGN>
 static const void* fftp_fn_n(int mode, int sign, int out4) {
@@ -1668,28 +1591,3 @@ extern "C" int md_ewald_self_energy(md_system* sys, double beta, double* out) {
   }
   return MD_OK;
 }
-
-extern "C" int md_ewald_exact(md_system* sys, const int K[3], double beta, double* energy, int add_forces) {
-  if (!sys || !K || !(beta > 0)) return MD_ERR_BADARG;
-  const int M0 = K[0] / 2, M1 = K[1] / 2, M2 = K[2] / 2;
-  const long nm = (long)(2 * M0 + 1) * (2 * M1 + 1) * (2 * M2 + 1);
-  double2* S = nullptr;
-  double* e = nullptr;
-  MD_CUDA(cudaMallocAsync((void**)&S, sizeof(double2) * nm, sys->stream));
-  MD_CUDA(cudaMallocAsync((void**)&e, sizeof(double), sys->stream));
-  k_ewald_sk<<<(unsigned)nm, 256, 0, sys->stream>>>(sys->N, (double4a*)sys->pos, (float4*)sys->pos, sys->prec, M0, M1,
-                                                     M2, sys->st, S);
-  MD_CHECK_LAUNCH("ewald sk");
-  k_ewald_force<<<ceil_div(sys->N, 128), 128, 0, sys->stream>>>(sys->N, (double4a*)sys->pos, (float4*)sys->pos,
-                                                                 sys->prec, M0, M1, M2, beta, sys->st, S, sys->force,
-                                                                 add_forces, nullptr, nullptr, e);
-  MD_CHECK_LAUNCH("ewald force");
-  double h = 0;
-  MD_CUDA(cudaMemcpyAsync(&h, e, sizeof(double), cudaMemcpyDeviceToHost, sys->stream));
-  MD_CUDA(cudaFreeAsync(S, sys->stream));
-  MD_CUDA(cudaFreeAsync(e, sys->stream));
-  MD_CUDA(cudaStreamSynchronize(sys->stream));
-  if (energy) *energy = h;
-  return MD_OK;
-}
-
