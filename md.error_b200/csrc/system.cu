@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 #include "device_common.cuh"
 
@@ -242,6 +243,53 @@ static int ensure_stage(md_system* s, size_t bytes) {
   return MD_OK;
 }
 
+struct DevicePool {
+  cudaMemPool_t pool = nullptr;
+  int users = 0;
+  void* host = nullptr;  // page-locked staging shared by the device's systems, one lease at a time
+  size_t host_bytes = 0;
+  bool host_busy = false;
+};
+static std::mutex g_pool_mutex;
+static DevicePool g_pool[64];
+
+int pool_retain(int device) {
+  if (device < 0 || device >= 64) { md_set_error("device %d out of range", device); return MD_ERR_BADARG; }
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  DevicePool& d = g_pool[device];
+  if (!d.pool) {
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    MD_CUDA(cudaMemPoolCreate(&d.pool, &props));
+    unsigned long long keep = POOL_KEEP;
+    MD_CUDA(cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  }
+  d.users += 1;
+  return MD_OK;
+}
+
+void pool_release(int device) {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  DevicePool& d = g_pool[device];
+  if (--d.users > 0) return;
+  cudaMemPoolTrimTo(d.pool, 0);
+  if (d.host && !d.host_busy) {
+    cudaFreeHost(d.host);
+    d.host = nullptr;
+    d.host_bytes = 0;
+  }
+}
+
+int pool_alloc(int device, size_t bytes, cudaStream_t stream, void** p) {
+  MD_CUDA(cudaMallocFromPoolAsync(p, bytes, g_pool[device].pool, stream));
+  return MD_OK;
+}
+
+void pool_free(int, void* p, cudaStream_t stream) { cudaFreeAsync(p, stream); }
+
 int sys_scratch(md_system* s, size_t bytes, void** p, bool* owned) {
   *p = nullptr;
   *owned = bytes > SYS_SCRATCH_KEEP;
@@ -250,12 +298,11 @@ int sys_scratch(md_system* s, size_t bytes, void** p, bool* owned) {
     return MD_OK;
   }
   if (s->d_stage_bytes < bytes) {
-    MD_CUDA(cudaSetDevice(s->device));
     MD_CUDA(cudaStreamSynchronize(s->stream));  // the old buffer's last use
-    if (s->d_stage) cudaFree(s->d_stage);
+    if (s->d_stage) pool_free(s->device, s->d_stage, s->stream);
     s->d_stage = nullptr;
     s->d_stage_bytes = 0;
-    MD_CUDA(cudaMalloc(&s->d_stage, bytes));
+    if (int r = pool_alloc(s->device, bytes, s->stream, &s->d_stage)) return r;
     s->d_stage_bytes = bytes;
   }
   *p = s->d_stage;
@@ -264,6 +311,65 @@ int sys_scratch(md_system* s, size_t bytes, void** p, bool* owned) {
 
 int sys_scratch_done(md_system* s, void* p, bool owned) {
   if (owned && p) MD_CUDA(cudaFreeAsync(p, s->stream));
+  return MD_OK;
+}
+
+// Page-locked memory for one read-back: the device's shared buffer (grown up
+// to SYS_SCRATCH_KEEP, freed with the last system) unless another thread holds
+// it, then the system's own; none (p null) where neither can be had.  Locking
+// pages takes about 1 ms per MB, which every new system would pay on its
+// first frame.
+struct HostLease {
+  void* p = nullptr;
+  int device = -1;
+  HostLease(md_system* s, size_t bytes) {
+    if (bytes > SYS_SCRATCH_KEEP) return;
+    {
+      std::lock_guard<std::mutex> lock(g_pool_mutex);
+      DevicePool& d = g_pool[s->device];
+      if (!d.host_busy) {
+        if (d.host_bytes < bytes) {
+          if (d.host) cudaFreeHost(d.host);
+          d.host = nullptr;
+          d.host_bytes = 0;
+          if (cudaMallocHost(&d.host, bytes) == cudaSuccess) d.host_bytes = bytes;
+          else { cudaGetLastError(); d.host = nullptr; }
+        }
+        if (d.host) {
+          d.host_busy = true;
+          device = s->device;
+          p = d.host;
+        }
+      }
+    }
+    if (!p && ensure_stage(s, bytes) == MD_OK) p = s->h_stage;
+  }
+  ~HostLease() {
+    if (device < 0) return;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    g_pool[device].host_busy = false;
+  }
+};
+
+int sys_read_back(md_system* s, cudaStream_t stream, void* const* dst, const void* const* src, const size_t* bytes,
+                  int n) {
+  size_t total = 0;
+  for (int k = 0; k < n; ++k) total += (bytes[k] + 15) & ~(size_t)15;
+  HostLease lease(s, total);
+  char* stage = (char*)lease.p;
+  size_t at = 0;
+  for (int k = 0; k < n; ++k) {
+    void* to = stage ? stage + at : dst[k];
+    MD_CUDA(cudaMemcpyAsync(to, src[k], bytes[k], cudaMemcpyDeviceToHost, stream));
+    at += (bytes[k] + 15) & ~(size_t)15;
+  }
+  MD_CUDA(cudaStreamSynchronize(stream));
+  at = 0;
+  if (stage)
+    for (int k = 0; k < n; ++k) {
+      memcpy(dst[k], stage + at, bytes[k]);
+      at += (bytes[k] + 15) & ~(size_t)15;
+    }
   return MD_OK;
 }
 
@@ -342,6 +448,8 @@ extern "C" int md_system_create(md_system** out, int n, const double box[3], con
   s->device = device;
   int rc = MD_OK;
   auto fail = [&](int code) { md_system_destroy(s); return code; };
+  if (int r = pool_retain(device)) return fail(r);
+  s->pooled = true;
   if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(md_cuda_fail(cudaGetLastError(), "stream"));
   s->own_stream = true;
   size_t r4 = s->r4_size();
@@ -401,11 +509,14 @@ extern "C" int md_system_destroy(md_system* s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   void* ptrs[] = {s->pos, s->vel, s->force, s->image, s->id, s->rcut, s->t_pos, s->t_vel,
                   s->t_force, s->t_image, s->t_id, s->t_rcut, s->st, s->partials, s->nb_rows, s->d_lattice,
-                  s->type_by_id, s->type, s->d_stage};
+                  s->type_by_id, s->type};
   for (void* p : ptrs) if (p) cudaFree(p);
   topo_destroy(s->topo);
   if (s->h_stage) cudaFreeHost(s->h_stage);
+  // the stream is idle (synchronised above) and may be a caller's that is gone by now
+  if (s->d_stage) pool_free(s->device, s->d_stage, cudaStreamPerThread);
   if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
+  if (s->pooled) pool_release(s->device);
   delete s;
   return MD_OK;
 }
@@ -454,12 +565,11 @@ static int download(md_system* s, int what, double* out) {
   else
     k_download<float><<<nb, 256, 0, s->stream>>>(s->N, what, (float4*)s->pos, (float4*)s->vel, s->force, s->image, s->id, s->st, d);
   MD_CHECK_LAUNCH("download");
-  if (int r = ensure_stage(s, bytes)) return r;
-  MD_CUDA(cudaMemcpyAsync(s->h_stage, d, bytes, cudaMemcpyDeviceToHost, s->stream));
-  if (int r = sys_scratch_done(s, buf, owned)) return r;
-  MD_CUDA(cudaStreamSynchronize(s->stream));
-  memcpy(out, s->h_stage, bytes);
-  return MD_OK;
+  void* dst[1] = {out};
+  const void* src[1] = {d};
+  const int r = sys_read_back(s, s->stream, dst, src, &bytes, 1);
+  if (int q = sys_scratch_done(s, buf, owned)) return q;
+  return r;
 }
 
 static int upload_vec(md_system* s, int what, const double* in) {
