@@ -419,6 +419,9 @@ int md_errmap_ana_fconv(md_errmap* h, int k, double* out);
 /* print_meanf of the maps: the signed mean force error field
    e1_d = Re IFFT(k1_d FFT(rho1 V/N)) charge / V of the current profile, out [3][K0][K1][K2] */
 int md_errmap_mean_force(md_errmap* h, double charge, double* out);
+/* the RMS force error of every grid point, sqrt(error1[..][0] + error2[..][0] + self),
+   out [K0][K1][K2] (self: self_error * charge^4 of the analytic map, else 0) */
+int md_errmap_rms(md_errmap* h, double charge, double self, double* out);
 
 /* ------------------------------------------------------- per-atom cutoff
  * Replaces AssignRCut::getRCut + assign (ENG/src/AssignRCut.cu:46-117):

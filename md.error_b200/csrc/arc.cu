@@ -12,8 +12,7 @@
 // point of the k-grid octant runs the adaptive Gauss-4 quadrature (explicit
 // stack, same subdivision rule as the reference) for every rc interval and
 // writes the kernel values of all sign images.  The 3D transforms of the
-// (odd-sized) bin grid are batched direct DFTs along each axis with the line
-// and its twiddles in shared memory.  Error map, bisection and refinement are
+// (odd-sized) bin grid are the batched FP64 grid transforms of dft.cu.  Error map, bisection and refinement are
 // element-wise kernels; nothing returns to the host until asked.
 #include <cmath>
 #include <cstring>
@@ -228,176 +227,8 @@ __global__ void k_arc_tables(ArcDims g, const double* rc, const double* ints, do
   }
 }
 
-// ------------------------------------------------------------ batched DFT
-// One block per line; lines of all `batch` arrays of the grid along `axis`.
-// out[k] = sum_j in[j] exp(sign 2 pi i jk/n), in place.  n <= 1024.
-// A block takes `per` lines of one axis (several short lines per block, so
-// that lanes are not idle on 41-point lines).  A line of composite length
-// n = n1 n2 (n1 its smallest prime factor) is transformed in two stages
-// (Cooley-Tukey: n2 inner DFTs of length n1, the twiddles W_n^{j2 k1}, n1
-// DFTs of length n2), n (n1 + n2) products instead of n^2; a prime length
-// is summed directly.  All factors come from one table of W_n^m.
-__global__ void k_dft_axis(double2* data, ArcDims g, int axis, int sign, int batch, int n1, int per) {
-  extern __shared__ double2 sm[];
-  const int n = g.n[axis], n2 = n / n1;
-  double2* tw = sm;                  // [n]
-  double2* lines_sm = sm + n;        // [per][n] input, then stage-1 output
-  double2* tmp = lines_sm + per * n; // [per][n] stage-1 results (two-stage only)
-  const long nele = (long)g.n[0] * g.n[1] * g.n[2];
-  const int a1 = (axis + 1) % 3, a2 = (axis + 2) % 3;
-  const long lines = (long)g.n[a1] * g.n[a2];
-  const long stride[3] = {(long)g.n[1] * g.n[2], (long)g.n[2], 1};
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    double s, c;
-    sincospi(2.0 * j / n, &s, &c);
-    tw[j] = make_double2(c, sign * s);
-  }
-  // load the block's lines
-  double2* base[8];
-  for (int q = 0; q < per; ++q) {
-    const long lid = (long)blockIdx.x * per + q;
-    base[q] = nullptr;
-    if (lid < lines * batch) {
-      const int b = (int)(lid / lines);
-      const long r = lid % lines;
-      const int i1 = (int)(r / g.n[a2]), i2 = (int)(r % g.n[a2]);
-      base[q] = data + (long)b * nele + i1 * stride[a1] + i2 * stride[a2];
-    }
-  }
-  for (int t = threadIdx.x; t < per * n; t += blockDim.x) {
-    const int q = t / n, j = t - q * n;
-    lines_sm[t] = base[q] ? base[q][j * stride[axis]] : make_double2(0.0, 0.0);
-  }
-  __syncthreads();
-  auto cmul_acc = [](double2& acc, const double2 x, const double2 w) {
-    acc.x += x.x * w.x - x.y * w.y;
-    acc.y += x.x * w.y + x.y * w.x;
-  };
-  if (n1 == n) {
-    for (int t = threadIdx.x; t < per * n; t += blockDim.x) {
-      const int q = t / n, kk = t - q * n;
-      if (!base[q]) continue;
-      const double2* line = lines_sm + q * n;
-      double2 acc = make_double2(0.0, 0.0);
-      int m = 0;
-      for (int j = 0; j < n; ++j) {
-        cmul_acc(acc, line[j], tw[m]);
-        m += kk;
-        if (m >= n) m -= n;
-      }
-      base[q][kk * stride[axis]] = acc;
-    }
-    return;
-  }
-  // stage 1: y[k1][j2] = W_n^{j2 k1} sum_j1 x[n2 j1 + j2] W_n1^{j1 k1}
-  for (int t = threadIdx.x; t < per * n; t += blockDim.x) {
-    const int q = t / n, r = t - q * n, k1 = r / n2, j2 = r - k1 * n2;
-    const double2* line = lines_sm + q * n;
-    double2 acc = make_double2(0.0, 0.0);
-    const int step = (k1 * n2) % n;  // W_n1^{k1} = W_n^{k1 n2}
-    int m = 0;
-    for (int j1 = 0; j1 < n1; ++j1) {
-      cmul_acc(acc, line[n2 * j1 + j2], tw[m]);
-      m += step;
-      if (m >= n) m -= n;
-    }
-    const double2 w = tw[(j2 * k1) % n];
-    tmp[q * n + r] = make_double2(acc.x * w.x - acc.y * w.y, acc.x * w.y + acc.y * w.x);
-  }
-  __syncthreads();
-  // stage 2: X[k1 + n1 k2] = sum_j2 y[k1][j2] W_n2^{j2 k2}
-  for (int t = threadIdx.x; t < per * n; t += blockDim.x) {
-    const int q = t / n, r = t - q * n, k1 = r % n1, k2 = r / n1;
-    if (!base[q]) continue;
-    const double2* y = tmp + q * n + k1 * n2;
-    double2 acc = make_double2(0.0, 0.0);
-    const int step = (k2 * n1) % n;  // W_n2^{k2} = W_n^{k2 n1}
-    int m = 0;
-    for (int j2 = 0; j2 < n2; ++j2) {
-      cmul_acc(acc, y[j2], tw[m]);
-      m += step;
-      if (m >= n) m -= n;
-    }
-    base[q][(k1 + n1 * k2) * stride[axis]] = acc;
-  }
-}
-
-// Power-of-two lines: radix-2 Stockham FFT of one line per block in shared
-// memory (autosorting, natural order in and out; Govindaraju et al., SC'08),
-// same convention and result as k_dft_axis.  Stage Ns (1, 2, 4, ...): for
-// butterfly j < n/2, k = j mod Ns, v1 = x[j + n/2] exp(sign i pi k / Ns);
-// y[2 Ns floor(j/Ns) + k] = x[j] + v1, y[... + Ns] = x[j] - v1.  Twiddles
-// exp(sign 2 pi i t / n), t < n/2, from FP64 sincospi once per block.
-__global__ void k_fft2_axis(double2* data, ArcDims g, int axis, int sign, int batch, int logn) {
-  extern __shared__ double2 sm[];
-  const int n = 1 << logn, h = n >> 1;
-  double2* x = sm;
-  double2* y = sm + n;
-  double2* tw = sm + 2 * n;
-  const int a1 = (axis + 1) % 3, a2 = (axis + 2) % 3;
-  const long lines = (long)g.n[a1] * g.n[a2];
-  const long lid = blockIdx.x;
-  if (lid >= lines * batch) return;
-  const long nele = (long)g.n[0] * g.n[1] * g.n[2];
-  const int b = (int)(lid / lines);
-  const long r = lid % lines;
-  const int i1 = (int)(r / g.n[a2]), i2 = (int)(r % g.n[a2]);
-  const long stride[3] = {(long)g.n[1] * g.n[2], (long)g.n[2], 1};
-  double2* base = data + (long)b * nele + i1 * stride[a1] + i2 * stride[a2];
-  const long st = stride[axis];
-  for (int j = threadIdx.x; j < n; j += blockDim.x) x[j] = base[j * st];
-  for (int t = threadIdx.x; t < h; t += blockDim.x) {
-    double sn, cs;
-    sincospi(2.0 * t / n, &sn, &cs);
-    tw[t] = make_double2(cs, sign * sn);
-  }
-  __syncthreads();
-  for (int ls = 0; ls < logn; ++ls) {
-    const int Ns = 1 << ls;
-    for (int j = threadIdx.x; j < h; j += blockDim.x) {
-      const int k = j & (Ns - 1);
-      const double2 w = tw[k << (logn - 1 - ls)];  // exp(sign i pi k / Ns)
-      const double2 v0 = x[j], u = x[j + h];
-      const double2 v1 = make_double2(u.x * w.x - u.y * w.y, u.x * w.y + u.y * w.x);
-      const int d = ((j >> ls) << (ls + 1)) + k;
-      y[d] = make_double2(v0.x + v1.x, v0.y + v1.y);
-      y[d + Ns] = make_double2(v0.x - v1.x, v0.y - v1.y);
-    }
-    __syncthreads();
-    double2* t = x;
-    x = y;
-    y = t;
-  }
-  for (int j = threadIdx.x; j < n; j += blockDim.x) base[j * st] = x[j];
-}
-
-// unnormalised 3D DFT (sign -1 forward, +1 backward) of `batch` consecutive
-// complex grids [n0][n1][n2], in place, any sizes up to 1024 per axis;
-// power-of-two axes by the FFT above, others by the direct sum
-int dft3_grid(double2* data, const int n[3], int sign, int batch, cudaStream_t stream) {
-  ArcDims g;
-  for (int d = 0; d < 3; ++d) g.n[d] = n[d];
-  for (int axis = 2; axis >= 0; --axis) {
-    const int na = g.n[axis];
-    long lines = (long)g.n[(axis + 1) % 3] * g.n[(axis + 2) % 3] * batch;
-    if (na >= 2 && (na & (na - 1)) == 0) {
-      int logn = 0;
-      while ((1 << logn) < na) ++logn;
-      const size_t smem = sizeof(double2) * (2 * na + na / 2);
-      k_fft2_axis<<<(unsigned)lines, 128, smem, stream>>>(data, g, axis, sign, batch, logn);
-      MD_CHECK_LAUNCH("fft axis");
-    } else {
-      int n1 = na;  // smallest prime factor
-      for (int f = 2; f * f <= na; ++f)
-        if (na % f == 0) { n1 = f; break; }
-      const int per = std::max(1, std::min(8, 128 / na));  // lines per block
-      size_t smem = sizeof(double2) * (na + 2 * (size_t)per * na);
-      k_dft_axis<<<(unsigned)((lines + per - 1) / per), 128, smem, stream>>>(data, g, axis, sign, batch, n1, per);
-      MD_CHECK_LAUNCH("dft axis");
-    }
-  }
-  return MD_OK;
-}
+// ------------------------------------------------------------ transforms (dft.cu)
+int dft3_grid(double2* data, const int n[3], int sign, int batch, cudaStream_t stream);
 
 static int dft3(md_adapt_rcut* a, double2* data, int sign, int batch) {
   return dft3_grid(data, a->n, sign, batch, a->sys->stream);
@@ -735,10 +566,14 @@ extern "C" int md_arc_get_error(md_adapt_rcut* a, double* err) {
 
 extern "C" int md_arc_get_rcut(md_adapt_rcut* a, double* rcut, int* idx, double* result_error) {
   if (!a) return MD_ERR_BADARG;
-  if (rcut) MD_CUDA(cudaMemcpyAsync(rcut, a->rcut, sizeof(double) * a->nele, cudaMemcpyDeviceToHost, a->sys->stream));
-  if (idx) MD_CUDA(cudaMemcpyAsync(idx, a->rcidx, sizeof(int) * a->nele, cudaMemcpyDeviceToHost, a->sys->stream));
-  if (result_error) MD_CUDA(cudaMemcpyAsync(result_error, a->rerr, sizeof(double) * a->nele, cudaMemcpyDeviceToHost, a->sys->stream));
-  MD_CUDA(cudaStreamSynchronize(a->sys->stream));
+  void* dst[3];
+  const void* src[3];
+  size_t bytes[3];
+  int n = 0;
+  if (rcut) { dst[n] = rcut; src[n] = a->rcut; bytes[n++] = sizeof(double) * a->nele; }
+  if (idx) { dst[n] = idx; src[n] = a->rcidx; bytes[n++] = sizeof(int) * a->nele; }
+  if (result_error) { dst[n] = result_error; src[n] = a->rerr; bytes[n++] = sizeof(double) * a->nele; }
+  if (int r = sys_read_back(a->sys, a->sys->stream, dst, src, bytes, n)) return r;
   DevState hs;
   if (int r = a->sys->read_state(hs)) return r;
   if (hs.flags & FLAG_QUADRATURE) { md_set_error("adaptive quadrature reached its depth bound"); return MD_ERR_BADARG; }

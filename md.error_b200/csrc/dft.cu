@@ -1,0 +1,241 @@
+// Batched FP64 transforms of complex grids [n0][n1][n2], unnormalised, any
+// sizes up to 1024 per axis, one pass per axis.
+//
+// Power-of-two axes: radix-8 Stockham lines in shared memory (fft_lines.cuh),
+// 1,024 points per block of 128 threads; lines adjacent in memory share a
+// block, so strided axes load coalesced.  Bound: latency of two or three
+// shared-memory exchanges per pass; the radix-2 line per block it replaces
+// made log2 n of them and loaded strided axes 16 bytes at a time (64^3 grids,
+// batches of 1 to 4: 21 us a pass before, 6 us now).
+//
+// Other sizes (the odd bin grids of AdaptRCut): a length p is summed over the
+// (p-1)/2 pairs x_j +- x_{p-j}, which gives outputs k and p-k together from
+// 4 real products per pair where the direct sum takes 16; composite lengths
+// n = n1 n2 with a prime n1 <= 11 take two such stages (Cooley-Tukey).  Lanes
+// hold different lines, so a twiddle is one broadcast and six outputs share
+// each loaded pair.  Bound: shared-memory bandwidth and FP64 issue.
+#include <algorithm>
+#include "fft_lines.cuh"
+
+namespace {
+
+// line L of an axis of n points: elements `inner` apart from (L / inner) n inner + L % inner
+__device__ __forceinline__ size_t line_base(long L, int n, long inner) {
+  return (size_t)(L / inner) * n * inner + (size_t)(L % inner);
+}
+
+template <int LOGN>
+__global__ void __launch_bounds__(FFT_THREADS)
+k_fft_grid(const double2* in, double2* out, long nlines, long inner, int sign) {
+  typedef FftGeom<LOGN> G;
+  constexpr int n = G::n, LPB = G::LPB, LS = G::LS, EPT = G::EPT;
+  extern __shared__ __align__(16) unsigned char fg_smem[];
+  double2* tw = reinterpret_cast<double2*>(fg_smem);
+  double2* X = tw + n;
+  for (int m = threadIdx.x; m < n; m += FFT_THREADS) {
+    double s, c;
+    sincospi(2.0 * m / n, &s, &c);
+    tw[m] = make_double2(c, sign * s);
+  }
+  const long line0 = (long)blockIdx.x * LPB;
+  double2 v[EPT];
+#pragma unroll
+  for (int s = 0; s < EPT; ++s) {
+    const int e = threadIdx.x + s * FFT_THREADS;
+    const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
+    const long L = line0 + l;
+    v[s] = L < nlines ? in[line_base(L, n, inner) + k * inner] : make_double2(0.0, 0.0);
+  }
+#pragma unroll
+  for (int s = 0; s < EPT; ++s) {
+    const int e = threadIdx.x + s * FFT_THREADS;
+    const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
+    X[l * LS + fft_pad(k)] = v[s];
+  }
+  __syncthreads();
+  double2* x = X + (threadIdx.x / G::TPL) * LS;
+  if (sign < 0) fft_stages<double, LOGN, 0, -1>(x, tw, threadIdx.x % G::TPL);
+  else fft_stages<double, LOGN, 0, 1>(x, tw, threadIdx.x % G::TPL);
+#pragma unroll
+  for (int s = 0; s < EPT; ++s) {
+    const int e = threadIdx.x + s * FFT_THREADS;
+    const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
+    const long L = line0 + l;
+    if (L < nlines) out[line_base(L, n, inner) + k * inner] = X[l * LS + fft_pad(k)];
+  }
+}
+
+template <int LOGN>
+int fft_grid_launch(const double2* in, double2* out, long nlines, long inner, int sign, cudaStream_t s) {
+  typedef FftGeom<LOGN> G;
+  const size_t smem = sizeof(double2) * (G::n + (size_t)G::LPB * G::LS);
+  k_fft_grid<LOGN><<<(unsigned)((nlines + G::LPB - 1) / G::LPB), FFT_THREADS, smem, s>>>(in, out, nlines, inner, sign);
+  MD_CHECK_LAUNCH("fft axis");
+  return MD_OK;
+}
+
+constexpr int DA_THREADS = 128;
+constexpr int DA_KB = 6;  // output pairs (k, p - k) a thread forms at a time
+
+// the pair sums of outputs k0 .. k0 + DA_KB - 1 (<= p / 2) of the length-p
+// transform whose point j sits at x[j * xs]: A_k = sum_j a_j cos, B_k = sum_j b_j sin,
+// X_k = x_0 + A_k + i B_k, X_{p-k} = x_0 + A_k - i B_k; tw holds (cos, sin) of
+// 2 pi m / n, st = n / p.  ready: x already holds a_j at j and b_j at p - j.
+template <bool READY>
+__device__ __forceinline__ void pair_sums(const double2* x, int xs, int p, int k0, const double2* tw, int n, int st,
+                                          double2 (&A)[DA_KB], double2 (&B)[DA_KB]) {
+  int m[DA_KB], dm[DA_KB];
+  const double2 x0 = x[0];
+#pragma unroll
+  for (int q = 0; q < DA_KB; ++q) {
+    A[q] = x0;
+    B[q] = make_double2(0.0, 0.0);
+    dm[q] = min(k0 + q, p / 2) * st;
+    m[q] = 0;
+  }
+  const int h = (p - 1) / 2;
+  for (int j = 1; j <= h; ++j) {
+    double2 a = x[(size_t)j * xs], b = x[(size_t)(p - j) * xs];
+    if (!READY) {
+      const double2 t = a;
+      a = make_double2(t.x + b.x, t.y + b.y);
+      b = make_double2(t.x - b.x, t.y - b.y);
+    }
+#pragma unroll
+    for (int q = 0; q < DA_KB; ++q) {
+      m[q] += dm[q];
+      if (m[q] >= n) m[q] -= n;
+      const double2 w = tw[m[q]];
+      A[q].x = fma(a.x, w.x, A[q].x);
+      A[q].y = fma(a.y, w.x, A[q].y);
+      B[q].x = fma(-b.y, w.y, B[q].x);
+      B[q].y = fma(b.x, w.y, B[q].y);
+    }
+  }
+  if ((p & 1) == 0) {  // the unpaired middle point
+    const double2 c = x[(size_t)(p / 2) * xs];
+#pragma unroll
+    for (int q = 0; q < DA_KB; ++q) {
+      const double sg = ((k0 + q) & 1) ? -1.0 : 1.0;
+      A[q].x += sg * c.x;
+      A[q].y += sg * c.y;
+    }
+  }
+}
+
+// LN lines per block, one per lane; n = n1 n2 (n1 = 1: a single stage of length n)
+template <int LN>
+__global__ void __launch_bounds__(DA_THREADS)
+k_dft_any(const double2* in, double2* out, long nlines, long inner, int n, int n1, int sign) {
+  extern __shared__ __align__(16) unsigned char da_smem[];
+  constexpr int LS = LN + 1, NG = DA_THREADS / LN;
+  double2* tw = reinterpret_cast<double2*>(da_smem);  // (cos, sign sin) of 2 pi m / n
+  double2* x = tw + n;                                // [n][LS]
+  const int n2 = n / n1;
+  const long line0 = (long)blockIdx.x * LN;
+  for (int m = threadIdx.x; m < n; m += DA_THREADS) {
+    double s, c;
+    sincospi(2.0 * m / n, &s, &c);
+    tw[m] = make_double2(c, sign * s);
+  }
+  for (int t = threadIdx.x; t < n * LN; t += DA_THREADS) {
+    const int l = inner > 1 ? t % LN : t / n, j = inner > 1 ? t / LN : t % n;
+    const long L = line0 + l;
+    x[j * LS + l] = L < nlines ? in[line_base(L, n, inner) + j * inner] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  const int l = threadIdx.x % LN, g = threadIdx.x / LN;
+  const long L = line0 + l;
+  const bool live = L < nlines;
+  double2* dst = out + (live ? line_base(L, n, inner) : 0);
+  double2 A[DA_KB], B[DA_KB];
+  if (n1 > 1) {
+    // stage 1, in place: a thread holds all outputs of a length-n1 transform
+    // (n1 <= 11: k <= 5), times W_n^{j2 k1}
+    for (int j2 = g; j2 < n2; j2 += NG) {
+      double2* c = x + j2 * LS + l;
+      pair_sums<false>(c, n2 * LS, n1, 0, tw, n, n2, A, B);
+#pragma unroll
+      for (int q = 0; q < DA_KB; ++q) {
+        if (q > n1 / 2) break;
+        const double2 w = tw[(j2 * q) % n];
+        const double2 u = make_double2(A[q].x + B[q].x, A[q].y + B[q].y);
+        c[(size_t)q * n2 * LS] = make_double2(u.x * w.x - u.y * w.y, u.x * w.y + u.y * w.x);
+        if (q > 0 && 2 * q < n1) {
+          const int k = n1 - q;
+          const double2 z = tw[(j2 * k) % n];
+          const double2 v = make_double2(A[q].x - B[q].x, A[q].y - B[q].y);
+          c[(size_t)k * n2 * LS] = make_double2(v.x * z.x - v.y * z.y, v.x * z.y + v.y * z.x);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // the last stage: n1 transforms of length n2 (point j2 of transform k1 at
+  // row k1 n2 + j2); pairs first, in place, then the outputs
+  const int h = (n2 - 1) / 2;
+  for (int t = threadIdx.x; t < n1 * h * LN; t += DA_THREADS) {
+    const int ll = t % LN, r = t / LN, k1 = r / h, j = 1 + r - k1 * h;
+    double2* a = x + (k1 * n2 + j) * LS + ll;
+    double2* b = x + (k1 * n2 + n2 - j) * LS + ll;
+    const double2 u = *a, v = *b;
+    *a = make_double2(u.x + v.x, u.y + v.y);
+    *b = make_double2(u.x - v.x, u.y - v.y);
+  }
+  __syncthreads();
+  const int nk = n2 / 2 + 1, nt = (nk + DA_KB - 1) / DA_KB;
+  for (int t = g; t < n1 * nt; t += NG) {
+    const int k1 = t / nt, k0 = (t - k1 * nt) * DA_KB;
+    pair_sums<true>(x + k1 * n2 * LS + l, LS, n2, k0, tw, n, n1, A, B);
+    if (!live) continue;
+#pragma unroll
+    for (int q = 0; q < DA_KB; ++q) {
+      const int k2 = k0 + q;
+      if (k2 >= nk) break;
+      dst[(size_t)(k1 + n1 * k2) * inner] = make_double2(A[q].x + B[q].x, A[q].y + B[q].y);
+      if (k2 > 0 && 2 * k2 < n2)
+        dst[(size_t)(k1 + n1 * (n2 - k2)) * inner] = make_double2(A[q].x - B[q].x, A[q].y - B[q].y);
+    }
+  }
+}
+
+template <int LN>
+int dft_any_launch(const double2* in, double2* out, long nlines, long inner, int n, int n1, int sign, cudaStream_t s) {
+  const size_t smem = sizeof(double2) * (n + (size_t)n * (LN + 1));
+  if (smem > 48 * 1024)
+    MD_CUDA(cudaFuncSetAttribute(k_dft_any<LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  k_dft_any<LN><<<(unsigned)((nlines + LN - 1) / LN), DA_THREADS, smem, s>>>(in, out, nlines, inner, n, n1, sign);
+  MD_CHECK_LAUNCH("dft axis");
+  return MD_OK;
+}
+
+}  // namespace
+
+// one pass (sign -1 forward, +1 backward) over `batch` consecutive grids along
+// `axis`; in may equal out
+int dft3_axis(const double2* in, double2* out, const int n[3], int axis, int sign, int batch, cudaStream_t s) {
+  const int na = n[axis];
+  const long inner = axis == 2 ? 1 : axis == 1 ? n[2] : (long)n[1] * n[2];
+  const long nlines = (long)n[0] * n[1] * n[2] / na * batch;
+  switch (na) {
+#define FFT_CASE(L) case 1 << L: return fft_grid_launch<L>(in, out, nlines, inner, sign, s);
+    FFT_CASE(1) FFT_CASE(2) FFT_CASE(3) FFT_CASE(4) FFT_CASE(5) FFT_CASE(6) FFT_CASE(7) FFT_CASE(8) FFT_CASE(9) FFT_CASE(10)
+#undef FFT_CASE
+  }
+  int n1 = 1;  // the smallest prime factor when it is at most 11 and proper
+  for (int f = 2; f <= 11 && f < na; ++f)
+    if (na % f == 0) { n1 = f; break; }
+  // lines per block: all lanes of a warp where several blocks' lines still fit
+  // on an SM (41 points: 23 KB, 161 points: 46 KB of the 228 KB)
+  if (na <= 96) return dft_any_launch<32>(in, out, nlines, inner, na, n1, sign, s);
+  if (na <= 192) return dft_any_launch<16>(in, out, nlines, inner, na, n1, sign, s);
+  if (na <= 384) return dft_any_launch<8>(in, out, nlines, inner, na, n1, sign, s);
+  return dft_any_launch<4>(in, out, nlines, inner, na, n1, sign, s);
+}
+
+// unnormalised 3D transform of `batch` consecutive grids, in place
+int dft3_grid(double2* data, const int n[3], int sign, int batch, cudaStream_t s) {
+  for (int axis = 2; axis >= 0; --axis)
+    if (int r = dft3_axis(data, data, n, axis, sign, batch, s)) return r;
+  return MD_OK;
+}

@@ -30,10 +30,7 @@
 #include <type_traits>
 #include <vector>
 #include "device_common.cuh"
-
-template <class R> struct C2;
-template <> struct C2<float> { typedef float2 T; };
-template <> struct C2<double> { typedef double2 T; };
+#include "fft_lines.cuh"
 
 struct md_spme {
   md_system* sys = nullptr;
@@ -231,157 +228,7 @@ k_spme_spread_t(int N, const typename V4<R>::T* __restrict__ pos, int K0, int K1
   }
 }
 
-// ---------------------------------------------------------------- FFT
-// Stockham transform of whole lines in shared memory, in the formulation of
-// Govindaraju et al. (SC'08): with Ns the length already transformed, stage
-// (radix R) takes butterfly j < n/R, reads its R inputs at stride n/R,
-// multiplies input r by W_n^{r k n/(Ns R)} (k = j mod Ns), applies an R-point
-// DFT in registers and writes output r to (j / Ns) Ns R + k + r Ns.  Stages
-// of radix 8, then one of radix 4 or 2, cover n = 2^LOGN and leave the line
-// in natural order.  One stage reads all its inputs, synchronises and then
-// writes, so a single buffer per line suffices.  A block of FFT_THREADS
-// threads holds FFT_THREADS / TPL lines (TPL = n/8 threads per line), each
-// padded by one element; twiddles come from a per-axis table computed once
-// in FP64 (conjugated for the inverse transform).
-constexpr int FFT_THREADS = 128;
-
-template <class T2>
-__device__ __forceinline__ T2 cmul(T2 a, T2 b) {
-  T2 r;
-  r.x = a.x * b.x - a.y * b.y;
-  r.y = a.x * b.y + a.y * b.x;
-  return r;
-}
-template <class T2>
-__device__ __forceinline__ T2 c_add(T2 a, T2 b) {
-  T2 r;
-  r.x = a.x + b.x;
-  r.y = a.y + b.y;
-  return r;
-}
-template <class T2>
-__device__ __forceinline__ T2 c_sub(T2 a, T2 b) {
-  T2 r;
-  r.x = a.x - b.x;
-  r.y = a.y - b.y;
-  return r;
-}
-// a * (SIGN i)
-template <int SIGN, class T2>
-__device__ __forceinline__ T2 c_mul_si(T2 a) {
-  T2 r;
-  r.x = SIGN > 0 ? -a.y : a.y;
-  r.y = SIGN > 0 ? a.x : -a.x;
-  return r;
-}
-
-// X_s = sum_r v_r exp(SIGN 2 pi i r s / 4)
-template <int SIGN, class T2>
-__device__ __forceinline__ void dft4(T2& v0, T2& v1, T2& v2, T2& v3) {
-  const T2 s0 = c_add(v0, v2), d0 = c_sub(v0, v2), s1 = c_add(v1, v3), d1 = c_mul_si<SIGN>(c_sub(v1, v3));
-  v0 = c_add(s0, s1);
-  v2 = c_sub(s0, s1);
-  v1 = c_add(d0, d1);
-  v3 = c_sub(d0, d1);
-}
-
-template <class R, int RR, int SIGN>
-__device__ __forceinline__ void dft_reg(typename C2<R>::T (&v)[RR]) {
-  typedef typename C2<R>::T T2;
-  if constexpr (RR == 2) {
-    const T2 a = v[0];
-    v[0] = c_add(a, v[1]);
-    v[1] = c_sub(a, v[1]);
-  } else if constexpr (RR == 4) {
-    dft4<SIGN>(v[0], v[1], v[2], v[3]);
-  } else {
-    // radix 8 = two radix-4 DFTs of the even and odd inputs, odd ones
-    // multiplied by W^k, W = exp(SIGN 2 pi i / 8)
-    T2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
-    dft4<SIGN>(e0, e1, e2, e3);
-    dft4<SIGN>(o0, o1, o2, o3);
-    const R h = R(0.70710678118654752440);  // 1/sqrt(2)
-    T2 t;
-    t.x = (SIGN > 0 ? o1.x - o1.y : o1.x + o1.y) * h;
-    t.y = (SIGN > 0 ? o1.y + o1.x : o1.y - o1.x) * h;
-    o1 = t;
-    o2 = c_mul_si<SIGN>(o2);
-    t.x = (SIGN > 0 ? -o3.x - o3.y : -o3.x + o3.y) * h;
-    t.y = (SIGN > 0 ? -o3.y + o3.x : -o3.y - o3.x) * h;
-    o3 = t;
-    v[0] = c_add(e0, o0);
-    v[4] = c_sub(e0, o0);
-    v[1] = c_add(e1, o1);
-    v[5] = c_sub(e1, o1);
-    v[2] = c_add(e2, o2);
-    v[6] = c_sub(e2, o2);
-    v[3] = c_add(e3, o3);
-    v[7] = c_sub(e3, o3);
-  }
-}
-
-template <int LOGN>
-struct FftGeom {
-  static constexpr int n = 1 << LOGN;
-  static constexpr int TPL = n >= 8 ? n / 8 : 1;  // threads per line
-  static constexpr int LPB = FFT_THREADS / TPL;   // lines per block
-  static constexpr int LS = n + 1;                // padded line stride
-  static constexpr int EPT = LPB * n / FFT_THREADS;  // elements per thread
-};
-
-// the stages from Ns = 2^LOGNS on, for the line x of this thread (lane tl of
-// the line's TPL threads); every thread of the block takes part
-template <class R, int LOGN, int LOGNS, int SIGN>
-__device__ __forceinline__ void fft_stages(typename C2<R>::T* x, const typename C2<R>::T* tw, int tl) {
-  typedef typename C2<R>::T T2;
-  constexpr int n = 1 << LOGN, TPL = FftGeom<LOGN>::TPL;
-  constexpr int LR = (LOGN - LOGNS) >= 3 ? 3 : (LOGN - LOGNS);
-  constexpr int RR = 1 << LR, NS = 1 << LOGNS, NBF = n / RR, BPT = NBF / TPL;
-  static_assert(BPT >= 1, "at least one butterfly per thread");
-  T2 v[BPT][RR];
-#pragma unroll
-  for (int q = 0; q < BPT; ++q) {
-    const int j = tl + q * TPL;
-#pragma unroll
-    for (int r = 0; r < RR; ++r) v[q][r] = x[j + r * NBF];
-    if constexpr (LOGNS > 0) {
-      const int k = j & (NS - 1);
-#pragma unroll
-      for (int r = 1; r < RR; ++r) v[q][r] = cmul(v[q][r], tw[(r * k) << (LOGN - LOGNS - LR)]);
-    }
-    dft_reg<R, RR, SIGN>(v[q]);
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < BPT; ++q) {
-    const int j = tl + q * TPL;
-    const int d = ((j >> LOGNS) << (LOGNS + LR)) + (j & (NS - 1));
-#pragma unroll
-    for (int r = 0; r < RR; ++r) x[d + r * NS] = v[q][r];
-  }
-  __syncthreads();
-  if constexpr (LOGNS + LR < LOGN) fft_stages<R, LOGN, LOGNS + LR, SIGN>(x, tw, tl);
-}
-
-// the block barriers of fft_stages<R, LOGN, LOGNS, *> without the work: a
-// group with nothing to transform meets the others' barriers
-template <int LOGN, int LOGNS>
-__device__ __forceinline__ void fft_stage_barriers() {
-  constexpr int LR = (LOGN - LOGNS) >= 3 ? 3 : (LOGN - LOGNS);
-  __syncthreads();
-  __syncthreads();
-  if constexpr (LOGNS + LR < LOGN) fft_stage_barriers<LOGN, LOGNS + LR>();
-}
-
-template <class R, int SIGN>
-__device__ __forceinline__ void load_tw(typename C2<R>::T* tw, const typename C2<R>::T* __restrict__ twg, int n) {
-  for (int m = threadIdx.x; m < n; m += blockDim.x) {
-    typename C2<R>::T w = twg[m];
-    if (SIGN > 0) w.y = -w.y;
-    tw[m] = w;
-  }
-}
-
+// ---------------------------------------------------------------- FFT passes (fft_lines.cuh)
 // One transform pass over lines of one axis.
 //   MODE 0: real lines along z (contiguous) -> half-complex lines (n/2+1);
 //           the input lines are cleared after they are read
@@ -478,7 +325,7 @@ k_fftp(const void* in, void* out, const typename C2<R>::T* __restrict__ twg, lon
         if (L < nlc) src[2 * L * n + k] = R(0);
         if (2 * L + 1 < nlines) src[(2 * L + 1) * n + k] = R(0);
       }
-      Xb[l * LS + k] = vv[s];
+      Xb[l * LS + fft_pad(k)] = vv[s];
     }
   }
   __syncthreads();
@@ -490,10 +337,10 @@ k_fftp(const void* in, void* out, const typename C2<R>::T* __restrict__ twg, lon
       const long L = line0 + l2;
       if (L >= nlines) continue;
       R4 o;
-      const T2 xy = X[l2 * LS + k];
+      const T2 xy = X[l2 * LS + fft_pad(k)];
       o.x = xy.x;
       o.y = xy.y;
-      o.z = X[LPB * LS + l2 * LS + k].x;
+      o.z = X[LPB * LS + l2 * LS + fft_pad(k)].x;
       o.w = R(0);
       reinterpret_cast<R4*>(out)[L * n + k] = o;
     }
@@ -505,10 +352,10 @@ k_fftp(const void* in, void* out, const typename C2<R>::T* __restrict__ twg, lon
     else { l2 = e >> LOGN; k = e & (n - 1); }
     const long L = line0 + l2;
     if (L >= nlc) continue;
-    const T2 v = X[l2 * LS + k];
+    const T2 v = X[l2 * LS + fft_pad(k)];
     if (MODE == 0) {
       if (k < nh) {
-        const T2 w = X[l2 * LS + ((n - k) & (n - 1))];
+        const T2 w = X[l2 * LS + fft_pad((n - k) & (n - 1))];
         T2 a, b;
         a.x = R(0.5) * (v.x + w.x);
         a.y = R(0.5) * (v.y - w.y);
@@ -529,7 +376,7 @@ k_fftp(const void* in, void* out, const typename C2<R>::T* __restrict__ twg, lon
 template <class R>
 static size_t fftp_smem(int logn, int nbuf) {
   const int n = 1 << logn, tpl = n >= 8 ? n / 8 : 1, lpb = FFT_THREADS / tpl;
-  return sizeof(typename C2<R>::T) * ((size_t)n + (size_t)nbuf * lpb * (n + 1)) + sizeof(long) * lpb;
+  return sizeof(typename C2<R>::T) * ((size_t)n + (size_t)nbuf * lpb * fft_line_stride(n)) + sizeof(long) * lpb;
 }
 
 // Forward transform along x, the k-space step and the inverse transform(s)
@@ -611,7 +458,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
 #pragma unroll
     for (int s = 0; s < EPT; ++s) {
       const int e = gt + s * FFT_THREADS;
-      X[(e % LPB) * LS + e / LPB] = vv[s];
+      X[(e % LPB) * LS + fft_pad(e / LPB)] = vv[s];
     }
   }
   __syncthreads();
@@ -634,7 +481,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
       PS[le * LS + i] = ps;
       if (with_stats && live) {
         // E = 1/2 sum_m |Q^|^2 psi over the full spectrum: interior z planes count twice
-        const T2 q = X[le * LS + i];
+        const T2 q = X[le * LS + fft_pad(i)];
         const double wgt = (k == 0 || (2 * k == K2)) ? 1.0 : 2.0;
         const double e2 = 0.5 * wgt * ((double)q.x * q.x + (double)q.y * q.y) * (double)ps;
         // f = 2 (1 + pi^2 m^2 / beta^2) / m^2
@@ -652,7 +499,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
 #pragma unroll
   for (int s = 0; s < EPT; ++s) {
     const int e = gt + s * FFT_THREADS, le = e % LPB, i = e / LPB;
-    const T2 q = X[le * LS + i];
+    const T2 q = X[le * LS + fft_pad(i)];
     const R ps = PS[le * LS + i];
     T2 g;
     if (METHOD == 0 && grp == 0) {
@@ -668,7 +515,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
       g.x = q.x * (R(0.5) * ps);
       g.y = q.y * (R(0.5) * ps);
     }
-    Yg[le * LS + i] = g;
+    Yg[le * LS + fft_pad(i)] = g;
   }
   __syncthreads();
   fft_stages<R, LOGN, 0, 1>(Yg + l * LS, twi, tl);
@@ -682,7 +529,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
       if (L >= nlines) continue;
       const int jp = lj[le] <= K1 / 2 ? lj[le] : lj[le] - K1;
       const R cy = (R)(-2.0 * M_PI * (jp * st->Li[1])), cz = (R)(-2.0 * M_PI * (lk[le] * st->Li[2]));
-      const T2 v = Yg[le * LS + i];
+      const T2 v = Yg[le * LS + fft_pad(i)];
       T2 a, b;
       a.x = -v.y * cy;
       a.y = v.x * cy;
@@ -696,7 +543,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
     for (int e = gt; e < LPB * n; e += FFT_THREADS) {
       const int le = e % LPB, i = e / LPB;
       const long L = line0 + le;
-      if (L < nlines) out[L + i * stride] = Yg[le * LS + i];
+      if (L < nlines) out[L + i * stride] = Yg[le * LS + fft_pad(i)];
     }
   }
   if (with_stats && block_reduce_finish<4>(v, partials, &st->red_counter[RED_SPME], st->scratch, true) && merge) {
@@ -709,8 +556,8 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
 template <class R>
 static size_t fftx_smem(int logn, int method) {
   const int n = 1 << logn, tpl = n >= 8 ? n / 8 : 1, lpb = FFT_THREADS / tpl, ng = method == 0 ? 2 : 1;
-  return sizeof(typename C2<R>::T) * (2 * (size_t)n + (1 + (size_t)ng) * lpb * (n + 1)) +
-         sizeof(R) * (size_t)lpb * (n + 1) + 8 + sizeof(double) * ((size_t)n + 2 * lpb) + 2 * sizeof(int) * lpb;
+  return sizeof(typename C2<R>::T) * (2 * (size_t)n + (1 + (size_t)ng) * lpb * fft_line_stride(n)) +
+         sizeof(R) * (size_t)lpb * fft_line_stride(n) + 8 + sizeof(double) * ((size_t)n + 2 * lpb) + 2 * sizeof(int) * lpb;
 }
 
 // per-axis forward twiddle table exp(-2 pi i m / n), m < n, from FP64

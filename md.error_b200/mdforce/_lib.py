@@ -185,6 +185,7 @@ _SIGS = {
     "md_errmap_mean_force": (i32, [vp, f64, P(f64)]),
     "md_errmap_set_profile": (i32, [vp, P(f64), P(f64)]),
     "md_errmap_deposit": (i32, [vp, vp]),
+    "md_errmap_rms": (i32, [vp, f64, f64, P(f64)]),
     "md_errmap_get_profile": (i32, [vp, P(f64), P(f64)]),
     "md_errmap_compute": (i32, [vp, f64, P(f64), P(f64)]),
     "md_ikerr_create":(i32, [P(vp), P(i32), P(f64), f64, f64, i32, i32, i32, i32, f64, f64, i32]),

@@ -578,9 +578,13 @@ class ErrorEstimate_SPME_Ik:
         check(lib.md_errmap_compute(self.h, float(charge), _p(e1), _p(e2)), "calError")
         return e1, e2
 
+    def _rms(self, charge, self_error):
+        out = np.empty(self.K)
+        check(lib.md_errmap_rms(self.h, float(charge), float(self_error), _p(out)), "rms")
+        return out
+
     def rms(self, charge=1.0):
-        e1, e2 = self.calError(charge)
-        return np.sqrt(e1[..., 0] + e2[..., 0])
+        return self._rms(charge, 0.0)
 
     def mean_force(self, charge=1.0):
         """The signed mean force error field e1_d (print_meanf): [3, K...]."""
@@ -628,8 +632,7 @@ class ErrorEstimate_SPME_Ana(ErrorEstimate_SPME_Ik):
         return self.self_error() * charge ** 4
 
     def rms(self, charge=1.0):
-        e1, e2 = self.calError(charge)
-        return np.sqrt(e1[..., 0] + e2[..., 0] + self.qself_error(charge))
+        return self._rms(charge, self.qself_error(charge))
 
     def fconv(self, k):
         """FConvRho1_{x,y,z} for alias index k (0 < |k| <= 2): [3, K..., 2]."""
