@@ -6,8 +6,8 @@
 //   analytic differentiation         RE/src/EleRecFBSpline.cpp:771-907, 1146-1195
 //
 // Chain of one force evaluation (each step one kernel):
-//   spread      charges into a shared-memory tile per block of 64 charges,
-//               the tile added to the mesh with 4-wide atomics
+//   spread      charges into a shared-memory tile per warp, the tile added to
+//               the mesh with 4-wide atomics (spme_pm.cu)
 //   z pass      R2C along z (real lines -> half-complex lines)
 //   y pass      forward C2C along y
 //   x pass      forward C2C along x, k-space step (energy and virial in FP64,
@@ -18,7 +18,7 @@
 //               spectrum (the FFTW c2r convention the reference relies on);
 //               for ik the three meshes are written interleaved, one Real4
 //               per mesh point
-//   gather      order-templated, LPA lanes per atom
+//   gather      a warp per atom, lanes along its stencil rows (spme_pm.cu)
 // The FFT passes are radix-8 Stockham transforms of whole lines in shared
 // memory; a block holds several lines adjacent in memory so that strided
 // axes load coalesced.  Mixed precision: mesh, FFT and gather in FP32,
@@ -31,6 +31,7 @@
 #include <vector>
 #include "device_common.cuh"
 #include "fft_lines.cuh"
+#include "spme_pm.cuh"
 
 struct md_spme {
   md_system* sys = nullptr;
@@ -73,159 +74,6 @@ __device__ __forceinline__ void bspline_w(int n, R f, R* w, R* dw) {
     }
   }
   if (n == 2 && dw) { dw[0] = R(1); dw[1] = R(-1); }
-}
-
-template <class R>
-__device__ __forceinline__ void grid_coord(R x, R Linv, int K, int& base, R& frac) {
-  R u = R(K) * x * Linv;
-  u -= floor_r(u / R(K)) * R(K);
-  R b = floor_r(u);
-  frac = u - b;
-  base = (int)b;
-  if (base >= K) { base -= K; }
-}
-
-// The same recursion with the order a compile-time constant, so that the
-// weight arrays stay in registers (a runtime order spills them to local
-// memory).  D: also the derivatives dM_n/du.
-template <class R, int NO, bool D>
-__device__ __forceinline__ void bsp_t(R f, R (&w)[NO], R (&dw)[NO]) {
-  w[0] = f;
-  w[1] = R(1) - f;
-#pragma unroll
-  for (int j = 2; j < NO; ++j) w[j] = R(0);
-#pragma unroll
-  for (int k = 3; k <= NO; ++k) {
-    if (D && k == NO) {
-#pragma unroll
-      for (int j = 0; j < NO; ++j) dw[j] = (j < NO - 1 ? w[j] : R(0)) - (j > 0 ? w[j - 1] : R(0));
-    }
-    const R inv = R(1) / R(k - 1);
-#pragma unroll
-    for (int j = k - 1; j >= 0; --j) {
-      const R u = f + R(j);
-      const R a = (j < k - 1) ? w[j] : R(0);
-      const R b = (j > 0) ? w[j - 1] : R(0);
-      w[j] = (u * a + (R(k) - u) * b) * inv;
-    }
-  }
-  if (D && NO == 2) { dw[0] = R(1); dw[1] = R(-1); }
-}
-
-// Orders with a compiled spread / gather (md_spme_create accepts 2..14).
-#define SPME_ORDERS(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14)
-
-// ---------------------------------------------------------------- spread
-// A block takes SPREAD_ATOMS consecutive charges (cell order, hence compact
-// in space) and spreads them into a shared-memory tile that covers their
-// stencils, with shared-memory atomics; the tile is then added to the mesh
-// with one 4-wide atomic per 4 z points (binary32) or scalar atomics
-// (binary64), skipping empty groups.  Each charge's stencil base is taken in
-// the periodic image closest to the block's first charge, so that a block
-// next to a periodic face still has a compact tile.  The tile's z origin and
-// extent are multiples of 4 (K2 is a power of two >= 4, so a group never
-// wraps); rows are padded by one element against bank conflicts.  A block
-// whose tile does not fit adds every stencil point with a global atomic.
-constexpr int SPREAD_ATOMS = 64;
-constexpr int SPREAD_THREADS = 256;
-constexpr int SPREAD_TILE_BYTES = 64 * 1024;
-
-template <class R>
-__device__ __forceinline__ void mesh_add4(R* dst, R a, R b, R c, R d);
-template <>
-__device__ __forceinline__ void mesh_add4<float>(float* dst, float a, float b, float c, float d) {
-  atomicAdd(reinterpret_cast<float4*>(dst), make_float4(a, b, c, d));
-}
-template <>
-__device__ __forceinline__ void mesh_add4<double>(double* dst, double a, double b, double c, double d) {
-  if (a != 0.0) atomicAdd(dst, a);
-  if (b != 0.0) atomicAdd(dst + 1, b);
-  if (c != 0.0) atomicAdd(dst + 2, c);
-  if (d != 0.0) atomicAdd(dst + 3, d);
-}
-
-template <class R, int NO>
-__global__ void __launch_bounds__(SPREAD_THREADS)
-k_spme_spread_t(int N, const typename V4<R>::T* __restrict__ pos, int K0, int K1, int K2,
-                const DevState* __restrict__ st, R* __restrict__ Q, int tile_cap) {
-  extern __shared__ __align__(16) unsigned char sp_smem[];
-  R* tile = reinterpret_cast<R*>(sp_smem);
-  __shared__ R sw[3][NO][SPREAD_ATOMS];
-  __shared__ R sq[SPREAD_ATOMS];
-  __shared__ int sb[3][SPREAD_ATOMS];
-  __shared__ int sbox[6];
-  const int i0 = blockIdx.x * SPREAD_ATOMS;
-  const int na = min(SPREAD_ATOMS, N - i0);
-  const int K[3] = {K0, K1, K2};
-  if (threadIdx.x < 6) sbox[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
-  __syncthreads();
-  if ((int)threadIdx.x < na) {
-    const typename V4<R>::T p = pos[i0 + threadIdx.x], p0 = pos[i0];
-    const R x[3] = {p.x, p.y, p.z}, x0[3] = {p0.x, p0.y, p0.z};
-    const R q = p.w;
-    sq[threadIdx.x] = q;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      int b, r;
-      R f, fr;
-      grid_coord<R>(x[d], (R)st->Li[d], K[d], b, f);
-      grid_coord<R>(x0[d], (R)st->Li[d], K[d], r, fr);
-      const int dv = b - r;
-      if (2 * dv > K[d]) b -= K[d];
-      else if (2 * dv < -K[d]) b += K[d];
-      sb[d][threadIdx.x] = b;
-      R w[NO], dw[NO];
-      bsp_t<R, NO, false>(f, w, dw);
-#pragma unroll
-      for (int j = 0; j < NO; ++j) sw[d][j][threadIdx.x] = w[j];
-      if (q != R(0)) {
-        atomicMin(&sbox[d], b);
-        atomicMax(&sbox[3 + d], b);
-      }
-    }
-  }
-  __syncthreads();
-  if (sbox[0] > sbox[3]) return;  // no charge in this block
-  const int o0 = sbox[0] - (NO - 1), o1 = sbox[1] - (NO - 1);
-  const int o2 = (sbox[2] - (NO - 1)) & ~3;
-  const long e0 = sbox[3] - o0 + 1, e1 = sbox[4] - o1 + 1;
-  const long e2 = (sbox[5] - o2 + 4) & ~3;
-  const long rs = e2 + 1;
-  const int nab = na * NO * NO;
-  if (e0 * e1 * rs <= tile_cap) {
-    const int tsz = (int)(e0 * e1 * rs), ie1 = (int)e1, irs = (int)rs;
-    for (int e = threadIdx.x; e < tsz; e += SPREAD_THREADS) tile[e] = R(0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < nab; e += SPREAD_THREADS) {
-      const int at = e / (NO * NO), ab = e - at * (NO * NO), a = ab / NO, b = ab - a * NO;
-      const R q = sq[at];
-      if (q == R(0)) continue;
-      const R qab = q * sw[0][a][at] * sw[1][b][at];
-      R* row = tile + ((sb[0][at] - a - o0) * ie1 + (sb[1][at] - b - o1)) * irs + (sb[2][at] - o2);
-#pragma unroll
-      for (int c = 0; c < NO; ++c) atomicAdd(row - c, qab * sw[2][c][at]);
-    }
-    __syncthreads();
-    const int g2 = (int)(e2 >> 2), ng = (int)(e0 * e1) * g2;
-    for (int g = threadIdx.x; g < ng; g += SPREAD_THREADS) {
-      const int z4 = g % g2, xy = g / g2, y = xy % ie1, x = xy / ie1;
-      const R* s = tile + (x * ie1 + y) * irs + 4 * z4;
-      const R v0 = s[0], v1 = s[1], v2 = s[2], v3 = s[3];
-      if (v0 == R(0) && v1 == R(0) && v2 == R(0) && v3 == R(0)) continue;
-      const int gx = (o0 + x) & (K0 - 1), gy = (o1 + y) & (K1 - 1), gz = (o2 + 4 * z4) & (K2 - 1);
-      mesh_add4<R>(Q + ((size_t)gx * K1 + gy) * K2 + gz, v0, v1, v2, v3);
-    }
-  } else {
-    for (int e = threadIdx.x; e < nab; e += SPREAD_THREADS) {
-      const int at = e / (NO * NO), ab = e - at * (NO * NO), a = ab / NO, b = ab - a * NO;
-      const R q = sq[at];
-      if (q == R(0)) continue;
-      const R qab = q * sw[0][a][at] * sw[1][b][at];
-      const size_t row = ((size_t)((sb[0][at] - a) & (K0 - 1)) * K1 + ((sb[1][at] - b) & (K1 - 1))) * K2;
-#pragma unroll
-      for (int c = 0; c < NO; ++c) atomicAdd(Q + row + ((sb[2][at] - c) & (K2 - 1)), qab * sw[2][c][at]);
-    }
-  }
 }
 
 // ---------------------------------------------------------------- FFT passes (fft_lines.cuh)
@@ -621,236 +469,6 @@ __global__ void k_spme_bmod(int K0, int K1, int K2, int n, double* bm) {
   else if (t < K0 + K1 + K2 / 2 + 1) bm[t] = bmod_d(n, K2, t - K0 - K1);
 }
 
-// ---------------------------------------------------------------- gather
-// A block takes GATHER_ATOMS consecutive atoms (cell order) with LPA lanes
-// each (the power of two >= order, at least 4); lane a takes the stencil
-// plane b0 - a and runs over its order^2 points, and the lanes' sums are
-// combined by shuffles.  The block first stages the mesh region covering its
-// charges' stencils (image-adjusted as in the spread) into shared memory
-// with coalesced, independent row loads, then gathers from there; a block
-// whose region does not fit reads the mesh directly.
-//   MODE 0: ik, the three convolved meshes interleaved, one Real4 per point
-//   MODE 1: analytic differentiation of the single convolved mesh
-//   MODE 2: adjoint gather of Phi: potential dE/dq_i and exact position
-//           gradient dE/dx_i, written in the caller's atom order
-// store (MODES 0, 1): force is a separate buffer that receives every atom's
-// reciprocal force (zero for neutral atoms) instead of accumulating it.
-// MD_SPME_GATHER_TILE_KB: shared-memory budget of the staged region (0: read
-// the mesh directly)
-#ifndef MD_SPME_GATHER_TILE_KB
-#define MD_SPME_GATHER_TILE_KB 64
-#endif
-constexpr int GATHER_ATOMS = 32;
-constexpr int GATHER_TILE_BYTES = MD_SPME_GATHER_TILE_KB * 1024;
-
-__host__ __device__ constexpr int gather_lanes(int order) { return order <= 4 ? 4 : (order <= 8 ? 8 : 16); }
-
-// one stencil row of order points: point c at G[-c] (the staged region) or
-// at G[kz[c]] (the mesh, wrapped indices)
-template <class R, int NO, int MODE, class GT, class A>
-__device__ __forceinline__ void gather_row(const GT* G, R wa, R da, R w1b, R d1b, const R (&w2)[NO],
-                                           const R (&d2)[NO], A& s0, A& s1, A& s2, A& s3) {
-  const R wab = wa * w1b;
-  if constexpr (MODE == 0) {
-#pragma unroll
-    for (int c = 0; c < NO; ++c) {
-      const GT g = G[-c];
-      const R w = wab * w2[c];
-      s0 += g.x * w;
-      s1 += g.y * w;
-      s2 += g.z * w;
-    }
-  } else {
-    const R dab = da * w1b, wdb = wa * d1b;
-#pragma unroll
-    for (int c = 0; c < NO; ++c) {
-      const R g = G[-c];
-      if (MODE == 1) {
-        s0 -= g * dab * w2[c];
-        s1 -= g * wdb * w2[c];
-        s2 -= g * wab * d2[c];
-      } else {
-        s0 += (double)(g * wab * w2[c]);
-        s1 += (double)(g * dab * w2[c]);
-        s2 += (double)(g * wdb * w2[c]);
-        s3 += (double)(g * wab * d2[c]);
-      }
-    }
-  }
-}
-
-template <class R, int NO, int MODE, class GT, class A>
-__device__ __forceinline__ void gather_row_idx(const GT* G, const int (&kz)[NO], R wa, R da, R w1b, R d1b,
-                                               const R (&w2)[NO], const R (&d2)[NO], A& s0, A& s1, A& s2, A& s3) {
-  const R wab = wa * w1b;
-  if constexpr (MODE == 0) {
-#pragma unroll
-    for (int c = 0; c < NO; ++c) {
-      const GT g = G[kz[c]];
-      const R w = wab * w2[c];
-      s0 += g.x * w;
-      s1 += g.y * w;
-      s2 += g.z * w;
-    }
-  } else {
-    const R dab = da * w1b, wdb = wa * d1b;
-#pragma unroll
-    for (int c = 0; c < NO; ++c) {
-      const R g = G[kz[c]];
-      if (MODE == 1) {
-        s0 -= g * dab * w2[c];
-        s1 -= g * wdb * w2[c];
-        s2 -= g * wab * d2[c];
-      } else {
-        s0 += (double)(g * wab * w2[c]);
-        s1 += (double)(g * dab * w2[c]);
-        s2 += (double)(g * wdb * w2[c]);
-        s3 += (double)(g * wab * d2[c]);
-      }
-    }
-  }
-}
-
-template <class R, int NO, int MODE>
-__global__ void __launch_bounds__(GATHER_ATOMS * gather_lanes(NO))
-k_spme_gather_t(int N, const typename V4<R>::T* __restrict__ pos, const int* __restrict__ id, int K0, int K1,
-                int K2, const DevState* __restrict__ st, const void* __restrict__ Gv, double4a* __restrict__ force,
-                double* __restrict__ dq, double* __restrict__ dr, int tile_cap, int store) {
-  typedef typename V4<R>::T R4;
-  typedef typename std::conditional<MODE == 0, R4, R>::type GT;  // mesh element
-  constexpr int LPA = gather_lanes(NO), NT = GATHER_ATOMS * LPA;
-  extern __shared__ __align__(32) unsigned char g_smem[];
-  GT* tile = reinterpret_cast<GT*>(g_smem);
-  __shared__ int sbox[6];
-  const int i0 = blockIdx.x * GATHER_ATOMS;
-  const int i = i0 + (int)threadIdx.x / LPA, a = threadIdx.x & (LPA - 1);
-  const bool act = i < N;
-  const int K[3] = {K0, K1, K2};
-  if (threadIdx.x < 6) sbox[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
-  R4 p;
-  if (act) p = pos[i];
-  else { p.x = R(0); p.y = R(0); p.z = R(0); p.w = R(0); }
-  const R4 p0 = pos[i0];
-  const R x[3] = {p.x, p.y, p.z}, x0[3] = {p0.x, p0.y, p0.z};
-  int bb[3];
-  R ff[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    int r;
-    R fr;
-    grid_coord<R>(x[d], (R)st->Li[d], K[d], bb[d], ff[d]);
-    grid_coord<R>(x0[d], (R)st->Li[d], K[d], r, fr);
-    const int dv = bb[d] - r;
-    if (2 * dv > K[d]) bb[d] -= K[d];
-    else if (2 * dv < -K[d]) bb[d] += K[d];
-  }
-  // a neutral atom feels no force, but its potential is the adjoint's dE/dq
-  const bool live = act && (MODE == 2 || p.w != R(0));
-  __syncthreads();
-  if (live && a == 0) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      atomicMin(&sbox[d], bb[d]);
-      atomicMax(&sbox[3 + d], bb[d]);
-    }
-  }
-  R w0[NO], w1[NO], w2[NO], d0[NO], d1[NO], d2[NO];
-  bsp_t<R, NO, MODE != 0>(ff[0], w0, d0);
-  bsp_t<R, NO, MODE != 0>(ff[1], w1, d1);
-  bsp_t<R, NO, MODE != 0>(ff[2], w2, d2);
-  R wa = R(0), da = R(0);
-#pragma unroll
-  for (int j = 0; j < NO; ++j)
-    if (j == a) { wa = w0[j]; da = d0[j]; }
-  __syncthreads();
-  if (sbox[0] > sbox[3]) {  // no charge in this block
-    if (MODE != 2 && store && act && a == 0) force[i] = double4a{0.0, 0.0, 0.0, 0.0};
-    return;
-  }
-  const int o0 = sbox[0] - (NO - 1), o1 = sbox[1] - (NO - 1), o2 = sbox[2] - (NO - 1);
-  const long e0 = sbox[3] - o0 + 1, e1 = sbox[4] - o1 + 1, e2 = sbox[5] - o2 + 1;
-  // odd plane stride: the lanes of an atom (one x plane each) then fall on
-  // different shared-memory banks
-  const long ps = (e1 * e2) | 1;
-  const bool staged = e0 * ps <= tile_cap;
-  const GT* Gm = reinterpret_cast<const GT*>(Gv);
-  if (staged) {
-    // one mesh row (e2 points along z) per warp pass, lanes along z
-    // row (xx, y) = warp + k * (NT / 32), stepped without divisions
-    const int nrow = (int)(e0 * e1), ie1 = (int)e1, ie2 = (int)e2, ips = (int)ps;
-    constexpr int NWARP = NT >> 5;
-    const int w0 = threadIdx.x >> 5;
-    int y = w0 % ie1, xx = w0 / ie1;
-    for (int row = w0; row < nrow; row += NWARP) {
-      const size_t g = ((size_t)((o0 + xx) & (K0 - 1)) * K1 + ((o1 + y) & (K1 - 1))) * K2;
-      GT* t = tile + xx * ips + y * ie2;
-      for (int z = threadIdx.x & 31; z < ie2; z += 32) t[z] = Gm[g + ((o2 + z) & (K2 - 1))];
-      y += NWARP;
-      while (y >= ie1) { y -= ie1; ++xx; }
-    }
-    __syncthreads();
-  }
-  // the lane's order^2 points are summed in the working precision (FP64 for
-  // the adjoint), the lanes in FP64
-  typedef typename std::conditional<MODE == 2, double, R>::type A;
-  A s0 = A(0), s1 = A(0), s2 = A(0), s3 = A(0);
-  if (live && a < NO) {
-    if (staged) {
-      // row b of plane a starts at tp - b e2; point c of the row at -c
-      const int ie2 = (int)e2;
-      const GT* tp = tile + (bb[0] - a - o0) * (int)ps + (bb[1] - o1) * ie2 + (bb[2] - o2);
-#pragma unroll
-      for (int b = 0; b < NO; ++b)
-        gather_row<R, NO, MODE>(tp - b * ie2, wa, da, w1[b], d1[b], w2, d2, s0, s1, s2, s3);
-    } else {
-      int kz[NO];
-#pragma unroll
-      for (int c = 0; c < NO; ++c) kz[c] = (bb[2] - c) & (K2 - 1);
-      const size_t xrow = (size_t)((bb[0] - a) & (K0 - 1)) * K1;
-#pragma unroll
-      for (int b = 0; b < NO; ++b)
-        gather_row_idx<R, NO, MODE>(Gm + (xrow + ((bb[1] - b) & (K1 - 1))) * K2, kz, wa, da, w1[b], d1[b], w2, d2,
-                                    s0, s1, s2, s3);
-    }
-  }
-  double F0 = s0, F1 = s1, F2 = s2, F3 = s3;
-#pragma unroll
-  for (int o = LPA / 2; o > 0; o >>= 1) {
-    F0 += __shfl_xor_sync(0xffffffffu, F0, o);
-    F1 += __shfl_xor_sync(0xffffffffu, F1, o);
-    F2 += __shfl_xor_sync(0xffffffffu, F2, o);
-    if (MODE == 2) F3 += __shfl_xor_sync(0xffffffffu, F3, o);
-  }
-  if (!act || a != 0) return;
-  const double q = (double)p.w;
-  if (MODE == 2) {
-    const int o = id[i];  // results in the caller's atom order
-    if (dq) dq[o] = F0;
-    if (dr) {
-      dr[3 * o] = q * F1 * K0 * st->Li[0];
-      dr[3 * o + 1] = q * F2 * K1 * st->Li[1];
-      dr[3 * o + 2] = q * F3 * K2 * st->Li[2];
-    }
-    return;
-  }
-  double4a f = {0.0, 0.0, 0.0, 0.0};
-  if (!live) {
-    if (store) force[i] = f;
-    return;
-  }
-  if (!store) f = force[i];
-  if (MODE == 0) {
-    f.x += q * F0;
-    f.y += q * F1;
-    f.z += q * F2;
-  } else {
-    f.x += 2.0 * q * F0 * K0 * st->Li[0];
-    f.y += 2.0 * q * F1 * K1 * st->Li[1];
-    f.z += 2.0 * q * F2 * K2 * st->Li[2];
-  }
-  force[i] = f;
-}
-
 // ---------------------------------------------------------------- adjoint
 // The reciprocal energy is the quadratic form E = 1/2 sum_m psi(m) |Q^(m)|^2
 // = 1/2 sum_k Q(k) Phi(k) with Phi = IFFT(psi Q^) (unnormalised transforms),
@@ -1018,29 +636,6 @@ static const void* fftx_fn(int logn, int method) {
   return nullptr;
 }
 
-template <class R>
-static const void* spread_fn(int order) {
-  switch (order) {
-#define ORDER_CASE(NO) case NO: return (const void*)k_spme_spread_t<R, NO>;
-    SPME_ORDERS(ORDER_CASE)
-#undef ORDER_CASE
-  }
-  return nullptr;
-}
-
-template <class R>
-static const void* gather_fn(int order, int mode) {
-  switch (order) {
-#define ORDER_CASE(NO)                                                                          \
-  case NO:                                                                                      \
-    return mode == 0 ? (const void*)k_spme_gather_t<R, NO, 0>                                   \
-                     : (mode == 1 ? (const void*)k_spme_gather_t<R, NO, 1> : (const void*)k_spme_gather_t<R, NO, 2>);
-    SPME_ORDERS(ORDER_CASE)
-#undef ORDER_CASE
-  }
-  return nullptr;
-}
-
 static int ilog2i(int k) {
   int l = 0;
   while ((1 << l) < k) ++l;
@@ -1101,7 +696,7 @@ static int spme_prepare(md_spme* s) {
     MD_CHECK_LAUNCH("fft twiddles");
   }
   const int l0 = ilog2i(s->K[0]), l1 = ilog2i(s->K[1]), l2 = ilog2i(s->K[2]);
-  if (int r = smem_optin(spread_fn<R>(s->order), SPREAD_TILE_BYTES)) return r;
+  if (int r = pm_prepare(s->sys->prec, s->order)) return r;
   if (int r = smem_optin(fftp_fn<R>(l2, 0, -1, 0), fftp_smem<R>(l2, 1))) return r;
   if (int r = smem_optin(fftp_fn<R>(l2, 2, 1, 0), fftp_smem<R>(l2, 1))) return r;
   if (int r = smem_optin(fftp_fn<R>(l2, 2, 1, 1), fftp_smem<R>(l2, 2))) return r;
@@ -1110,8 +705,6 @@ static int spme_prepare(md_spme* s) {
     if (int r = smem_optin(fftp_fn<R>(l0, 1, sg, 0), fftp_smem<R>(l0, 1))) return r;
   }
   if (int r = smem_optin(fftx_fn<R>(l0, s->method), fftx_smem<R>(l0, s->method))) return r;
-  for (int m = 0; m < 3; ++m)
-    if (int r = smem_optin(gather_fn<R>(s->order, m), GATHER_TILE_BYTES)) return r;
   return MD_OK;
 }
 
@@ -1133,20 +726,6 @@ static int influence_launch(md_spme* s, Recorder* rec) {
   return rec_launch(rec, (const void*)k_spme_box_tab, dim3(1), dim3(1), 0, a);
 }
 
-// charges onto the (cleared) real mesh
-template <class R>
-static int spread_launch(md_spme* s, Recorder* rec) {
-  md_system* sys = s->sys;
-  int K0 = s->K[0], K1 = s->K[1], K2 = s->K[2], N = sys->N;
-  R* Q = (R*)s->Q;
-  DevState* st = sys->st;
-  const void* pos = sys->pos;
-  int cap = SPREAD_TILE_BYTES / (int)sizeof(R);
-  void* a[] = {&N, &pos, &K0, &K1, &K2, &st, &Q, &cap};
-  return rec_launch(rec, spread_fn<R>(s->order), dim3(ceil_div(N, SPREAD_ATOMS)), dim3(SPREAD_THREADS),
-                    SPREAD_TILE_BYTES, a);
-}
-
 // spread and the forward transform along z (which clears the real mesh for
 // the next spread), y and (with_x) x: C[0] = Q^ on the half spectrum.  Every
 // launch goes through the recorder, so the chain is either run on the stream
@@ -1156,28 +735,12 @@ static int spme_forward_mesh(md_spme* s, Recorder* rec, bool with_x) {
   typedef typename C2<R>::T T2;
   R* Q = (R*)s->Q;
   T2* C = (T2*)s->C;
-  if (int r = spread_launch<R>(s, rec)) return r;
+  if (int r = pm_spread(s->sys, s->K, s->order, Q, rec)) return r;
   if (int r = fft_launch<R>(s, rec, Q, C, 0, 2, -1, 1, 0)) return r;
   if (int r = fft_launch<R>(s, rec, C, C, 1, 1, -1, 1, 0)) return r;
   if (with_x)
     if (int r = fft_launch<R>(s, rec, C, C, 1, 0, -1, 1, 0)) return r;
   return MD_OK;
-}
-
-template <class R>
-static int gather_launch(md_spme* s, Recorder* rec, int mode, double* dq, double* dr, bool store) {
-  md_system* sys = s->sys;
-  int N = sys->N, K0 = s->K[0], K1 = s->K[1], K2 = s->K[2];
-  const void* pos = sys->pos;
-  const void* G = s->G;
-  DevState* st = sys->st;
-  const size_t el = mode == 0 ? sizeof(typename V4<R>::T) : sizeof(R);
-  int cap = (int)(GATHER_TILE_BYTES / el);
-  double4a* force = store ? s->frec : sys->force;
-  int st_ = store ? 1 : 0;
-  void* a[] = {&N, &pos, &sys->id, &K0, &K1, &K2, &st, &G, &force, &dq, &dr, &cap, &st_};
-  return rec_launch(rec, gather_fn<R>(s->order, mode), dim3(ceil_div(N, GATHER_ATOMS)),
-                    dim3(GATHER_ATOMS * gather_lanes(s->order)), GATHER_TILE_BYTES, a);
 }
 
 template <class R>
@@ -1203,7 +766,7 @@ static int spme_run(md_spme* s, bool with_stats, Recorder* rec, bool concurrent)
   T2* Cp = C + s->nhalf;
   if (int r = fft_launch<R>(s, rec, Cp, Cp, 1, 1, +1, nconv, 0)) return r;
   if (int r = fft_launch<R>(s, rec, Cp, s->G, 2, 2, +1, nconv, method == 0 ? 1 : 0)) return r;
-  return gather_launch<R>(s, rec, method, nullptr, nullptr, concurrent);
+  return pm_gather(sys, s->K, s->order, method, s->G, concurrent ? s->frec : sys->force, concurrent ? 1 : 0, rec);
 }
 
 bool spme_belongs_to(const md_spme* s, const md_system* sys) { return s && s->sys == sys; }
@@ -1254,7 +817,7 @@ static int spme_energy_grad(md_spme* s, double* energy, double* dq, double* dr, 
     if (int r = fft_launch<R>(s, &rec, Cp, Cp, 1, 0, +1, 1, 0)) return r;
     if (int r = fft_launch<R>(s, &rec, Cp, Cp, 1, 1, +1, 1, 0)) return r;
     if (int r = fft_launch<R>(s, &rec, Cp, s->G, 2, 2, +1, 1, 0)) return r;
-    if (int r = gather_launch<R>(s, &rec, 2, d_q, d_r, false)) return r;
+    if (int r = pm_gather_adjoint(sys, s->K, s->order, s->G, d_q, d_r, &rec)) return r;
   }
   if (dev) {
     k_adj_out<<<1, 1, 0, st_>>>(sys->st, energy, dbeta);
@@ -1402,7 +965,7 @@ extern "C" int md_spme_get_mesh(md_spme* s, double* Q) {
   Recorder rec;
   rec.stream = sys->stream;
   const bool f = sys->prec != MD_PREC_FP64;
-  if (int r = f ? spread_launch<float>(s, &rec) : spread_launch<double>(s, &rec)) return r;
+  if (int r = pm_spread(sys, s->K, s->order, s->Q, &rec)) return r;
   double* d = nullptr;
   MD_CUDA(cudaMallocAsync((void**)&d, sizeof(double) * s->nreal, sys->stream));
   k_mesh_out<<<(unsigned)((s->nreal + 255) / 256), 256, 0, sys->stream>>>(
