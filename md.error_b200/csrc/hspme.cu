@@ -37,9 +37,22 @@
 //   Lam     = -Re IFFT(sum_a i 2 pi m_a/L_a G Bh_a),
 //   H_d     = marginals of Re(sum_a conj(Bh_a) i 2 pi m_a/L_a Qh) G
 // (all inverse transforms unnormalised).
-// Weights, their position and coefficient derivatives are evaluated in the
-// spread and gather kernels; the 3D transforms are the FP64 grid transforms
-// (radix-2 FFT for power-of-two meshes).
+// Candidates go through in batches of up to four, one launch per step.  All
+// meshes are real, so the FP64 grid transforms (dft.cu) carry two each, as the
+// real and imaginary parts: the charge meshes of two candidates forward,
+// (E_0, E_1) and (E_2, phi_pot) back -- for the force error (E_0, E_1), and E_2,
+// B_2 and Lam of two candidates -- 6.5 complex transforms per candidate for
+// both functionals where one per mesh takes 14; separate spectra come from
+// Z(m) and Z(-m).  Spread and gather give a warp to an atom with lanes along
+// its stencil rows; the gather leaves the scalar field of the stencil in shared
+// memory and contracts it by axis, which yields dE/dq, dE/dr and the
+// coefficient sums together (for the force error all three need only the
+// scalar Lam - R.E).  Sums over blocks and the marginals are block reductions
+// in a fixed order.  Bound: FP64 mesh atomics in the spread, latency and L2
+// reads in the gather.  8 candidates of order-6 support, 20,736 charges, 64^3,
+// energy and force error with every gradient: 11.8 ms when each candidate ran
+// by itself with serial finishing sums and atomic marginals.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -52,9 +65,8 @@ namespace {
 constexpr int HS_MAX_S = 16;      // stencil points per axis (2 ceil(CC))
 constexpr int HS_MAX_NBIN = 64;
 constexpr int HS_MAX_COEF = 2 * HS_MAX_NBIN;
-constexpr int HS_THREADS = 128;
-constexpr int HS_G = 8;                        // lanes per atom in the spread and gather
-constexpr int HS_ATOMS = HS_THREADS / HS_G;    // atoms per spread / gather block
+constexpr int HS_BATCH = 4;  // candidates per launch (two where four would not stay in L2)
+constexpr int HS_ATOMS = 4;  // atoms per warp of the spread and the gather
 
 struct HsGeom {
   int K[3];
@@ -116,53 +128,54 @@ __device__ __forceinline__ PhiEval phi_eval(const HsGeom& g, const double* c, do
   return e;
 }
 
-__device__ __forceinline__ long mesh_index(const HsGeom& g, const int k[3]) {
-  return (long)k[2] + (long)g.K[2] * ((long)k[1] + (long)g.K[1] * k[0]);
-}
-
-// stencil of one atom, shared by its HS_G lanes: first point k0_d and the
-// weights phi and phi' per axis; the lanes evaluate the 3 S entries between
-// them.  u_d is returned to every lane (the coefficient derivatives are
-// re-evaluated from it at the end).
-struct GroupStencil {
-  int k0[3];
-  double v[3][HS_MAX_S], dv[3][HS_MAX_S];
-};
-
-__device__ void group_stencil(const HsGeom& g, const double* c, const double* r, int sub, GroupStencil& s,
-                              double u[3], int k0[3]) {
-  for (int d = 0; d < 3; ++d) {
-    double f = r[d] / g.L[d];
-    f -= floor(f);
-    u[d] = g.K[d] * f;
-    k0[d] = (int)floor(u[d]) - g.half + 1;
-  }
-  if (sub == 0)
-    for (int d = 0; d < 3; ++d) s.k0[d] = k0[d];
-  for (int t = sub; t < 3 * g.S; t += HS_G) {
-    const int d = t / g.S, j = t - d * g.S;
-    const PhiEval e = phi_eval(g, c, u[d] - (double)(k0[d] + j));
-    s.v[d][j] = e.v;
-    s.dv[d][j] = e.dv;
-  }
-}
-
-template <int W>
-__device__ __forceinline__ double group_sum(double v) {
-#pragma unroll
-  for (int o = W / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, W);
-  return v;
-}
-
 __device__ __forceinline__ int wrap(int k, int K) {
   k %= K;
   return k < 0 ? k + K : k;
 }
 
-// b_d(m) and db_d(m)/dc_b for one candidate: one thread per (axis, m)
+// warps per block: the larger stencils' scalar field fills shared memory
+__host__ __device__ constexpr int hs_warps(int S) { return S <= 8 ? 4 : 1; }
+
+// An atom's stencil in shared memory, evaluated by its warp: the weights phi
+// and phi' and the wrapped mesh offsets of the 3 S one-dimensional points.
+template <int S>
+struct HsStencil {
+  double v[3][S], dv[3][S];
+  int off[3][S];
+};
+
+template <int S>
+__device__ __forceinline__ PhiEval hs_entry(const HsGeom& g, const double* c, const double* r, int t, HsStencil<S>& st) {
+  const int d = t / S, j = t - d * S;
+  double f = r[d] / g.L[d];
+  f -= floor(f);
+  const double u = g.K[d] * f;
+  const int k = (int)floor(u) - g.half + 1 + j;
+  const PhiEval e = phi_eval(g, c, u - (double)k);
+  st.v[d][j] = e.v;
+  st.dv[d][j] = e.dv;
+  st.off[d][j] = wrap(k, g.K[d]) * (d == 0 ? g.K[1] * g.K[2] : d == 1 ? g.K[2] : 1);
+  return e;
+}
+
+__device__ __forceinline__ double hs_block_sum(double v, double* sh) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s = 0.0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += sh[w];
+  return s;  // thread 0
+}
+
+// b_d(m) and db_d(m)/dc_b: one thread per (axis, m), a candidate per blockIdx.z
 __global__ void k_hs_factor(HsGeom g, const double* __restrict__ c, double* __restrict__ bfac,
                             double* __restrict__ dbfac, int Kmax) {
   const int d = blockIdx.y;
+  c += (long)blockIdx.z * g.ncoef;
+  bfac += (long)blockIdx.z * 3 * Kmax;
+  dbfac += (long)blockIdx.z * 3 * g.ncoef * Kmax;
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= g.K[d]) return;
   double b = 0.0;
@@ -180,306 +193,368 @@ __global__ void k_hs_factor(HsGeom g, const double* __restrict__ c, double* __re
   for (int t = 0; t < g.ncoef; ++t) dbfac[((long)d * g.ncoef + t) * Kmax + m] = db[t];
 }
 
-// spread: mode 0: Q += q_i W_i; mode 1: B_a -= q_i R_i,a W_i (three meshes).
-// HS_G lanes per atom share its S^3 stencil points (lane l: points l, l + HS_G, ...).
-__global__ void __launch_bounds__(HS_THREADS)
+// Spread, a candidate per blockIdx.y, a warp per atom with lanes along its
+// stencil rows.  MODE 0: Q += q_i W_i into part c & 1 of mesh c / 2; MODE 1:
+// B_a -= q_i R_i,a W_i, B_0 and B_1 as the parts of mesh c of `mesh`, B_2 into
+// part c & 1 of mesh c / 2 of `mesh2`.
+template <int S, int MODE>
+__global__ void __launch_bounds__(32 * hs_warps(S))
 k_hs_spread(HsGeom g, int N, const double* __restrict__ q, const double* __restrict__ r,
-            const double* __restrict__ c, int mode, const double* __restrict__ R, double2* __restrict__ mesh) {
-  __shared__ GroupStencil gs[HS_ATOMS];
-  const int grp = threadIdx.x / HS_G, sub = threadIdx.x % HS_G;
-  const int i = blockIdx.x * HS_ATOMS + grp;
-  if (i >= N) return;  // whole groups leave together; no block barrier below
-  GroupStencil& s = gs[grp];
-  double u[3];
-  int k0[3];
-  group_stencil(g, c, r + 3 * (long)i, sub, s, u, k0);
-  __syncwarp(((1u << HS_G) - 1u) << (threadIdx.x & 31 & ~(HS_G - 1)));  // the group's lanes
-  double a[3] = {q[i], 0.0, 0.0};
-  if (mode == 1) for (int d = 0; d < 3; ++d) a[d] = -q[i] * R[3 * (long)i + d];
-  const int S = g.S, S2 = S * S, S3 = S2 * S;
-  for (int t = sub; t < S3; t += HS_G) {
-    const int j0 = t / S2, j1 = (t / S) % S, j2 = t % S;
-    const double w = s.v[0][j0] * s.v[1][j1] * s.v[2][j2];
-    if (w == 0.0) continue;
-    const int k[3] = {wrap(k0[0] + j0, g.K[0]), wrap(k0[1] + j1, g.K[1]), wrap(k0[2] + j2, g.K[2])};
-    const long p = mesh_index(g, k);
-    if (mode == 0) {
-      atomicAdd(&mesh[p].x, a[0] * w);
-    } else {
-      for (int d = 0; d < 3; ++d) atomicAdd(&mesh[d * g.Kt + p].x, a[d] * w);
+            const double* __restrict__ coeffs, const double* __restrict__ R, double2* __restrict__ mesh,
+            double2* __restrict__ mesh2) {
+  constexpr int RP = 32 / S, NR = S * S, NI = (NR + RP - 1) / RP, W = hs_warps(S);
+  __shared__ HsStencil<S> sst[W];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cand = blockIdx.y;
+  HsStencil<S>& st = sst[warp];
+  const double* c = coeffs + (long)cand * g.ncoef;
+  const int k = lane / S, z = lane - k * S;
+  double* m0 = MODE == 0 ? reinterpret_cast<double*>(mesh + (long)(cand >> 1) * g.Kt) + (cand & 1)
+                         : reinterpret_cast<double*>(mesh + (long)cand * g.Kt);
+  double* m2 = MODE == 0 ? nullptr : reinterpret_cast<double*>(mesh2 + (long)(cand >> 1) * g.Kt) + (cand & 1);
+  for (int n = 0; n < HS_ATOMS; ++n) {
+    const int i = (blockIdx.x * W + warp) * HS_ATOMS + n;
+    if (i >= N) return;  // the whole warp
+    __syncwarp();
+    for (int t = lane; t < 3 * S; t += 32) hs_entry<S>(g, c, r + 3 * (long)i, t, st);
+    __syncwarp();
+    if (k >= RP) continue;
+    double a[3];
+    a[0] = q[i];
+    if (MODE == 1) {
+      const double* Ri = R + 3 * ((long)cand * N + i);
+      a[1] = -a[0] * Ri[1];
+      a[2] = -a[0] * Ri[2];
+      a[0] = -a[0] * Ri[0];
+    }
+    const double wz = st.v[2][z];
+    const int oz = st.off[2][z];
+#pragma unroll 4
+    for (int j = 0; j < NI; ++j) {
+      const int row = j * RP + k;
+      if (row >= NR) break;
+      const int x = row / S, y = row - x * S;
+      const double w = st.v[0][x] * st.v[1][y] * wz;
+      if (w == 0.0) continue;
+      const long p = 2 * (long)(st.off[0][x] + st.off[1][y] + oz);
+      atomicAdd(m0 + p, a[0] * w);
+      if (MODE == 1) {
+        atomicAdd(m0 + p + 1, a[1] * w);
+        atomicAdd(m2 + p, a[2] * w);
+      }
     }
   }
 }
 
-__device__ __forceinline__ void mvec(const HsGeom& g, long p, int m[3], double mv[3], bool nyq[3]) {
-  const int i2 = (int)(p % g.K[2]);
-  const int i1 = (int)((p / g.K[2]) % g.K[1]);
-  const int i0 = (int)(p / ((long)g.K[2] * g.K[1]));
-  const int id[3] = {i0, i1, i2};
-  for (int d = 0; d < 3; ++d) {
-    m[d] = id[d];
-    const int md = id[d] <= g.K[d] / 2 ? id[d] : id[d] - g.K[d];
-    mv[d] = md / g.L[d];
-    nyq[d] = (g.K[d] % 2 == 0) && id[d] == g.K[d] / 2;
-  }
-}
+struct HsPoint {
+  int m[3];
+  double k[3];  // 2 pi m_a / L_a, zero at the axis' own Nyquist index
+  double G;     // e^{-pi^2 |m|^2 / beta^2} / (pi V |m|^2), without the interpolation factors
+  long q;       // index of -m
+};
 
-__device__ __forceinline__ double influence(const HsGeom& g, const int m[3], const double mv[3],
-                                            const double* __restrict__ bfac, int Kmax) {
-  const double m2 = mv[0] * mv[0] + mv[1] * mv[1] + mv[2] * mv[2];
-  if (m2 == 0.0) return 0.0;
+__device__ __forceinline__ HsPoint hs_point(const HsGeom& g, long p) {
+  HsPoint h;
+  h.m[2] = (int)(p % g.K[2]);
+  h.m[1] = (int)((p / g.K[2]) % g.K[1]);
+  h.m[0] = (int)(p / ((long)g.K[2] * g.K[1]));
+  double m2 = 0.0;
+  h.q = 0;
+  for (int d = 0; d < 3; ++d) {
+    const int md = h.m[d] <= g.K[d] / 2 ? h.m[d] : h.m[d] - g.K[d];
+    const double mv = md / g.L[d];
+    m2 += mv * mv;
+    h.k[d] = (g.K[d] % 2 == 0) && h.m[d] == g.K[d] / 2 ? 0.0 : 2.0 * M_PI * mv;
+    h.q = h.q * g.K[d] + (h.m[d] ? g.K[d] - h.m[d] : 0);
+  }
   const double V = g.L[0] * g.L[1] * g.L[2];
-  double b2 = 1.0;
-  for (int d = 0; d < 3; ++d) {
-    const double b = bfac[d * Kmax + m[d]];
-    b2 *= b * b;
-  }
-  return exp(-M_PI * M_PI * m2 / (g.beta * g.beta)) / (M_PI * V * m2) / b2;
+  h.G = m2 == 0.0 ? 0.0 : exp(-M_PI * M_PI * m2 / (g.beta * g.beta)) / (M_PI * V * m2);
+  return h;
 }
 
-// k space of the forward pass: energy partials, the field transforms
-// (i 2 pi m_a G Qh, a = 0..2), the potential transform G Qh, and the marginals
-// P_d(m_d) of G |Qh|^2 (atomics)
-__global__ void k_hs_kspace_fwd(HsGeom g, const double2* __restrict__ Qh, const double* __restrict__ bfac, int Kmax,
-                                double2* __restrict__ field /* [4][Kt] */, double* __restrict__ marg,
-                                double* __restrict__ epart) {
-  const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  double e = 0.0;
-  if (p < g.Kt) {
-    int m[3];
-    double mv[3];
-    bool nyq[3];
-    mvec(g, p, m, mv, nyq);
-    const double G = influence(g, m, mv, bfac, Kmax);
-    const double2 z = Qh[p];
-    const double a2 = z.x * z.x + z.y * z.y;
-    e = 0.5 * G * a2;
-    for (int d = 0; d < 3; ++d) {
-      const double k = nyq[d] ? 0.0 : 2.0 * M_PI * mv[d] * G;  // i k z = (-k z.y, k z.x)
-      field[d * g.Kt + p] = make_double2(-k * z.y, k * z.x);
-    }
-    field[3 * g.Kt + p] = make_double2(G * z.x, G * z.y);
-    if (marg && G != 0.0)
-      for (int d = 0; d < 3; ++d) atomicAdd(&marg[d * Kmax + m[d]], G * a2);
-  }
-  for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-  __shared__ double sh[32];
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = e;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
-    epart[blockIdx.x] = t;
-  }
+__device__ __forceinline__ double hs_factor2(const HsPoint& h, const double* bfac, int Kmax) {
+  const double b = bfac[h.m[0]] * bfac[Kmax + h.m[1]] * bfac[2 * Kmax + h.m[2]];
+  return h.G / (b * b);
 }
 
-// k space of the loss adjoint: Lam transform -sum_a i k_a G Bh_a, and the
-// marginals of Re(sum_a conj(Bh_a) i k_a Qh) G
-__global__ void k_hs_kspace_adj(HsGeom g, const double2* __restrict__ Qh, const double2* __restrict__ Bh,
-                                const double* __restrict__ bfac, int Kmax, double2* __restrict__ lam,
-                                double* __restrict__ marg) {
+// spectra of the two real meshes packed as a complex one: z = Z(m), y = Z(-m)
+__device__ __forceinline__ double2 hs_first(double2 z, double2 y) { return make_double2(0.5 * (z.x + y.x), 0.5 * (z.y - y.y)); }
+__device__ __forceinline__ double2 hs_second(double2 z, double2 y) { return make_double2(0.5 * (z.y + y.y), 0.5 * (y.x - z.x)); }
+
+// k space of the forward pass, a point per thread, nb candidates: with
+// g = G Qh, F[c] = transform of E_0 + i E_1 = (i k_0 - k_1) g; energy pass
+// (pair = 0) F[nb + c] = E_2 + i phi = i (k_2 + 1) g; force error (pair = 1)
+// F[nb + c / 2] = E_2 of two candidates.  w[c] = G |Qh|^2 (or null).
+__global__ void __launch_bounds__(256)
+k_hs_kspace_fwd(HsGeom g, int nb, int pair, const double2* __restrict__ Z, const double* __restrict__ bfac, int Kmax,
+                double2* __restrict__ F, double* __restrict__ w) {
   const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (p >= g.Kt) return;
-  int m[3];
-  double mv[3];
-  bool nyq[3];
-  mvec(g, p, m, mv, nyq);
-  const double G = influence(g, m, mv, bfac, Kmax);
-  const double2 z = Qh[p];
-  double lx = 0.0, ly = 0.0, h = 0.0;
-  for (int d = 0; d < 3; ++d) {
-    if (nyq[d]) continue;
-    const double k = 2.0 * M_PI * mv[d];
-    const double2 b = Bh[d * g.Kt + p];
-    lx += k * G * b.y;   // -i k G b = (k G b.y, -k G b.x)
-    ly -= k * G * b.x;
-    // Re(conj(b) i k z) = k (b.x (-z.y) + b.y z.x)... conj(b) = (b.x, -b.y); i k z = (-k z.y, k z.x)
-    h += k * (-b.x * z.y + b.y * z.x);
-  }
-  lam[p] = make_double2(lx, ly);
-  if (marg && G != 0.0) {
-    const double v = h * G;
-    for (int d = 0; d < 3; ++d) atomicAdd(&marg[d * Kmax + m[d]], v);
+  const HsPoint h = hs_point(g, p);
+  for (int c = 0; c < nb; c += 2) {
+    const double2 z = Z[(c >> 1) * g.Kt + p], y = Z[(c >> 1) * g.Kt + h.q];
+    double2 e2 = make_double2(0.0, 0.0);
+    for (int s = 0; s < 2 && c + s < nb; ++s) {
+      const double2 Q = s ? hs_second(z, y) : hs_first(z, y);
+      const double G = hs_factor2(h, bfac + (long)(c + s) * 3 * Kmax, Kmax);
+      const double2 a = make_double2(G * Q.x, G * Q.y);
+      F[(c + s) * g.Kt + p] = make_double2(-h.k[0] * a.y - h.k[1] * a.x, h.k[0] * a.x - h.k[1] * a.y);
+      if (!pair) {
+        const double k = h.k[2] + 1.0;
+        F[(nb + c + s) * g.Kt + p] = make_double2(-k * a.y, k * a.x);
+      } else if (s == 0) {
+        e2 = make_double2(-h.k[2] * a.y, h.k[2] * a.x);
+      } else {
+        e2.x -= h.k[2] * a.x;
+        e2.y -= h.k[2] * a.y;
+      }
+      if (w) w[(c + s) * g.Kt + p] = G * (Q.x * Q.x + Q.y * Q.y);
+    }
+    if (pair) F[(nb + (c >> 1)) * g.Kt + p] = e2;
   }
 }
 
-// The real parts of three field meshes and one scalar mesh interleaved per
-// point (one 32-byte read per stencil point in the gather)
-__global__ void k_hs_pack4(long Kt, const double2* __restrict__ a, const double2* __restrict__ s,
-                           double4a* __restrict__ out) {
+// k space of the loss adjoint: Lam = -sum_a i k_a G Bh_a of two candidates per
+// mesh, w[c] = Re(sum_a conj(Bh_a) i k_a Qh) G
+__global__ void __launch_bounds__(256)
+k_hs_kspace_adj(HsGeom g, int nb, const double2* __restrict__ Z, const double2* __restrict__ Y,
+                const double2* __restrict__ Y2, const double* __restrict__ bfac, int Kmax, double2* __restrict__ lam,
+                double* __restrict__ w) {
   const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (p < Kt) out[p] = double4a{a[p].x, a[Kt + p].x, a[2 * Kt + p].x, s[p].x};
+  if (p >= g.Kt) return;
+  const HsPoint h = hs_point(g, p);
+  for (int c = 0; c < nb; c += 2) {
+    const long o = (c >> 1) * g.Kt;
+    const double2 z = Z[o + p], y = Z[o + h.q], z2 = Y2[o + p], y2 = Y2[o + h.q];
+    double2 l = make_double2(0.0, 0.0);
+    for (int s = 0; s < 2 && c + s < nb; ++s) {
+      const double2 Q = s ? hs_second(z, y) : hs_first(z, y);
+      const double2 zb = Y[(c + s) * g.Kt + p], yb = Y[(c + s) * g.Kt + h.q];
+      const double2 b[3] = {hs_first(zb, yb), hs_second(zb, yb), s ? hs_second(z2, y2) : hs_first(z2, y2)};
+      const double G = hs_factor2(h, bfac + (long)(c + s) * 3 * Kmax, Kmax);
+      double2 a = make_double2(0.0, 0.0);
+      double v = 0.0;
+      for (int d = 0; d < 3; ++d) {
+        a.x += h.k[d] * G * b[d].y;  // -i k G b
+        a.y -= h.k[d] * G * b[d].x;
+        v += h.k[d] * (-b[d].x * Q.y + b[d].y * Q.x);  // Re(conj(b) i k Q)
+      }
+      if (s == 0) {
+        l = a;
+      } else {  // + i times the second candidate's
+        l.x -= a.y;
+        l.y += a.x;
+      }
+      if (w) w[(c + s) * g.Kt + p] = v * G;
+    }
+    lam[o + p] = l;
+  }
 }
 
-// Gather.  mode 0 (energy): F_i, dE/dq_i, dE/dr_i, dE/dc partials from the
-// field meshes E_a and the potential (f4 = (E_0, E_1, E_2, phi)).  mode 1
-// (loss, first pass): F_i only (into F).  mode 2 (loss, adjoint): dL/dq_i,
-// dL/dr_i, dL/dc partials from f4 = (E_0, E_1, E_2, Lam).  HS_G lanes per atom
-// split its S^3 stencil points; their sums are combined by shuffles in a
-// fixed order.
-__global__ void __launch_bounds__(HS_THREADS)
+// marginals of w[c]: block (m, d, c) sums the plane m_d = m
+__global__ void __launch_bounds__(256)
+k_hs_marginal(HsGeom g, const double* __restrict__ w, int Kmax, double* __restrict__ marg) {
+  __shared__ double sh[8];
+  const int m = blockIdx.x, d = blockIdx.y, c = blockIdx.z;
+  if (m >= g.K[d]) return;
+  const double* wc = w + c * g.Kt;
+  const int n1 = d == 0 ? g.K[1] : g.K[0], n2 = d == 2 ? g.K[1] : g.K[2];  // the other two axes
+  const long s0 = d == 0 ? (long)g.K[1] * g.K[2] : d == 1 ? g.K[2] : 1;   // strides
+  const long s1 = d == 0 ? g.K[2] : (long)g.K[1] * g.K[2], s2 = d == 2 ? g.K[2] : 1;
+  double v = 0.0;
+  for (int t = threadIdx.x; t < n1 * n2; t += 256) v += wc[m * s0 + (t / n2) * s1 + (t % n2) * s2];
+  v = hs_block_sum(v, sh);
+  if (threadIdx.x == 0) marg[(c * 3 + d) * (long)Kmax + m] = v;
+}
+
+struct HsOut {
+  double *F, *dq, *dr;  // [nb][N][3], [nb][N], [nb][N][3]; null where not asked
+  double* cpart;        // [nb][blocks][ncoef]
+};
+
+// Gather, a candidate per blockIdx.y, a warp per atom.
+//   MODE 0 (energy): f1 = (E_0, E_1), f2 = (E_2, phi): F_i, dE/dq_i, dE/dr_i and
+//     the coefficient partials of the scalar phi
+//   MODE 1 (loss): f2 = E_2 of two candidates: F_i, the residual R_i = 2 (F_i - Fref_i) / N
+//     and the block's part of the loss
+//   MODE 2 (loss adjoint): dL/dq_i, dL/dr_i and the coefficient partials of the
+//     scalar Lam - R_i.E (dL/dr_i = q_i sum grad W_i (Lam - R_i.E), and so for dq, dc)
+// Per atom the lanes read the field along the stencil rows and leave the scalar
+// s(a, b, c) in shared memory; u(a, b) = sum_c w s, then lane (d, j) forms
+// T[d][j] = sum over the other two axes of w w s, whose products with the
+// weights, their derivatives and their coefficient derivatives are the results.
+template <int S, int MODE>
+__global__ void __launch_bounds__(32 * hs_warps(S))
 k_hs_gather(HsGeom g, int N, const double* __restrict__ q, const double* __restrict__ r,
-            const double* __restrict__ c, int mode, const double4a* __restrict__ f4,
-            const double* __restrict__ R, double* __restrict__ F, double* __restrict__ dq, double* __restrict__ dr,
-            double* __restrict__ cpart) {
-  __shared__ double csum[HS_MAX_COEF];
-  __shared__ GroupStencil gs[HS_ATOMS];
-  for (int t = threadIdx.x; t < g.ncoef; t += blockDim.x) csum[t] = 0.0;
-  const int grp = threadIdx.x / HS_G, sub = threadIdx.x % HS_G;
-  const int i = blockIdx.x * HS_ATOMS + grp;
-  const bool live = i < N;
-  GroupStencil& s = gs[grp];
-  double u[3] = {0, 0, 0};
-  int k0[3] = {0, 0, 0};
-  if (live) group_stencil(g, c, r + 3 * (long)i, sub, s, u, k0);
-  __syncthreads();
-  const int S = g.S, S2 = S * S, S3 = S2 * S;
-  const double qi = live ? q[i] : 0.0;
-  double Ri[3] = {0, 0, 0};
-  if (live && mode == 2)
-    for (int d = 0; d < 3; ++d) Ri[d] = R[3 * (long)i + d];
-  double Ef[3] = {0, 0, 0};    // sum W E_a
-  double pot = 0.0;            // sum W phi (mode 0) or sum W Lam (mode 2)
-  double gpot[3] = {0, 0, 0};  // sum grad W phi / Lam
-  double M[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};  // sum d_b W E_a
-  // partial contractions per axis for the coefficient gradient: T[d][j] =
-  // sum over the other two axes of (scalar field) prod_{d' != d} w
-  double T[3][HS_MAX_S];
-  for (int d = 0; d < 3; ++d)
-    for (int j = 0; j < S; ++j) T[d][j] = 0.0;
-  const double kl[3] = {g.K[0] / g.L[0], g.K[1] / g.L[1], g.K[2] / g.L[2]};
-  if (live)
-    for (int t = sub; t < S3; t += HS_G) {
-      const int j0 = t / S2, j1 = (t / S) % S, j2 = t % S;
-      const double av = s.v[0][j0], adv = s.dv[0][j0], bv = s.v[1][j1], bdv = s.dv[1][j1];
-      const double ev = s.v[2][j2], edv = s.dv[2][j2];
-      const bool any = (av != 0.0 || adv != 0.0) && (bv != 0.0 || bdv != 0.0) && (ev != 0.0 || edv != 0.0);
-      if (!any) continue;
-      const double w12 = bv * ev, w02 = av * ev, w01 = av * bv;
-      const double w = av * w12;
-      const int k[3] = {wrap(k0[0] + j0, g.K[0]), wrap(k0[1] + j1, g.K[1]), wrap(k0[2] + j2, g.K[2])};
-      const long p = mesh_index(g, k);
-      const double gw[3] = {adv * kl[0] * w12, bdv * kl[1] * w02, edv * kl[2] * w01};
-      const double4a fv = f4[p];  // E_0, E_1, E_2 and the scalar field (phi or Lam)
-      const double E3[3] = {fv.x, fv.y, fv.z};
-      for (int d = 0; d < 3; ++d) Ef[d] += w * E3[d];
-      double sc = 0.0;  // the scalar field whose coefficient contraction is needed
-      if (mode == 0) {
-        const double ph = fv.w;
-        pot += w * ph;
-        for (int d = 0; d < 3; ++d) gpot[d] += gw[d] * ph;
-        sc = ph;
-      } else if (mode == 2) {
-        const double lm = fv.w;
-        pot += w * lm;
-        for (int d = 0; d < 3; ++d) gpot[d] += gw[d] * lm;
-        for (int a2 = 0; a2 < 3; ++a2)
-          for (int b2 = 0; b2 < 3; ++b2) M[a2][b2] += gw[b2] * E3[a2];
-        sc = lm - (Ri[0] * E3[0] + Ri[1] * E3[1] + Ri[2] * E3[2]);
-      }
-      if (mode != 1) {
-        T[0][j0] += sc * w12;
-        T[1][j1] += sc * w02;
-        T[2][j2] += sc * w01;
-      }
-    }
-  // group sums (every lane of the group ends with the totals)
-  for (int d = 0; d < 3; ++d) Ef[d] = group_sum<HS_G>(Ef[d]);
-  if (mode != 1) {
-    pot = group_sum<HS_G>(pot);
-    for (int d = 0; d < 3; ++d) gpot[d] = group_sum<HS_G>(gpot[d]);
-    for (int d = 0; d < 3; ++d)
-      for (int j = 0; j < S; ++j) T[d][j] = group_sum<HS_G>(T[d][j]);
+            const double* __restrict__ coeffs, const double2* __restrict__ f1, const double2* __restrict__ f2,
+            const double2* __restrict__ lam, const double* __restrict__ fref, double* __restrict__ R,
+            double* __restrict__ lpart, HsOut out) {
+  constexpr int RP = 32 / S, NR = S * S, NI = (NR + RP - 1) / RP, W = hs_warps(S), LD = S + 1;
+  __shared__ HsStencil<S> sst[W];
+  __shared__ double ss[W][MODE == 1 ? 1 : NR * LD], su[W][MODE == 1 ? 1 : NR], sp[W][MODE == 1 ? 1 : 32 + 4 * S];
+  __shared__ double csum[MODE == 1 ? 1 : HS_MAX_COEF], sl[W];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cand = blockIdx.y;
+  if (MODE != 1) {
+    for (int t = threadIdx.x; t < g.ncoef; t += blockDim.x) csum[t] = 0.0;
+    __syncthreads();
   }
-  if (mode == 2)
-    for (int a2 = 0; a2 < 3; ++a2)
-      for (int b2 = 0; b2 < 3; ++b2) M[a2][b2] = group_sum<HS_G>(M[a2][b2]);
-  if (live && sub == 0) {
-    if (mode == 0 || mode == 1)
-      for (int d = 0; d < 3; ++d) F[3 * (long)i + d] = -qi * Ef[d];
-    if (mode == 0) {
-      if (dq) dq[i] = pot;
-      if (dr) for (int d = 0; d < 3; ++d) dr[3 * (long)i + d] = qi * gpot[d];
-    } else if (mode == 2) {
-      // dL/dq_i = R_i . g_i + sum W Lam, g_i = -sum W E
-      if (dq) dq[i] = -(Ri[0] * Ef[0] + Ri[1] * Ef[1] + Ri[2] * Ef[2]) + pot;
-      if (dr)
-        for (int b2 = 0; b2 < 3; ++b2) {
-          double v = 0.0;
-          for (int a2 = 0; a2 < 3; ++a2) v += Ri[a2] * M[a2][b2];
-          dr[3 * (long)i + b2] = -qi * v + qi * gpot[b2];
+  HsStencil<S>& st = sst[warp];
+  const double* c = coeffs + (long)cand * g.ncoef;
+  const int k = lane / S, z = lane - k * S;
+  const double2* e01 = f1 + (long)cand * g.Kt;
+  const double2* e2p = f2 + (long)(MODE == 0 ? cand : cand >> 1) * g.Kt;
+  const double2* lm = MODE == 2 ? lam + (long)(cand >> 1) * g.Kt : nullptr;
+  const bool second = cand & 1;
+  double loss = 0.0;
+  for (int n = 0; n < HS_ATOMS; ++n) {
+    const int i = (blockIdx.x * W + warp) * HS_ATOMS + n;
+    if (i >= N) break;  // the whole warp
+    __syncwarp();
+    PhiEval e;
+    if (lane < 3 * S) e = hs_entry<S>(g, c, r + 3 * (long)i, lane, st);
+    if (3 * S > 32 && lane + 32 < 3 * S) hs_entry<S>(g, c, r + 3 * (long)i, lane + 32, st);
+    __syncwarp();
+    const double qi = q[i];
+    const long ia = (long)cand * N + i;
+    double Ri[3] = {0.0, 0.0, 0.0};
+    if (MODE == 2)
+      for (int d = 0; d < 3; ++d) Ri[d] = R[3 * ia + d];
+    double Ef[3] = {0.0, 0.0, 0.0}, t2 = 0.0;
+    if (k < RP) {
+      const int oz = st.off[2][z];
+#pragma unroll 4
+      for (int j = 0; j < NI; ++j) {
+        const int row = j * RP + k;
+        if (row >= NR) break;
+        const int x = row / S, y = row - x * S, p = st.off[0][x] + st.off[1][y] + oz;
+        const double wxy = st.v[0][x] * st.v[1][y];
+        const double2 a = e01[p], b = e2p[p];
+        if (MODE == 2) {
+          const double2 l = lm[p];
+          const double s = (second ? l.y : l.x) - (Ri[0] * a.x + Ri[1] * a.y + Ri[2] * (second ? b.y : b.x));
+          ss[warp][row * LD + z] = s;
+          t2 += wxy * s;
+        } else {
+          Ef[0] += wxy * a.x;
+          Ef[1] += wxy * a.y;
+          Ef[2] += wxy * (MODE == 0 || !second ? b.x : b.y);
+          if (MODE == 0) {
+            ss[warp][row * LD + z] = b.y;
+            t2 += wxy * b.y;
+          }
         }
+      }
+      if (MODE != 2) {
+        const double wz = st.v[2][z];
+        for (int d = 0; d < 3; ++d) Ef[d] *= wz;
+      }
     }
-  }
-  if (live && mode != 1 && cpart) {
-    // the group's lanes split the 3 S stencil entries, re-evaluating which
-    // coefficients each weight depends on
-    for (int t = sub; t < 3 * S; t += HS_G) {
+    if (MODE != 2) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        for (int d = 0; d < 3; ++d) Ef[d] += __shfl_xor_sync(0xffffffffu, Ef[d], o);
+      if (lane < 3) {
+        const double F = -qi * (lane == 0 ? Ef[0] : lane == 1 ? Ef[1] : Ef[2]);
+        if (out.F) out.F[3 * ia + lane] = F;
+        if (MODE == 1) {
+          const double dF = F - fref[3 * (long)i + lane];
+          R[3 * ia + lane] = 2.0 * dF / N;
+          loss += dF * dF / N;
+        }
+      }
+    }
+    if (MODE == 1) continue;
+    sp[warp][lane] = t2;
+    __syncwarp();
+    for (int row = lane; row < NR; row += 32) {
+      double u = 0.0;
+#pragma unroll
+      for (int j = 0; j < S; ++j) u += st.v[2][j] * ss[warp][row * LD + j];
+      su[warp][row] = u;
+    }
+    __syncwarp();
+    for (int t = lane; t < 3 * S; t += 32) {
       const int d = t / S, j = t - d * S;
-      const double tv = qi * T[d][j];
-      if (tv == 0.0) continue;
-      const PhiEval e = phi_eval(g, c, u[d] - (double)(k0[d] + j));
-      for (int b2 = 0; b2 < 4; ++b2)
-        if (e.idx[b2] >= 0) atomicAdd(&csum[e.idx[b2]], tv * e.dc[b2]);
+      double T = 0.0;
+      if (d == 0) {
+#pragma unroll
+        for (int b = 0; b < S; ++b) T += st.v[1][b] * su[warp][j * S + b];
+      } else if (d == 1) {
+#pragma unroll
+        for (int a = 0; a < S; ++a) T += st.v[0][a] * su[warp][a * S + j];
+      } else {
+#pragma unroll
+        for (int a = 0; a < RP; ++a) T += sp[warp][a * S + j];
+      }
+      sp[warp][32 + t] = st.dv[d][j] * T;
+      if (d == 0) sp[warp][32 + 3 * S + j] = st.v[0][j] * T;
+      if (out.cpart) {
+        // which coefficients the weight depends on
+        const double tv = qi * T;
+        if (t >= 32) {
+          HsStencil<S>& same = st;  // re-evaluated: the same values are stored again
+          e = hs_entry<S>(g, c, r + 3 * (long)i, t, same);
+        }
+        for (int b = 0; b < 4; ++b)
+          if (e.idx[b] >= 0) atomicAdd(&csum[e.idx[b]], tv * e.dc[b]);
+      }
+    }
+    __syncwarp();
+    if (lane < 4) {
+      double v = 0.0;
+#pragma unroll
+      for (int j = 0; j < S; ++j) v += sp[warp][32 + lane * S + j];
+      if (lane < 3) {
+        if (out.dr) out.dr[3 * ia + lane] = qi * v * g.K[lane] / g.L[lane];
+      } else if (out.dq) {
+        out.dq[ia] = v;
+      }
     }
   }
-  __syncthreads();
-  if (cpart)
-    for (int t = threadIdx.x; t < g.ncoef; t += blockDim.x) cpart[(long)blockIdx.x * g.ncoef + t] = csum[t];
+  if (MODE == 1) {
+    for (int o = 2; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if (lane == 0) sl[warp] = loss;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double v = 0.0;
+      for (int w = 0; w < W; ++w) v += sl[w];
+      lpart[(long)cand * gridDim.x + blockIdx.x] = v;
+    }
+  } else if (out.cpart) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < g.ncoef; t += blockDim.x)
+      out.cpart[((long)cand * gridDim.x + blockIdx.x) * g.ncoef + t] = csum[t];
+  }
 }
 
-// coefficient gradient: block partials in a fixed order, plus the
-// interpolation factor term -w sum_d sum_m marg_d(m) db_d(m)/dc / b_d(m)
-__global__ void k_hs_coef_finish(HsGeom g, const double* __restrict__ cpart, int nblk, const double* __restrict__ marg,
-                                 const double* __restrict__ bfac, const double* __restrict__ dbfac, int Kmax,
-                                 double wfac, double* __restrict__ out, const double* __restrict__ epart, int neblk,
-                                 double* __restrict__ energy) {
-  const int t = threadIdx.x;
-  if (out && t < g.ncoef) {
-    double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += cpart[(long)b * g.ncoef + t];
+// Block (t, c): coefficient t's gradient of candidate c, the gather's block
+// partials plus the interpolation factor term -wfac sum_d sum_m marg_d(m) db_d(m)/dc / b_d(m);
+// t = ncoef: the energy, half the sum of a marginal, or the loss from its parts
+__global__ void __launch_bounds__(128)
+k_hs_finish(HsGeom g, const double* __restrict__ cpart, int nblk, const double* __restrict__ marg,
+            const double* __restrict__ bfac, const double* __restrict__ dbfac, int Kmax, double wfac,
+            double* __restrict__ out, const double* __restrict__ lpart, double* __restrict__ scalar) {
+  __shared__ double sh[4];
+  const int t = blockIdx.x, c = blockIdx.y;
+  double s = 0.0;
+  if (t < g.ncoef) {
+    if (!out) return;
+    for (int b = threadIdx.x; b < nblk; b += 128) s += cpart[((long)c * nblk + b) * g.ncoef + t];
     double f = 0.0;
     for (int d = 0; d < 3; ++d)
-      for (int m = 0; m < g.K[d]; ++m) {
-        const double b = bfac[d * Kmax + m];
-        f += marg[d * Kmax + m] * dbfac[((long)d * g.ncoef + t) * Kmax + m] / b;
-      }
-    out[t] = s - wfac * f;
+      for (int m = threadIdx.x; m < g.K[d]; m += 128)
+        f += marg[(c * 3 + d) * (long)Kmax + m] * dbfac[(((long)c * 3 + d) * g.ncoef + t) * Kmax + m] /
+             bfac[(c * 3 + d) * (long)Kmax + m];
+    s = hs_block_sum(s - wfac * f, sh);
+    if (threadIdx.x == 0) out[(long)c * g.ncoef + t] = s;
+    return;
   }
-  if (t == 0 && energy) {
-    double e = 0.0;
-    for (int b = 0; b < neblk; ++b) e += epart[b];
-    *energy = e;
-  }
-}
-
-__global__ void k_hs_residual(int N, const double* __restrict__ F, const double* __restrict__ Fref,
-                              double* __restrict__ R, double* __restrict__ part) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double l = 0.0;
-  if (i < N)
-    for (int d = 0; d < 3; ++d) {
-      const double e = F[3 * (long)i + d] - Fref[3 * (long)i + d];
-      R[3 * (long)i + d] = 2.0 * e / N;
-      l += e * e / N;
-    }
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  __shared__ double sh[32];
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = l;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
-    part[blockIdx.x] = t;
-  }
-}
-
-__global__ void k_hs_sum(const double* __restrict__ part, int n, double* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int b = 0; b < n; ++b) s += part[b];
-    *out = s;
-  }
+  if (!scalar) return;
+  if (lpart)
+    for (int b = threadIdx.x; b < nblk; b += 128) s += lpart[(long)c * nblk + b];
+  else
+    for (int m = threadIdx.x; m < g.K[0]; m += 128) s += 0.5 * marg[c * 3 * (long)Kmax + m];
+  s = hs_block_sum(s, sh);
+  if (threadIdx.x == 0) scalar[c] = s;
 }
 
 }  // namespace
@@ -489,22 +564,23 @@ struct md_hspme {
   int N = 0;
   HsGeom g;
   int Kmax = 0;
-  double2* mesh = nullptr;   // [4][Kt]: Q / Qh, then field and potential [4][Kt] below
-  double2* fld = nullptr;    // [4][Kt]
-  double2* bmesh = nullptr;  // [3][Kt] residual spread / transforms
-  double2* lam = nullptr;    // [Kt]
-  double4a* f4 = nullptr;    // [Kt] gather input: fields and one scalar mesh, real parts
-  double* bfac = nullptr;    // [3][Kmax]
-  double* dbfac = nullptr;   // [3][ncoef][Kmax]
-  double* marg = nullptr;    // [3][Kmax]
-  double* epart = nullptr;   // [k-space blocks]
-  double* cpart = nullptr;   // [atom blocks][ncoef]
-  double* R = nullptr;       // [N][3] residual weights
-  double* Fw = nullptr;      // [N][3] forces of the loss pass
+  int B = HS_BATCH;          // candidates per batch
+  int nab = 0;               // blocks of the spread and the gather
+  double2* Z = nullptr;      // [B/2][Kt] charge meshes of two candidates each, transformed in place
+  double2* F = nullptr;      // [2B][Kt] fields
+  double2* Y = nullptr;      // [B + B/2][Kt] residual meshes
+  double2* lam = nullptr;    // [B/2][Kt]
+  double* w = nullptr;       // [B][Kt] summand of the marginals
+  double* bfac = nullptr;    // [B][3][Kmax]
+  double* dbfac = nullptr;   // [B][3][ncoef][Kmax]
+  double* marg = nullptr;    // [B][3][Kmax]
+  double* cpart = nullptr;   // [B][nab][ncoef]
+  double* lpart = nullptr;   // [B][nab]
+  double* R = nullptr;       // [B][N][3] residual weights
 };
 
 static void hs_free(md_hspme* h) {
-  void* p[] = {h->mesh, h->fld, h->bmesh, h->lam, h->f4, h->bfac, h->dbfac, h->marg, h->epart, h->cpart, h->R, h->Fw};
+  void* p[] = {h->Z, h->F, h->Y, h->lam, h->w, h->bfac, h->dbfac, h->marg, h->cpart, h->lpart, h->R};
   for (void* x : p) if (x) cudaFree(x);
 }
 
@@ -538,19 +614,23 @@ extern "C" int md_hspme_create(md_hspme** out, int natoms, const int K[3], const
   g.Kt = (long)K[0] * K[1] * K[2];
   h->Kmax = std::max(K[0], std::max(K[1], K[2]));
   const long Kt = g.Kt;
-  const long nkb = (Kt + 255) / 256, nab = (natoms + HS_ATOMS - 1) / HS_ATOMS;
-  bool ok = cudaMalloc(&h->mesh, sizeof(double2) * Kt) == cudaSuccess &&
-            cudaMalloc(&h->fld, sizeof(double2) * 4 * Kt) == cudaSuccess &&
-            cudaMalloc(&h->bmesh, sizeof(double2) * 3 * Kt) == cudaSuccess &&
-            cudaMalloc(&h->lam, sizeof(double2) * Kt) == cudaSuccess &&
-            cudaMalloc(&h->f4, sizeof(double4a) * Kt) == cudaSuccess &&
-            cudaMalloc(&h->bfac, sizeof(double) * 3 * h->Kmax) == cudaSuccess &&
-            cudaMalloc(&h->dbfac, sizeof(double) * 3 * std::max(g.ncoef, 1) * h->Kmax) == cudaSuccess &&
-            cudaMalloc(&h->marg, sizeof(double) * 3 * h->Kmax) == cudaSuccess &&
-            cudaMalloc(&h->epart, sizeof(double) * std::max(nkb, nab)) == cudaSuccess &&
-            cudaMalloc(&h->cpart, sizeof(double) * nab * std::max(g.ncoef, 1)) == cudaSuccess &&
-            cudaMalloc(&h->R, sizeof(double) * 3 * natoms) == cudaSuccess &&
-            cudaMalloc(&h->Fw, sizeof(double) * 3 * natoms) == cudaSuccess;
+  const int per = HS_ATOMS * hs_warps(g.S), nco = std::max(g.ncoef, 1);
+  h->nab = (natoms + per - 1) / per;
+  // the meshes of a batch (80 bytes per point and candidate) stay in the 126 MB
+  // L2 with four candidates up to 64^3
+  h->B = Kt * 80 * HS_BATCH <= (96L << 20) ? HS_BATCH : 2;
+  const long B = h->B;
+  bool ok = cudaMalloc(&h->Z, sizeof(double2) * B / 2 * Kt) == cudaSuccess &&
+            cudaMalloc(&h->F, sizeof(double2) * 2 * B * Kt) == cudaSuccess &&
+            cudaMalloc(&h->Y, sizeof(double2) * (B + B / 2) * Kt) == cudaSuccess &&
+            cudaMalloc(&h->lam, sizeof(double2) * B / 2 * Kt) == cudaSuccess &&
+            cudaMalloc(&h->w, sizeof(double) * B * Kt) == cudaSuccess &&
+            cudaMalloc(&h->bfac, sizeof(double) * B * 3 * h->Kmax) == cudaSuccess &&
+            cudaMalloc(&h->dbfac, sizeof(double) * B * 3 * nco * h->Kmax) == cudaSuccess &&
+            cudaMalloc(&h->marg, sizeof(double) * B * 3 * h->Kmax) == cudaSuccess &&
+            cudaMalloc(&h->cpart, sizeof(double) * B * h->nab * nco) == cudaSuccess &&
+            cudaMalloc(&h->lpart, sizeof(double) * B * h->nab) == cudaSuccess &&
+            cudaMalloc(&h->R, sizeof(double) * B * 3 * natoms) == cudaSuccess;
   if (!ok) {
     md_cuda_fail(cudaGetLastError(), "md_hspme_create");
     hs_free(h);
@@ -575,25 +655,62 @@ extern "C" int md_hspme_num_coeffs(md_hspme* h, int* out) {
   return MD_OK;
 }
 
-// forward pass of candidate c: factors, spread, transform, k space, the four
-// inverse transforms (three field components and the potential)
-static int hs_forward(md_hspme* h, const double* q, const double* r, const double* c, cudaStream_t s,
-                      bool want_marg) {
-  HsGeom& g = h->g;
-  const long Kt = g.Kt;
-  const int nab = (h->N + HS_ATOMS - 1) / HS_ATOMS;
-  const int nkb = (int)((Kt + 255) / 256);
-  k_hs_factor<<<dim3((h->Kmax + 63) / 64, 3), 64, 0, s>>>(g, c, h->bfac, h->dbfac, h->Kmax);
-  MD_CHECK_LAUNCH("hspme factor");
-  MD_CUDA(cudaMemsetAsync(h->mesh, 0, sizeof(double2) * Kt, s));
-  k_hs_spread<<<nab, HS_THREADS, 0, s>>>(g, h->N, q, r, c, 0, nullptr, h->mesh);
+// stencil widths 2 ceil(CC)
+#define HS_WIDTHS(X) X(2) X(4) X(6) X(8) X(10) X(12) X(14) X(16)
+
+template <int MODE>
+static int hs_spread(md_hspme* h, int nb, const double* q, const double* r, const double* c, double2* mesh,
+                     double2* mesh2, cudaStream_t s) {
+  switch (h->g.S) {
+#define HS_CASE(W)                                                                                               \
+  case W:                                                                                                        \
+    k_hs_spread<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), 0, s>>>(h->g, h->N, q, r, c, h->R, mesh, mesh2);    \
+    break;
+    HS_WIDTHS(HS_CASE)
+#undef HS_CASE
+  }
   MD_CHECK_LAUNCH("hspme spread");
-  if (int e = dft3_grid(h->mesh, g.K, -1, 1, s)) return e;
-  if (want_marg) MD_CUDA(cudaMemsetAsync(h->marg, 0, sizeof(double) * 3 * h->Kmax, s));
-  k_hs_kspace_fwd<<<nkb, 256, 0, s>>>(g, h->mesh, h->bfac, h->Kmax, h->fld, want_marg ? h->marg : nullptr,
-                                      h->epart);
+  return MD_OK;
+}
+
+template <int MODE>
+static int hs_gather(md_hspme* h, int nb, const double* q, const double* r, const double* c, const double* fref,
+                     const HsOut& out, cudaStream_t s) {
+  const double2* f2 = h->F + (long)nb * h->g.Kt;
+  switch (h->g.S) {
+#define HS_CASE(W)                                                                                               \
+  case W:                                                                                                        \
+    k_hs_gather<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), 0, s>>>(h->g, h->N, q, r, c, h->F, f2, h->lam,      \
+                                                                      fref, h->R, h->lpart, out);                  \
+    break;
+    HS_WIDTHS(HS_CASE)
+#undef HS_CASE
+  }
+  MD_CHECK_LAUNCH("hspme gather");
+  return MD_OK;
+}
+
+static int hs_marginals(md_hspme* h, int nb, int axes, cudaStream_t s) {
+  k_hs_marginal<<<dim3(axes == 1 ? h->g.K[0] : h->Kmax, axes, nb), 256, 0, s>>>(h->g, h->w, h->Kmax, h->marg);
+  MD_CHECK_LAUNCH("hspme marginals");
+  return MD_OK;
+}
+
+// forward pass of nb candidates: factors, spread, transform, k space and the
+// inverse transforms of the fields (pair: as the force error wants them)
+static int hs_forward(md_hspme* h, int nb, const double* q, const double* r, const double* c, bool pair, bool want_w,
+                      cudaStream_t s) {
+  HsGeom& g = h->g;
+  const int np = (nb + 1) / 2;
+  k_hs_factor<<<dim3((h->Kmax + 63) / 64, 3, nb), 64, 0, s>>>(g, c, h->bfac, h->dbfac, h->Kmax);
+  MD_CHECK_LAUNCH("hspme factor");
+  MD_CUDA(cudaMemsetAsync(h->Z, 0, sizeof(double2) * np * g.Kt, s));
+  if (int e = hs_spread<0>(h, nb, q, r, c, h->Z, nullptr, s)) return e;
+  if (int e = dft3_grid(h->Z, g.K, -1, np, s)) return e;
+  k_hs_kspace_fwd<<<(unsigned)((g.Kt + 255) / 256), 256, 0, s>>>(g, nb, pair ? 1 : 0, h->Z, h->bfac, h->Kmax, h->F,
+                                                                 want_w ? h->w : nullptr);
   MD_CHECK_LAUNCH("hspme kspace");
-  return dft3_grid(h->fld, g.K, +1, 4, s);
+  return dft3_grid(h->F, g.K, +1, nb + (pair ? np : nb), s);
 }
 
 extern "C" int md_hspme_energy(md_hspme* h, const double* q, const double* r, const double* coeffs, int C,
@@ -603,23 +720,20 @@ extern "C" int md_hspme_energy(md_hspme* h, const double* q, const double* r, co
   MD_CUDA(cudaSetDevice(h->device));
   cudaStream_t s = (cudaStream_t)stream;
   HsGeom& g = h->g;
-  const int N = h->N;
-  const int nab = (N + HS_ATOMS - 1) / HS_ATOMS;
-  const int nkb = (int)((g.Kt + 255) / 256);
-  for (int b = 0; b < C; ++b) {
+  const long N = h->N;
+  for (int b = 0; b < C; b += h->B) {
+    const int nb = std::min(h->B, C - b);
     const double* c = coeffs + (long)b * g.ncoef;
-    if (int e = hs_forward(h, q, r, c, s, dE_dc != nullptr)) return e;
-    double* F = forces ? forces + 3L * N * b : h->Fw;
-    k_hs_pack4<<<nkb, 256, 0, s>>>(g.Kt, h->fld, h->fld + 3 * g.Kt, h->f4);
-    MD_CHECK_LAUNCH("hspme pack");
-    k_hs_gather<<<nab, HS_THREADS, 0, s>>>(g, N, q, r, c, 0, h->f4, nullptr, F,
-                                           dE_dq ? dE_dq + (long)N * b : nullptr, dE_dr ? dE_dr + 3L * N * b : nullptr,
-                                           dE_dc ? h->cpart : nullptr);
-    MD_CHECK_LAUNCH("hspme gather");
+    if (int e = hs_forward(h, nb, q, r, c, false, true, s)) return e;
+    if (int e = hs_marginals(h, nb, dE_dc ? 3 : 1, s)) return e;
+    if (forces || dE_dq || dE_dr || dE_dc) {
+      HsOut o = {forces ? forces + 3 * N * b : nullptr, dE_dq ? dE_dq + N * b : nullptr,
+                 dE_dr ? dE_dr + 3 * N * b : nullptr, dE_dc ? h->cpart : nullptr};
+      if (int e = hs_gather<0>(h, nb, q, r, c, nullptr, o, s)) return e;
+    }
     // the factor term of dE/dc: 1/2 sum G|Qh|^2 (-2 db/b) = -sum P db / b
-    k_hs_coef_finish<<<1, std::max(32, ((g.ncoef + 31) / 32) * 32), 0, s>>>(
-        g, h->cpart, nab, h->marg, h->bfac, h->dbfac, h->Kmax, 1.0, dE_dc ? dE_dc + (long)g.ncoef * b : nullptr,
-        h->epart, nkb, energy + b);
+    k_hs_finish<<<dim3(g.ncoef + 1, nb), 128, 0, s>>>(g, h->cpart, h->nab, h->marg, h->bfac, h->dbfac, h->Kmax, 1.0,
+                                                      dE_dc ? dE_dc + (long)g.ncoef * b : nullptr, nullptr, energy + b);
     MD_CHECK_LAUNCH("hspme finish");
   }
   return MD_OK;
@@ -635,46 +749,33 @@ extern "C" int md_hspme_force_error(md_hspme* h, const double* q, const double* 
   MD_CUDA(cudaSetDevice(h->device));
   cudaStream_t s = (cudaStream_t)stream;
   HsGeom& g = h->g;
-  const int N = h->N;
-  const long Kt = g.Kt;
-  const int nab = (N + HS_ATOMS - 1) / HS_ATOMS;       // spread / gather blocks
-  const int nrb = (N + HS_THREADS - 1) / HS_THREADS;   // residual blocks
-  const int nkb = (int)((Kt + 255) / 256);
+  const long N = h->N, Kt = g.Kt;
   const bool grads = dL_dq || dL_dr || dL_dc;
-  for (int b = 0; b < C; ++b) {
+  for (int b = 0; b < C; b += h->B) {
+    const int nb = std::min(h->B, C - b), np = (nb + 1) / 2;
     const double* c = coeffs + (long)b * g.ncoef;
-    if (int e = hs_forward(h, q, r, c, s, false)) return e;
-    k_hs_pack4<<<nkb, 256, 0, s>>>(Kt, h->fld, h->fld + 3 * Kt, h->f4);
-    MD_CHECK_LAUNCH("hspme pack");
-    k_hs_gather<<<nab, HS_THREADS, 0, s>>>(g, N, q, r, c, 1, h->f4, nullptr, h->Fw, nullptr, nullptr, nullptr);
-    MD_CHECK_LAUNCH("hspme gather");
-    k_hs_residual<<<nrb, HS_THREADS, 0, s>>>(N, h->Fw, fref, h->R, h->epart);
-    MD_CHECK_LAUNCH("hspme residual");
-    k_hs_sum<<<1, 32, 0, s>>>(h->epart, nrb, loss + b);
-    MD_CHECK_LAUNCH("hspme loss");
-    if (!grads) continue;
-    // adjoint: residuals spread, transformed, Lam and the factor marginals
-    MD_CUDA(cudaMemsetAsync(h->bmesh, 0, sizeof(double2) * 3 * Kt, s));
-    k_hs_spread<<<nab, HS_THREADS, 0, s>>>(g, N, q, r, c, 1, h->R, h->bmesh);
-    MD_CHECK_LAUNCH("hspme residual spread");
-    if (int e = dft3_grid(h->bmesh, g.K, -1, 3, s)) return e;
-    MD_CUDA(cudaMemsetAsync(h->marg, 0, sizeof(double) * 3 * h->Kmax, s));
-    k_hs_kspace_adj<<<nkb, 256, 0, s>>>(g, h->mesh, h->bmesh, h->bfac, h->Kmax, h->lam, h->marg);
-    MD_CHECK_LAUNCH("hspme adjoint kspace");
-    if (int e = dft3_grid(h->lam, g.K, +1, 1, s)) return e;
-    k_hs_pack4<<<nkb, 256, 0, s>>>(Kt, h->fld, h->lam, h->f4);
-    MD_CHECK_LAUNCH("hspme pack");
-    k_hs_gather<<<nab, HS_THREADS, 0, s>>>(g, N, q, r, c, 2, h->f4, h->R, nullptr,
-                                           dL_dq ? dL_dq + (long)N * b : nullptr, dL_dr ? dL_dr + 3L * N * b : nullptr,
-                                           dL_dc ? h->cpart : nullptr);
-    MD_CHECK_LAUNCH("hspme adjoint gather");
-    if (dL_dc) {
-      // factor term of dL/dc through G: sum_m H(m) dG/dc = -2 sum_d sum_m H_d db/b
-      k_hs_coef_finish<<<1, std::max(32, ((g.ncoef + 31) / 32) * 32), 0, s>>>(
-          g, h->cpart, nab, h->marg, h->bfac, h->dbfac, h->Kmax, 2.0, dL_dc + (long)g.ncoef * b, nullptr, 0,
-          nullptr);
-      MD_CHECK_LAUNCH("hspme adjoint finish");
+    if (int e = hs_forward(h, nb, q, r, c, true, false, s)) return e;
+    if (int e = hs_gather<1>(h, nb, q, r, c, fref, HsOut{}, s)) return e;
+    if (grads) {
+      // adjoint: residuals spread, transformed, Lam and the factor marginals
+      double2* Y2 = h->Y + nb * Kt;
+      MD_CUDA(cudaMemsetAsync(h->Y, 0, sizeof(double2) * (nb + np) * Kt, s));
+      if (int e = hs_spread<1>(h, nb, q, r, c, h->Y, Y2, s)) return e;
+      if (int e = dft3_grid(h->Y, g.K, -1, nb + np, s)) return e;
+      k_hs_kspace_adj<<<(unsigned)((Kt + 255) / 256), 256, 0, s>>>(g, nb, h->Z, h->Y, Y2, h->bfac, h->Kmax, h->lam,
+                                                                   dL_dc ? h->w : nullptr);
+      MD_CHECK_LAUNCH("hspme adjoint kspace");
+      if (dL_dc)
+        if (int e = hs_marginals(h, nb, 3, s)) return e;
+      if (int e = dft3_grid(h->lam, g.K, +1, np, s)) return e;
+      HsOut o = {nullptr, dL_dq ? dL_dq + N * b : nullptr, dL_dr ? dL_dr + 3 * N * b : nullptr,
+                 dL_dc ? h->cpart : nullptr};
+      if (int e = hs_gather<2>(h, nb, q, r, c, nullptr, o, s)) return e;
     }
+    // factor term of dL/dc through G: sum_m H(m) dG/dc = -2 sum_d sum_m H_d db/b
+    k_hs_finish<<<dim3(g.ncoef + 1, nb), 128, 0, s>>>(g, h->cpart, h->nab, h->marg, h->bfac, h->dbfac, h->Kmax, 2.0,
+                                                      dL_dc ? dL_dc + (long)g.ncoef * b : nullptr, h->lpart, loss + b);
+    MD_CHECK_LAUNCH("hspme finish");
   }
   return MD_OK;
 }
