@@ -50,7 +50,7 @@ k_fft_grid(const double2* in, double2* out, long nlines, long inner, int sign) {
   for (int s = 0; s < EPT; ++s) {
     const int e = threadIdx.x + s * FFT_THREADS;
     const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
-    X[l * LS + fft_pad(k)] = v[s];
+    X[l * LS + fft_pad<double>(k)] = v[s];
   }
   __syncthreads();
   double2* x = X + (threadIdx.x / G::TPL) * LS;
@@ -61,7 +61,7 @@ k_fft_grid(const double2* in, double2* out, long nlines, long inner, int sign) {
     const int e = threadIdx.x + s * FFT_THREADS;
     const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
     const long L = line0 + l;
-    if (L < nlines) out[line_base(L, n, inner) + k * inner] = X[l * LS + fft_pad(k)];
+    if (L < nlines) out[line_base(L, n, inner) + k * inner] = X[l * LS + fft_pad<double>(k)];
   }
 }
 

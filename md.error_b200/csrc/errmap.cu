@@ -158,7 +158,7 @@ k_em_alias_sq(EmGrid g, const double2* __restrict__ T, const double* __restrict_
     const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
     const long L = line0 + l;
     at[s] = L < nlines ? (size_t)(L / inner) * n * inner + (size_t)(L % inner) + k * inner : (size_t)-1;
-    xs[s] = l * LS + fft_pad(k);
+    xs[s] = l * LS + fft_pad<double>(k);
     km[s] = k;
     sq[s] = 0.0;
   }

@@ -18,10 +18,11 @@ template <> struct C2<double> { typedef double2 T; };
 // writes, so a single buffer per line suffices.  A block of FFT_THREADS
 // threads holds FFT_THREADS / TPL lines (TPL = n/8 threads per line); twiddles
 // come from a per-axis table computed once in FP64 (conjugated for the inverse
-// transform).  Element i of a line sits at fft_pad(i) = i + i/8: the outputs of
-// a radix-8 stage are 8 apart from lane to lane, which without the padding
-// falls on one bank (8-way conflicts in 64 and 128 bits); the odd line stride
-// keeps the loads and stores across lines conflict free.
+// transform).  Element i of a line sits at fft_pad(i): the outputs of a radix-8
+// stage are 8 apart from lane to lane (and, the next 64, from eighth to ninth
+// lane), which fall on one bank where they lie in order (8-way conflicts).
+// binary64: one element of padding per 8.  binary32: a permutation within each
+// 16 elements; padding would split every aligned run over two wavefronts.
 constexpr int FFT_THREADS = 128;
 
 template <class T2>
@@ -99,8 +100,13 @@ __device__ __forceinline__ void dft_reg(typename C2<R>::T (&v)[RR]) {
   }
 }
 
-__host__ __device__ __forceinline__ constexpr int fft_pad(int i) { return i + (i >> 3); }
-__host__ __device__ __forceinline__ constexpr int fft_line_stride(int n) { return n + (n >> 3) + 1; }
+template <class R>
+__host__ __device__ __forceinline__ constexpr int fft_pad(int i) {
+  return sizeof(R) == 4 ? i ^ ((i >> 4) & 7) ^ (((i >> 6) & 1) << 3) : i + (i >> 3);
+}
+// lines shorter than 256 share a warp: odd, so that accesses across lines fall
+// on different banks; longer ones pair up in the real passes (2 modulo 8)
+__host__ __device__ __forceinline__ constexpr int fft_line_stride(int n) { return n < 256 ? n + (n >> 3) + 1 : n + (n >> 3) + 2; }
 
 template <int LOGN>
 struct FftGeom {
@@ -125,7 +131,7 @@ __device__ __forceinline__ void fft_stages(typename C2<R>::T* x, const typename 
   for (int q = 0; q < BPT; ++q) {
     const int j = tl + q * TPL;
 #pragma unroll
-    for (int r = 0; r < RR; ++r) v[q][r] = x[fft_pad(j + r * NBF)];
+    for (int r = 0; r < RR; ++r) v[q][r] = x[fft_pad<R>(j + r * NBF)];
     if constexpr (LOGNS > 0) {
       const int k = j & (NS - 1);
 #pragma unroll
@@ -139,7 +145,7 @@ __device__ __forceinline__ void fft_stages(typename C2<R>::T* x, const typename 
     const int j = tl + q * TPL;
     const int d = ((j >> LOGNS) << (LOGNS + LR)) + (j & (NS - 1));
 #pragma unroll
-    for (int r = 0; r < RR; ++r) x[fft_pad(d + r * NS)] = v[q][r];
+    for (int r = 0; r < RR; ++r) x[fft_pad<R>(d + r * NS)] = v[q][r];
   }
   __syncthreads();
   if constexpr (LOGNS + LR < LOGN) fft_stages<R, LOGN, LOGNS + LR, SIGN>(x, tw, tl);

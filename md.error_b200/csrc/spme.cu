@@ -31,6 +31,7 @@
 #include <vector>
 #include "device_common.cuh"
 #include "fft_lines.cuh"
+#include "spme_plane.cuh"
 #include "spme_pm.cuh"
 
 struct md_spme {
@@ -50,6 +51,7 @@ struct md_spme {
   double4a* frec = nullptr;   // reciprocal forces of a concurrent evaluation (stored, not added)
   double* partials = nullptr; // block partials of the x pass (its own: it may run beside other reductions)
   int max_blocks = 0;
+  bool planes = false;        // equal x and y sizes: the transforms run by planes (spme_plane.cu)
   double* d_box_tab = nullptr;  // box psi was computed for (device; 0 = never)
 };
 
@@ -173,7 +175,7 @@ k_fftp(const void* in, void* out, const typename C2<R>::T* __restrict__ twg, lon
         if (L < nlc) src[2 * L * n + k] = R(0);
         if (2 * L + 1 < nlines) src[(2 * L + 1) * n + k] = R(0);
       }
-      Xb[l * LS + fft_pad(k)] = vv[s];
+      Xb[l * LS + fft_pad<R>(k)] = vv[s];
     }
   }
   __syncthreads();
@@ -185,10 +187,10 @@ k_fftp(const void* in, void* out, const typename C2<R>::T* __restrict__ twg, lon
       const long L = line0 + l2;
       if (L >= nlines) continue;
       R4 o;
-      const T2 xy = X[l2 * LS + fft_pad(k)];
+      const T2 xy = X[l2 * LS + fft_pad<R>(k)];
       o.x = xy.x;
       o.y = xy.y;
-      o.z = X[LPB * LS + l2 * LS + fft_pad(k)].x;
+      o.z = X[LPB * LS + l2 * LS + fft_pad<R>(k)].x;
       o.w = R(0);
       reinterpret_cast<R4*>(out)[L * n + k] = o;
     }
@@ -200,10 +202,10 @@ k_fftp(const void* in, void* out, const typename C2<R>::T* __restrict__ twg, lon
     else { l2 = e >> LOGN; k = e & (n - 1); }
     const long L = line0 + l2;
     if (L >= nlc) continue;
-    const T2 v = X[l2 * LS + fft_pad(k)];
+    const T2 v = X[l2 * LS + fft_pad<R>(k)];
     if (MODE == 0) {
       if (k < nh) {
-        const T2 w = X[l2 * LS + fft_pad((n - k) & (n - 1))];
+        const T2 w = X[l2 * LS + fft_pad<R>((n - k) & (n - 1))];
         T2 a, b;
         a.x = R(0.5) * (v.x + w.x);
         a.y = R(0.5) * (v.y - w.y);
@@ -306,7 +308,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
 #pragma unroll
     for (int s = 0; s < EPT; ++s) {
       const int e = gt + s * FFT_THREADS;
-      X[(e % LPB) * LS + fft_pad(e / LPB)] = vv[s];
+      X[(e % LPB) * LS + fft_pad<R>(e / LPB)] = vv[s];
     }
   }
   __syncthreads();
@@ -329,7 +331,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
       PS[le * LS + i] = ps;
       if (with_stats && live) {
         // E = 1/2 sum_m |Q^|^2 psi over the full spectrum: interior z planes count twice
-        const T2 q = X[le * LS + fft_pad(i)];
+        const T2 q = X[le * LS + fft_pad<R>(i)];
         const double wgt = (k == 0 || (2 * k == K2)) ? 1.0 : 2.0;
         const double e2 = 0.5 * wgt * ((double)q.x * q.x + (double)q.y * q.y) * (double)ps;
         // f = 2 (1 + pi^2 m^2 / beta^2) / m^2
@@ -347,7 +349,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
 #pragma unroll
   for (int s = 0; s < EPT; ++s) {
     const int e = gt + s * FFT_THREADS, le = e % LPB, i = e / LPB;
-    const T2 q = X[le * LS + fft_pad(i)];
+    const T2 q = X[le * LS + fft_pad<R>(i)];
     const R ps = PS[le * LS + i];
     T2 g;
     if (METHOD == 0 && grp == 0) {
@@ -363,7 +365,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
       g.x = q.x * (R(0.5) * ps);
       g.y = q.y * (R(0.5) * ps);
     }
-    Yg[le * LS + fft_pad(i)] = g;
+    Yg[le * LS + fft_pad<R>(i)] = g;
   }
   __syncthreads();
   fft_stages<R, LOGN, 0, 1>(Yg + l * LS, twi, tl);
@@ -377,7 +379,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
       if (L >= nlines) continue;
       const int jp = lj[le] <= K1 / 2 ? lj[le] : lj[le] - K1;
       const R cy = (R)(-2.0 * M_PI * (jp * st->Li[1])), cz = (R)(-2.0 * M_PI * (lk[le] * st->Li[2]));
-      const T2 v = Yg[le * LS + fft_pad(i)];
+      const T2 v = Yg[le * LS + fft_pad<R>(i)];
       T2 a, b;
       a.x = -v.y * cy;
       a.y = v.x * cy;
@@ -391,7 +393,7 @@ k_fft_x_kspace(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, 
     for (int e = gt; e < LPB * n; e += FFT_THREADS) {
       const int le = e % LPB, i = e / LPB;
       const long L = line0 + le;
-      if (L < nlines) out[L + i * stride] = Yg[le * LS + fft_pad(i)];
+      if (L < nlines) out[L + i * stride] = Yg[le * LS + fft_pad<R>(i)];
     }
   }
   if (with_stats && block_reduce_finish<4>(v, partials, &st->red_counter[RED_SPME], st->scratch, true) && merge) {
@@ -684,7 +686,8 @@ static int spme_prepare(md_spme* s) {
   // the real mesh starts cleared; every z pass clears it again after reading
   MD_CUDA(cudaMemsetAsync(s->Q, 0, sizeof(R) * s->nreal, str));
   MD_CUDA(cudaMalloc(&s->frec, sizeof(double4a) * s->sys->N));
-  s->max_blocks = ceil_div((long)s->K[1] * s->K2h, fft_lpb(s->K[0]));
+  // blocks of the x pass, or a plane each
+  s->max_blocks = std::max(ceil_div((long)s->K[1] * s->K2h, fft_lpb(s->K[0])), s->K2h);
   MD_CUDA(cudaMalloc(&s->partials, sizeof(double) * 4 * s->max_blocks));
   const int nbm = s->K[0] + s->K[1] + s->K2h;
   MD_CUDA(cudaMalloc(&s->bm, sizeof(double) * nbm));
@@ -697,6 +700,9 @@ static int spme_prepare(md_spme* s) {
   }
   const int l0 = ilog2i(s->K[0]), l1 = ilog2i(s->K[1]), l2 = ilog2i(s->K[2]);
   if (int r = pm_prepare(s->sys->prec, s->order)) return r;
+  s->planes = plane_chain_ok(s->sys->prec, s->K);
+  if (s->planes)
+    if (int r = plane_prepare(s->sys->prec, s->K, s->method)) return r;
   if (int r = smem_optin(fftp_fn<R>(l2, 0, -1, 0), fftp_smem<R>(l2, 1))) return r;
   if (int r = smem_optin(fftp_fn<R>(l2, 2, 1, 0), fftp_smem<R>(l2, 1))) return r;
   if (int r = smem_optin(fftp_fn<R>(l2, 2, 1, 1), fftp_smem<R>(l2, 2))) return r;
@@ -743,6 +749,25 @@ static int spme_forward_mesh(md_spme* s, Recorder* rec, bool with_x) {
   return MD_OK;
 }
 
+static PlaneChain plane_args(md_spme* s, int method) {
+  PlaneChain p;
+  p.n = s->K[0];
+  p.K2 = s->K[2];
+  p.method = method;
+  p.Q = s->Q;
+  p.C = s->C;
+  p.G = s->G;
+  p.bm = s->bm;
+  p.tw_n = s->tw[0];
+  p.tw_z = s->tw[2];
+  p.beta = s->beta;
+  p.partials = s->partials;
+  p.with_stats = 1;
+  p.merge = 0;
+  p.energy = p.dbeta = nullptr;
+  return p;
+}
+
 template <class R>
 static int spme_run(md_spme* s, bool with_stats, Recorder* rec, bool concurrent) {
   typedef typename C2<R>::T T2;
@@ -750,6 +775,14 @@ static int spme_run(md_spme* s, bool with_stats, Recorder* rec, bool concurrent)
   int K1 = s->K[1], K2 = s->K[2], method = s->method;
   T2* C = (T2*)s->C;
   DevState* st = sys->st;
+  if (s->planes) {
+    PlaneChain p = plane_args(s, method);
+    p.with_stats = with_stats ? 1 : 0;
+    p.merge = concurrent ? 0 : 1;
+    if (int r = pm_spread(sys, s->K, s->order, s->Q, rec)) return r;
+    if (int r = plane_chain(sys, p, rec)) return r;
+    return pm_gather(sys, s->K, s->order, method, s->G, concurrent ? s->frec : sys->force, concurrent ? 1 : 0, rec);
+  }
   if (int r = spme_forward_mesh<R>(s, rec, false)) return r;
   const int l0 = ilog2i(s->K[0]);
   const int nb = ceil_div((long)K1 * s->K2h, fft_lpb(s->K[0]));
@@ -807,17 +840,33 @@ static int spme_energy_grad(md_spme* s, double* energy, double* dq, double* dr, 
   double* d_p = dev ? nullptr : (dpsi ? d + nq + nr : nullptr);
   Recorder rec;
   rec.stream = st_;
-  if (int r = influence_launch<R>(s, &rec)) return r;
-  if (int r = spme_forward_mesh<R>(s, &rec, true)) return r;
-  k_spme_adj_kspace<R><<<nb, 256, 0, st_>>>(K0, K1, K2, s->beta, (const R*)s->psi, C, s->nhalf, sys->st,
-                                             sys->partials, d_p);
-  MD_CHECK_LAUNCH("spme adjoint kspace");
-  if (dq || dr) {
-    T2* Cp = C + s->nhalf;
-    if (int r = fft_launch<R>(s, &rec, Cp, Cp, 1, 0, +1, 1, 0)) return r;
-    if (int r = fft_launch<R>(s, &rec, Cp, Cp, 1, 1, +1, 1, 0)) return r;
-    if (int r = fft_launch<R>(s, &rec, Cp, s->G, 2, 2, +1, 1, 0)) return r;
-    if (int r = pm_gather_adjoint(sys, s->K, s->order, s->G, d_q, d_r, &rec)) return r;
+  const bool planes = s->planes && !dpsi;
+  if (planes) {
+    // energy and dE/dbeta leave the plane pass for their device outputs
+    PlaneChain p = plane_args(s, 2);
+    if (dev) {
+      p.energy = energy;
+      p.dbeta = dbeta;
+    }
+    if (int r = pm_spread(sys, s->K, s->order, s->Q, &rec)) return r;
+    if (int r = plane_chain(sys, p, &rec)) return r;
+    if (dq || dr)
+      if (int r = pm_gather_adjoint(sys, s->K, s->order, s->G, d_q, d_r, &rec)) return r;
+    if (dev) return MD_OK;
+  }
+  if (!planes) {
+    if (int r = influence_launch<R>(s, &rec)) return r;
+    if (int r = spme_forward_mesh<R>(s, &rec, true)) return r;
+    k_spme_adj_kspace<R><<<nb, 256, 0, st_>>>(K0, K1, K2, s->beta, (const R*)s->psi, C, s->nhalf, sys->st,
+                                               sys->partials, d_p);
+    MD_CHECK_LAUNCH("spme adjoint kspace");
+    if (dq || dr) {
+      T2* Cp = C + s->nhalf;
+      if (int r = fft_launch<R>(s, &rec, Cp, Cp, 1, 0, +1, 1, 0)) return r;
+      if (int r = fft_launch<R>(s, &rec, Cp, Cp, 1, 1, +1, 1, 0)) return r;
+      if (int r = fft_launch<R>(s, &rec, Cp, s->G, 2, 2, +1, 1, 0)) return r;
+      if (int r = pm_gather_adjoint(sys, s->K, s->order, s->G, d_q, d_r, &rec)) return r;
+    }
   }
   if (dev) {
     k_adj_out<<<1, 1, 0, st_>>>(sys->st, energy, dbeta);
