@@ -38,20 +38,21 @@
 //   H_d     = marginals of Re(sum_a conj(Bh_a) i 2 pi m_a/L_a Qh) G
 // (all inverse transforms unnormalised).
 // Candidates go through in batches of up to four, one launch per step.  All
-// meshes are real, so the FP64 grid transforms (dft.cu) carry two each, as the
-// real and imaginary parts: the charge meshes of two candidates forward,
-// (E_0, E_1) and (E_2, phi_pot) back -- for the force error (E_0, E_1), and E_2,
-// B_2 and Lam of two candidates -- 6.5 complex transforms per candidate for
-// both functionals where one per mesh takes 14; separate spectra come from
-// Z(m) and Z(-m).  Spread and gather give a warp to an atom with lanes along
-// its stencil rows; the gather leaves the scalar field of the stencil in shared
+// meshes are real, so the FP64 grid transforms (dft.cu) carry two fields of a
+// candidate each where it has two, as the real and imaginary parts: (E_0, E_1)
+// and (E_2, phi_pot) back, (B_0, B_1) forward -- 9 complex transforms per
+// candidate for both functionals where one per mesh takes 14.  Two candidates
+// never share a transform: the rounding of one (or its infinities) would reach
+// the other, 4 to 10 times the error in the gradient of the smaller.  Spread
+// and gather give a warp to an atom with lanes along its
+// stencil rows; the gather leaves the scalar field of the stencil in shared
 // memory and contracts it by axis, which yields dE/dq, dE/dr and the
 // coefficient sums together (for the force error all three need only the
 // scalar Lam - R.E).  Sums over blocks and the marginals are block reductions
 // in a fixed order.  Bound: FP64 mesh atomics in the spread, latency and L2
 // reads in the gather.  8 candidates of order-6 support, 20,736 charges, 64^3,
-// energy and force error with every gradient: 11.8 ms when each candidate ran
-// by itself with serial finishing sums and atomic marginals.
+// energy and force error with every gradient: 2.2 ms, 11.8 ms when each
+// candidate ran by itself with serial finishing sums and atomic marginals.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -194,9 +195,9 @@ __global__ void k_hs_factor(HsGeom g, const double* __restrict__ c, double* __re
 }
 
 // Spread, a candidate per blockIdx.y, a warp per atom with lanes along its
-// stencil rows.  MODE 0: Q += q_i W_i into part c & 1 of mesh c / 2; MODE 1:
+// stencil rows.  MODE 0: Q += q_i W_i into the real part of mesh c; MODE 1:
 // B_a -= q_i R_i,a W_i, B_0 and B_1 as the parts of mesh c of `mesh`, B_2 into
-// part c & 1 of mesh c / 2 of `mesh2`.
+// the real part of mesh c of `mesh2`.
 template <int S, int MODE>
 __global__ void __launch_bounds__(32 * hs_warps(S))
 k_hs_spread(HsGeom g, int N, const double* __restrict__ q, const double* __restrict__ r,
@@ -208,9 +209,8 @@ k_hs_spread(HsGeom g, int N, const double* __restrict__ q, const double* __restr
   HsStencil<S>& st = sst[warp];
   const double* c = coeffs + (long)cand * g.ncoef;
   const int k = lane / S, z = lane - k * S;
-  double* m0 = MODE == 0 ? reinterpret_cast<double*>(mesh + (long)(cand >> 1) * g.Kt) + (cand & 1)
-                         : reinterpret_cast<double*>(mesh + (long)cand * g.Kt);
-  double* m2 = MODE == 0 ? nullptr : reinterpret_cast<double*>(mesh2 + (long)(cand >> 1) * g.Kt) + (cand & 1);
+  double* m0 = reinterpret_cast<double*>(mesh + (long)cand * g.Kt);
+  double* m2 = MODE == 0 ? nullptr : reinterpret_cast<double*>(mesh2 + (long)cand * g.Kt);
   for (int n = 0; n < HS_ATOMS; ++n) {
     const int i = (blockIdx.x * W + warp) * HS_ATOMS + n;
     if (i >= N) return;  // the whole warp
@@ -282,71 +282,47 @@ __device__ __forceinline__ double2 hs_second(double2 z, double2 y) { return make
 
 // k space of the forward pass, a point per thread, nb candidates: with
 // g = G Qh, F[c] = transform of E_0 + i E_1 = (i k_0 - k_1) g; energy pass
-// (pair = 0) F[nb + c] = E_2 + i phi = i (k_2 + 1) g; force error (pair = 1)
-// F[nb + c / 2] = E_2 of two candidates.  w[c] = G |Qh|^2 (or null).
+// (loss = 0) F[nb + c] = E_2 + i phi = i (k_2 + 1) g; force error (loss = 1)
+// F[nb + c] = E_2 = i k_2 g.  w[c] = G |Qh|^2 (or null).
 __global__ void __launch_bounds__(256)
-k_hs_kspace_fwd(HsGeom g, int nb, int pair, const double2* __restrict__ Z, const double* __restrict__ bfac, int Kmax,
+k_hs_kspace_fwd(HsGeom g, int nb, int loss, const double2* __restrict__ Z, const double* __restrict__ bfac, int Kmax,
                 double2* __restrict__ F, double* __restrict__ w) {
   const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (p >= g.Kt) return;
   const HsPoint h = hs_point(g, p);
-  for (int c = 0; c < nb; c += 2) {
-    const double2 z = Z[(c >> 1) * g.Kt + p], y = Z[(c >> 1) * g.Kt + h.q];
-    double2 e2 = make_double2(0.0, 0.0);
-    for (int s = 0; s < 2 && c + s < nb; ++s) {
-      const double2 Q = s ? hs_second(z, y) : hs_first(z, y);
-      const double G = hs_factor2(h, bfac + (long)(c + s) * 3 * Kmax, Kmax);
-      const double2 a = make_double2(G * Q.x, G * Q.y);
-      F[(c + s) * g.Kt + p] = make_double2(-h.k[0] * a.y - h.k[1] * a.x, h.k[0] * a.x - h.k[1] * a.y);
-      if (!pair) {
-        const double k = h.k[2] + 1.0;
-        F[(nb + c + s) * g.Kt + p] = make_double2(-k * a.y, k * a.x);
-      } else if (s == 0) {
-        e2 = make_double2(-h.k[2] * a.y, h.k[2] * a.x);
-      } else {
-        e2.x -= h.k[2] * a.x;
-        e2.y -= h.k[2] * a.y;
-      }
-      if (w) w[(c + s) * g.Kt + p] = G * (Q.x * Q.x + Q.y * Q.y);
-    }
-    if (pair) F[(nb + (c >> 1)) * g.Kt + p] = e2;
+  const double k2 = loss ? h.k[2] : h.k[2] + 1.0;
+  for (int c = 0; c < nb; ++c) {
+    const double2 Q = Z[c * g.Kt + p];
+    const double G = hs_factor2(h, bfac + (long)c * 3 * Kmax, Kmax);
+    const double2 a = make_double2(G * Q.x, G * Q.y);
+    F[c * g.Kt + p] = make_double2(-h.k[0] * a.y - h.k[1] * a.x, h.k[0] * a.x - h.k[1] * a.y);
+    F[(nb + c) * g.Kt + p] = make_double2(-k2 * a.y, k2 * a.x);
+    if (w) w[c * g.Kt + p] = G * (Q.x * Q.x + Q.y * Q.y);
   }
 }
 
-// k space of the loss adjoint: Lam = -sum_a i k_a G Bh_a of two candidates per
-// mesh, w[c] = Re(sum_a conj(Bh_a) i k_a Qh) G
+// k space of the loss adjoint: Lam = -sum_a i k_a G Bh_a in place of Bh_2,
+// w[c] = Re(sum_a conj(Bh_a) i k_a Qh) G
 __global__ void __launch_bounds__(256)
-k_hs_kspace_adj(HsGeom g, int nb, const double2* __restrict__ Z, const double2* __restrict__ Y,
-                const double2* __restrict__ Y2, const double* __restrict__ bfac, int Kmax, double2* __restrict__ lam,
-                double* __restrict__ w) {
+k_hs_kspace_adj(HsGeom g, int nb, const double2* __restrict__ Z, const double2* __restrict__ Y, double2* Y2,
+                const double* __restrict__ bfac, int Kmax, double* __restrict__ w) {
   const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (p >= g.Kt) return;
   const HsPoint h = hs_point(g, p);
-  for (int c = 0; c < nb; c += 2) {
-    const long o = (c >> 1) * g.Kt;
-    const double2 z = Z[o + p], y = Z[o + h.q], z2 = Y2[o + p], y2 = Y2[o + h.q];
-    double2 l = make_double2(0.0, 0.0);
-    for (int s = 0; s < 2 && c + s < nb; ++s) {
-      const double2 Q = s ? hs_second(z, y) : hs_first(z, y);
-      const double2 zb = Y[(c + s) * g.Kt + p], yb = Y[(c + s) * g.Kt + h.q];
-      const double2 b[3] = {hs_first(zb, yb), hs_second(zb, yb), s ? hs_second(z2, y2) : hs_first(z2, y2)};
-      const double G = hs_factor2(h, bfac + (long)(c + s) * 3 * Kmax, Kmax);
-      double2 a = make_double2(0.0, 0.0);
-      double v = 0.0;
-      for (int d = 0; d < 3; ++d) {
-        a.x += h.k[d] * G * b[d].y;  // -i k G b
-        a.y -= h.k[d] * G * b[d].x;
-        v += h.k[d] * (-b[d].x * Q.y + b[d].y * Q.x);  // Re(conj(b) i k Q)
-      }
-      if (s == 0) {
-        l = a;
-      } else {  // + i times the second candidate's
-        l.x -= a.y;
-        l.y += a.x;
-      }
-      if (w) w[(c + s) * g.Kt + p] = v * G;
+  for (int c = 0; c < nb; ++c) {
+    const long o = c * g.Kt;
+    const double2 Q = Z[o + p], zb = Y[o + p], yb = Y[o + h.q];
+    const double2 b[3] = {hs_first(zb, yb), hs_second(zb, yb), Y2[o + p]};
+    const double G = hs_factor2(h, bfac + (long)c * 3 * Kmax, Kmax);
+    double2 a = make_double2(0.0, 0.0);
+    double v = 0.0;
+    for (int d = 0; d < 3; ++d) {
+      a.x += h.k[d] * G * b[d].y;  // -i k G b
+      a.y -= h.k[d] * G * b[d].x;
+      v += h.k[d] * (-b[d].x * Q.y + b[d].y * Q.x);  // Re(conj(b) i k Q)
     }
-    lam[o + p] = l;
+    if (w) w[o + p] = v * G;
+    Y2[o + p] = a;
   }
 }
 
@@ -374,7 +350,7 @@ struct HsOut {
 // Gather, a candidate per blockIdx.y, a warp per atom.
 //   MODE 0 (energy): f1 = (E_0, E_1), f2 = (E_2, phi): F_i, dE/dq_i, dE/dr_i and
 //     the coefficient partials of the scalar phi
-//   MODE 1 (loss): f2 = E_2 of two candidates: F_i, the residual R_i = 2 (F_i - Fref_i) / N
+//   MODE 1 (loss): f2 = E_2: F_i, the residual R_i = 2 (F_i - Fref_i) / N
 //     and the block's part of the loss
 //   MODE 2 (loss adjoint): dL/dq_i, dL/dr_i and the coefficient partials of the
 //     scalar Lam - R_i.E (dL/dr_i = q_i sum grad W_i (Lam - R_i.E), and so for dq, dc)
@@ -401,9 +377,8 @@ k_hs_gather(HsGeom g, int N, const double* __restrict__ q, const double* __restr
   const double* c = coeffs + (long)cand * g.ncoef;
   const int k = lane / S, z = lane - k * S;
   const double2* e01 = f1 + (long)cand * g.Kt;
-  const double2* e2p = f2 + (long)(MODE == 0 ? cand : cand >> 1) * g.Kt;
-  const double2* lm = MODE == 2 ? lam + (long)(cand >> 1) * g.Kt : nullptr;
-  const bool second = cand & 1;
+  const double2* e2p = f2 + (long)cand * g.Kt;
+  const double2* lm = MODE == 2 ? lam + (long)cand * g.Kt : nullptr;
   double loss = 0.0;
   for (int n = 0; n < HS_ATOMS; ++n) {
     const int i = (blockIdx.x * W + warp) * HS_ATOMS + n;
@@ -429,14 +404,13 @@ k_hs_gather(HsGeom g, int N, const double* __restrict__ q, const double* __restr
         const double wxy = st.v[0][x] * st.v[1][y];
         const double2 a = e01[p], b = e2p[p];
         if (MODE == 2) {
-          const double2 l = lm[p];
-          const double s = (second ? l.y : l.x) - (Ri[0] * a.x + Ri[1] * a.y + Ri[2] * (second ? b.y : b.x));
+          const double s = lm[p].x - (Ri[0] * a.x + Ri[1] * a.y + Ri[2] * b.x);
           ss[warp][row * LD + z] = s;
           t2 += wxy * s;
         } else {
           Ef[0] += wxy * a.x;
           Ef[1] += wxy * a.y;
-          Ef[2] += wxy * (MODE == 0 || !second ? b.x : b.y);
+          Ef[2] += wxy * b.x;
           if (MODE == 0) {
             ss[warp][row * LD + z] = b.y;
             t2 += wxy * b.y;
@@ -566,10 +540,9 @@ struct md_hspme {
   int Kmax = 0;
   int B = HS_BATCH;          // candidates per batch
   int nab = 0;               // blocks of the spread and the gather
-  double2* Z = nullptr;      // [B/2][Kt] charge meshes of two candidates each, transformed in place
+  double2* Z = nullptr;      // [B][Kt] charge meshes, transformed in place
   double2* F = nullptr;      // [2B][Kt] fields
-  double2* Y = nullptr;      // [B + B/2][Kt] residual meshes
-  double2* lam = nullptr;    // [B/2][Kt]
+  double2* Y = nullptr;      // [2B][Kt] residual meshes, then Lam in place of B_2
   double* w = nullptr;       // [B][Kt] summand of the marginals
   double* bfac = nullptr;    // [B][3][Kmax]
   double* dbfac = nullptr;   // [B][3][ncoef][Kmax]
@@ -580,7 +553,7 @@ struct md_hspme {
 };
 
 static void hs_free(md_hspme* h) {
-  void* p[] = {h->Z, h->F, h->Y, h->lam, h->w, h->bfac, h->dbfac, h->marg, h->cpart, h->lpart, h->R};
+  void* p[] = {h->Z, h->F, h->Y, h->w, h->bfac, h->dbfac, h->marg, h->cpart, h->lpart, h->R};
   for (void* x : p) if (x) cudaFree(x);
 }
 
@@ -616,14 +589,13 @@ extern "C" int md_hspme_create(md_hspme** out, int natoms, const int K[3], const
   const long Kt = g.Kt;
   const int per = HS_ATOMS * hs_warps(g.S), nco = std::max(g.ncoef, 1);
   h->nab = (natoms + per - 1) / per;
-  // the meshes of a batch (80 bytes per point and candidate) stay in the 126 MB
+  // the meshes of a batch (88 bytes per point and candidate) stay in the 126 MB
   // L2 with four candidates up to 64^3
-  h->B = Kt * 80 * HS_BATCH <= (96L << 20) ? HS_BATCH : 2;
+  h->B = Kt * 88 * HS_BATCH <= (96L << 20) ? HS_BATCH : 2;
   const long B = h->B;
-  bool ok = cudaMalloc(&h->Z, sizeof(double2) * B / 2 * Kt) == cudaSuccess &&
+  bool ok = cudaMalloc(&h->Z, sizeof(double2) * B * Kt) == cudaSuccess &&
             cudaMalloc(&h->F, sizeof(double2) * 2 * B * Kt) == cudaSuccess &&
-            cudaMalloc(&h->Y, sizeof(double2) * (B + B / 2) * Kt) == cudaSuccess &&
-            cudaMalloc(&h->lam, sizeof(double2) * B / 2 * Kt) == cudaSuccess &&
+            cudaMalloc(&h->Y, sizeof(double2) * 2 * B * Kt) == cudaSuccess &&
             cudaMalloc(&h->w, sizeof(double) * B * Kt) == cudaSuccess &&
             cudaMalloc(&h->bfac, sizeof(double) * B * 3 * h->Kmax) == cudaSuccess &&
             cudaMalloc(&h->dbfac, sizeof(double) * B * 3 * nco * h->Kmax) == cudaSuccess &&
@@ -676,11 +648,11 @@ static int hs_spread(md_hspme* h, int nb, const double* q, const double* r, cons
 template <int MODE>
 static int hs_gather(md_hspme* h, int nb, const double* q, const double* r, const double* c, const double* fref,
                      const HsOut& out, cudaStream_t s) {
-  const double2* f2 = h->F + (long)nb * h->g.Kt;
+  const double2 *f2 = h->F + (long)nb * h->g.Kt, *lam = h->Y + (long)nb * h->g.Kt;
   switch (h->g.S) {
 #define HS_CASE(W)                                                                                               \
   case W:                                                                                                        \
-    k_hs_gather<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), 0, s>>>(h->g, h->N, q, r, c, h->F, f2, h->lam,      \
+    k_hs_gather<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), 0, s>>>(h->g, h->N, q, r, c, h->F, f2, lam,         \
                                                                       fref, h->R, h->lpart, out);                  \
     break;
     HS_WIDTHS(HS_CASE)
@@ -697,20 +669,19 @@ static int hs_marginals(md_hspme* h, int nb, int axes, cudaStream_t s) {
 }
 
 // forward pass of nb candidates: factors, spread, transform, k space and the
-// inverse transforms of the fields (pair: as the force error wants them)
-static int hs_forward(md_hspme* h, int nb, const double* q, const double* r, const double* c, bool pair, bool want_w,
+// inverse transforms of the fields (loss: as the force error wants them)
+static int hs_forward(md_hspme* h, int nb, const double* q, const double* r, const double* c, bool loss, bool want_w,
                       cudaStream_t s) {
   HsGeom& g = h->g;
-  const int np = (nb + 1) / 2;
   k_hs_factor<<<dim3((h->Kmax + 63) / 64, 3, nb), 64, 0, s>>>(g, c, h->bfac, h->dbfac, h->Kmax);
   MD_CHECK_LAUNCH("hspme factor");
-  MD_CUDA(cudaMemsetAsync(h->Z, 0, sizeof(double2) * np * g.Kt, s));
+  MD_CUDA(cudaMemsetAsync(h->Z, 0, sizeof(double2) * nb * g.Kt, s));
   if (int e = hs_spread<0>(h, nb, q, r, c, h->Z, nullptr, s)) return e;
-  if (int e = dft3_grid(h->Z, g.K, -1, np, s)) return e;
-  k_hs_kspace_fwd<<<(unsigned)((g.Kt + 255) / 256), 256, 0, s>>>(g, nb, pair ? 1 : 0, h->Z, h->bfac, h->Kmax, h->F,
+  if (int e = dft3_grid(h->Z, g.K, -1, nb, s)) return e;
+  k_hs_kspace_fwd<<<(unsigned)((g.Kt + 255) / 256), 256, 0, s>>>(g, nb, loss ? 1 : 0, h->Z, h->bfac, h->Kmax, h->F,
                                                                  want_w ? h->w : nullptr);
   MD_CHECK_LAUNCH("hspme kspace");
-  return dft3_grid(h->F, g.K, +1, nb + (pair ? np : nb), s);
+  return dft3_grid(h->F, g.K, +1, 2 * nb, s);
 }
 
 extern "C" int md_hspme_energy(md_hspme* h, const double* q, const double* r, const double* coeffs, int C,
@@ -752,22 +723,22 @@ extern "C" int md_hspme_force_error(md_hspme* h, const double* q, const double* 
   const long N = h->N, Kt = g.Kt;
   const bool grads = dL_dq || dL_dr || dL_dc;
   for (int b = 0; b < C; b += h->B) {
-    const int nb = std::min(h->B, C - b), np = (nb + 1) / 2;
+    const int nb = std::min(h->B, C - b);
     const double* c = coeffs + (long)b * g.ncoef;
     if (int e = hs_forward(h, nb, q, r, c, true, false, s)) return e;
     if (int e = hs_gather<1>(h, nb, q, r, c, fref, HsOut{}, s)) return e;
     if (grads) {
       // adjoint: residuals spread, transformed, Lam and the factor marginals
       double2* Y2 = h->Y + nb * Kt;
-      MD_CUDA(cudaMemsetAsync(h->Y, 0, sizeof(double2) * (nb + np) * Kt, s));
+      MD_CUDA(cudaMemsetAsync(h->Y, 0, sizeof(double2) * 2 * nb * Kt, s));
       if (int e = hs_spread<1>(h, nb, q, r, c, h->Y, Y2, s)) return e;
-      if (int e = dft3_grid(h->Y, g.K, -1, nb + np, s)) return e;
-      k_hs_kspace_adj<<<(unsigned)((Kt + 255) / 256), 256, 0, s>>>(g, nb, h->Z, h->Y, Y2, h->bfac, h->Kmax, h->lam,
+      if (int e = dft3_grid(h->Y, g.K, -1, 2 * nb, s)) return e;
+      k_hs_kspace_adj<<<(unsigned)((Kt + 255) / 256), 256, 0, s>>>(g, nb, h->Z, h->Y, Y2, h->bfac, h->Kmax,
                                                                    dL_dc ? h->w : nullptr);
       MD_CHECK_LAUNCH("hspme adjoint kspace");
       if (dL_dc)
         if (int e = hs_marginals(h, nb, 3, s)) return e;
-      if (int e = dft3_grid(h->lam, g.K, +1, np, s)) return e;
+      if (int e = dft3_grid(Y2, g.K, +1, nb, s)) return e;
       HsOut o = {nullptr, dL_dq ? dL_dq + N * b : nullptr, dL_dr ? dL_dr + 3 * N * b : nullptr,
                  dL_dc ? h->cpart : nullptr};
       if (int e = hs_gather<2>(h, nb, q, r, c, nullptr, o, s)) return e;
