@@ -31,16 +31,20 @@ struct NlGeom {
   int nc[3];
 };
 
-#define NL_TILE_CAP 2304
+// bytes of the tile: 2,752 packed entries, so that the 125 cells of a liquid
+// stencil (2,270 atoms at density 0.78 and cells of 2.86; 2,600 at 0.8 and
+// 2.96) fit with four blocks on an SM
+#define NL_TILE_BYTES 44032
 #define NL_MAX_RUNS 160
 #define NL_RUN_MAXZ 7   // z cells of a run with per-atom z windows (longer runs are scanned whole)
+#define NL_LIGHT 4      // home cells below this many atoms are built warp per cell
 
 // Runs of a home cell, one array per field (the 32 lanes of a warp read the
 // fields of 32 different runs at once, which a struct per run would turn
 // into 16-way shared-memory bank conflicts)
 struct RunTable {
   int jb[NL_MAX_RUNS], cnt[NL_MAX_RUNS], off[NL_MAX_RUNS];  // global start, length, tile offset
-  int sx[NL_MAX_RUNS], sy[NL_MAX_RUNS], sz[NL_MAX_RUNS];    // periodic images of the run
+  int code[NL_MAX_RUNS];                                    // periodic image of the run (img_code)
   float b0[3][NL_MAX_RUNS], b1[3][NL_MAX_RUNS];             // run box (unwrapped frame of the home cell)
   int zc0[NL_MAX_RUNS], nz[NL_MAX_RUNS];  // first z cell (unwrapped); z cells with offsets in zoff (0 = none)
   // zoff[k][r]: offset in run r of the first atom of its k-th z cell (k = nz: cnt)
@@ -50,6 +54,12 @@ struct RunTable {
 __device__ __forceinline__ int img_code(int kx, int ky, int kz) {
   return ((kx + 1) << 26) | ((ky + 1) << 28) | ((kz + 1) << 30);
 }
+// the shift k_d L of axis d of an image code
+template <class R> __device__ __forceinline__ R img_shift(int code, int d, R L) {
+  const unsigned b = ((unsigned)code >> (26 + 2 * d)) & 3u;
+  return b == 1u ? R(0) : b == 2u ? L : -L;
+}
+#define NL_SLOT_MASK 0x03FFFFFF
 
 // the slot index carried in the w component of a staged position (bit copy)
 template <class R> __device__ __forceinline__ R slot_as_w(int j);
@@ -58,6 +68,161 @@ template <> __device__ __forceinline__ double slot_as_w<double>(int j) { return 
 template <class R> __device__ __forceinline__ int slot_of_w(R w);
 template <> __device__ __forceinline__ int slot_of_w<float>(float w) { return __float_as_int(w); }
 template <> __device__ __forceinline__ int slot_of_w<double>(double w) { return (int)__double_as_longlong(w); }
+
+// cells along one axis whose box comes within rle of home cell hc's box
+__device__ __forceinline__ void nl_stencil_axis(double L, int nc, int hc, double rle, double& h, int& lo, int& hi,
+                                                int& full) {
+  h = L / nc;
+  int a = (int)floor((hc * h - rle) / h), b = (int)floor(((hc + 1) * h + rle) / h);
+  full = (b - a + 1) >= nc;
+  if (full) { a = 0; b = nc - 1; }
+  lo = a; hi = b;
+}
+__device__ __forceinline__ double nl_stencil_radius(float rl_max) { return (double)rl_max * (1.0 + 1e-6) + 2e-3; }
+// Columns of a stencil may be cut to the sphere around the home cell, and
+// light cells may go warp per cell, only where no home cell can need more
+// than NL_MAX_RUNS runs: the limit refuses the same builds either way.
+__device__ __forceinline__ bool nl_runs_bounded(int ncols) { return ncols > 0 && 2 * ncols <= NL_MAX_RUNS; }
+
+// the reference's difference r_j - r_i - k L, operation for operation, and
+// its square in binary32 (or binary64) without contraction
+template <class R>
+__device__ __forceinline__ R nl_exact_d2(const typename V4<R>::T& pj, const typename V4<R>::T& pi, int code,
+                                         const R (&L)[3]) {
+  const R dx = sub_rn(sub_rn(pj.x, pi.x), img_shift<R>(code, 0, L[0]));
+  const R dy = sub_rn(sub_rn(pj.y, pi.y), img_shift<R>(code, 1, L[1]));
+  const R dz = sub_rn(sub_rn(pj.z, pi.z), img_shift<R>(code, 2, L[2]));
+  return add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
+}
+
+__device__ __forceinline__ float nl_enum_radius(float rl) { return rl * (1.0f + 1e-5f) + 2e-3f; }
+
+// The lists of a light home cell (1 to NL_LIGHT - 1 atoms), by one warp and
+// without block barriers; false (nothing written) where the stencil spans the
+// box or may need more runs than a home cell has, which the block path then
+// builds.  A vapour cell has a handful of candidates, so what bounds it is the
+// chain of dependent loads, not the tests: its lanes take the (x, y) columns,
+// cut to the atom's sphere, and each candidate finds its column by a search
+// over the prefix sums.  The enumeration order is the block path's (columns
+// in order, z ascending, each cell in z order), so the rows are the same.
+template <class R>
+__device__ __forceinline__ bool nl_light_cell(int c, int i0, int i1, bool per_atom_rc,
+                                              const typename V4<R>::T* __restrict__ pos,
+                                              const float* __restrict__ rcut, const uint32_t* __restrict__ start,
+                                              const uint32_t* __restrict__ zord, const NlGeom& g,
+                                              const DevState* __restrict__ st, double rlist_uniform, double skin,
+                                              int cap, bool test_only, int* __restrict__ list, int* __restrict__ nnb,
+                                              typename V4<R>::T* __restrict__ backup, DevState* stw) {
+  typedef typename V4<R>::T T4;
+  const int lane = threadIdx.x & 31;
+  float rl_max = per_atom_rc ? 0.f : (float)rlist_uniform;
+  if (per_atom_rc)
+    for (int i = i0; i < i1; ++i) rl_max = fmaxf(rl_max, __fadd_rn(rcut[i], (float)skin));
+  const double rle = nl_stencil_radius(rl_max);
+  const int hc[3] = {c / (g.nc[2] * g.nc[1]), (c / g.nc[2]) % g.nc[1], c % g.nc[2]};
+  // lanes 0..2 take one axis each (two binary64 divisions)
+  double hd = 1.0;
+  int slo = 0, shi = 0, sfull = 0;
+  {
+    const int d = lane < 3 ? lane : 0;
+    nl_stencil_axis(st->L[d], d == 0 ? g.nc[0] : d == 1 ? g.nc[1] : g.nc[2],
+                    d == 0 ? hc[0] : d == 1 ? hc[1] : hc[2], rle, hd, slo, shi, sfull);
+  }
+  double h[3];
+  int lo[3], hi[3];
+  bool any_full = false;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    h[d] = __shfl_sync(0xffffffffu, hd, d);
+    lo[d] = __shfl_sync(0xffffffffu, slo, d);
+    hi[d] = __shfl_sync(0xffffffffu, shi, d);
+    any_full |= __shfl_sync(0xffffffffu, sfull, d) != 0;
+  }
+  const int ncy = hi[1] - lo[1] + 1, ncols = (hi[0] - lo[0] + 1) * ncy;
+  if (any_full || !nl_runs_bounded(ncols)) return false;
+  if (test_only) return true;
+  const R L[3] = {boxL<R>(st, 0), boxL<R>(st, 1), boxL<R>(st, 2)};
+  const float hx = (float)h[0], hy = (float)h[1], hzi = 1.0f / (float)h[2];
+  const unsigned ltmask = (1u << lane) - 1u;
+  for (int i = i0; i < i1; ++i) {
+    const T4 pi = pos[i];
+    const R rl = per_atom_rc ? add_rn((R)rcut[i], (R)skin) : (R)rlist_uniform;
+    const R rl2 = mul_rn(rl, rl);
+    const float xe[3] = {(float)pi.x, (float)pi.y, (float)pi.z};
+    const float rle_i = nl_enum_radius((float)rl);
+    int n = 0;
+    int* rowp = list + (size_t)i * cap;
+    for (int col0 = 0; col0 < ncols; col0 += 32) {
+      const int col = col0 + lane;
+      // up to two z segments (the second past the periodic boundary)
+      int ja = 0, ca = 0, jb = 0, cb = 0, code_a = 0, code_b = 0;
+      if (col < ncols) {
+        const int ix = lo[0] + col / ncy, iy = lo[1] + col % ncy;
+        const float ex = fmaxf(0.f, fmaxf(ix * hx - xe[0], xe[0] - (ix + 1) * hx));
+        const float ey = fmaxf(0.f, fmaxf(iy * hy - xe[1], xe[1] - (iy + 1) * hy));
+        const float w2 = rle_i * rle_i - (ex * ex + ey * ey);
+        if (w2 >= 0.f) {
+          const float wz = sqrtf(w2);
+          const int k0 = max((int)floorf((xe[2] - wz) * hzi), lo[2]), k1 = min((int)floorf((xe[2] + wz) * hzi), hi[2]);
+          int cx = ix, cy = iy, sx = 0, sy = 0;
+          if (cx < 0) { cx += g.nc[0]; sx = 1; } else if (cx >= g.nc[0]) { cx -= g.nc[0]; sx = -1; }
+          if (cy < 0) { cy += g.nc[1]; sy = 1; } else if (cy >= g.nc[1]) { cy -= g.nc[1]; sy = -1; }
+          const uint32_t* sc = start + g.nc[2] * (cy + g.nc[1] * cx);
+          const int zmid = k0 < 0 ? 0 : k0 >= g.nc[2] ? k0 : min(k1, g.nc[2] - 1) + 1;  // first cell of the second segment
+          auto seg = [&](int z0, int z1, int& j, int& cnt, int& code) {
+            if (z0 > z1) return;
+            const int sz = z0 < 0 ? 1 : z0 >= g.nc[2] ? -1 : 0;
+            j = (int)sc[z0 + sz * g.nc[2]];
+            cnt = (int)sc[z1 + sz * g.nc[2] + 1] - j;
+            code = img_code(sx, sy, sz);
+          };
+          seg(k0, min(k1, zmid - 1), ja, ca, code_a);
+          seg(max(k0, zmid), k1, jb, cb, code_b);
+        }
+      }
+      const int len = ca + cb;
+      int incl = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int total = __shfl_sync(0xffffffffu, incl, 31);
+      const int excl = incl - len;
+      for (int t0 = 0; t0 < total; t0 += 32) {
+        const int x = t0 + lane;
+        int o = 0;  // the first column whose range ends beyond x
+#pragma unroll
+        for (int w = 16; w; w >>= 1)
+          if (__shfl_sync(0xffffffffu, incl, o + w - 1) <= x) o += w;
+        const int q = x - __shfl_sync(0xffffffffu, excl, o);
+        const int oja = __shfl_sync(0xffffffffu, ja, o), oca = __shfl_sync(0xffffffffu, ca, o);
+        const int ojb = __shfl_sync(0xffffffffu, jb, o);
+        const int oka = __shfl_sync(0xffffffffu, code_a, o), okb = __shfl_sync(0xffffffffu, code_b, o);
+        bool ok = false;
+        int j = 0, code = 0;
+        if (x < total) {
+          j = (int)zord[q < oca ? oja + q : ojb + (q - oca)];
+          code = q < oca ? oka : okb;
+          ok = nl_exact_d2<R>(pos[j], pi, code, L) < rl2 && j != i;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, ok);
+        if (ok) {
+          const int p = n + __popc(m & ltmask);
+          if (p < cap) rowp[nl_slot(p)] = j | code;
+        }
+        n += __popc(m);
+      }
+    }
+    if (lane == 0) {
+      nnb[i] = n;
+      backup[i] = pi;
+      if (n > cap) atomicOr(&stw->flags, FLAG_NL_OVERFLOW);
+      if (n > __ldcg(&stw->max_nnb)) atomicMax(&stw->max_nnb, n);
+    }
+  }
+  return true;
+}
 
 // The lists of the atoms of home cell c, by one block of 8 warps.  Every
 // exit is uniform over the block; the shared state is first written after a
@@ -72,10 +237,9 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
                                               DevState* stw) {
   typedef typename V4<R>::T T4;
   extern __shared__ __align__(16) unsigned char nl_smem[];
-  T4* tile = reinterpret_cast<T4*>(nl_smem);  // w carries the atom's slot (charges are not needed here)
+  float4* ftile = reinterpret_cast<float4*>(nl_smem);  // home frame, w carries the list entry (slot and image)
+  T4* tile = reinterpret_cast<T4*>(nl_smem);           // stored positions, w carries the slot
   __shared__ RunTable rt;
-  __shared__ int nruns, tile_n, use_global;
-  __shared__ float rl_max_sh;
   const int i0 = (int)start[c], i1 = (int)start[c + 1];
   if (i0 == i1) return;  // empty home cell (uniform exit for the whole block)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
@@ -84,141 +248,196 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
   const bool minimg = (MODE == MD_NL_MINIMAGE) || force_minimage;
   const int hc[3] = {c / (g.nc[2] * g.nc[1]), (c / g.nc[2]) % g.nc[1], c % g.nc[2]};
 
-  // largest list radius among the home atoms
-  if (threadIdx.x == 0) rl_max_sh = 0.f;
-  __syncthreads();
-  if (MODE == MD_NL_MINIMAGE) {
-    float m = 0.f;
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) m = fmaxf(m, __fadd_rn(rcut[i], (float)skin));
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) atomicMax((int*)&rl_max_sh, __float_as_int(m));  // non-negative floats order as ints
-  } else if (threadIdx.x == 0) {
-    rl_max_sh = (float)rlist_uniform;
-  }
-  __syncthreads();
-
-  // the stencil of the home cell (cells per axis whose box comes within the
-  // largest radius), worked out once by thread 0
+  // largest list radius among the home atoms, from it the stencil of the home
+  // cell (cells per axis whose box comes within that radius), and from that
+  // the runs of candidate cells: warp 0, its lanes first taking an axis each,
+  // then an (x, y) column each of at most 3 z segments, whose slots and tile
+  // offsets come from warp scans in column order.  (All 8 warps with block
+  // scans took five barriers a cell for work that 25 lanes do.)
   __shared__ double s_h[3];
-  __shared__ int s_lo[3], s_hi[3], s_full[3];
-  if (threadIdx.x == 0) {
-    const double rle = (double)rl_max_sh * (1.0 + 1e-6) + 2e-3;
-    for (int d = 0; d < 3; ++d) {
-      const double hd = st->L[d] / g.nc[d];
-      s_h[d] = hd;
+  __shared__ int s_nr, s_atoms, s_flags;  // runs, their atoms; 1: box spanned per axis excluded (shift per run), 2: too many runs
+  const bool per_atom = MODE == MD_NL_MINIMAGE;
+  if (warp == 0) {
+    float m = per_atom ? 0.f : (float)rlist_uniform;
+    if (per_atom) {
+      for (int i = i0 + lane; i < i1; i += 32) m = fmaxf(m, __fadd_rn(rcut[i], (float)skin));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    }
+    const double rle = nl_stencil_radius(m);
+    double h[3], hd;
+    int lo[3], hi[3], a, b, f;
+    bool full[3];
+    {
+      const int d = lane < 3 ? lane : 0;
+      const int ncd = d == 0 ? g.nc[0] : d == 1 ? g.nc[1] : g.nc[2];
+      const int hcd = d == 0 ? hc[0] : d == 1 ? hc[1] : hc[2];
       if (!minimg) {
+        hd = st->L[d] / ncd;
         const int reach = (hd >= rlist_uniform) ? 1 : (int)ceil(rlist_uniform / hd);
-        s_lo[d] = hc[d] - reach; s_hi[d] = hc[d] + reach; s_full[d] = 0;
+        a = hcd - reach; b = hcd + reach; f = 0;
       } else {
-        int a = (int)floor((hc[d] * hd - rle) / hd), b = (int)floor(((hc[d] + 1) * hd + rle) / hd);
-        s_full[d] = (b - a + 1) >= g.nc[d];
-        if (s_full[d]) { a = 0; b = g.nc[d] - 1; }
-        s_lo[d] = a; s_hi[d] = b;
+        nl_stencil_axis(st->L[d], ncd, hcd, rle, hd, a, b, f);
       }
+      if (lane < 3) s_h[d] = hd;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      h[d] = __shfl_sync(0xffffffffu, hd, d);
+      lo[d] = __shfl_sync(0xffffffffu, a, d);
+      hi[d] = __shfl_sync(0xffffffffu, b, d);
+      full[d] = __shfl_sync(0xffffffffu, f, d) != 0;
+    }
+    const int ncy = hi[1] - lo[1] + 1;
+    const int ncols = (hi[0] - lo[0] + 1) * ncy;
+    // When the stencil spans less than the box along every axis, each cell
+    // appears in exactly one run, at that run's periodic image k_run, and
+    // 2 rlist < L.  For any pair within rlist the reference's image
+    // floor((r_j - r_i)/L + 1/2) is then k_run (it can differ only where
+    // |d| is within rounding of L/2 > rlist, where both reject), so
+    // d = (r_j - r_i) - k_run L repeats the reference's binary32 operations and
+    // the image code is the run's.
+    const bool runshift = minimg && !full[0] && !full[1] && !full[2];
+    // columns are then cut to the cells within the largest radius of the home
+    // cell: at 4.0 with cells of 2.86, 81 cells of 125 remain
+    const bool trim = runshift && nl_runs_bounded(ncols);
+    int base_r = 0, base_a = 0;
+    bool over = false;
+    for (int col0 = 0; col0 < ncols; col0 += 32) {
+      const int col = col0 + lane;
+      int jb_s[3], cnt_s[3], rs[3], rz0[3], len_s[3], ra_s[3], nseg = 0;
+      int ix = 0, iy = 0, sx = 0, sy = 0, colbase = 0;
+      if (col < ncols) {
+        ix = lo[0] + col / ncy;
+        iy = lo[1] + col % ncy;
+        int cx = ix, cy = iy;
+        if (cx < 0) { cx += g.nc[0]; sx = 1; } else if (cx >= g.nc[0]) { cx -= g.nc[0]; sx = -1; }
+        if (cy < 0) { cy += g.nc[1]; sy = 1; } else if (cy >= g.nc[1]) { cy -= g.nc[1]; sy = -1; }
+        colbase = g.nc[2] * (cy + g.nc[1] * cx);
+        int ra[3], rb[3], ns = 0;
+        if (full[2]) { ra[0] = 0; rb[0] = g.nc[2] - 1; rs[0] = 0; rz0[0] = 0; ns = 1; }
+        else {
+          int zlo = lo[2], zhi = hi[2];
+          if (trim) {
+            const float gx = (float)h[0] * (float)max(0, max(ix - hc[0], hc[0] - ix) - 1);
+            const float gy = (float)h[1] * (float)max(0, max(iy - hc[1], hc[1] - iy) - 1);
+            const float rf = (float)rle, w2 = rf * rf - (gx * gx + gy * gy);
+            const float zc = sqrtf(fmaxf(w2, 0.f)) / (float)h[2];  // reach along z in cells
+            zlo = max(zlo, hc[2] - (int)ceilf(zc));
+            zhi = w2 < 0.f ? zlo - 1 : min(zhi, hc[2] + 1 + (int)floorf(zc));
+          }
+          if (zlo <= zhi) {
+            if (zlo < 0) {
+              ra[ns] = zlo + g.nc[2]; rb[ns] = min(zhi, -1) + g.nc[2]; rs[ns] = 1; rz0[ns] = zlo; ++ns;
+            }
+            const int za = max(zlo, 0), zb = min(zhi, g.nc[2] - 1);
+            if (za <= zb) { ra[ns] = za; rb[ns] = zb; rs[ns] = 0; rz0[ns] = za; ++ns; }
+            if (zhi >= g.nc[2]) {
+              const int z0 = max(zlo, g.nc[2]);
+              ra[ns] = z0 - g.nc[2]; rb[ns] = zhi - g.nc[2]; rs[ns] = -1; rz0[ns] = z0; ++ns;
+            }
+          }
+        }
+        for (int s = 0; s < ns; ++s) {
+          const int jb = (int)start[colbase + ra[s]], je = (int)start[colbase + rb[s] + 1];
+          if (je == jb) continue;
+          jb_s[nseg] = jb; cnt_s[nseg] = je - jb; len_s[nseg] = rb[s] - ra[s];
+          rs[nseg] = rs[s]; rz0[nseg] = rz0[s]; ra_s[nseg] = ra[s];
+          ++nseg;
+        }
+      }
+      int atoms = 0;
+      for (int s = 0; s < nseg; ++s) atoms += cnt_s[s];
+      int ir = nseg, ia = atoms;  // inclusive scans
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int vr = __shfl_up_sync(0xffffffffu, ir, o), va = __shfl_up_sync(0xffffffffu, ia, o);
+        if (lane >= o) { ir += vr; ia += va; }
+      }
+      int r_off = base_r + ir - nseg, a_off = base_a + ia - atoms;
+      for (int s = 0; s < nseg; ++s) {
+        if (r_off >= NL_MAX_RUNS) { over = true; break; }
+        const int q = r_off;
+        rt.jb[q] = jb_s[s]; rt.cnt[q] = cnt_s[s]; rt.off[q] = a_off;
+        rt.code[q] = img_code(sx, sy, rs[s]);
+        const int zc0 = rz0[s], zc1 = rz0[s] + len_s[s];
+        rt.b0[0][q] = full[0] ? -1e30f : (float)(ix * h[0]); rt.b1[0][q] = full[0] ? 1e30f : (float)((ix + 1) * h[0]);
+        rt.b0[1][q] = full[1] ? -1e30f : (float)(iy * h[1]); rt.b1[1][q] = full[1] ? 1e30f : (float)((iy + 1) * h[1]);
+        rt.b0[2][q] = full[2] ? -1e30f : (float)(zc0 * h[2]); rt.b1[2][q] = full[2] ? 1e30f : (float)((zc1 + 1) * h[2]);
+        // per-cell offsets for the per-atom z window (runs that do not wrap the
+        // whole z axis and have at most NL_RUN_MAXZ cells)
+        rt.zc0[q] = zc0;
+        const int nzq = (!full[2] && len_s[s] + 1 <= NL_RUN_MAXZ && cnt_s[s] <= 65535) ? len_s[s] + 1 : 0;
+        rt.nz[q] = nzq;
+        for (int k = 0; k < nzq; ++k)
+          rt.zoff[k][q] = (unsigned short)((int)start[colbase + ra_s[s] + k] - jb_s[s]);
+        if (nzq) rt.zoff[nzq][q] = (unsigned short)cnt_s[s];
+        ++r_off;
+        a_off += cnt_s[s];
+      }
+      base_r += __shfl_sync(0xffffffffu, ir, 31);
+      base_a += __shfl_sync(0xffffffffu, ia, 31);
+    }
+    over = __any_sync(0xffffffffu, over);
+    if (lane == 0) {
+      s_nr = min(base_r, NL_MAX_RUNS);
+      s_atoms = base_a;
+      s_flags = (runshift ? 1 : 0) | (over ? 2 : 0);
+      if (over) atomicOr(&stw->flags, FLAG_NL_OVERFLOW);
     }
   }
   __syncthreads();
-  // runs of candidate cells: one thread per (x, y) column of the stencil
-  // computes its (at most 3) z segments; block-wide exclusive scans give
-  // each run its slot and tile offset in column order
   const double h[3] = {s_h[0], s_h[1], s_h[2]};
-  const int lo[3] = {s_lo[0], s_lo[1], s_lo[2]}, hi[3] = {s_hi[0], s_hi[1], s_hi[2]};
-  const bool full[3] = {s_full[0] != 0, s_full[1] != 0, s_full[2] != 0};
-  __shared__ int scan_r[32], scan_a[32];
-  __shared__ int base_r, base_a, overflow_runs;
-  if (threadIdx.x == 0) { base_r = 0; base_a = 0; overflow_runs = 0; }
-  __syncthreads();
-  const int ncy = hi[1] - lo[1] + 1;
-  const int ncols = (hi[0] - lo[0] + 1) * ncy;
-  for (int col0 = 0; col0 < ncols; col0 += blockDim.x) {
-    const int col = col0 + threadIdx.x;
-    int jb_s[3], cnt_s[3], rs[3], rz0[3], len_s[3], ra_s[3], nseg = 0;
-    int ix = 0, iy = 0, sx = 0, sy = 0, colbase = 0;
-    if (col < ncols) {
-      ix = lo[0] + col / ncy;
-      iy = lo[1] + col % ncy;
-      int cx = ix, cy = iy;
-      if (cx < 0) { cx += g.nc[0]; sx = 1; } else if (cx >= g.nc[0]) { cx -= g.nc[0]; sx = -1; }
-      if (cy < 0) { cy += g.nc[1]; sy = 1; } else if (cy >= g.nc[1]) { cy -= g.nc[1]; sy = -1; }
-      colbase = g.nc[2] * (cy + g.nc[1] * cx);
-      int ra[3], rb[3], ns = 0;
-      if (full[2]) { ra[0] = 0; rb[0] = g.nc[2] - 1; rs[0] = 0; rz0[0] = 0; ns = 1; }
-      else {
-        const int zlo = lo[2], zhi = hi[2];
-        if (zlo < 0) { ra[ns] = zlo + g.nc[2]; rb[ns] = g.nc[2] - 1; rs[ns] = 1; rz0[ns] = zlo; ++ns; }
-        const int a = max(zlo, 0), b = min(zhi, g.nc[2] - 1);
-        if (a <= b) { ra[ns] = a; rb[ns] = b; rs[ns] = 0; rz0[ns] = a; ++ns; }
-        if (zhi >= g.nc[2]) { ra[ns] = 0; rb[ns] = zhi - g.nc[2]; rs[ns] = -1; rz0[ns] = g.nc[2]; ++ns; }
-      }
-      for (int s = 0; s < ns; ++s) {
-        const int jb = (int)start[colbase + ra[s]], je = (int)start[colbase + rb[s] + 1];
-        if (je == jb) continue;
-        jb_s[nseg] = jb; cnt_s[nseg] = je - jb; len_s[nseg] = rb[s] - ra[s];
-        rs[nseg] = rs[s]; rz0[nseg] = rz0[s]; ra_s[nseg] = ra[s];
-        ++nseg;
-      }
-    }
-    int atoms = 0;
-    for (int s = 0; s < nseg; ++s) atoms += cnt_s[s];
-    // inclusive warp scans of (runs, atoms), then across warps
-    int ir = nseg, ia = atoms;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int vr = __shfl_up_sync(0xffffffffu, ir, o), va = __shfl_up_sync(0xffffffffu, ia, o);
-      if (lane >= o) { ir += vr; ia += va; }
-    }
-    if (lane == 31) { scan_r[warp] = ir; scan_a[warp] = ia; }
-    __syncthreads();
-    int wr = base_r, wa = base_a;
-    for (int w = 0; w < warp; ++w) { wr += scan_r[w]; wa += scan_a[w]; }
-    int r_off = wr + ir - nseg, a_off = wa + ia - atoms;
-    for (int s = 0; s < nseg; ++s) {
-      if (r_off >= NL_MAX_RUNS) { overflow_runs = 1; break; }
-      const int q = r_off;
-      rt.jb[q] = jb_s[s]; rt.cnt[q] = cnt_s[s]; rt.off[q] = a_off;
-      rt.sx[q] = sx; rt.sy[q] = sy; rt.sz[q] = rs[s];
-      const int zc0 = rz0[s], zc1 = rz0[s] + len_s[s];
-      rt.b0[0][q] = full[0] ? -1e30f : (float)(ix * h[0]); rt.b1[0][q] = full[0] ? 1e30f : (float)((ix + 1) * h[0]);
-      rt.b0[1][q] = full[1] ? -1e30f : (float)(iy * h[1]); rt.b1[1][q] = full[1] ? 1e30f : (float)((iy + 1) * h[1]);
-      rt.b0[2][q] = full[2] ? -1e30f : (float)(zc0 * h[2]); rt.b1[2][q] = full[2] ? 1e30f : (float)((zc1 + 1) * h[2]);
-      // per-cell offsets for the per-atom z window (runs that do not wrap the
-      // whole z axis and have at most NL_RUN_MAXZ cells)
-      rt.zc0[q] = zc0;
-      const int nzq = (!full[2] && len_s[s] + 1 <= NL_RUN_MAXZ && cnt_s[s] <= 65535) ? len_s[s] + 1 : 0;
-      rt.nz[q] = nzq;
-      for (int k = 0; k < nzq; ++k)
-        rt.zoff[k][q] = (unsigned short)((int)start[colbase + ra_s[s] + k] - jb_s[s]);
-      if (nzq) rt.zoff[nzq][q] = (unsigned short)cnt_s[s];
-      ++r_off;
-      a_off += cnt_s[s];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 0; w < nwarp; ++w) { base_r += scan_r[w]; base_a += scan_a[w]; }
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    nruns = min(base_r, NL_MAX_RUNS);
-    tile_n = base_a;
-    use_global = (base_a > NL_TILE_CAP) ? 1 : 0;
-    if (overflow_runs) atomicOr(&stw->flags, FLAG_NL_OVERFLOW);
-  }
-  __syncthreads();
-  const int nr = nruns;
-  // stage the runs into the tile, one warp per run; a home cell with fewer
-  // than 4 atoms reads its candidates from L2 instead (staging would cost
-  // more than the few reads it saves)
-  const bool stage = !use_global && (i1 - i0) >= 4;
-  // a run's cells are staged in their z order (zord), so each cell of the run
-  // is a z-sorted slice of the tile
+  const int nr = s_nr, tile_n = s_atoms;
+  const bool runshift = s_flags & 1;
+  // stage the runs into the tile; a home cell with fewer than NL_LIGHT atoms
+  // reads its candidates from L2 instead (staging would cost more than the
+  // few reads it saves).  A run's cells are staged in their z order (zord),
+  // so each cell of the run is a z-sorted slice of the tile.
+  const int fit = runshift ? NL_TILE_BYTES / (int)sizeof(float4) : NL_TILE_BYTES / (int)sizeof(T4);
+  const bool stage = tile_n <= fit && !(s_flags & 2) && (i1 - i0) >= NL_LIGHT;
+  const bool fast = stage && runshift;
+  // frame of the packed tile: the box (binary32), or the home cell's corner,
+  // so that binary64 positions lose nothing but their last binary32 digit
+  R corner[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) corner[d] = (fast && sizeof(R) == 8) ? (R)(hc[d] * h[d]) : R(0);
   if (stage) {
-    for (int r = warp; r < nr; r += nwarp) {
-      const int c = rt.cnt[r], o = rt.off[r], jb = rt.jb[r];
-      for (int t = lane; t < c; t += 32) {
-        const int j = (int)zord[jb + t];
-        T4 v = pos[j];
-        v.w = slot_as_w<R>(j);
-        tile[o + t] = v;
+    // a warp takes four runs at a time, so that four of the two dependent
+    // loads of an entry (its slot, then the position) are in flight per lane
+    constexpr int U = 4;
+    for (int r0 = warp; r0 < nr; r0 += U * nwarp) {
+      int cnt[U], off[U], jb[U], code[U], longest = 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int r = min(r0 + u * nwarp, nr - 1);
+        cnt[u] = r0 + u * nwarp < nr ? rt.cnt[r] : 0;
+        off[u] = rt.off[r];
+        jb[u] = rt.jb[r];
+        code[u] = rt.code[r];
+        longest = max(longest, cnt[u]);
+      }
+      for (int t = lane; t < longest; t += 32) {
+        int jj[U];
+        T4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) jj[u] = t < cnt[u] ? (int)zord[jb[u] + t] : -1;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (jj[u] >= 0) v[u] = pos[jj[u]];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (jj[u] < 0) continue;
+          if (runshift) {
+            ftile[off[u] + t] = make_float4((float)(v[u].x - img_shift<R>(code[u], 0, L[0]) - corner[0]),
+                                            (float)(v[u].y - img_shift<R>(code[u], 1, L[1]) - corner[1]),
+                                            (float)(v[u].z - img_shift<R>(code[u], 2, L[2]) - corner[2]),
+                                            __int_as_float(jj[u] | code[u]));
+          } else {
+            v[u].w = slot_as_w<R>(jj[u]);
+            tile[off[u] + t] = v[u];
+          }
+        }
       }
     }
   }
@@ -228,21 +447,19 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
   const unsigned lemask = (2u << lane) - 1u;  // lanes 0..lane (all 32 for lane 31)
   // per-warp table of the current run group's non-empty runs (rank order)
   __shared__ int wdelta[8][32];
-  __shared__ T4 wshift[8][32];
-  // When the stencil spans less than the box along every axis, each cell
-  // appears in exactly one run, at that run's periodic image k_run, and
-  // 2 rlist < L.  For any pair within rlist the reference's image
-  // floor((r_j - r_i)/L + 1/2) is then k_run (it can differ only where
-  // |d| is within rounding of L/2 > rlist, where both reject), so
-  // d = (r_j - r_i) - k_run L repeats the reference's binary32 operations and
-  // the image code is the run's.
-  const bool runshift = minimg && !full[0] && !full[1] && !full[2];
+  __shared__ int wcode[8][32];
   const float hz = (float)h[2], hzi = 1.0f / hz;
-  const float Lzf = (float)st->L[2];
-  // z of entry t of a run (z order) in the stored, wrapped frame
+  const float Lzf = (float)st->L[2], cz = (float)corner[2];
+  // z of entry t of a run (z order) in the frame of the run: the stored,
+  // wrapped one, or the packed tile's
   auto zat = [&](int roff, int rjb, int t) -> float {
-    return glob ? (float)pos[zord[rjb + t]].z : (float)tile[roff + t].z;
+    return fast ? ftile[roff + t].z : glob ? (float)pos[zord[rjb + t]].z : (float)tile[roff + t].z;
   };
+  // Bound on the difference between the packed tile's squared distance and
+  // the reference's (coordinates and differences rounded to binary32, each
+  // within 4 units of 2^-24 of the longest edge); inside it the reference's own operations decide.
+  const float delta = 2.4e-7f * fmaxf((float)st->L[0], fmaxf((float)st->L[1], Lzf));
+  int nmax = 0;
 
   for (int i = i0 + warp; i < i1; i += nwarp) {
     const T4 pi = pos[i];
@@ -250,17 +467,13 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
     if (MODE == MD_NL_MINIMAGE) rl = add_rn((R)rcut[i], (R)skin);
     else rl = (R)rlist_uniform;
     const R rl2 = mul_rn(rl, rl);
-    // enumeration coordinates of i in the home cell's frame
-    float xe[3];
-    {
-      const double xi[3] = {(double)pi.x, (double)pi.y, (double)pi.z};
-      for (int d = 0; d < 3; ++d) {
-        double w = xi[d] - floor(xi[d] * st->Li[d]) * st->L[d];
-        if (!(w >= 0.0) || w >= st->L[d]) w = 0.0;
-        xe[d] = (float)w;
-      }
-    }
-    const float rle_i = (float)rl * (1.0f + 1e-5f) + 2e-3f;
+    // enumeration coordinates of i (binning left it inside the box)
+    const float xe[3] = {(float)pi.x, (float)pi.y, (float)pi.z};
+    const float rle_i = nl_enum_radius((float)rl);
+    const float eps = 4.f * delta * ((float)rl + delta) + 4.8e-7f * (float)rl2;
+    const float in2 = (float)rl2 - eps, out2 = (float)rl2 + eps;
+    const float3 ri = make_float3((float)(pi.x - corner[0]), (float)(pi.y - corner[1]), (float)(pi.z - corner[2]));
+    const int self = i | img_code(0, 0, 0);
     int n = 0;
     int* rowp = list + (size_t)i * cap;
     // the 32 lanes test 32 runs at a time against i's box distance and z
@@ -280,7 +493,8 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
           }
           const float ez = fmaxf(0.f, fmaxf(rt.b0[2][r] - xe[2], xe[2] - rt.b1[2][r]));
           keep = dxy + ez * ez <= rle_i * rle_i;
-          wz = sqrtf(fmaxf(rle_i * rle_i - dxy, 0.f));
+          const float w2 = fmaxf(rle_i * rle_i - dxy, 1e-12f);
+          wz = w2 * rsqrtf(w2);  // (a few 1e-7 of the root: inside the margin)
         }
         // the cells of the run that meet i's z window [z - wz, z + wz]; the
         // first and last of them are cut to the window by binary search in
@@ -297,8 +511,8 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
           keep = k0 <= k1;
           if (keep) {
             const int roff = rt.off[r], rjb = rt.jb[r];
-            // window in the stored frame: z_stored = z_run + sz L_z
-            const float shift = (float)rt.sz[r] * Lzf;
+            // window in the run's frame; stored: z_stored = z_run + sz L_z
+            const float shift = fast ? -cz : img_shift<float>(rt.code[r], 2, Lzf);
             const float zlo = xe[2] - wz - 1e-3f + shift, zhi = xe[2] + wz + 1e-3f + shift;
             int lo = rt.zoff[k0][r], hi = rt.zoff[k0 + 1][r];  // first index with z >= zlo
             while (lo < hi) {
@@ -321,10 +535,10 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
       // 32-lane chunks: lane l of a chunk takes candidate c = t0 + l, owned by
       // the last non-empty run whose range starts at or before c.  The
       // non-empty runs are compacted (in run order) into the warp's table:
-      // the offset taking c to its tile (or zord) index, and the run's image
-      // shift k L with its code.  Within a chunk the owner's rank is the number
-      // of non-empty runs starting before the chunk plus those starting inside
-      // it at or before c (a 32-bit start mask).
+      // the offset taking c to its tile (or zord) index, and the run's image.
+      // Within a chunk the owner's rank is the number of non-empty runs
+      // starting before the chunk plus those starting inside it at or before
+      // c (a 32-bit start mask).
       const int len = keep ? tel - tbl : 0;
       int incl = len;
 #pragma unroll
@@ -333,25 +547,60 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
         if (lane >= o) incl += v;
       }
       const int total = __shfl_sync(0xffffffffu, incl, 31);
-      const int excl = incl - len;
       const bool ne = len > 0;
+      const int excl = incl - len;
       const unsigned nem = __ballot_sync(0xffffffffu, ne);
       __syncwarp();  // the previous group's table has been read
       if (ne) {
         const int r = rb + lane;
         const int k = __popc(nem & ltmask);
         wdelta[warp][k] = (glob ? rt.jb[r] : rt.off[r]) + tbl - excl;
-        const int rsx = rt.sx[r], rsy = rt.sy[r], rsz = rt.sz[r];
-        wshift[warp][k] = T4{mul_rn((R)rsx, L[0]), mul_rn((R)rsy, L[1]), mul_rn((R)rsz, L[2]),
-                             slot_as_w<R>(img_code(rsx, rsy, rsz))};
+        wcode[warp][k] = rt.code[r];
       }
       __syncwarp();
-      int before = 0;  // non-empty runs starting before the chunk
+      const int first = ne ? excl : 0x7fffffff;  // where the lane's range starts
+      int before = -1;  // rank of the run that owns the candidate before the chunk
+      if (fast) {
+        // two chunks a turn: their loads and votes overlap
+        for (int t0 = 0; t0 < total; t0 += 64) {
+          const unsigned rel = (unsigned)(first - t0);
+          const unsigned sm0 = __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
+          const unsigned sm1 = __reduce_or_sync(0xffffffffu, rel - 32u < 32u ? 1u << (rel - 32u) : 0u);
+          const int mid = before + __popc(sm0);
+          const int k[2] = {before + __popc(sm0 & lemask), mid + __popc(sm1 & lemask)};
+          before = mid + __popc(sm1);
+          float d2[2] = {3e38f, 3e38f};
+          int entry[2] = {self, self};
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int x = t0 + 32 * u + lane;
+            if (x < total) {
+              const float4 pj = ftile[x + wdelta[warp][k[u]]];
+              entry[u] = __float_as_int(pj.w);
+              const float dx = pj.x - ri.x, dy = pj.y - ri.y, dz = pj.z - ri.z;
+              d2[u] = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+            }
+          }
+          bool ok[2] = {d2[0] < in2, d2[1] < in2};
+          const bool e0 = d2[0] < out2 && !ok[0], e1 = d2[1] < out2 && !ok[1];
+          if (__any_sync(0xffffffffu, e0 || e1)) {
+            if (e0) ok[0] = nl_exact_d2<R>(pos[entry[0] & NL_SLOT_MASK], pi, entry[0], L) < rl2;
+            if (e1) ok[1] = nl_exact_d2<R>(pos[entry[1] & NL_SLOT_MASK], pi, entry[1], L) < rl2;
+          }
+          const unsigned m0 = __ballot_sync(0xffffffffu, ok[0] && entry[0] != self);
+          const unsigned m1 = __ballot_sync(0xffffffffu, ok[1] && entry[1] != self);
+          const int p0 = n + __popc(m0 & ltmask), n1 = n + __popc(m0), p1 = n1 + __popc(m1 & ltmask);
+          if (ok[0] && entry[0] != self && p0 < cap) rowp[nl_slot(p0)] = entry[0];
+          if (ok[1] && entry[1] != self && p1 < cap) rowp[nl_slot(p1)] = entry[1];
+          n = n1 + __popc(m1);
+        }
+        continue;
+      }
       for (int t0 = 0; t0 < total; t0 += 32) {
         const int cidx = t0 + lane;
-        const unsigned smask =
-            __reduce_or_sync(0xffffffffu, (ne && excl >= t0 && excl < t0 + 32) ? (1u << (excl - t0)) : 0u);
-        const int k = before + __popc(smask & lemask) - 1;
+        const unsigned rel = (unsigned)(first - t0);
+        const unsigned smask = __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
+        const int k = before + __popc(smask & lemask);
         before += __popc(smask);
         bool ok = false;
         int j = 0, code = 0;
@@ -365,35 +614,24 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
             pj = tile[x];
             j = slot_of_w<R>(pj.w);
           }
-          const T4 sh = wshift[warp][k];
-          R dx, dy, dz, d2;
+          code = wcode[warp][k];
+          R d2;
           if (runshift) {
-            dz = sub_rn(sub_rn(pj.z, pi.z), sh.z);
-            if constexpr (std::is_same<R, float>::value) {
-              // x and y as one packed binary32 pair: the same roundings
-              const F2 dxy = f2_sub(f2_sub(f2(pj.x, pj.y), f2(pi.x, pi.y)), f2(sh.x, sh.y));
-              float sx, sy;
-              f2_split(f2_mul(dxy, dxy), sx, sy);
-              d2 = __fadd_rn(__fadd_rn(sx, sy), __fmul_rn(dz, dz));
-            } else {
-              dx = sub_rn(sub_rn(pj.x, pi.x), sh.x);
-              dy = sub_rn(sub_rn(pj.y, pi.y), sh.y);
-              d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
-            }
-            code = slot_of_w<R>(sh.w);
+            d2 = nl_exact_d2<R>(pj, pi, code, L);
           } else {
             const R rx = sub_rn(pj.x, pi.x), ry = sub_rn(pj.y, pi.y), rz = sub_rn(pj.z, pi.z);
             const R kx = floor_r(add_rn(mul_rn(rx, Li[0]), R(0.5)));
             const R ky = floor_r(add_rn(mul_rn(ry, Li[1]), R(0.5)));
             const R kz = floor_r(add_rn(mul_rn(rz, Li[2]), R(0.5)));
+            R dx, dy, dz;
             if (minimg) {
               dx = sub_rn(rx, mul_rn(kx, L[0]));
               dy = sub_rn(ry, mul_rn(ky, L[1]));
               dz = sub_rn(rz, mul_rn(kz, L[2]));
             } else {
-              dx = sub_rn(sub_rn(pj.x, sh.x), pi.x);
-              dy = sub_rn(sub_rn(pj.y, sh.y), pi.y);
-              dz = sub_rn(sub_rn(pj.z, sh.z), pi.z);
+              dx = sub_rn(sub_rn(pj.x, img_shift<R>(code, 0, L[0])), pi.x);
+              dy = sub_rn(sub_rn(pj.y, img_shift<R>(code, 1, L[1])), pi.y);
+              dz = sub_rn(sub_rn(pj.z, img_shift<R>(code, 2, L[2])), pi.z);
             }
             code = img_code((int)kx, (int)ky, (int)kz);
             d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
@@ -408,12 +646,17 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
         n += __popc(m);
       }
     }
+    nmax = max(nmax, n);
     if (lane == 0) {
       nnb[i] = n;
       backup[i] = pi;
-      if (n > cap) atomicOr(&stw->flags, FLAG_NL_OVERFLOW);
-      atomicMax(&stw->max_nnb, n);
     }
+  }
+  // the largest list: an atomic only where it grows (one per atom would queue
+  // 65,536 of them at one address)
+  if (lane == 0 && nmax > 0) {
+    if (nmax > cap) atomicOr(&stw->flags, FLAG_NL_OVERFLOW);
+    if (nmax > __ldcg(&stw->max_nnb)) atomicMax(&stw->max_nnb, nmax);
   }
 }
 
@@ -425,7 +668,23 @@ k_nl_build(int N, const typename V4<R>::T* __restrict__ pos, const float* __rest
            int* __restrict__ nnb, typename V4<R>::T* __restrict__ backup, int force_minimage, DevState* stw,
            int gate) {
   if (gate && !(st->flags & FLAG_REBUILD)) return;
-  nl_build_cell<R, MODE>(blockIdx.x, pos, rcut, start, zord, g, st, rlist_uniform, skin, cap, list, nnb, backup,
+  const bool minimg = (MODE == MD_NL_MINIMAGE) || force_minimage;
+  const int c = blockIdx.x;
+  if (minimg) {
+    // the light cells among 8 neighbouring ones, a warp each
+    const int ntot = g.nc[0] * g.nc[1] * g.nc[2], cw = c + (int)(threadIdx.x >> 5);
+    if ((c & 7) == 0 && cw < ntot) {
+      const int a = (int)start[cw], n = (int)start[cw + 1] - a;
+      if (n > 0 && n < NL_LIGHT)
+        nl_light_cell<R>(cw, a, a + n, MODE == MD_NL_MINIMAGE, pos, rcut, start, zord, g, st, rlist_uniform, skin, cap,
+                         false, list, nnb, backup, stw);
+    }
+    const int a = (int)start[c], n = (int)start[c + 1] - a;
+    if (n < NL_LIGHT && (n == 0 || nl_light_cell<R>(c, a, a + n, MODE == MD_NL_MINIMAGE, pos, rcut, start, zord, g, st,
+                                                    rlist_uniform, skin, cap, true, list, nnb, backup, stw)))
+      return;
+  }
+  nl_build_cell<R, MODE>(c, pos, rcut, start, zord, g, st, rlist_uniform, skin, cap, list, nnb, backup,
                          force_minimage, stw);
 }
 
@@ -435,7 +694,7 @@ static const void* nl_kernel() {
   const void* f = (const void*)k_nl_build<R, MODE>;
   if (!attr) {
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(NL_TILE_CAP * sizeof(typename V4<R>::T)));
+                         NL_TILE_BYTES);
     attr = true;
   }
   return f;
@@ -472,13 +731,11 @@ int nlist_build_impl(md_nlist* nl, md_system* sys, md_cell_list* cl, Recorder* r
   void* a[] = {&N, &sys->pos, &sys->rcut, &cl->start, &cl->zord, &g, &st, &rl, &skin, &cap, &nl->list,
                &nl->nnb, &nl->backup, &force_mi, &st, &gate};
   const void* f;
-  size_t smem;
+  const size_t smem = NL_TILE_BYTES;
   if (sys->prec == MD_PREC_FP64) {
     f = nl->mode == MD_NL_MINIMAGE ? nl_kernel<double, MD_NL_MINIMAGE>() : nl_kernel<double, MD_NL_CELLSHIFT>();
-    smem = NL_TILE_CAP * sizeof(double4a);
   } else {
     f = nl->mode == MD_NL_MINIMAGE ? nl_kernel<float, MD_NL_MINIMAGE>() : nl_kernel<float, MD_NL_CELLSHIFT>();
-    smem = NL_TILE_CAP * sizeof(float4);
   }
   if (int r = rec_launch(rec, f, grid, block, smem, a)) return r;
   if (int r = topo_exclude_launch(sys, nl, rec, gated)) return r;
@@ -518,9 +775,9 @@ struct RebuildArgs {
   T4* backup;
 };
 
-// resident blocks per SM the kernels are built for: the list tile of the
-// FP64 path (72 KB) leaves room for two
-template <class R> constexpr int rebuild_min_blocks() { return sizeof(R) == 4 ? 4 : 2; }
+// resident blocks per SM the kernels are built for (the list tile leaves room
+// for four)
+#define REBUILD_MIN_BLOCKS 4
 
 // the atoms of this block in the per-atom phases: a contiguous share of
 // ceil(N / blocks), so that every block (and every SM) takes part
@@ -548,21 +805,21 @@ __device__ __forceinline__ void rebuild_phases(const RebuildArgs<R>& a) {
   if (blockIdx.x == 0) scan_block<16>(a.ntot, a.count, a.start);
   if (!grid_barrier(st)) return;
   // 3. member lists; the non-empty cells listed for the list build, cells of
-  // 4 atoms or more from the front of the list and the others from its back,
-  // so that the costly cells are handed out first and the cheap ones fill
-  // the end (a slab has many empty or near-empty vapour cells)
+  // NL_LIGHT atoms or more from the front of the list and the others from its
+  // back, so that the costly cells are handed out first and the cheap ones
+  // fill the end (a slab has many empty or near-empty vapour cells)
   for (int i = k0 + threadIdx.x; i < k1; i += blockDim.x) scatter_atom(i, a.t_cell, a.slot, a.start, a.members);
   for (int cb = gw * 32; cb < a.ntot; cb += nw * 32) {
     const int c = cb + lane;
     const uint32_t n = c < a.ntot ? a.start[c + 1] - a.start[c] : 0u;
-    const unsigned mh = __ballot_sync(0xffffffffu, n >= 4u), ml = __ballot_sync(0xffffffffu, n > 0u && n < 4u);
+    const unsigned mh = __ballot_sync(0xffffffffu, n >= NL_LIGHT), ml = __ballot_sync(0xffffffffu, n > 0u && n < NL_LIGHT);
     unsigned bh = 0, bl = 0;
     if (lane == 0 && mh) bh = atomicAdd(&st->ncell_busy, (unsigned)__popc(mh));
     if (lane == 0 && ml) bl = atomicAdd(&st->ncell_light, (unsigned)__popc(ml));
     bh = __shfl_sync(0xffffffffu, bh, 0);
     bl = __shfl_sync(0xffffffffu, bl, 0);
     const unsigned below = (1u << lane) - 1u;
-    if (n >= 4u) a.busy[bh + __popc(mh & below)] = (uint32_t)c;
+    if (n >= NL_LIGHT) a.busy[bh + __popc(mh & below)] = (uint32_t)c;
     else if (n > 0u) a.busy[a.ntot - 1 - (int)(bl + __popc(ml & below))] = (uint32_t)c;
   }
   if (!grid_barrier(st)) return;
@@ -585,19 +842,40 @@ __device__ __forceinline__ void rebuild_phases(const RebuildArgs<R>& a) {
   if (!grid_barrier(st)) return;
   // 7. lists, the non-empty home cells handed out by a counter (cells differ
   // in work by tens of times across a slab; the order of the cells does not
-  // change any list); the next cell is fetched while this one is built
-  const int nfull = (int)__ldcg(&st->ncell_busy);
-  const int nbusy = nfull + (int)__ldcg(&st->ncell_light);
+  // change any list), the light ones eight at a time, a warp each; the next
+  // share is fetched while this one is built
+  const int nfull = (int)__ldcg(&st->ncell_busy), nlight = (int)__ldcg(&st->ncell_light);
+  const int nbusy = nfull + (nlight + 7) / 8;
+  const bool minimg = (MODE == MD_NL_MINIMAGE) || a.force_mi;
   __shared__ int s_work;
+  __shared__ unsigned s_left;  // light cells of a share that need the whole block
   if (threadIdx.x == 0) s_work = (int)atomicAdd(&st->red_counter[RED_NLWORK], 1u);
   __syncthreads();
   int w = s_work;
   while (w < nbusy) {
     int nxt = 0;
-    if (threadIdx.x == 0) nxt = (int)atomicAdd(&st->red_counter[RED_NLWORK], 1u);
-    const int c = (int)__ldcg(&a.busy[w < nfull ? w : a.ntot - 1 - (w - nfull)]);
-    nl_build_cell<R, MODE>(c, a.pos, a.rcut, a.start, a.zord, a.ng, st, a.rlist, a.skin, a.cap, a.list, a.nnb,
-                           a.backup, a.force_mi, st);
+    if (threadIdx.x == 0) { nxt = (int)atomicAdd(&st->red_counter[RED_NLWORK], 1u); s_left = 0u; }
+    unsigned left = 1u;  // cells of this share for the whole block
+    const int l0 = 8 * (w - nfull);
+    if (w >= nfull) {
+      __syncthreads();
+      const int l = l0 + (int)(threadIdx.x >> 5);
+      if (l < nlight) {
+        const int c = (int)__ldcg(&a.busy[a.ntot - 1 - l]), i0 = (int)a.start[c], i1 = (int)a.start[c + 1];
+        const bool done = minimg && nl_light_cell<R>(c, i0, i1, MODE == MD_NL_MINIMAGE, a.pos, a.rcut, a.start, a.zord,
+                                                     a.ng, st, a.rlist, a.skin, a.cap, false, a.list, a.nnb, a.backup,
+                                                     st);
+        if (!done && lane == 0) atomicOr(&s_left, 1u << (threadIdx.x >> 5));
+      }
+      __syncthreads();
+      left = s_left;
+    }
+    for (; left; left &= left - 1u) {
+      const int b = w < nfull ? w : a.ntot - 1 - (l0 + __ffs((int)left) - 1);
+      nl_build_cell<R, MODE>((int)__ldcg(&a.busy[b]), a.pos, a.rcut, a.start, a.zord, a.ng, st, a.rlist, a.skin, a.cap,
+                             a.list, a.nnb, a.backup, a.force_mi, st);
+      __syncthreads();
+    }
     __syncthreads();
     if (threadIdx.x == 0) s_work = nxt;
     __syncthreads();
@@ -606,7 +884,7 @@ __device__ __forceinline__ void rebuild_phases(const RebuildArgs<R>& a) {
 }
 
 template <class R, int MODE>
-__global__ void __launch_bounds__(256, rebuild_min_blocks<R>()) k_rebuild(RebuildArgs<R> a) {
+__global__ void __launch_bounds__(256, REBUILD_MIN_BLOCKS) k_rebuild(RebuildArgs<R> a) {
   // FLAG_REBUILD does not change while this kernel runs (it is set by the
   // step's first kernel and cleared by its last), so every block takes the
   // same branch
@@ -620,7 +898,7 @@ __global__ void __launch_bounds__(256, rebuild_min_blocks<R>()) k_rebuild(Rebuil
 // atom has moved more than half the skin, the rebuild phases.  This saves the
 // step a kernel node against k_lv_step1 followed by k_rebuild.
 template <class R, int MODE>
-__global__ void __launch_bounds__(256, rebuild_min_blocks<R>())
+__global__ void __launch_bounds__(256, REBUILD_MIN_BLOCKS)
 k_lv_step1_rebuild(typename V4<R>::T* __restrict__ vel, const double4a* __restrict__ force, LvDev p,
                    RebuildArgs<R> a) {
   DevState* st = a.st;
@@ -650,7 +928,6 @@ static const void* rebuild_kernel(int prec, int mode, size_t* smem, int* blocks,
     else
       f = mode == MD_NL_MINIMAGE ? (const void*)k_rebuild<double, MD_NL_MINIMAGE>
                                  : (const void*)k_rebuild<double, MD_NL_CELLSHIFT>;
-    *smem = NL_TILE_CAP * sizeof(double4a);
   } else {
     if (with_lv)
       f = mode == MD_NL_MINIMAGE ? (const void*)k_lv_step1_rebuild<float, MD_NL_MINIMAGE>
@@ -658,8 +935,8 @@ static const void* rebuild_kernel(int prec, int mode, size_t* smem, int* blocks,
     else
       f = mode == MD_NL_MINIMAGE ? (const void*)k_rebuild<float, MD_NL_MINIMAGE>
                                  : (const void*)k_rebuild<float, MD_NL_CELLSHIFT>;
-    *smem = NL_TILE_CAP * sizeof(float4);
   }
+  *smem = NL_TILE_BYTES;
   *blocks = 0;
   int dev = 0, coop = 0, nsm = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
@@ -711,11 +988,13 @@ static int rebuild_fused_t(md_cell_list* cl, md_nlist* nl, md_system* sys, Recor
   int blocks, sms = 1;
   const void* f = rebuild_kernel(sys->prec, nl->mode, &smem, &blocks, with_lv, &sms);
   if (blocks <= 0) { md_set_error("fused rebuild: no cooperative launch on this device"); return MD_ERR_CUDA; }
-  // a block per 8 cells, at least one per SM: every launch pays the grid
-  // barrier and the block launches, and a small system has few cells to
-  // share out (4,000-atom fluid, 216 cells: 30,500 steps/s at one block per
-  // SM against 26,200 at four; the 65,536-atom slab keeps all four)
-  blocks = std::min(blocks, std::max(sms, (cl->ntot + 7) / 8));
+  // a block per 2 cells, at least one per SM: more blocks cost every launch
+  // (block starts, the grid barrier), fewer leave the list build waiting on
+  // latency.  20,736-atom fluid, 1,000 cells: 166 us a rebuild and 4.5 a step
+  // without at a block per 8, 126 and 4.8 per 4, 97 and 5.4 per 2, 97 and 5.6
+  // per 1; 4,000 atoms, 216 cells: 54 and 4.6 at one block per SM, 59 and 4.7 at
+  // a block per cell
+  blocks = std::min(blocks, std::max(sms, (cl->ntot + 1) / 2));
   if (!with_lv) {
     void* args[] = {&a};
     return rec_launch_coop(rec, f, dim3(blocks), dim3(256), smem, args);
