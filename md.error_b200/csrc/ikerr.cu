@@ -111,13 +111,20 @@ struct IkMesh {
   double Li[3];
   double beta;
 };
+// mesh indices |m| <= K/2 of an axis: K + 1, or K where K is odd
+__host__ __device__ __forceinline__ int ik_span(int K) { return 2 * (K / 2) + 1; }
+
 __global__ void __launch_bounds__(IK_THREADS)
 k_ikerr_weights(IkMesh g, double* W0, double* W1, double* W2) {
   const int d = blockIdx.y;
   const int i = blockIdx.x;
   if (i > g.K[d]) return;  // whole block leaves before any barrier
+  if (i >= ik_span(g.K[d])) {  // the entry an odd axis does not use
+    if (threadIdx.x == 0) (d == 0 ? W0 : d == 1 ? W1 : W2)[i] = 0.0;
+    return;
+  }
   const int a = (d + 1) % 3, b = (d + 2) % 3;
-  const int na = g.K[a] + 1, nb = g.K[b] + 1;
+  const int na = ik_span(g.K[a]), nb = ik_span(g.K[b]);
   int m[3];
   m[d] = i - g.K[d] / 2;
   const double pb2 = M_PI * M_PI / (g.beta * g.beta);
@@ -182,10 +189,10 @@ k_ikerr_eval(IkEval e, const double* __restrict__ coeff, double* __restrict__ va
       phi[e.off[d] + k] = v;
     }
   __syncthreads();
-  const int npair = e.K[0] + e.K[1] + e.K[2] + 3;
+  const int n0 = ik_span(e.K[0]), n1 = ik_span(e.K[1]), npair = n0 + n1 + ik_span(e.K[2]);
   auto pair_of = [&](int p, int& d, int& m) {
-    d = p <= e.K[0] ? 0 : (p <= e.K[0] + e.K[1] + 1 ? 1 : 2);
-    const int i = d == 0 ? p : (d == 1 ? p - e.K[0] - 1 : p - e.K[0] - e.K[1] - 2);
+    d = p < n0 ? 0 : p < n0 + n1 ? 1 : 2;
+    const int i = d == 0 ? p : d == 1 ? p - n0 : p - n0 - n1;
     m = i - e.K[d] / 2;
     return i;
   };
