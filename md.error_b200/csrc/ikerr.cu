@@ -20,6 +20,7 @@
 // grid x_n = n K/M (folded to (-K/2, K/2]), the same samples np.fft sees in
 // the reference; here a direct sum over each function's support with exact
 // integer reduction of the phase k n mod M.
+#include <cooperative_groups.h>
 #include <cmath>
 #include <vector>
 #include "device_common.cuh"
@@ -170,25 +171,46 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return s;  // valid in thread 0
 }
 
-// block (c, y): candidate c; y = 0 its value, y = 1 + b its gradient in
-// coefficient b.  Every block forms phi_d = hat0_d + c . hats_d in shared
-// memory and the value sum over the (axis, m) pairs (a gradient block needs it
-// for the square root's derivative); sums are block-reduced in a fixed order.
-__global__ void __launch_bounds__(IK_THREADS)
+// A cluster of IK_CTAS blocks per candidate.  Each block forms its share of
+// phi_d = hat0_d + c . hats_d, the blocks read one another's shares from shared
+// memory, so that each holds phi whole, and each forms the value sum over the
+// (axis, m) pairs (the gradient needs it for the square root's derivative).
+// The gradient goes through phi: A_d(k) = d sum_o1 / d phi_d(k), and
+// d / d c_b = sum_d sum_k A_d(k) hat_{d,b}(k), four coefficients at a time,
+// dealt to the blocks, so that the hats are read twice a candidate and not once
+// per coefficient (a block per coefficient formed phi from all of them).  Sums
+// are block-reduced in a fixed order.  Bound: latency (the chain of phi, its
+// exchange, the sums), not bytes.  Candidates of 32
+// coefficients, l_cut 10: 8 on 64^3 16 us (31 with a block per coefficient), 16
+// on 128^3 29 (64), 64 on 128^3 43 (207).
+constexpr int IK_CTAS = 8;
+constexpr int IK_GROUP = 4;  // coefficients per pass of a block
+
+__global__ void __cluster_dims__(IK_CTAS, 1, 1) __launch_bounds__(IK_THREADS)
 k_ikerr_eval(IkEval e, const double* __restrict__ coeff, double* __restrict__ value,
              double* __restrict__ grad) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ double phi[];  // concatenated phi_0, phi_1, phi_2
   __shared__ double sh[IK_THREADS / 32];
-  const int c = blockIdx.x;
-  if (blockIdx.y > 0 && !grad) return;
+  const int c = blockIdx.x / IK_CTAS, rank = (int)cluster.block_rank();
   const double* cc = coeff + (size_t)c * e.ncoef;
-  for (int d = 0; d < 3; ++d)
-    for (int k = threadIdx.x; k <= e.kmax[d]; k += blockDim.x) {
-      double v = e.hat0[d][k];
-      for (int b = 0; b < e.ncoef; ++b) v += cc[b] * e.hats[d][(size_t)b * (e.kmax[d] + 1) + k];
-      phi[e.off[d] + k] = v;
-    }
-  __syncthreads();
+  const int ntot = e.off[2] + e.kmax[2] + 1, share = (ntot + IK_CTAS - 1) / IK_CTAS;
+  auto axis_of = [&](int x) { return x >= e.off[2] ? 2 : x >= e.off[1] ? 1 : 0; };
+  for (int x = rank * share + threadIdx.x; x < min((rank + 1) * share, ntot); x += blockDim.x) {
+    const int d = axis_of(x), k = x - e.off[d];
+    const size_t ld = e.kmax[d] + 1;
+    double v = e.hat0[d][k];
+#pragma unroll 16
+    for (int b = 0; b < e.ncoef; ++b) v += cc[b] * e.hats[d][b * ld + k];
+    phi[x] = v;
+  }
+  cluster.sync();
+  for (int x = threadIdx.x; x < ntot; x += blockDim.x) {
+    const int owner = x / share;
+    if (owner != rank) phi[x] = cluster.map_shared_rank(phi, owner)[x];
+  }
+  cluster.sync();  // every block holds phi, and none is read by another any more
   const int n0 = ik_span(e.K[0]), n1 = ik_span(e.K[1]), npair = n0 + n1 + ik_span(e.K[2]);
   auto pair_of = [&](int p, int& d, int& m) {
     d = p < n0 ? 0 : p < n0 + n1 ? 1 : 2;
@@ -215,34 +237,48 @@ k_ikerr_eval(IkEval e, const double* __restrict__ coeff, double* __restrict__ va
   __shared__ double s_o1;
   if (threadIdx.x == 0) {
     s_o1 = s_tot * e.norm;
-    if (blockIdx.y == 0) value[c] = sqrt(s_o1) * e.scale;
+    if (rank == 0) value[c] = sqrt(s_o1) * e.scale;
   }
   __syncthreads();
-  if (blockIdx.y == 0) return;
-  // d T / d c_b = sum_l 2 phi_l B_l / phi_0^2 - 2 phi_l^2 B_0 / phi_0^3
+  if (!grad) return;
   const double gpref = e.norm * 0.5 / sqrt(s_o1) * e.scale;
-  {
-    const int b = blockIdx.y - 1;
-    double g = 0.0;
-    for (int p = threadIdx.x; p < npair; p += blockDim.x) {
-      int d, m;
-      const int i = pair_of(p, d, m);
+  for (int b0 = rank * IK_GROUP; b0 < e.ncoef; b0 += IK_CTAS * IK_GROUP) {
+    double g[IK_GROUP] = {0.0, 0.0, 0.0, 0.0};
+    for (int x = threadIdx.x; x < ntot; x += blockDim.x) {
+      const int d = axis_of(x), k = x - e.off[d], K = e.K[d], h = K / 2;
       const double* ph = phi + e.off[d];
-      const double* hb = e.hats[d] + (size_t)b * (e.kmax[d] + 1);
-      const double p0 = ph[abs(m)];
-      const double p02i = 1.0 / (p0 * p0), p03i = 1.0 / (p0 * p0 * p0);
-      const double b0 = hb[abs(m)];
-      double dT = 0.0;
-      for (int l = -e.l_cut; l <= e.l_cut; ++l) {
-        if (l == 0) continue;
-        const int idx = abs(m + l * e.K[d]);
-        const double pl = ph[idx];
-        dT += 2 * pl * p02i * hb[idx] - 2 * pl * pl * (p03i * b0);
+      const double* W = e.W[d];
+      // pairs (m, l != 0) with |m + l K| = k, and their mirror images (-m, -l):
+      // 2 W phi(k) / phi_0(m)^2
+      double A = 0.0;
+      const int l0 = (k + h) / K;
+      for (int l = l0 - 1; l <= l0; ++l) {
+        const int m = k - l * K;
+        if (l < 1 || l > e.l_cut || m > h) continue;
+        const double p0 = ph[abs(m)];
+        A += 2.0 * (W[h + m] + W[h - m]) * ph[k] / (p0 * p0);
       }
-      g += e.W[d][i] * dT;
+      // phi_0 of the pairs m = k and m = -k: -2 W phi(m + l K)^2 / phi_0^3
+      if (k <= h) {
+        const double p0 = ph[k];
+        double T = 0.0;
+        for (int l = 1; l <= e.l_cut; ++l) {
+          const double a = ph[l * K + k], b = ph[l * K - k];
+          T += a * a + b * b;
+        }
+        A -= 2.0 * (k == 0 ? W[h] : W[h + k] + W[h - k]) * T / (p0 * p0 * p0);
+      }
+      const size_t ld = e.kmax[d] + 1;
+      const double* hb = e.hats[d] + b0 * ld + k;
+#pragma unroll
+      for (int q = 0; q < IK_GROUP; ++q)
+        if (b0 + q < e.ncoef) g[q] += A * hb[q * ld];
     }
-    const double gs = block_sum(g, sh);
-    if (threadIdx.x == 0) grad[(size_t)c * e.ncoef + b] = gs * gpref;
+#pragma unroll
+    for (int q = 0; q < IK_GROUP; ++q) {
+      const double gs = block_sum(g[q], sh);
+      if (threadIdx.x == 0 && b0 + q < e.ncoef) grad[(size_t)c * e.ncoef + b0 + q] = gs * gpref;
+    }
   }
 }
 
@@ -400,7 +436,7 @@ static int ikerr_launch(md_ikerr* h, int C, const double* d_coeff, double* d_val
   const double V = h->L[0] * h->L[1] * h->L[2];
   e.norm = 1.0 / (2. * M_PI * V * 2. * M_PI * V);
   e.scale = sqrt(h->q2 * h->q2 / h->natoms) * 138.93545756169981341199;
-  k_ikerr_eval<<<dim3(C, d_grad ? 1 + h->ncoef : 1), IK_THREADS, h->smem, s>>>(e, d_coeff, d_val, d_grad);
+  k_ikerr_eval<<<(unsigned)C * IK_CTAS, IK_THREADS, h->smem, s>>>(e, d_coeff, d_val, d_grad);
   MD_CHECK_LAUNCH("k_ikerr_eval");
   return MD_OK;
 }
