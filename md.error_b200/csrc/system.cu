@@ -523,6 +523,9 @@ extern "C" int md_system_destroy(md_system* s) {
 
 extern "C" int md_system_set_stream(md_system* s, void* stream) {
   if (int r = check_sys(s)) return r;
+  // nothing to wait for when the stream stays: its work is in order already (a
+  // caller on torch's current stream sets it again before every call)
+  if (stream && !s->own_stream && s->stream == (cudaStream_t)stream) return MD_OK;
   MD_CUDA(cudaStreamSynchronize(s->stream));
   if (stream) {
     if (s->own_stream) cudaStreamDestroy(s->stream);

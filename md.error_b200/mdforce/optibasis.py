@@ -10,6 +10,8 @@ scipy.optimize.minimize unchanged.  The coefficient vector is
 [v_1..v_n, d_1..d_n] (optiBasis/basis_common.py unpack_v_d).
 """
 import ctypes as C
+import functools
+import types
 
 import numpy as np
 
@@ -114,15 +116,39 @@ def _torch():
     return torch
 
 
-def ik_error_loss(coeffs, functional):
-    """Force-error estimates of a batch of candidate bases, differentiable
-    with respect to the coefficients: coeffs is a float64 tensor [C, n] (or
-    [n]) on the CPU or on the functional's GPU; returns [C] (or a scalar)."""
+def _spme_run(spme, qq, rr, grads):
+    """Energy and, with grads, its gradients for spme_energy's Function."""
+    torch = _torch()
+    sys_ = spme.sys
+    if qq.is_cuda:
+        qd = qq.detach().to(torch.float64).contiguous()
+        rd = rr.detach().to(torch.float64).contiguous()
+        sys_.set_stream(torch.cuda.current_stream(qd.device).cuda_stream)
+        sys_.set_device_view(rd.data_ptr(), qd.data_ptr())
+        e = torch.empty(2, dtype=torch.float64, device=qd.device)
+        gq = torch.empty_like(qd) if grads else None
+        gr = torch.empty_like(rd) if grads else None
+        spme.energy_grad_device(e.data_ptr(), gq.data_ptr() if grads else None,
+                                gr.data_ptr() if grads else None, e[1:].data_ptr())
+        return e[0], gq, gr
+    sys_.set_charges(qq.detach().numpy())
+    sys_.set_positions(rr.detach().numpy())
+    out = spme.energy_grad(dq=grads, dr=grads)
+    e = torch.tensor(out["energy"], dtype=torch.float64)
+    if not grads:
+        return e, None, None
+    return e, torch.from_numpy(out["dE_dq"]), torch.from_numpy(out["dE_dr"])
+
+
+@functools.lru_cache(maxsize=None)
+def _functions():
+    """The autograd Functions, made once (a class a call costs more host time
+    than the small kernels that it launches take)."""
     torch = _torch()
 
     class _IkErrorLoss(torch.autograd.Function):
         @staticmethod
-        def forward(ctx, x):
+        def forward(ctx, x, functional):
             squeeze = x.dim() == 1
             xb = x.detach().reshape(-1, functional.ncoef).to(torch.float64).contiguous()
             nc = xb.shape[0]
@@ -142,10 +168,69 @@ def ik_error_loss(coeffs, functional):
         def backward(ctx, gout):
             (grad,) = ctx.saved_tensors
             if ctx.squeeze:
-                return (gout * grad[0]).to(gout.dtype)
-            return (gout.reshape(-1, 1) * grad).to(gout.dtype)
+                return (gout * grad[0]).to(gout.dtype), None
+            return (gout.reshape(-1, 1) * grad).to(gout.dtype), None
 
-    return _IkErrorLoss.apply(coeffs)
+    class _SPMEEnergy(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, qq, rr, spme, recompute):
+            e, gq, gr = _spme_run(spme, qq, rr, not recompute)
+            ctx.spme = spme if recompute else None
+            if recompute:
+                ctx.save_for_backward(qq, rr)
+            else:
+                ctx.save_for_backward(gq, gr)
+            return e
+
+        @staticmethod
+        def backward(ctx, g):
+            a, b = ctx.saved_tensors
+            if ctx.spme is not None:
+                _, gq, gr = _spme_run(ctx.spme, a, b, True)
+            else:
+                gq, gr = a, b
+            return (g * gq).to(gq.dtype), (g * gr).to(gr.dtype), None, None
+
+    class _HermiteEnergy(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, qq, rr, cc, hspme):
+            out = hspme.energy(qq, rr, cc, grads=True)
+            ctx.save_for_backward(out["dE_dq"], out["dE_dr"], out["dE_dc"])
+            ctx.cshape = cc.shape
+            return out["energy"]
+
+        @staticmethod
+        def backward(ctx, g):
+            gq, gr, gc = ctx.saved_tensors
+            g = g.reshape(-1)
+            return ((g[:, None] * gq).sum(0), (g[:, None, None] * gr).sum(0),
+                    (g[:, None] * gc).reshape(ctx.cshape), None)
+
+    class _HermiteError(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, qq, rr, cc, const):
+            hspme, fref = const
+            out = hspme.force_error(qq, rr, cc, fref, grads=True)
+            ctx.save_for_backward(out["dL_dq"], out["dL_dr"], out["dL_dc"])
+            ctx.cshape = cc.shape
+            return out["loss"]
+
+        @staticmethod
+        def backward(ctx, g):
+            gq, gr, gc = ctx.saved_tensors
+            g = g.reshape(-1)
+            return ((g[:, None] * gq).sum(0), (g[:, None, None] * gr).sum(0),
+                    (g[:, None] * gc).reshape(ctx.cshape), None)
+
+    return types.SimpleNamespace(ik_error=_IkErrorLoss, spme=_SPMEEnergy, hermite_energy=_HermiteEnergy,
+                                 hermite_error=_HermiteError)
+
+
+def ik_error_loss(coeffs, functional):
+    """Force-error estimates of a batch of candidate bases, differentiable
+    with respect to the coefficients: coeffs is a float64 tensor [C, n] (or
+    [n]) on the CPU or on the functional's GPU; returns [C] (or a scalar)."""
+    return _functions().ik_error.apply(coeffs, functional)
 
 
 def spme_energy(q, r, spme, recompute=False):
@@ -158,49 +243,7 @@ def spme_energy(q, r, spme, recompute=False):
     the forward keeps nothing but the inputs and the backward recomputes
     spread, transforms and gather (memory-lean); by default the gradient comes
     with the forward pass and is kept for the backward."""
-    torch = _torch()
-    sys_ = spme.sys
-
-    def run(qq, rr, grads):
-        if qq.is_cuda:
-            qd = qq.detach().to(torch.float64).contiguous()
-            rd = rr.detach().to(torch.float64).contiguous()
-            sys_.set_stream(torch.cuda.current_stream(qd.device).cuda_stream)
-            sys_.set_device_view(rd.data_ptr(), qd.data_ptr())
-            e = torch.empty(2, dtype=torch.float64, device=qd.device)
-            gq = torch.empty_like(qd) if grads else None
-            gr = torch.empty_like(rd) if grads else None
-            spme.energy_grad_device(e.data_ptr(), gq.data_ptr() if grads else None,
-                                    gr.data_ptr() if grads else None, e[1:].data_ptr())
-            return e[0], gq, gr
-        sys_.set_charges(qq.detach().numpy())
-        sys_.set_positions(rr.detach().numpy())
-        out = spme.energy_grad(dq=grads, dr=grads)
-        e = torch.tensor(out["energy"], dtype=torch.float64)
-        if not grads:
-            return e, None, None
-        return e, torch.from_numpy(out["dE_dq"]), torch.from_numpy(out["dE_dr"])
-
-    class _SPMEEnergy(torch.autograd.Function):
-        @staticmethod
-        def forward(ctx, qq, rr):
-            e, gq, gr = run(qq, rr, not recompute)
-            if recompute:
-                ctx.save_for_backward(qq, rr)
-            else:
-                ctx.save_for_backward(gq, gr)
-            return e
-
-        @staticmethod
-        def backward(ctx, g):
-            a, b = ctx.saved_tensors
-            if recompute:
-                _, gq, gr = run(a, b, True)
-            else:
-                gq, gr = a, b
-            return (g * gq).to(gq.dtype), (g * gr).to(gr.dtype)
-
-    return _SPMEEnergy.apply(q, r)
+    return _functions().spme.apply(q, r, spme, recompute)
 
 
 class HermiteSPME:
@@ -272,48 +315,14 @@ def hermite_spme_energy(q, r, coeffs, hspme):
     """Reciprocal energies [C] of the candidate bases coeffs [C, ncoef], as a
     torch.autograd.Function differentiable in q [N], r [N, 3] and coeffs (the
     gradients come from the hand-written adjoint in the same pass)."""
-    torch = _torch()
-
-    class _E(torch.autograd.Function):
-        @staticmethod
-        def forward(ctx, qq, rr, cc):
-            out = hspme.energy(qq, rr, cc, grads=True)
-            ctx.save_for_backward(out["dE_dq"], out["dE_dr"], out["dE_dc"])
-            ctx.cshape = cc.shape
-            return out["energy"]
-
-        @staticmethod
-        def backward(ctx, g):
-            gq, gr, gc = ctx.saved_tensors
-            g = g.reshape(-1)
-            return ((g[:, None] * gq).sum(0), (g[:, None, None] * gr).sum(0),
-                    (g[:, None] * gc).reshape(ctx.cshape))
-
-    return _E.apply(q, r, coeffs)
+    return _functions().hermite_energy.apply(q, r, coeffs, hspme)
 
 
 def hermite_spme_force_error(q, r, coeffs, fref, hspme):
     """Force-error functional [C] (1/N sum |F_ik - fref|^2 per candidate) as a
     torch.autograd.Function differentiable in q, r and coeffs (second adjoint of
     the SPME chain, md_hspme_force_error); fref is a constant."""
-    torch = _torch()
-
-    class _L(torch.autograd.Function):
-        @staticmethod
-        def forward(ctx, qq, rr, cc):
-            out = hspme.force_error(qq, rr, cc, fref, grads=True)
-            ctx.save_for_backward(out["dL_dq"], out["dL_dr"], out["dL_dc"])
-            ctx.cshape = cc.shape
-            return out["loss"]
-
-        @staticmethod
-        def backward(ctx, g):
-            gq, gr, gc = ctx.saved_tensors
-            g = g.reshape(-1)
-            return ((g[:, None] * gq).sum(0), (g[:, None, None] * gr).sum(0),
-                    (g[:, None] * gc).reshape(ctx.cshape))
-
-    return _L.apply(q, r, coeffs)
+    return _functions().hermite_error.apply(q, r, coeffs, (hspme, fref))
 
 
 def bspline_initial_basis(CC, nbin, order, bound0=False):
