@@ -24,9 +24,34 @@ __device__ __forceinline__ size_t line_base(long L, int n, long inner) {
   return (size_t)(L / inner) * n * inner + (size_t)(L % inner);
 }
 
-template <int LOGN>
+// Where a pass reads and writes its grids (element p of all grids end to end):
+// complex in and out; or, first pass of real grids, (re[p], im[p]) with im = 0
+// from element n_im on; or, last pass, the real parts alone from element n_c on,
+// to outr[p - n_c].
+struct DftIo {
+  const double2* in = nullptr;
+  double2* out = nullptr;
+  const double *re = nullptr, *im = nullptr;
+  long n_im = 0;
+  double* outr = nullptr;
+  long n_c = 0;
+};
+enum { IO_PLAIN = 0, IO_REAL_IN = 1, IO_REAL_OUT = 2 };
+
+template <int IO>
+__device__ __forceinline__ double2 io_load(const DftIo& io, size_t p) {
+  if (IO != IO_REAL_IN) return io.in[p];
+  return make_double2(io.re[p], (long)p < io.n_im ? io.im[p] : 0.0);
+}
+template <int IO>
+__device__ __forceinline__ void io_store(const DftIo& io, size_t p, double2 v) {
+  if (IO == IO_REAL_OUT && (long)p >= io.n_c) io.outr[p - io.n_c] = v.x;
+  else io.out[p] = v;
+}
+
+template <int LOGN, int IO>
 __global__ void __launch_bounds__(FFT_THREADS)
-k_fft_grid(const double2* in, double2* out, long nlines, long inner, int sign) {
+k_fft_grid(DftIo io, long nlines, long inner, int sign) {
   typedef FftGeom<LOGN> G;
   constexpr int n = G::n, LPB = G::LPB, LS = G::LS, EPT = G::EPT;
   extern __shared__ __align__(16) unsigned char fg_smem[];
@@ -44,7 +69,7 @@ k_fft_grid(const double2* in, double2* out, long nlines, long inner, int sign) {
     const int e = threadIdx.x + s * FFT_THREADS;
     const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
     const long L = line0 + l;
-    v[s] = L < nlines ? in[line_base(L, n, inner) + k * inner] : make_double2(0.0, 0.0);
+    v[s] = L < nlines ? io_load<IO>(io, line_base(L, n, inner) + k * inner) : make_double2(0.0, 0.0);
   }
 #pragma unroll
   for (int s = 0; s < EPT; ++s) {
@@ -61,15 +86,15 @@ k_fft_grid(const double2* in, double2* out, long nlines, long inner, int sign) {
     const int e = threadIdx.x + s * FFT_THREADS;
     const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
     const long L = line0 + l;
-    if (L < nlines) out[line_base(L, n, inner) + k * inner] = X[l * LS + fft_pad<double>(k)];
+    if (L < nlines) io_store<IO>(io, line_base(L, n, inner) + k * inner, X[l * LS + fft_pad<double>(k)]);
   }
 }
 
-template <int LOGN>
-int fft_grid_launch(const double2* in, double2* out, long nlines, long inner, int sign, cudaStream_t s) {
+template <int LOGN, int IO>
+int fft_grid_launch(const DftIo& io, long nlines, long inner, int sign, cudaStream_t s) {
   typedef FftGeom<LOGN> G;
   const size_t smem = sizeof(double2) * (G::n + (size_t)G::LPB * G::LS);
-  k_fft_grid<LOGN><<<(unsigned)((nlines + G::LPB - 1) / G::LPB), FFT_THREADS, smem, s>>>(in, out, nlines, inner, sign);
+  k_fft_grid<LOGN, IO><<<(unsigned)((nlines + G::LPB - 1) / G::LPB), FFT_THREADS, smem, s>>>(io, nlines, inner, sign);
   MD_CHECK_LAUNCH("fft axis");
   return MD_OK;
 }
@@ -124,9 +149,9 @@ __device__ __forceinline__ void pair_sums(const double2* x, int xs, int p, int k
 }
 
 // LN lines per block, one per lane; n = n1 n2 (n1 = 1: a single stage of length n)
-template <int LN>
+template <int LN, int IO>
 __global__ void __launch_bounds__(DA_THREADS)
-k_dft_any(const double2* in, double2* out, long nlines, long inner, int n, int n1, int sign) {
+k_dft_any(DftIo io, long nlines, long inner, int n, int n1, int sign) {
   extern __shared__ __align__(16) unsigned char da_smem[];
   constexpr int LS = LN + 1, NG = DA_THREADS / LN;
   double2* tw = reinterpret_cast<double2*>(da_smem);  // (cos, sign sin) of 2 pi m / n
@@ -141,13 +166,13 @@ k_dft_any(const double2* in, double2* out, long nlines, long inner, int n, int n
   for (int t = threadIdx.x; t < n * LN; t += DA_THREADS) {
     const int l = inner > 1 ? t % LN : t / n, j = inner > 1 ? t / LN : t % n;
     const long L = line0 + l;
-    x[j * LS + l] = L < nlines ? in[line_base(L, n, inner) + j * inner] : make_double2(0.0, 0.0);
+    x[j * LS + l] = L < nlines ? io_load<IO>(io, line_base(L, n, inner) + j * inner) : make_double2(0.0, 0.0);
   }
   __syncthreads();
   const int l = threadIdx.x % LN, g = threadIdx.x / LN;
   const long L = line0 + l;
   const bool live = L < nlines;
-  double2* dst = out + (live ? line_base(L, n, inner) : 0);
+  const size_t dst = live ? line_base(L, n, inner) : 0;
   double2 A[DA_KB], B[DA_KB];
   if (n1 > 1) {
     // stage 1, in place: a thread holds all outputs of a length-n1 transform
@@ -192,33 +217,30 @@ k_dft_any(const double2* in, double2* out, long nlines, long inner, int n, int n
     for (int q = 0; q < DA_KB; ++q) {
       const int k2 = k0 + q;
       if (k2 >= nk) break;
-      dst[(size_t)(k1 + n1 * k2) * inner] = make_double2(A[q].x + B[q].x, A[q].y + B[q].y);
+      io_store<IO>(io, dst + (size_t)(k1 + n1 * k2) * inner, make_double2(A[q].x + B[q].x, A[q].y + B[q].y));
       if (k2 > 0 && 2 * k2 < n2)
-        dst[(size_t)(k1 + n1 * (n2 - k2)) * inner] = make_double2(A[q].x - B[q].x, A[q].y - B[q].y);
+        io_store<IO>(io, dst + (size_t)(k1 + n1 * (n2 - k2)) * inner, make_double2(A[q].x - B[q].x, A[q].y - B[q].y));
     }
   }
 }
 
-template <int LN>
-int dft_any_launch(const double2* in, double2* out, long nlines, long inner, int n, int n1, int sign, cudaStream_t s) {
+template <int LN, int IO>
+int dft_any_launch(const DftIo& io, long nlines, long inner, int n, int n1, int sign, cudaStream_t s) {
   const size_t smem = sizeof(double2) * (n + (size_t)n * (LN + 1));
   if (smem > 48 * 1024)
-    MD_CUDA(cudaFuncSetAttribute(k_dft_any<LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  k_dft_any<LN><<<(unsigned)((nlines + LN - 1) / LN), DA_THREADS, smem, s>>>(in, out, nlines, inner, n, n1, sign);
+    MD_CUDA(cudaFuncSetAttribute(k_dft_any<LN, IO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  k_dft_any<LN, IO><<<(unsigned)((nlines + LN - 1) / LN), DA_THREADS, smem, s>>>(io, nlines, inner, n, n1, sign);
   MD_CHECK_LAUNCH("dft axis");
   return MD_OK;
 }
 
-}  // namespace
-
-// one pass (sign -1 forward, +1 backward) over `batch` consecutive grids along
-// `axis`; in may equal out
-int dft3_axis(const double2* in, double2* out, const int n[3], int axis, int sign, int batch, cudaStream_t s) {
+template <int IO>
+int dft_pass(const DftIo& io, const int n[3], int axis, int sign, int batch, cudaStream_t s) {
   const int na = n[axis];
   const long inner = axis == 2 ? 1 : axis == 1 ? n[2] : (long)n[1] * n[2];
   const long nlines = (long)n[0] * n[1] * n[2] / na * batch;
   switch (na) {
-#define FFT_CASE(L) case 1 << L: return fft_grid_launch<L>(in, out, nlines, inner, sign, s);
+#define FFT_CASE(L) case 1 << L: return fft_grid_launch<L, IO>(io, nlines, inner, sign, s);
     FFT_CASE(1) FFT_CASE(2) FFT_CASE(3) FFT_CASE(4) FFT_CASE(5) FFT_CASE(6) FFT_CASE(7) FFT_CASE(8) FFT_CASE(9) FFT_CASE(10)
 #undef FFT_CASE
   }
@@ -227,10 +249,21 @@ int dft3_axis(const double2* in, double2* out, const int n[3], int axis, int sig
     if (na % f == 0) { n1 = f; break; }
   // lines per block: all lanes of a warp where several blocks' lines still fit
   // on an SM (41 points: 23 KB, 161 points: 46 KB of the 228 KB)
-  if (na <= 96) return dft_any_launch<32>(in, out, nlines, inner, na, n1, sign, s);
-  if (na <= 192) return dft_any_launch<16>(in, out, nlines, inner, na, n1, sign, s);
-  if (na <= 384) return dft_any_launch<8>(in, out, nlines, inner, na, n1, sign, s);
-  return dft_any_launch<4>(in, out, nlines, inner, na, n1, sign, s);
+  if (na <= 96) return dft_any_launch<32, IO>(io, nlines, inner, na, n1, sign, s);
+  if (na <= 192) return dft_any_launch<16, IO>(io, nlines, inner, na, n1, sign, s);
+  if (na <= 384) return dft_any_launch<8, IO>(io, nlines, inner, na, n1, sign, s);
+  return dft_any_launch<4, IO>(io, nlines, inner, na, n1, sign, s);
+}
+
+}  // namespace
+
+// one pass (sign -1 forward, +1 backward) over `batch` consecutive grids along
+// `axis`; in may equal out
+int dft3_axis(const double2* in, double2* out, const int n[3], int axis, int sign, int batch, cudaStream_t s) {
+  DftIo io;
+  io.in = in;
+  io.out = out;
+  return dft_pass<IO_PLAIN>(io, n, axis, sign, batch, s);
 }
 
 // unnormalised 3D transform of `batch` consecutive grids, in place
@@ -238,4 +271,32 @@ int dft3_grid(double2* data, const int n[3], int sign, int batch, cudaStream_t s
   for (int axis = 2; axis >= 0; --axis)
     if (int r = dft3_axis(data, data, n, axis, sign, batch, s)) return r;
   return MD_OK;
+}
+
+// forward transforms out of the `batch` real grids re, the first n_im of them
+// with the grids im as imaginary parts
+int dft3_from_real(const double* re, const double* im, int n_im, double2* out, const int n[3], int batch,
+                   cudaStream_t s) {
+  DftIo io;
+  io.re = re;
+  io.im = im;
+  io.n_im = (long)n_im * n[0] * n[1] * n[2];
+  io.out = out;
+  if (int r = dft_pass<IO_REAL_IN>(io, n, 2, -1, batch, s)) return r;
+  for (int axis = 1; axis >= 0; --axis)
+    if (int r = dft3_axis(out, out, n, axis, -1, batch, s)) return r;
+  return MD_OK;
+}
+
+// backward transforms of `batch` grids, the first n_c in place, of the others
+// the real parts to outr
+int dft3_to_real(double2* data, int n_c, double* outr, const int n[3], int batch, cudaStream_t s) {
+  for (int axis = 2; axis >= 1; --axis)
+    if (int r = dft3_axis(data, data, n, axis, +1, batch, s)) return r;
+  DftIo io;
+  io.in = data;
+  io.out = data;
+  io.outr = outr;
+  io.n_c = (long)n_c * n[0] * n[1] * n[2];
+  return dft_pass<IO_REAL_OUT>(io, n, 0, +1, batch, s);
 }

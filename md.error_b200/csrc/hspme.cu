@@ -60,6 +60,9 @@
 #include "device_common.cuh"
 
 int dft3_grid(double2* data, const int n[3], int sign, int batch, cudaStream_t stream);
+int dft3_from_real(const double* re, const double* im, int n_im, double2* out, const int n[3], int batch,
+                   cudaStream_t stream);
+int dft3_to_real(double2* data, int n_c, double* outr, const int n[3], int batch, cudaStream_t stream);
 
 namespace {
 
@@ -195,22 +198,24 @@ __global__ void k_hs_factor(HsGeom g, const double* __restrict__ c, double* __re
 }
 
 // Spread, a candidate per blockIdx.y, a warp per atom with lanes along its
-// stencil rows.  MODE 0: Q += q_i W_i into the real part of mesh c; MODE 1:
-// B_a -= q_i R_i,a W_i, B_0 and B_1 as the parts of mesh c of `mesh`, B_2 into
-// the real part of mesh c of `mesh2`.
+// stencil rows, onto real meshes (a row of 6 points is then two or three 32-byte
+// sectors an instruction; as parts of complex meshes it was four, and the atomics
+// are what bounds this).  MODE 0: Q += q_i W_i into grid c of im; MODE 1:
+// B_a -= q_i R_i,a W_i, B_0 and B_2 into grids c and nb + c of re, B_1 into im.
 template <int S, int MODE>
 __global__ void __launch_bounds__(32 * hs_warps(S))
 k_hs_spread(HsGeom g, int N, const double* __restrict__ q, const double* __restrict__ r,
-            const double* __restrict__ coeffs, const double* __restrict__ R, double2* __restrict__ mesh,
-            double2* __restrict__ mesh2) {
+            const double* __restrict__ coeffs, const double* __restrict__ R, double* __restrict__ re,
+            double* __restrict__ im) {
   constexpr int RP = 32 / S, NR = S * S, NI = (NR + RP - 1) / RP, W = hs_warps(S);
   __shared__ HsStencil<S> sst[W];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cand = blockIdx.y;
   HsStencil<S>& st = sst[warp];
   const double* c = coeffs + (long)cand * g.ncoef;
   const int k = lane / S, z = lane - k * S;
-  double* m0 = reinterpret_cast<double*>(mesh + (long)cand * g.Kt);
-  double* m2 = MODE == 0 ? nullptr : reinterpret_cast<double*>(mesh2 + (long)cand * g.Kt);
+  double* m0 = (MODE == 0 ? im : re) + (long)cand * g.Kt;
+  double* m2 = re + (long)(gridDim.y + cand) * g.Kt;
+  double* m1 = im + (long)cand * g.Kt;
   for (int n = 0; n < HS_ATOMS; ++n) {
     const int i = (blockIdx.x * W + warp) * HS_ATOMS + n;
     if (i >= N) return;  // the whole warp
@@ -235,10 +240,10 @@ k_hs_spread(HsGeom g, int N, const double* __restrict__ q, const double* __restr
       const int x = row / S, y = row - x * S;
       const double w = st.v[0][x] * st.v[1][y] * wz;
       if (w == 0.0) continue;
-      const long p = 2 * (long)(st.off[0][x] + st.off[1][y] + oz);
+      const int p = st.off[0][x] + st.off[1][y] + oz;
       atomicAdd(m0 + p, a[0] * w);
       if (MODE == 1) {
-        atomicAdd(m0 + p + 1, a[1] * w);
+        atomicAdd(m1 + p, a[1] * w);
         atomicAdd(m2 + p, a[2] * w);
       }
     }
@@ -350,7 +355,7 @@ struct HsOut {
 // Gather, a candidate per blockIdx.y, a warp per atom.
 //   MODE 0 (energy): f1 = (E_0, E_1), f2 = (E_2, phi): F_i, dE/dq_i, dE/dr_i and
 //     the coefficient partials of the scalar phi
-//   MODE 1 (loss): f2 = E_2: F_i, the residual R_i = 2 (F_i - Fref_i) / N
+//   MODE 1 (loss): E_2 from the real grid e2: F_i, the residual R_i = 2 (F_i - Fref_i) / N
 //     and the block's part of the loss
 //   MODE 2 (loss adjoint): dL/dq_i, dL/dr_i and the coefficient partials of the
 //     scalar Lam - R_i.E (dL/dr_i = q_i sum grad W_i (Lam - R_i.E), and so for dq, dc)
@@ -362,7 +367,7 @@ template <int S, int MODE>
 __global__ void __launch_bounds__(32 * hs_warps(S))
 k_hs_gather(HsGeom g, int N, const double* __restrict__ q, const double* __restrict__ r,
             const double* __restrict__ coeffs, const double2* __restrict__ f1, const double2* __restrict__ f2,
-            const double2* __restrict__ lam, const double* __restrict__ fref, double* __restrict__ R,
+            const double* __restrict__ e2, const double* __restrict__ lam, const double* __restrict__ fref, double* __restrict__ R,
             double* __restrict__ lpart, HsOut out) {
   constexpr int RP = 32 / S, NR = S * S, NI = (NR + RP - 1) / RP, W = hs_warps(S), LD = S + 1;
   __shared__ HsStencil<S> sst[W];
@@ -378,7 +383,7 @@ k_hs_gather(HsGeom g, int N, const double* __restrict__ q, const double* __restr
   const int k = lane / S, z = lane - k * S;
   const double2* e01 = f1 + (long)cand * g.Kt;
   const double2* e2p = f2 + (long)cand * g.Kt;
-  const double2* lm = MODE == 2 ? lam + (long)cand * g.Kt : nullptr;
+  const double *e2r = e2 + (long)cand * g.Kt, *lm = lam + (long)cand * g.Kt;
   double loss = 0.0;
   for (int n = 0; n < HS_ATOMS; ++n) {
     const int i = (blockIdx.x * W + warp) * HS_ATOMS + n;
@@ -402,9 +407,9 @@ k_hs_gather(HsGeom g, int N, const double* __restrict__ q, const double* __restr
         if (row >= NR) break;
         const int x = row / S, y = row - x * S, p = st.off[0][x] + st.off[1][y] + oz;
         const double wxy = st.v[0][x] * st.v[1][y];
-        const double2 a = e01[p], b = e2p[p];
+        const double2 a = e01[p], b = MODE == 0 ? e2p[p] : make_double2(e2r[p], 0.0);
         if (MODE == 2) {
-          const double s = lm[p].x - (Ri[0] * a.x + Ri[1] * a.y + Ri[2] * b.x);
+          const double s = lm[p] - (Ri[0] * a.x + Ri[1] * a.y + Ri[2] * b.x);
           ss[warp][row * LD + z] = s;
           t2 += wxy * s;
         } else {
@@ -541,9 +546,10 @@ struct md_hspme {
   int B = HS_BATCH;          // candidates per batch
   int nab = 0;               // blocks of the spread and the gather
   double2* Z = nullptr;      // [B][Kt] charge meshes, transformed in place
-  double2* F = nullptr;      // [2B][Kt] fields
-  double2* Y = nullptr;      // [2B][Kt] residual meshes, then Lam in place of B_2
-  double* w = nullptr;       // [B][Kt] summand of the marginals
+  double2* F = nullptr;      // [2B][Kt] fields; B_0 and B_2 of the loss as [2B][Kt] real grids in its second half
+  double2* Y = nullptr;      // [2B][Kt] transforms of the residual meshes, then Lam in place of B_2
+  double* e2 = nullptr;      // [B][Kt] the loss's E_2
+  double* w = nullptr;       // [B][Kt] the spread Q or B_1, then the summand of the marginals, then the loss's Lam
   double* bfac = nullptr;    // [B][3][Kmax]
   double* dbfac = nullptr;   // [B][3][ncoef][Kmax]
   double* marg = nullptr;    // [B][3][Kmax]
@@ -553,7 +559,7 @@ struct md_hspme {
 };
 
 static void hs_free(md_hspme* h) {
-  void* p[] = {h->Z, h->F, h->Y, h->w, h->bfac, h->dbfac, h->marg, h->cpart, h->lpart, h->R};
+  void* p[] = {h->Z, h->F, h->Y, h->e2, h->w, h->bfac, h->dbfac, h->marg, h->cpart, h->lpart, h->R};
   for (void* x : p) if (x) cudaFree(x);
 }
 
@@ -589,13 +595,14 @@ extern "C" int md_hspme_create(md_hspme** out, int natoms, const int K[3], const
   const long Kt = g.Kt;
   const int per = HS_ATOMS * hs_warps(g.S), nco = std::max(g.ncoef, 1);
   h->nab = (natoms + per - 1) / per;
-  // the meshes of a batch (88 bytes per point and candidate) stay in the 126 MB
+  // the meshes of a batch (96 bytes per point and candidate) stay in the 126 MB
   // L2 with four candidates up to 64^3
-  h->B = Kt * 88 * HS_BATCH <= (96L << 20) ? HS_BATCH : 2;
+  h->B = Kt * 96 * HS_BATCH <= (96L << 20) ? HS_BATCH : 2;
   const long B = h->B;
   bool ok = cudaMalloc(&h->Z, sizeof(double2) * B * Kt) == cudaSuccess &&
             cudaMalloc(&h->F, sizeof(double2) * 2 * B * Kt) == cudaSuccess &&
             cudaMalloc(&h->Y, sizeof(double2) * 2 * B * Kt) == cudaSuccess &&
+            cudaMalloc(&h->e2, sizeof(double) * B * Kt) == cudaSuccess &&
             cudaMalloc(&h->w, sizeof(double) * B * Kt) == cudaSuccess &&
             cudaMalloc(&h->bfac, sizeof(double) * B * 3 * h->Kmax) == cudaSuccess &&
             cudaMalloc(&h->dbfac, sizeof(double) * B * 3 * nco * h->Kmax) == cudaSuccess &&
@@ -631,12 +638,12 @@ extern "C" int md_hspme_num_coeffs(md_hspme* h, int* out) {
 #define HS_WIDTHS(X) X(2) X(4) X(6) X(8) X(10) X(12) X(14) X(16)
 
 template <int MODE>
-static int hs_spread(md_hspme* h, int nb, const double* q, const double* r, const double* c, double2* mesh,
-                     double2* mesh2, cudaStream_t s) {
+static int hs_spread(md_hspme* h, int nb, const double* q, const double* r, const double* c, cudaStream_t s) {
+  double* re = reinterpret_cast<double*>(h->F + (long)nb * h->g.Kt);
   switch (h->g.S) {
 #define HS_CASE(W)                                                                                               \
   case W:                                                                                                        \
-    k_hs_spread<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), 0, s>>>(h->g, h->N, q, r, c, h->R, mesh, mesh2);    \
+    k_hs_spread<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), 0, s>>>(h->g, h->N, q, r, c, h->R, re, h->w);       \
     break;
     HS_WIDTHS(HS_CASE)
 #undef HS_CASE
@@ -648,11 +655,11 @@ static int hs_spread(md_hspme* h, int nb, const double* q, const double* r, cons
 template <int MODE>
 static int hs_gather(md_hspme* h, int nb, const double* q, const double* r, const double* c, const double* fref,
                      const HsOut& out, cudaStream_t s) {
-  const double2 *f2 = h->F + (long)nb * h->g.Kt, *lam = h->Y + (long)nb * h->g.Kt;
+  const double2* f2 = h->F + (long)nb * h->g.Kt;
   switch (h->g.S) {
 #define HS_CASE(W)                                                                                               \
   case W:                                                                                                        \
-    k_hs_gather<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), 0, s>>>(h->g, h->N, q, r, c, h->F, f2, lam,         \
+    k_hs_gather<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), 0, s>>>(h->g, h->N, q, r, c, h->F, f2, h->e2, h->w, \
                                                                       fref, h->R, h->lpart, out);                  \
     break;
     HS_WIDTHS(HS_CASE)
@@ -675,13 +682,13 @@ static int hs_forward(md_hspme* h, int nb, const double* q, const double* r, con
   HsGeom& g = h->g;
   k_hs_factor<<<dim3((h->Kmax + 63) / 64, 3, nb), 64, 0, s>>>(g, c, h->bfac, h->dbfac, h->Kmax);
   MD_CHECK_LAUNCH("hspme factor");
-  MD_CUDA(cudaMemsetAsync(h->Z, 0, sizeof(double2) * nb * g.Kt, s));
-  if (int e = hs_spread<0>(h, nb, q, r, c, h->Z, nullptr, s)) return e;
-  if (int e = dft3_grid(h->Z, g.K, -1, nb, s)) return e;
+  MD_CUDA(cudaMemsetAsync(h->w, 0, sizeof(double) * nb * g.Kt, s));
+  if (int e = hs_spread<0>(h, nb, q, r, c, s)) return e;
+  if (int e = dft3_from_real(h->w, nullptr, 0, h->Z, g.K, nb, s)) return e;
   k_hs_kspace_fwd<<<(unsigned)((g.Kt + 255) / 256), 256, 0, s>>>(g, nb, loss ? 1 : 0, h->Z, h->bfac, h->Kmax, h->F,
                                                                  want_w ? h->w : nullptr);
   MD_CHECK_LAUNCH("hspme kspace");
-  return dft3_grid(h->F, g.K, +1, 2 * nb, s);
+  return loss ? dft3_to_real(h->F, nb, h->e2, g.K, 2 * nb, s) : dft3_grid(h->F, g.K, +1, 2 * nb, s);
 }
 
 extern "C" int md_hspme_energy(md_hspme* h, const double* q, const double* r, const double* coeffs, int C,
@@ -729,16 +736,17 @@ extern "C" int md_hspme_force_error(md_hspme* h, const double* q, const double* 
     if (int e = hs_gather<1>(h, nb, q, r, c, fref, HsOut{}, s)) return e;
     if (grads) {
       // adjoint: residuals spread, transformed, Lam and the factor marginals
-      double2* Y2 = h->Y + nb * Kt;
-      MD_CUDA(cudaMemsetAsync(h->Y, 0, sizeof(double2) * 2 * nb * Kt, s));
-      if (int e = hs_spread<1>(h, nb, q, r, c, h->Y, Y2, s)) return e;
-      if (int e = dft3_grid(h->Y, g.K, -1, 2 * nb, s)) return e;
+      double2 *Y2 = h->Y + nb * Kt, *B02 = h->F + nb * Kt;
+      MD_CUDA(cudaMemsetAsync(B02, 0, sizeof(double) * 2 * nb * Kt, s));
+      MD_CUDA(cudaMemsetAsync(h->w, 0, sizeof(double) * nb * Kt, s));
+      if (int e = hs_spread<1>(h, nb, q, r, c, s)) return e;
+      if (int e = dft3_from_real((const double*)B02, h->w, nb, h->Y, g.K, 2 * nb, s)) return e;
       k_hs_kspace_adj<<<(unsigned)((Kt + 255) / 256), 256, 0, s>>>(g, nb, h->Z, h->Y, Y2, h->bfac, h->Kmax,
                                                                    dL_dc ? h->w : nullptr);
       MD_CHECK_LAUNCH("hspme adjoint kspace");
       if (dL_dc)
         if (int e = hs_marginals(h, nb, 3, s)) return e;
-      if (int e = dft3_grid(Y2, g.K, +1, nb, s)) return e;
+      if (int e = dft3_to_real(Y2, 0, h->w, g.K, nb, s)) return e;
       HsOut o = {nullptr, dL_dq ? dL_dq + N * b : nullptr, dL_dr ? dL_dr + 3 * N * b : nullptr,
                  dL_dc ? h->cpart : nullptr};
       if (int e = hs_gather<2>(h, nb, q, r, c, nullptr, o, s)) return e;
