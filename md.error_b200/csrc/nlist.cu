@@ -61,14 +61,6 @@ template <class R> __device__ __forceinline__ R img_shift(int code, int d, R L) 
 }
 #define NL_SLOT_MASK 0x03FFFFFF
 
-// the slot index carried in the w component of a staged position (bit copy)
-template <class R> __device__ __forceinline__ R slot_as_w(int j);
-template <> __device__ __forceinline__ float slot_as_w<float>(int j) { return __int_as_float(j); }
-template <> __device__ __forceinline__ double slot_as_w<double>(int j) { return __longlong_as_double((long long)j); }
-template <class R> __device__ __forceinline__ int slot_of_w(R w);
-template <> __device__ __forceinline__ int slot_of_w<float>(float w) { return __float_as_int(w); }
-template <> __device__ __forceinline__ int slot_of_w<double>(double w) { return (int)__double_as_longlong(w); }
-
 // cells along one axis whose box comes within rle of home cell hc's box
 __device__ __forceinline__ void nl_stencil_axis(double L, int nc, int hc, double rle, double& h, int& lo, int& hi,
                                                 int& full) {
@@ -237,8 +229,9 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
                                               DevState* stw) {
   typedef typename V4<R>::T T4;
   extern __shared__ __align__(16) unsigned char nl_smem[];
-  float4* ftile = reinterpret_cast<float4*>(nl_smem);  // home frame, w carries the list entry (slot and image)
-  T4* tile = reinterpret_cast<T4*>(nl_smem);           // stored positions, w carries the slot
+  // one image per run: home frame, w carries the list entry (slot and image);
+  // otherwise the stored position (rounded to binary32), w the slot
+  float4* ftile = reinterpret_cast<float4*>(nl_smem);
   __shared__ RunTable rt;
   const int i0 = (int)start[c], i1 = (int)start[c + 1];
   if (i0 == i1) return;  // empty home cell (uniform exit for the whole block)
@@ -394,8 +387,7 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
   // reads its candidates from L2 instead (staging would cost more than the
   // few reads it saves).  A run's cells are staged in their z order (zord),
   // so each cell of the run is a z-sorted slice of the tile.
-  const int fit = runshift ? NL_TILE_BYTES / (int)sizeof(float4) : NL_TILE_BYTES / (int)sizeof(T4);
-  const bool stage = tile_n <= fit && !(s_flags & 2) && (i1 - i0) >= NL_LIGHT;
+  const bool stage = tile_n <= NL_TILE_BYTES / (int)sizeof(float4) && !(s_flags & 2) && (i1 - i0) >= NL_LIGHT;
   const bool fast = stage && runshift;
   // frame of the packed tile: the box (binary32), or the home cell's corner,
   // so that binary64 positions lose nothing but their last binary32 digit
@@ -434,8 +426,7 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
                                             (float)(v[u].z - img_shift<R>(code[u], 2, L[2]) - corner[2]),
                                             __int_as_float(jj[u] | code[u]));
           } else {
-            v[u].w = slot_as_w<R>(jj[u]);
-            tile[off[u] + t] = v[u];
+            ftile[off[u] + t] = make_float4((float)v[u].x, (float)v[u].y, (float)v[u].z, __int_as_float(jj[u]));
           }
         }
       }
@@ -453,12 +444,14 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
   // z of entry t of a run (z order) in the frame of the run: the stored,
   // wrapped one, or the packed tile's
   auto zat = [&](int roff, int rjb, int t) -> float {
-    return fast ? ftile[roff + t].z : glob ? (float)pos[zord[rjb + t]].z : (float)tile[roff + t].z;
+    return glob ? (float)pos[zord[rjb + t]].z : ftile[roff + t].z;
   };
   // Bound on the difference between the packed tile's squared distance and
   // the reference's (coordinates and differences rounded to binary32, each
   // within 4 units of 2^-24 of the longest edge); inside it the reference's own operations decide.
   const float delta = 2.4e-7f * fmaxf((float)st->L[0], fmaxf((float)st->L[1], Lzf));
+  const float Lf[3] = {(float)st->L[0], (float)st->L[1], Lzf};
+  const float Lif[3] = {(float)st->Li[0], (float)st->Li[1], (float)st->Li[2]};
   int nmax = 0;
 
   for (int i = i0 + warp; i < i1; i += nwarp) {
@@ -602,19 +595,40 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
         const unsigned smask = __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
         const int k = before + __popc(smask & lemask);
         before += __popc(smask);
-        bool ok = false;
+        bool ok = false, test = cidx < total;
         int j = 0, code = 0;
-        if (cidx < total) {
+        T4 pj = pi;
+        if (test) {
           const int x = cidx + wdelta[warp][k];
-          T4 pj;
+          code = wcode[warp][k];
           if (glob) {
             j = (int)zord[x];
             pj = pos[j];
           } else {
-            pj = tile[x];
-            j = slot_of_w<R>(pj.w);
+            const float4 q = ftile[x];
+            j = __float_as_int(q.w);
+            if constexpr (sizeof(R) == 4) {
+              pj = T4{q.x, q.y, q.z, q.w};
+            } else {
+              // binary64: a binary32 distance (nearest image, or the run's in
+              // cell-shift mode) first; what is within its error bound of the
+              // radius, or nearer, is read and tested as stored
+              float dx = q.x - ri.x, dy = q.y - ri.y, dz = q.z - ri.z;
+              if (minimg) {
+                dx -= Lf[0] * rintf(dx * Lif[0]);
+                dy -= Lf[1] * rintf(dy * Lif[1]);
+                dz -= Lf[2] * rintf(dz * Lif[2]);
+              } else {
+                dx -= img_shift<float>(code, 0, Lf[0]);
+                dy -= img_shift<float>(code, 1, Lf[1]);
+                dz -= img_shift<float>(code, 2, Lf[2]);
+              }
+              test = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < out2;
+              if (test) pj = pos[j];
+            }
           }
-          code = wcode[warp][k];
+        }
+        if (test) {
           R d2;
           if (runshift) {
             d2 = nl_exact_d2<R>(pj, pi, code, L);
