@@ -4,18 +4,23 @@
 // NeighborList::mallocDeviceNeighborList (UNI/src/NeighborList_interface.cu:187-208),
 // Displacement_max (ENG/src/Displacement_interface.cu:80-126).
 //
-// One block per home cell.  The candidate cells of the home cell (every cell
+// One block per home cell of NL_LIGHT atoms or more, one warp per lighter cell.
+// The candidate cells of the home cell (every cell
 // whose box comes within the largest list radius of the home-cell box, or the
 // reference's c +- 1 stencil in cell-shift mode) are enumerated as (x, y)
 // columns of contiguous z runs -- each run one contiguous slice of the
 // cell-sorted arrays -- and staged into a shared-memory tile.  Each warp then
-// takes one home atom i at a time; its 32 lanes test 32 tile entries at once,
+// takes one home atom i at a time; its 32 lanes test 2 x 32 tile entries at once,
 // skipping runs whose box lies beyond rlist_i, and a ballot compacts the
 // accepted ones into row i of the list.  When the tile would not fit, the same
 // loop reads the runs from global memory.
-// The acceptance test repeats the reference's binary32 operations exactly
-// (no FMA contraction), so the neighbour SETS are bit-identical to the
-// reference criterion; only the enumeration (and list order) is ours.
+// A pair within rounding of the radius is decided by the reference's binary32
+// (or binary64) operations without FMA contraction, every other by a binary32
+// distance with a proven error bound, so the neighbour SETS are bit-identical to
+// the reference criterion; only the enumeration (and list order) is ours.
+// Bound: instruction issue and latency of the test loop (65,536-atom slab, 203
+// entries an atom: 118 M warp instructions, 172 us; test loop 72, windows 24,
+// staging 19, set-up and light cells 57).  Before: 227 us (binary64 421, now 198).
 // List layout: list[i*cap + k], k < nnb[i]; each entry packs the slot index j
 // (bits 0-25) and the periodic image k_d = floorf(d_d/L_d + 0.5) in {-1,0,1}
 // of the minimum-image vector, 2 bits per axis (bits 26-31, stored k+1), so
@@ -789,9 +794,11 @@ struct RebuildArgs {
   T4* backup;
 };
 
-// resident blocks per SM the kernels are built for (the list tile leaves room
-// for four)
-#define REBUILD_MIN_BLOCKS 4
+// Resident blocks per SM the kernels are built for: four, which is what the list
+// tile leaves room for, at 64 registers and some spills; or two, without spills,
+// where a launch has no more than two blocks per SM (rebuild_kernel)
+#define REBUILD_WIDE 4
+#define REBUILD_SMALL 2
 
 // the atoms of this block in the per-atom phases: a contiguous share of
 // ceil(N / blocks), so that every block (and every SM) takes part
@@ -897,8 +904,8 @@ __device__ __forceinline__ void rebuild_phases(const RebuildArgs<R>& a) {
   }
 }
 
-template <class R, int MODE>
-__global__ void __launch_bounds__(256, REBUILD_MIN_BLOCKS) k_rebuild(RebuildArgs<R> a) {
+template <class R, int MODE, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_rebuild(RebuildArgs<R> a) {
   // FLAG_REBUILD does not change while this kernel runs (it is set by the
   // step's first kernel and cleared by its last), so every block takes the
   // same branch
@@ -911,8 +918,8 @@ __global__ void __launch_bounds__(256, REBUILD_MIN_BLOCKS) k_rebuild(RebuildArgs
 // every atom, a grid barrier, the box of the step committed, and, when an
 // atom has moved more than half the skin, the rebuild phases.  This saves the
 // step a kernel node against k_lv_step1 followed by k_rebuild.
-template <class R, int MODE>
-__global__ void __launch_bounds__(256, REBUILD_MIN_BLOCKS)
+template <class R, int MODE, int MINB>
+__global__ void __launch_bounds__(256, MINB)
 k_lv_step1_rebuild(typename V4<R>::T* __restrict__ vel, const double4a* __restrict__ force, LvDev p,
                    RebuildArgs<R> a) {
   DevState* st = a.st;
@@ -932,24 +939,26 @@ k_lv_step1_rebuild(typename V4<R>::T* __restrict__ vel, const double4a* __restri
 // the kernel of a precision and list mode, its dynamic shared memory, the
 // most blocks one cooperative launch can hold (0: not possible on this
 // device) and the device's SM count
-static const void* rebuild_kernel(int prec, int mode, size_t* smem, int* blocks, bool with_lv = false,
-                                  int* sms = nullptr) {
-  const void* f;
+template <int MINB>
+static const void* rebuild_pick(int prec, int mode, bool with_lv) {
   if (prec == MD_PREC_FP64) {
     if (with_lv)
-      f = mode == MD_NL_MINIMAGE ? (const void*)k_lv_step1_rebuild<double, MD_NL_MINIMAGE>
-                                 : (const void*)k_lv_step1_rebuild<double, MD_NL_CELLSHIFT>;
-    else
-      f = mode == MD_NL_MINIMAGE ? (const void*)k_rebuild<double, MD_NL_MINIMAGE>
-                                 : (const void*)k_rebuild<double, MD_NL_CELLSHIFT>;
-  } else {
-    if (with_lv)
-      f = mode == MD_NL_MINIMAGE ? (const void*)k_lv_step1_rebuild<float, MD_NL_MINIMAGE>
-                                 : (const void*)k_lv_step1_rebuild<float, MD_NL_CELLSHIFT>;
-    else
-      f = mode == MD_NL_MINIMAGE ? (const void*)k_rebuild<float, MD_NL_MINIMAGE>
-                                 : (const void*)k_rebuild<float, MD_NL_CELLSHIFT>;
+      return mode == MD_NL_MINIMAGE ? (const void*)k_lv_step1_rebuild<double, MD_NL_MINIMAGE, MINB>
+                                    : (const void*)k_lv_step1_rebuild<double, MD_NL_CELLSHIFT, MINB>;
+    return mode == MD_NL_MINIMAGE ? (const void*)k_rebuild<double, MD_NL_MINIMAGE, MINB>
+                                  : (const void*)k_rebuild<double, MD_NL_CELLSHIFT, MINB>;
   }
+  if (with_lv)
+    return mode == MD_NL_MINIMAGE ? (const void*)k_lv_step1_rebuild<float, MD_NL_MINIMAGE, MINB>
+                                  : (const void*)k_lv_step1_rebuild<float, MD_NL_CELLSHIFT, MINB>;
+  return mode == MD_NL_MINIMAGE ? (const void*)k_rebuild<float, MD_NL_MINIMAGE, MINB>
+                                : (const void*)k_rebuild<float, MD_NL_CELLSHIFT, MINB>;
+}
+
+static const void* rebuild_kernel(int prec, int mode, size_t* smem, int* blocks, bool with_lv = false,
+                                  int* sms = nullptr, bool small = false) {
+  const void* f = small ? rebuild_pick<REBUILD_SMALL>(prec, mode, with_lv)
+                        : rebuild_pick<REBUILD_WIDE>(prec, mode, with_lv);
   *smem = NL_TILE_BYTES;
   *blocks = 0;
   int dev = 0, coop = 0, nsm = 0, per_sm = 0;
@@ -1008,7 +1017,18 @@ static int rebuild_fused_t(md_cell_list* cl, md_nlist* nl, md_system* sys, Recor
   // without at a block per 8, 126 and 4.8 per 4, 97 and 5.4 per 2, 97 and 5.6
   // per 1; 4,000 atoms, 216 cells: 54 and 4.6 at one block per SM, 59 and 4.7 at
   // a block per cell
-  blocks = std::min(blocks, std::max(sms, (cl->ntot + 1) / 2));
+  const int want = std::max(sms, (cl->ntot + 1) / 2);
+  // up to two blocks per SM: the build without spills (us a rebuild, a step
+  // without one: 4,000 atoms 51 and 4.4, with four blocks' registers 54 and 4.5;
+  // 12,000 63 and 4.6, 68 and 4.7; binary64 4,000 55 and 4.7, 60 and 4.9, and 33
+  // against 37 a whole step from a cold L2).  More blocks want the registers: the
+  // 65,536-atom slab in binary64 348 with four blocks an SM, 427 with two
+  if (want <= REBUILD_SMALL * sms && blocks >= want) {
+    int fit = 0;
+    const void* g = rebuild_kernel(sys->prec, nl->mode, &smem, &fit, with_lv, nullptr, true);
+    if (fit >= want) { f = g; blocks = fit; }
+  }
+  blocks = std::min(blocks, want);
   if (!with_lv) {
     void* args[] = {&a};
     return rec_launch_coop(rec, f, dim3(blocks), dim3(256), smem, args);
