@@ -41,7 +41,8 @@
 // meshes are real, so the FP64 grid transforms (dft.cu) carry two fields of a
 // candidate each where it has two, as the real and imaginary parts: (E_0, E_1)
 // and (E_2, phi_pot) back, (B_0, B_1) forward -- 9 complex transforms per
-// candidate for both functionals where one per mesh takes 14.  Two candidates
+// candidate for both functionals where one per mesh takes 14 -- and read and write
+// real grids where it has one.  Two candidates
 // never share a transform: the rounding of one (or its infinities) would reach
 // the other, 4 to 10 times the error in the gradient of the smaller.  Spread
 // and gather give a warp to an atom with lanes along its
@@ -51,7 +52,7 @@
 // scalar Lam - R.E).  Sums over blocks and the marginals are block reductions
 // in a fixed order.  Bound: FP64 mesh atomics in the spread, latency and L2
 // reads in the gather.  8 candidates of order-6 support, 20,736 charges, 64^3,
-// energy and force error with every gradient: 2.2 ms, 11.8 ms when each
+// energy and force error with every gradient: 2.0 ms, 11.8 ms when each
 // candidate ran by itself with serial finishing sums and atomic marginals.
 #include <algorithm>
 #include <cmath>
@@ -561,6 +562,24 @@ struct md_hspme {
 static void hs_free(md_hspme* h) {
   void* p[] = {h->Z, h->F, h->Y, h->e2, h->w, h->bfac, h->dbfac, h->marg, h->cpart, h->lpart, h->R};
   for (void* x : p) if (x) cudaFree(x);
+  h->Z = h->F = h->Y = nullptr;
+  h->e2 = h->w = h->bfac = h->dbfac = h->marg = h->cpart = h->lpart = h->R = nullptr;
+}
+
+// workspace for batches of B candidates
+static bool hs_alloc(md_hspme* h, long B) {
+  const long Kt = h->g.Kt, nco = std::max(h->g.ncoef, 1);
+  return cudaMalloc(&h->Z, sizeof(double2) * B * Kt) == cudaSuccess &&
+         cudaMalloc(&h->F, sizeof(double2) * 2 * B * Kt) == cudaSuccess &&
+         cudaMalloc(&h->Y, sizeof(double2) * 2 * B * Kt) == cudaSuccess &&
+         cudaMalloc(&h->e2, sizeof(double) * B * Kt) == cudaSuccess &&
+         cudaMalloc(&h->w, sizeof(double) * B * Kt) == cudaSuccess &&
+         cudaMalloc(&h->bfac, sizeof(double) * B * 3 * h->Kmax) == cudaSuccess &&
+         cudaMalloc(&h->dbfac, sizeof(double) * B * 3 * nco * h->Kmax) == cudaSuccess &&
+         cudaMalloc(&h->marg, sizeof(double) * B * 3 * h->Kmax) == cudaSuccess &&
+         cudaMalloc(&h->cpart, sizeof(double) * B * h->nab * nco) == cudaSuccess &&
+         cudaMalloc(&h->lpart, sizeof(double) * B * h->nab) == cudaSuccess &&
+         cudaMalloc(&h->R, sizeof(double) * B * 3 * h->N) == cudaSuccess;
 }
 
 extern "C" int md_hspme_create(md_hspme** out, int natoms, const int K[3], const double L[3], double beta, double CC,
@@ -592,29 +611,19 @@ extern "C" int md_hspme_create(md_hspme** out, int natoms, const int K[3], const
   g.S = 2 * half;
   g.Kt = (long)K[0] * K[1] * K[2];
   h->Kmax = std::max(K[0], std::max(K[1], K[2]));
-  const long Kt = g.Kt;
-  const int per = HS_ATOMS * hs_warps(g.S), nco = std::max(g.ncoef, 1);
+  const int per = HS_ATOMS * hs_warps(g.S);
   h->nab = (natoms + per - 1) / per;
   // the meshes of a batch (96 bytes per point and candidate) stay in the 126 MB
-  // L2 with four candidates up to 64^3
-  h->B = Kt * 96 * HS_BATCH <= (96L << 20) ? HS_BATCH : 2;
-  const long B = h->B;
-  bool ok = cudaMalloc(&h->Z, sizeof(double2) * B * Kt) == cudaSuccess &&
-            cudaMalloc(&h->F, sizeof(double2) * 2 * B * Kt) == cudaSuccess &&
-            cudaMalloc(&h->Y, sizeof(double2) * 2 * B * Kt) == cudaSuccess &&
-            cudaMalloc(&h->e2, sizeof(double) * B * Kt) == cudaSuccess &&
-            cudaMalloc(&h->w, sizeof(double) * B * Kt) == cudaSuccess &&
-            cudaMalloc(&h->bfac, sizeof(double) * B * 3 * h->Kmax) == cudaSuccess &&
-            cudaMalloc(&h->dbfac, sizeof(double) * B * 3 * nco * h->Kmax) == cudaSuccess &&
-            cudaMalloc(&h->marg, sizeof(double) * B * 3 * h->Kmax) == cudaSuccess &&
-            cudaMalloc(&h->cpart, sizeof(double) * B * h->nab * nco) == cudaSuccess &&
-            cudaMalloc(&h->lpart, sizeof(double) * B * h->nab) == cudaSuccess &&
-            cudaMalloc(&h->R, sizeof(double) * B * 3 * natoms) == cudaSuccess;
-  if (!ok) {
-    md_cuda_fail(cudaGetLastError(), "md_hspme_create");
+  // L2 with four candidates up to 64^3; fewer where memory holds no more
+  h->B = g.Kt * 96 * HS_BATCH <= (96L << 20) ? HS_BATCH : 2;
+  while (!hs_alloc(h, h->B)) {
+    const cudaError_t e = cudaGetLastError();
     hs_free(h);
-    delete h;
-    return MD_ERR_CUDA;
+    if (e != cudaErrorMemoryAllocation || h->B == 1) {
+      delete h;
+      return md_cuda_fail(e, "md_hspme_create");
+    }
+    h->B /= 2;
   }
   *out = h;
   return MD_OK;
