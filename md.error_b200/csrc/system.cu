@@ -358,12 +358,16 @@ int sys_read_back(md_system* s, cudaStream_t stream, void* const* dst, const voi
   HostLease lease(s, total);
   char* stage = (char*)lease.p;
   size_t at = 0;
-  for (int k = 0; k < n; ++k) {
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < n && e == cudaSuccess; ++k) {
     void* to = stage ? stage + at : dst[k];
-    MD_CUDA(cudaMemcpyAsync(to, src[k], bytes[k], cudaMemcpyDeviceToHost, stream));
+    e = cudaMemcpyAsync(to, src[k], bytes[k], cudaMemcpyDeviceToHost, stream);
     at += (bytes[k] + 15) & ~(size_t)15;
   }
-  MD_CUDA(cudaStreamSynchronize(stream));
+  // the copies issued so far end before the lease does, also after an error
+  const cudaError_t done = cudaStreamSynchronize(stream);
+  MD_CUDA(e);
+  MD_CUDA(done);
   at = 0;
   if (stage)
     for (int k = 0; k < n; ++k) {
