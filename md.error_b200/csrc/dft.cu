@@ -5,8 +5,8 @@
 // 1,024 points per block of 128 threads; lines adjacent in memory share a
 // block, so strided axes load coalesced.  Bound: latency of two or three
 // shared-memory exchanges per pass; the radix-2 line per block it replaces
-// made log2 n of them and loaded strided axes 16 bytes at a time (64^3 grids,
-// batches of 1 to 4: 21 us a pass before, 6 us now).
+// made log2 n of them and loaded strided axes 16 bytes at a time (64^3 grids:
+// 21 us a pass of one before, 8 us of three and 15 us of eight now).
 //
 // Other sizes (the odd bin grids of AdaptRCut): a length p is summed over the
 // (p-1)/2 pairs x_j +- x_{p-j}, which gives outputs k and p-k together from

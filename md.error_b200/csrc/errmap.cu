@@ -17,7 +17,7 @@
 // the summed kernel: per direction two passes over g (three components) and
 // one kernel that forms the nine fields along dir and adds their squares
 // without writing them (k_em_alias_sq).  64^3, order 6: 87 passes over the grids
-// (2.2 ms) became 21, and the map with its evaluation went from 3.0 to 0.31 ms
+// (2.2 ms) became 21, and the map with its evaluation went from 3.0 to 0.34 ms
 // of kernel time; memory comes from one allocation of the device's pool
 // (16 cudaMalloc / cudaFree calls took 5.2 ms).
 // rho1 is the density of charge signs, rho2 the number density of charges

@@ -6,8 +6,10 @@
 //   analytic differentiation         RE/src/EleRecFBSpline.cpp:771-907, 1146-1195
 //
 // Chain of one force evaluation (each step one kernel):
-//   spread      charges into a shared-memory tile per warp, the tile added to
-//               the mesh with 4-wide atomics (spme_pm.cu)
+//   spread      lanes along the stencil rows, mesh atomics; dense large systems
+//               through a shared-memory tile (spme_pm.cu)
+// then, where the x and y sizes are equal and a plane fits an SM, three passes by
+// planes (spme_plane.cu); on other meshes
 //   z pass      R2C along z (real lines -> half-complex lines)
 //   y pass      forward C2C along y
 //   x pass      forward C2C along x, k-space step (energy and virial in FP64,
