@@ -6,22 +6,26 @@
 // block, so strided axes load coalesced.  Bound: latency of two or three
 // shared-memory exchanges per pass; the radix-2 line per block it replaces
 // made log2 n of them and loaded strided axes 16 bytes at a time (64^3 grids:
-// 21 us a pass of one before, 8 us of three and 15 us of eight now).
+// 21 us a pass of one before, 5.7 us of three and 10 us of eight now).
 //
 // Other sizes (the odd bin grids of AdaptRCut): a length p is summed over the
 // (p-1)/2 pairs x_j +- x_{p-j}, which gives outputs k and p-k together from
 // 4 real products per pair where the direct sum takes 16; composite lengths
 // n = n1 n2 with a prime n1 <= 11 take two such stages (Cooley-Tukey).  Lanes
 // hold different lines, so a twiddle is one broadcast and six outputs share
-// each loaded pair.  Bound: shared-memory bandwidth and FP64 issue.
+// each loaded pair.  Bound: shared-memory bandwidth and FP64 issue (six grids of
+// 41 x 41 x 161: 31 us along the 41-point axes, 38 along the other).
 #include <algorithm>
 #include "fft_lines.cuh"
 
 namespace {
 
-// line L of an axis of n points: elements `inner` apart from (L / inner) n inner + L % inner
-__device__ __forceinline__ size_t line_base(long L, int n, long inner) {
-  return (size_t)(L / inner) * n * inner + (size_t)(L % inner);
+// line L of an axis of n points: elements `inner` apart from (L / inner) n inner + L % inner.
+// At most 2^20 lines a grid, so 32 bits hold any L; a 64-bit division here cost more
+// than the transform (one per point read and written).
+__device__ __forceinline__ size_t line_base(unsigned L, int n, unsigned inner) {
+  const unsigned q = L / inner;
+  return (size_t)q * n * inner + (L - q * inner);
 }
 
 // Where a pass reads and writes its grids (element p of all grids end to end):
@@ -51,7 +55,7 @@ __device__ __forceinline__ void io_store(const DftIo& io, size_t p, double2 v) {
 
 template <int LOGN, int IO>
 __global__ void __launch_bounds__(FFT_THREADS)
-k_fft_grid(DftIo io, long nlines, long inner, int sign) {
+k_fft_grid(DftIo io, unsigned nlines, unsigned inner, int sign) {
   typedef FftGeom<LOGN> G;
   constexpr int n = G::n, LPB = G::LPB, LS = G::LS, EPT = G::EPT;
   extern __shared__ __align__(16) unsigned char fg_smem[];
@@ -62,19 +66,30 @@ k_fft_grid(DftIo io, long nlines, long inner, int sign) {
     sincospi(2.0 * m / n, &s, &c);
     tw[m] = make_double2(c, sign * s);
   }
-  const long line0 = (long)blockIdx.x * LPB;
+  // element s of the thread: line l of the block, point k of it, element p of the
+  // grids (a thread's elements of a strided axis lie on one line: LPB divides
+  // the threads)
+  const unsigned line0 = blockIdx.x * LPB;
+  const size_t first = inner > 1 ? line_base(line0 + threadIdx.x % LPB, n, inner) : 0;
+  auto element = [&](int s, int& l, int& k, size_t& p) -> bool {
+    const int e = threadIdx.x + s * FFT_THREADS;
+    l = inner > 1 ? e % LPB : e >> LOGN;
+    k = inner > 1 ? e / LPB : e & (n - 1);
+    p = inner > 1 ? first + (size_t)k * inner : (size_t)line0 * n + e;
+    return line0 + l < nlines;
+  };
   double2 v[EPT];
 #pragma unroll
   for (int s = 0; s < EPT; ++s) {
-    const int e = threadIdx.x + s * FFT_THREADS;
-    const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
-    const long L = line0 + l;
-    v[s] = L < nlines ? io_load<IO>(io, line_base(L, n, inner) + k * inner) : make_double2(0.0, 0.0);
+    int l, k;
+    size_t p;
+    v[s] = element(s, l, k, p) ? io_load<IO>(io, p) : make_double2(0.0, 0.0);
   }
 #pragma unroll
   for (int s = 0; s < EPT; ++s) {
-    const int e = threadIdx.x + s * FFT_THREADS;
-    const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
+    int l, k;
+    size_t p;
+    element(s, l, k, p);
     X[l * LS + fft_pad<double>(k)] = v[s];
   }
   __syncthreads();
@@ -83,10 +98,9 @@ k_fft_grid(DftIo io, long nlines, long inner, int sign) {
   else fft_stages<double, LOGN, 0, 1>(x, tw, threadIdx.x % G::TPL);
 #pragma unroll
   for (int s = 0; s < EPT; ++s) {
-    const int e = threadIdx.x + s * FFT_THREADS;
-    const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
-    const long L = line0 + l;
-    if (L < nlines) io_store<IO>(io, line_base(L, n, inner) + k * inner, X[l * LS + fft_pad<double>(k)]);
+    int l, k;
+    size_t p;
+    if (element(s, l, k, p)) io_store<IO>(io, p, X[l * LS + fft_pad<double>(k)]);
   }
 }
 
@@ -151,28 +165,32 @@ __device__ __forceinline__ void pair_sums(const double2* x, int xs, int p, int k
 // LN lines per block, one per lane; n = n1 n2 (n1 = 1: a single stage of length n)
 template <int LN, int IO>
 __global__ void __launch_bounds__(DA_THREADS)
-k_dft_any(DftIo io, long nlines, long inner, int n, int n1, int sign) {
+k_dft_any(DftIo io, unsigned nlines, unsigned inner, int n, int n1, int sign) {
   extern __shared__ __align__(16) unsigned char da_smem[];
   constexpr int LS = LN + 1, NG = DA_THREADS / LN;
   double2* tw = reinterpret_cast<double2*>(da_smem);  // (cos, sign sin) of 2 pi m / n
   double2* x = tw + n;                                // [n][LS]
   const int n2 = n / n1;
-  const long line0 = (long)blockIdx.x * LN;
+  const unsigned line0 = blockIdx.x * LN;
   for (int m = threadIdx.x; m < n; m += DA_THREADS) {
     double s, c;
     sincospi(2.0 * m / n, &s, &c);
     tw[m] = make_double2(c, sign * s);
   }
-  for (int t = threadIdx.x; t < n * LN; t += DA_THREADS) {
-    const int l = inner > 1 ? t % LN : t / n, j = inner > 1 ? t / LN : t % n;
-    const long L = line0 + l;
-    x[j * LS + l] = L < nlines ? io_load<IO>(io, line_base(L, n, inner) + j * inner) : make_double2(0.0, 0.0);
+  const int l = threadIdx.x % LN, g = threadIdx.x / LN;
+  const bool live = line0 + l < nlines;
+  const size_t dst = live ? line_base(line0 + l, n, inner) : 0;
+  if (inner > 1) {  // the thread's line, a point in NG
+    for (int j = g; j < n; j += NG)
+      x[j * LS + l] = live ? io_load<IO>(io, dst + (size_t)j * inner) : make_double2(0.0, 0.0);
+  } else {  // whole lines end to end
+    const size_t p0 = (size_t)line0 * n;
+    for (int t = threadIdx.x; t < n * LN; t += DA_THREADS) {
+      const int q = t / n;
+      x[(t - q * n) * LS + q] = line0 + q < nlines ? io_load<IO>(io, p0 + t) : make_double2(0.0, 0.0);
+    }
   }
   __syncthreads();
-  const int l = threadIdx.x % LN, g = threadIdx.x / LN;
-  const long L = line0 + l;
-  const bool live = L < nlines;
-  const size_t dst = live ? line_base(L, n, inner) : 0;
   double2 A[DA_KB], B[DA_KB];
   if (n1 > 1) {
     // stage 1, in place: a thread holds all outputs of a length-n1 transform
@@ -183,12 +201,12 @@ k_dft_any(DftIo io, long nlines, long inner, int n, int n1, int sign) {
 #pragma unroll
       for (int q = 0; q < DA_KB; ++q) {
         if (q > n1 / 2) break;
-        const double2 w = tw[(j2 * q) % n];
+        const double2 w = tw[j2 * q];  // (j2 < n2, q < n1: below n)
         const double2 u = make_double2(A[q].x + B[q].x, A[q].y + B[q].y);
         c[(size_t)q * n2 * LS] = make_double2(u.x * w.x - u.y * w.y, u.x * w.y + u.y * w.x);
         if (q > 0 && 2 * q < n1) {
           const int k = n1 - q;
-          const double2 z = tw[(j2 * k) % n];
+          const double2 z = tw[j2 * k];
           const double2 v = make_double2(A[q].x - B[q].x, A[q].y - B[q].y);
           c[(size_t)k * n2 * LS] = make_double2(v.x * z.x - v.y * z.y, v.x * z.y + v.y * z.x);
         }

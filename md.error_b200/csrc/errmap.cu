@@ -17,7 +17,7 @@
 // the summed kernel: per direction two passes over g (three components) and
 // one kernel that forms the nine fields along dir and adds their squares
 // without writing them (k_em_alias_sq).  64^3, order 6: 87 passes over the grids
-// (2.2 ms) became 21, and the map with its evaluation went from 3.0 to 0.34 ms
+// (2.2 ms) became 21, and the map with its evaluation went from 3.0 to 0.30 ms
 // of kernel time; memory comes from one allocation of the device's pool
 // (16 cudaMalloc / cudaFree calls took 5.2 ms).
 // rho1 is the density of charge signs, rho2 the number density of charges
@@ -41,9 +41,11 @@ struct EmGrid {
 
 __device__ __forceinline__ int em_c(int i, int K) { return i > (K >> 1) ? i - K : i; }
 __device__ __forceinline__ void em_idx(long t, const EmGrid& g, int ii[3]) {
-  ii[2] = (int)(t % g.K[2]);
-  ii[1] = (int)((t / g.K[2]) % g.K[1]);
-  ii[0] = (int)(t / ((long)g.K[2] * g.K[1]));
+  // 32 bits hold any point of the grid (1,024^3 at most) and divide several times faster
+  const unsigned q = (unsigned)t / g.K[2], x = q / g.K[1];
+  ii[2] = (int)((unsigned)t - q * g.K[2]);
+  ii[1] = (int)(q - x * g.K[1]);
+  ii[0] = (int)x;
 }
 
 __device__ __forceinline__ double em_pow(double x, int n) {
@@ -148,7 +150,10 @@ k_em_alias_sq(EmGrid g, const double2* __restrict__ T, const double* __restrict_
     tw[m] = make_double2(c, s);
   }
   for (int t = threadIdx.x; t < (nk + 1) * n; t += FFT_THREADS) al[t] = tab[(size_t)(t / n) * Kmax + t % n];
-  const long nlines = g.N / n, line0 = (long)blockIdx.x * LPB;
+  const unsigned nlines = (unsigned)(g.N / n), line0 = blockIdx.x * LPB;
+  // a thread's elements of a strided axis lie on one line (LPB divides the threads)
+  const unsigned L0 = line0 + threadIdx.x % LPB, hi = L0 / (unsigned)inner;
+  const size_t base = (size_t)hi * n * inner + (L0 - hi * (unsigned)inner);
   size_t at[EPT];
   int xs[EPT], km[EPT];
   double sq[EPT];
@@ -156,8 +161,7 @@ k_em_alias_sq(EmGrid g, const double2* __restrict__ T, const double* __restrict_
   for (int s = 0; s < EPT; ++s) {
     const int e = threadIdx.x + s * FFT_THREADS;
     const int l = inner > 1 ? e % LPB : e >> LOGN, k = inner > 1 ? e / LPB : e & (n - 1);
-    const long L = line0 + l;
-    at[s] = L < nlines ? (size_t)(L / inner) * n * inner + (size_t)(L % inner) + k * inner : (size_t)-1;
+    at[s] = line0 + l >= nlines ? (size_t)-1 : inner > 1 ? base + (size_t)k * inner : (size_t)line0 * n + e;
     xs[s] = l * LS + fft_pad<double>(k);
     km[s] = k;
     sq[s] = 0.0;
