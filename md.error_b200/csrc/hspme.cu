@@ -52,7 +52,7 @@
 // scalar Lam - R.E).  Sums over blocks and the marginals are block reductions
 // in a fixed order.  Bound: FP64 mesh atomics in the spread, latency and L2
 // reads in the gather.  8 candidates of order-6 support, 20,736 charges, 64^3,
-// energy and force error with every gradient: 1.9 ms, 11.8 ms when each
+// energy and force error with every gradient: 1.8 ms, 11.8 ms when each
 // candidate ran by itself with serial finishing sums and atomic marginals.
 #include <algorithm>
 #include <cmath>
@@ -72,6 +72,7 @@ constexpr int HS_MAX_NBIN = 64;
 constexpr int HS_MAX_COEF = 2 * HS_MAX_NBIN;
 constexpr int HS_BATCH = 4;  // candidates per launch (two where four would not stay in L2)
 constexpr int HS_ATOMS = 4;  // atoms per warp of the spread and the gather
+constexpr int HS_COPIES = 8; // of a warp's coefficient sums: four lanes each
 
 struct HsGeom {
   int K[3];
@@ -375,10 +376,15 @@ k_hs_gather(HsGeom g, int N, const double* __restrict__ q, const double* __restr
   constexpr int RP = 32 / S, NR = S * S, NI = (NR + RP - 1) / RP, W = hs_warps(S), LD = S + 1;
   __shared__ HsStencil<S> sst[W];
   __shared__ double ss[W][MODE == 1 ? 1 : NR * LD], su[W][MODE == 1 ? 1 : NR], sp[W][MODE == 1 ? 1 : 32 + 4 * S];
-  __shared__ double csum[MODE == 1 ? 1 : HS_MAX_COEF], sl[W];
+  // the four coefficient terms of each one-dimensional point, and a warp's sums of
+  // them, HS_COPIES copies of [ncoef]
+  __shared__ double sv[W][MODE == 1 ? 1 : 12 * S], sl[W];
+  __shared__ int si[W][MODE == 1 ? 1 : 12 * S];
+  extern __shared__ double hs_csum[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cand = blockIdx.y;
   if (MODE != 1) {
-    for (int t = threadIdx.x; t < g.ncoef; t += blockDim.x) csum[t] = 0.0;
+    if (out.cpart)
+      for (int t = threadIdx.x; t < W * HS_COPIES * g.ncoef; t += blockDim.x) hs_csum[t] = 0.0;
     __syncthreads();
   }
   HsStencil<S>& st = sst[warp];
@@ -476,11 +482,26 @@ k_hs_gather(HsGeom g, int N, const double* __restrict__ q, const double* __restr
           HsStencil<S>& same = st;  // re-evaluated: the same values are stored again
           e = hs_entry<S>(g, c, r + 3 * (long)i, t, same);
         }
-        for (int b = 0; b < 4; ++b)
-          if (e.idx[b] >= 0) atomicAdd(&csum[e.idx[b]], tv * e.dc[b]);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          sv[warp][4 * t + b] = tv * e.dc[b];
+          si[warp][4 * t + b] = e.idx[b];
+        }
       }
     }
     __syncwarp();
+    if (out.cpart) {
+      // four lanes to a point, whose four coefficients differ, eight points at a
+      // time, each into its own copy: no two lanes meet (shared FP64 atomics, as
+      // before, retry where they do: 161 us a batch of four then, 145 now)
+      double* acc = hs_csum + (warp * HS_COPIES + (lane >> 2)) * g.ncoef;
+#pragma unroll
+      for (int t0 = 0; t0 < 12 * S; t0 += 32) {
+        const int t = t0 + lane;
+        if (t < 12 * S && si[warp][t] >= 0) acc[si[warp][t]] += sv[warp][t];
+        __syncwarp();
+      }
+    }
     if (lane < 4) {
       double v = 0.0;
 #pragma unroll
@@ -503,8 +524,11 @@ k_hs_gather(HsGeom g, int N, const double* __restrict__ q, const double* __restr
     }
   } else if (out.cpart) {
     __syncthreads();
-    for (int t = threadIdx.x; t < g.ncoef; t += blockDim.x)
-      out.cpart[((long)cand * gridDim.x + blockIdx.x) * g.ncoef + t] = csum[t];
+    for (int t = threadIdx.x; t < g.ncoef; t += blockDim.x) {
+      double v = 0.0;
+      for (int w = 0; w < W * HS_COPIES; ++w) v += hs_csum[w * g.ncoef + t];
+      out.cpart[((long)cand * gridDim.x + blockIdx.x) * g.ncoef + t] = v;
+    }
   }
 }
 
@@ -669,10 +693,14 @@ static int hs_gather(md_hspme* h, int nb, const double* q, const double* r, cons
   const double2* f2 = h->F + (long)nb * h->g.Kt;
   switch (h->g.S) {
 #define HS_CASE(W)                                                                                               \
-  case W:                                                                                                        \
-    k_hs_gather<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), 0, s>>>(h->g, h->N, q, r, c, h->F, f2, h->e2, h->w, \
-                                                                      fref, h->R, h->lpart, out);                  \
-    break;
+  case W: {                                                                                                      \
+    const size_t dyn = out.cpart ? sizeof(double) * hs_warps(W) * HS_COPIES * h->g.ncoef : 0;                      \
+    if (dyn > 4096)                                                                                                \
+      MD_CUDA(cudaFuncSetAttribute(k_hs_gather<W, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));  \
+    k_hs_gather<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), dyn, s>>>(h->g, h->N, q, r, c, h->F, f2, h->e2,     \
+                                                                      h->w, fref, h->R, h->lpart, out);            \
+    break;                                                                                                         \
+  }
     HS_WIDTHS(HS_CASE)
 #undef HS_CASE
   }
