@@ -20,7 +20,7 @@
 // the reference criterion; only the enumeration (and list order) is ours.
 // Bound: instruction issue and latency of the test loop (65,536-atom slab, 203
 // entries an atom: 118 M warp instructions, 172 us; test loop 72, windows 24,
-// staging 19, set-up and light cells 57).  Before: 227 us (binary64 421, now 198).
+// staging 19, set-up and light cells 57).  Before: 227 us (binary64 421, now 210).
 // List layout: list[i*cap + k], k < nnb[i]; each entry packs the slot index j
 // (bits 0-25) and the periodic image k_d = floorf(d_d/L_d + 0.5) in {-1,0,1}
 // of the minimum-image vector, 2 bits per axis (bits 26-31, stored k+1), so
