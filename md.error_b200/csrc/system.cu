@@ -19,6 +19,7 @@ void md_set_error(const char* fmt, ...) {
 }
 
 int md_cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here: the next call's launch check must not find it again
   md_set_error("CUDA error in %s: %s", what, cudaGetErrorString(e));
   return MD_ERR_CUDA;
 }

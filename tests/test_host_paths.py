@@ -1,0 +1,86 @@
+"""Host code of the library without a GPU: its objects linked against a CUDA
+runtime that carries out copies, only looks at kernels and can be told to fail
+(fake_cudart.c)."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "md.error_b200", "csrc")
+NO_FAILURE = -1
+
+
+@pytest.fixture(scope="module")
+def rt(tmp_path_factory):
+    """the library on the fake runtime"""
+    if not shutil.which("nvcc") or not shutil.which("g++"):
+        pytest.skip("no compiler for the objects of the library")
+    from mdforce._lib import _SIGS
+    subprocess.check_call(["make", "-s", "-j8", "-C", CSRC], stdout=subprocess.DEVNULL)
+    d = tmp_path_factory.mktemp("fake")
+    inc = os.path.join(os.path.dirname(os.path.dirname(shutil.which("nvcc"))), "include")
+    subprocess.check_call(["gcc", "-O1", "-fPIC", "-I" + inc, "-c", os.path.join(HERE, "fake_cudart.c"), "-o", d / "rt.o"])
+    objs = sorted(os.path.join(CSRC, "_build", f) for f in os.listdir(os.path.join(CSRC, "_build")) if f.endswith(".o"))
+    subprocess.check_call(["g++", "-shared", "-Wl,-Bsymbolic", "-o", d / "libfake.so", *objs, d / "rt.o", "-lpthread"])
+    lib = C.CDLL(str(d / "libfake.so"))
+    for name, (res, args) in _SIGS.items():
+        getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
+    for name, res in (("fake_calls", C.c_long), ("fake_live", C.c_long), ("fake_pinned", C.c_long),
+                      ("fake_pageable_dtoh", C.c_long), ("fake_launch_name", C.c_char_p), ("fake_lowered", C.c_char_p)):
+        getattr(lib, name).restype = res
+    lib.fake_fail_at.argtypes = [C.c_long]
+    lib.fake_limit.argtypes = [C.c_char_p, C.c_int]
+    return lib
+
+
+@pytest.fixture
+def lib(rt):
+    rt.fake_reset()
+    assert rt.fake_live() == 0
+    yield rt
+    rt.fake_reset()
+    assert rt.fake_live() == 0
+
+
+def dbl(a):
+    return a.ctypes.data_as(C.POINTER(C.c_double))
+
+
+def vec(t, *v):
+    return (t * len(v))(*v)
+
+
+def new_system(lib, n=64, device=0, box=8.0):
+    pos, h = np.zeros((n, 3)), C.c_void_p()
+    q = np.ones(n)
+    assert lib.md_system_create(C.byref(h), n, vec(C.c_double, box, box, box), dbl(pos), None, None, dbl(q), None, 1,
+                                device) == 0, lib.md_last_error_message()
+    return h
+
+
+def make_map(lib, K, kind="ik"):
+    h = C.c_void_p()
+    KK, LL = vec(C.c_int, *K), vec(C.c_double, 8.0, 8.0, 8.0)
+    if kind == "ik":
+        rc = lib.md_errmap_create(C.byref(h), KK, LL, 1.0, 6, 0)
+    elif kind == "ana":
+        rc = lib.md_errmap_create_ana(C.byref(h), KK, LL, 1.0, 6, 0)
+    else:
+        rc = lib.md_errmap_create_dir(C.byref(h), KK, LL, 1.0, 3.0, 0)
+    return rc, h
+
+
+@pytest.mark.parametrize("kind", ["ik", "ana", "dir"])
+def test_error_is_reported_once(lib, kind):
+    """after a map that memory does not hold, the next one is made"""
+    lib.fake_fail_at(1)  # the arrays' allocation (0: the stream)
+    assert make_map(lib, (16, 16, 16), kind)[0] != 0
+    assert b"out of memory" in lib.md_last_error_message()
+    lib.fake_fail_at(NO_FAILURE)
+    rc, h = make_map(lib, (8, 8, 8), kind)
+    assert rc == 0, lib.md_last_error_message()
+    lib.md_errmap_destroy(h)
