@@ -719,7 +719,7 @@ extern "C" int md_errmap_create(md_errmap** out, const int K[3], const double L[
   const EmAcc acc = {{h->cnt, h->cnt + N, (double*)(h->work + 3 * N)}};
   k_em_alias_tab<<<dim3(ceil_div(Kmax, 64), 3), 64, 0, s>>>(h->g, order, EM_KCUT_IK, Kmax, tab);
   k_em_ig<<<nb, 256, 0, s>>>(h->g, beta, S);
-  MD_CHECK_LAUNCH("errmap start");
+  if (const cudaError_t e = cudaGetLastError()) return done(md_cuda_fail(e, "errmap start"));
   if (int r = dft3_axis(S, T, K, 0, +1, 3, s)) return done(r);  // x, y: direction z
   if (int r = dft3_axis(T, T, K, 1, +1, 3, s)) return done(r);
   if (int r = em_alias_dir(h, 2, T, tab, Kmax, 1, W, acc, tmp)) return done(r);
@@ -731,7 +731,7 @@ extern "C" int md_errmap_create(md_errmap** out, const int K[3], const double L[
   k_em_k2<<<nb, 256, 0, s>>>(h->g, W, acc, h->k2a);
   k_em_ig<<<nb, 256, 0, s>>>(h->g, beta, S);
   k_em_k1<<<nb, 256, 0, s>>>(h->g, S, tab, Kmax, nk, h->k1);
-  MD_CHECK_LAUNCH("errmap kernels");
+  if (const cudaError_t e = cudaGetLastError()) return done(md_cuda_fail(e, "errmap kernels"));
   if (int r = dft3_grid(h->k2a, K, -1, 1, s)) return done(r);
   cudaError_t e = cudaMemsetAsync(h->rho, 0, sizeof(double) * 4 * N, s);  // rho and cnt
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -784,13 +784,13 @@ extern "C" int md_errmap_create_dir(md_errmap** out, const int K[3], const doubl
   };
   if (!ok) return fail(md_cuda_fail(cudaGetLastError(), "md_errmap_create_dir allocation"));
   cudaStream_t s = h->stream;
-  MD_CUDA(cudaMemsetAsync(h->cnt, 0, sizeof(double) * 2 * N, s));
-  MD_CUDA(cudaMemsetAsync(h->rho, 0, sizeof(double) * 2 * N, s));
-  MD_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned), s));
+  cudaError_t e = cudaMemsetAsync(h->rho, 0, sizeof(double) * 4 * N, s);  // rho and cnt
+  if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, sizeof(unsigned), s);
+  if (e != cudaSuccess) return fail(md_cuda_fail(e, "md_errmap_create_dir start"));
   const int oct = (K[0] / 2 + 1) * (K[1] / 2 + 1) * (K[2] / 2 + 1);
   k_em_dir_tables<<<ceil_div(oct, 64), 64, 0, s>>>(h->g, beta, rcut, h->k1, h->k2a, flag);
   unsigned hf = 0;
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(&hf, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail(md_cuda_fail(e, "md_errmap_create_dir kernel"));
@@ -860,9 +860,9 @@ extern "C" int md_errmap_create_ana(md_errmap** out, const int K[3], const doubl
   if (!ok) return fail(md_cuda_fail(cudaGetLastError(), "md_errmap_create_ana allocation"));
   cudaStream_t s = h->stream;
   const unsigned nb = (unsigned)((N + 255) / 256);
-  MD_CUDA(cudaMemsetAsync(k2b, 0, sizeof(double2) * N, s));
-  MD_CUDA(cudaMemsetAsync(h->cnt, 0, sizeof(double) * 2 * N, s));
-  MD_CUDA(cudaMemsetAsync(h->rho, 0, sizeof(double) * 2 * N, s));
+  cudaError_t e = cudaMemsetAsync(h->rho, 0, sizeof(double) * 4 * N, s);  // rho and cnt
+  if (e == cudaSuccess) e = cudaMemsetAsync(k2b, 0, sizeof(double2) * N, s);
+  if (e != cudaSuccess) return fail(md_cuda_fail(e, "md_errmap_create_ana start"));
   k_em_g<<<nb, 256, 0, s>>>(h->g, beta, gm, fm);
   k_ema_selfsum<<<NSELF, 256, 0, s>>>(h->g, order, EM_KCUT_ANA, fm, selfs);
   for (int k = -EM_KCUT_ANA; k <= EM_KCUT_ANA; ++k) {
@@ -883,7 +883,7 @@ extern "C" int md_errmap_create_ana(md_errmap** out, const int K[3], const doubl
   if (int r = dft3_grid(k2b, h->g.K, -1, 1, s)) return fail(r);
   k_em_axpy<<<nb, 256, 0, s>>>(N, h->k2a, k2b, 1.0);
   double hs[NSELF];
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(hs, selfs, sizeof(hs), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail(md_cuda_fail(e, "md_errmap_create_ana kernel"));

@@ -84,3 +84,31 @@ def test_error_is_reported_once(lib, kind):
     rc, h = make_map(lib, (8, 8, 8), kind)
     assert rc == 0, lib.md_last_error_message()
     lib.md_errmap_destroy(h)
+
+
+def with_each_call_failing(lib, op):
+    """op() once as it is, then once for each of its CUDA calls with that call failing"""
+    lib.fake_fail_at(NO_FAILURE)
+    op()
+    n = lib.fake_calls()
+    for k in range(n):
+        lib.fake_fail_at(k)
+        op()
+        lib.fake_fail_at(NO_FAILURE)
+        yield k
+
+
+@pytest.mark.parametrize("kind", ["ik", "ana", "dir"])
+@pytest.mark.parametrize("K", [(8, 8, 8), (8, 9, 12)])
+def test_failed_map_leaves_nothing(lib, kind, K):
+    """no memory, stream or pool reference stays after a map's creation fails at any of its calls"""
+    def op():
+        rc, h = make_map(lib, K, kind)
+        if rc == 0:
+            lib.md_errmap_destroy(h)
+
+    for k in with_each_call_failing(lib, op):
+        assert lib.fake_live() == 0, k
+    trims = lib.fake_trims()
+    op()
+    assert lib.fake_trims() == trims + 1  # the last user of the pool leaves: none of the failures kept a reference
