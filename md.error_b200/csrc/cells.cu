@@ -216,14 +216,12 @@ extern "C" int md_cell_list_get_cell_index(md_cell_list* cl, md_system* sys, uin
   if (!cl || !sys || !cell) return MD_ERR_BADARG;
   if (!cl->built) { md_set_error("cell list not built"); return MD_ERR_BADARG; }
   size_t bytes = sizeof(uint32_t) * sys->N;
-  void* buf;
-  bool owned;
-  if (int r = sys_scratch(sys, bytes, &buf, &owned)) return r;
-  uint32_t* d = (uint32_t*)buf;
+  SysScratch buf;
+  if (int r = buf.take(sys, bytes)) return r;
+  uint32_t* d = (uint32_t*)buf.p;
   k_cell_out<<<ceil_div(sys->N, 256), 256, 0, sys->stream>>>(sys->N, cl->cell_of, sys->id, d);
   MD_CHECK_LAUNCH("cell out");
   MD_CUDA(cudaMemcpyAsync(cell, d, bytes, cudaMemcpyDeviceToHost, sys->stream));
-  if (int r = sys_scratch_done(sys, buf, owned)) return r;
   MD_CUDA(cudaStreamSynchronize(sys->stream));
   return MD_OK;
 }

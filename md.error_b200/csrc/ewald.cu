@@ -245,10 +245,9 @@ extern "C" int md_ewald_exact(md_system* sys, const int K[3], double beta, doubl
   const size_t b_coef = sizeof(double4a) * (size_t)nm, b_tab = sizeof(double2) * (size_t)ntab * nmax,
                b_part = sizeof(double) * 4 * (size_t)ns * nm, b_f = sizeof(double) * 3 * (size_t)nf * nmax,
                b_red = sizeof(double) * ((size_t)nbc + 4);
-  void* buf;
-  bool owned;
-  if (int r = sys_scratch(sys, b_coef + b_tab + b_part + b_f + b_red, &buf, &owned)) return r;
-  char* p = (char*)buf;
+  SysScratch buf;
+  if (int r = buf.take(sys, b_coef + b_tab + b_part + b_f + b_red)) return r;
+  char* p = (char*)buf.p;
   double4a* coef = (double4a*)p;
   double2* tab = (double2*)(p += b_coef);
   double* part = (double*)(p += b_tab);
@@ -282,7 +281,6 @@ extern "C" int md_ewald_exact(md_system* sys, const int K[3], double beta, doubl
   }
   double h = 0;
   MD_CUDA(cudaMemcpyAsync(&h, e, sizeof(double), cudaMemcpyDeviceToHost, s));
-  if (int r = sys_scratch_done(sys, buf, owned)) return r;
   MD_CUDA(cudaStreamSynchronize(s));
   if (energy) *energy = h;
   return MD_OK;

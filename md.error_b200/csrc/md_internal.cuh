@@ -116,7 +116,7 @@ struct md_system {
   // pinned host staging
   void* h_stage = nullptr;
   size_t h_stage_bytes = 0;
-  // device staging of the calls that copy to or from the host (sys_scratch)
+  // device staging of the calls that copy to or from the host (SysScratch)
   void* d_stage = nullptr;
   bool pooled = false;  // holds a reference on the device's pool
   size_t d_stage_bytes = 0;
@@ -198,17 +198,24 @@ struct md_engine {
 // per-atom correction values (by atom id) of an md_fcorr
 const double4a* fcorr_values(const md_fcorr* f);
 
-// Device workspace of one host-synchronising call on the system's stream:
-// *p holds `bytes` until the next sys_scratch of this system, or until
-// sys_scratch_done when *owned is set.  Up to SYS_SCRATCH_KEEP the system keeps
+// Device workspace of one host-synchronising call on the system's stream: p
+// holds the bytes taken for as long as the object lives and no other takes
+// memory of the same system.  Up to SYS_SCRATCH_KEEP the system keeps
 // the buffer and frees it when it is destroyed: a stream-ordered allocation
 // per call had the pool return its memory at every synchronisation and map it
 // again, about 250 us of host time for 1.5 MB (frames of the 4,000-atom fluid
 // read after 50 steps: two such calls in 2.0 ms).  Larger requests are
-// allocated and freed with the call.
+// allocated with the call and freed with the object, on every way out of it.
 constexpr size_t SYS_SCRATCH_KEEP = 64u << 20;
-int sys_scratch(md_system* s, size_t bytes, void** p, bool* owned);
-int sys_scratch_done(md_system* s, void* p, bool owned);
+struct SysScratch {
+  void* p = nullptr;
+  md_system* owner = nullptr;  // of memory taken for this call alone
+  SysScratch() = default;
+  SysScratch(const SysScratch&) = delete;
+  SysScratch& operator=(const SysScratch&) = delete;
+  int take(md_system* s, size_t bytes);
+  ~SysScratch();
+};
 // n device arrays to host memory through a page-locked buffer, and
 // the wait for them: a copy to pageable memory is staged by the driver piece
 // by piece (5.4 MB of the cutoff map: 1.1 ms against 0.1 ms and the copies)

@@ -1201,10 +1201,9 @@ __global__ void k_max_disp(int N, const typename V4<R>::T* pos, const typename V
 extern "C" int md_nlist_max_displacement(md_nlist* nl, md_system* sys, double* out) {
   if (!nl || !sys || !out) return MD_ERR_BADARG;
   if (!nl->built) { md_set_error("list not built"); return MD_ERR_BADARG; }
-  void* buf;
-  bool owned;
-  if (int r = sys_scratch(sys, sizeof(double), &buf, &owned)) return r;
-  double* d = (double*)buf;
+  SysScratch buf;
+  if (int r = buf.take(sys, sizeof(double))) return r;
+  double* d = (double*)buf.p;
   MD_CUDA(cudaMemsetAsync(d, 0, sizeof(double), sys->stream));
   int nb = ceil_div(sys->N, 256);
   if (sys->prec == MD_PREC_FP64)
@@ -1214,7 +1213,6 @@ extern "C" int md_nlist_max_displacement(md_nlist* nl, md_system* sys, double* o
   MD_CHECK_LAUNCH("max disp");
   double h = 0;
   MD_CUDA(cudaMemcpyAsync(&h, d, sizeof(double), cudaMemcpyDeviceToHost, sys->stream));
-  if (int r = sys_scratch_done(sys, buf, owned)) return r;
   MD_CUDA(cudaStreamSynchronize(sys->stream));
   *out = sqrt(h);
   return MD_OK;

@@ -291,11 +291,10 @@ int pool_alloc(int device, size_t bytes, cudaStream_t stream, void** p) {
 
 void pool_free(int, void* p, cudaStream_t stream) { cudaFreeAsync(p, stream); }
 
-int sys_scratch(md_system* s, size_t bytes, void** p, bool* owned) {
-  *p = nullptr;
-  *owned = bytes > SYS_SCRATCH_KEEP;
-  if (*owned) {
-    MD_CUDA(cudaMallocAsync(p, bytes, s->stream));
+int SysScratch::take(md_system* s, size_t bytes) {
+  if (bytes > SYS_SCRATCH_KEEP) {
+    MD_CUDA(cudaMallocAsync(&p, bytes, s->stream));
+    owner = s;
     return MD_OK;
   }
   if (s->d_stage_bytes < bytes) {
@@ -306,13 +305,12 @@ int sys_scratch(md_system* s, size_t bytes, void** p, bool* owned) {
     if (int r = pool_alloc(s->device, bytes, s->stream, &s->d_stage)) return r;
     s->d_stage_bytes = bytes;
   }
-  *p = s->d_stage;
+  p = s->d_stage;
   return MD_OK;
 }
 
-int sys_scratch_done(md_system* s, void* p, bool owned) {
-  if (owned && p) MD_CUDA(cudaFreeAsync(p, s->stream));
-  return MD_OK;
+SysScratch::~SysScratch() {
+  if (owner) cudaFreeAsync(p, owner->stream);
 }
 
 // Page-locked memory for one read-back: the device's shared buffer (grown up
@@ -563,10 +561,9 @@ static int download(md_system* s, int what, double* out) {
   if (int r = check_sys(s)) return r;
   if (!out) return MD_ERR_BADARG;
   size_t bytes = sizeof(double) * 3 * (size_t)s->N;
-  void* buf;
-  bool owned;
-  if (int r = sys_scratch(s, bytes, &buf, &owned)) return r;
-  double* d = (double*)buf;
+  SysScratch buf;
+  if (int r = buf.take(s, bytes)) return r;
+  double* d = (double*)buf.p;
   int nb = ceil_div(s->N, 256);
   if (s->prec == MD_PREC_FP64)
     k_download<double><<<nb, 256, 0, s->stream>>>(s->N, what, (double4a*)s->pos, (double4a*)s->vel, s->force, s->image, s->id, s->st, d);
@@ -575,9 +572,7 @@ static int download(md_system* s, int what, double* out) {
   MD_CHECK_LAUNCH("download");
   void* dst[1] = {out};
   const void* src[1] = {d};
-  const int r = sys_read_back(s, s->stream, dst, src, &bytes, 1);
-  if (int q = sys_scratch_done(s, buf, owned)) return q;
-  return r;
+  return sys_read_back(s, s->stream, dst, src, &bytes, 1);
 }
 
 static int upload_vec(md_system* s, int what, const double* in) {
@@ -589,10 +584,9 @@ static int upload_vec(md_system* s, int what, const double* in) {
   if (int r = ensure_stage(s, bytes)) return r;
   MD_CUDA(cudaStreamSynchronize(s->stream));
   memcpy(s->h_stage, in, bytes);
-  void* buf;
-  bool owned;
-  if (int r = sys_scratch(s, bytes, &buf, &owned)) return r;
-  double* d = (double*)buf;
+  SysScratch buf;
+  if (int r = buf.take(s, bytes)) return r;
+  double* d = (double*)buf.p;
   MD_CUDA(cudaMemcpyAsync(d, s->h_stage, bytes, cudaMemcpyHostToDevice, s->stream));
   int nb = ceil_div(s->N, 256);
   if (s->prec == MD_PREC_FP64)
@@ -600,7 +594,6 @@ static int upload_vec(md_system* s, int what, const double* in) {
   else
     k_set_vec<float><<<nb, 256, 0, s->stream>>>(s->N, what, d, s->id, (float4*)s->pos, (float4*)s->vel);
   MD_CHECK_LAUNCH("set vec");
-  if (int r = sys_scratch_done(s, buf, owned)) return r;
   MD_CUDA(cudaStreamSynchronize(s->stream));
   return MD_OK;
 }
@@ -624,10 +617,9 @@ static int charge_io(md_system* s, int dir, double* q, int what = 0) {
   const size_t bytes = sizeof(double) * (size_t)s->N;
   if (int r = ensure_stage(s, bytes)) return r;
   MD_CUDA(cudaStreamSynchronize(s->stream));
-  void* buf;
-  bool owned;
-  if (int r = sys_scratch(s, bytes, &buf, &owned)) return r;
-  double* d = (double*)buf;
+  SysScratch buf;
+  if (int r = buf.take(s, bytes)) return r;
+  double* d = (double*)buf.p;
   if (dir == 0) {
     memcpy(s->h_stage, q, bytes);
     MD_CUDA(cudaMemcpyAsync(d, s->h_stage, bytes, cudaMemcpyHostToDevice, s->stream));
@@ -645,7 +637,6 @@ static int charge_io(md_system* s, int dir, double* q, int what = 0) {
   }
   MD_CHECK_LAUNCH("charge / mass io");
   if (dir == 1) MD_CUDA(cudaMemcpyAsync(s->h_stage, d, bytes, cudaMemcpyDeviceToHost, s->stream));
-  if (int r = sys_scratch_done(s, buf, owned)) return r;
   MD_CUDA(cudaStreamSynchronize(s->stream));
   if (dir == 1) memcpy(q, s->h_stage, bytes);
   return MD_OK;
@@ -695,15 +686,13 @@ static int rcut_io(md_system* s, int dir, float* host) {
   if (int r = check_sys(s)) return r;
   if (!host) return MD_ERR_BADARG;
   size_t bytes = sizeof(float) * s->N;
-  void* buf;
-  bool owned;
-  if (int r = sys_scratch(s, bytes, &buf, &owned)) return r;
-  float* d = (float*)buf;
+  SysScratch buf;
+  if (int r = buf.take(s, bytes)) return r;
+  float* d = (float*)buf.p;
   if (dir == 0) MD_CUDA(cudaMemcpyAsync(d, host, bytes, cudaMemcpyHostToDevice, s->stream));
   k_rcut_io<<<ceil_div(s->N, 256), 256, 0, s->stream>>>(s->N, dir, s->rcut, s->id, d);
   MD_CHECK_LAUNCH("rcut io");
   if (dir == 1) MD_CUDA(cudaMemcpyAsync(host, d, bytes, cudaMemcpyDeviceToHost, s->stream));
-  if (int r = sys_scratch_done(s, buf, owned)) return r;
   MD_CUDA(cudaStreamSynchronize(s->stream));
   return MD_OK;
 }

@@ -112,3 +112,35 @@ def test_failed_map_leaves_nothing(lib, kind, K):
     trims = lib.fake_trims()
     op()
     assert lib.fake_trims() == trims + 1  # the last user of the pool leaves: none of the failures kept a reference
+
+
+BIG = 3 << 20  # atoms whose positions take more than the scratch a system keeps (64 MB)
+
+
+@pytest.mark.parametrize("call", ["positions", "set_positions", "charges", "rcut", "ewald"])
+def test_failed_call_leaves_no_scratch(lib, call):
+    """workspace taken for one call is freed when any later call in it fails"""
+    n = {"charges": 9 << 20, "rcut": 17 << 20, "ewald": 64}.get(call, BIG)
+    h = new_system(lib, n)
+    buf = np.zeros(3 * n)
+    f32 = np.zeros(n, np.float32)
+    e = C.c_double()
+    K = vec(C.c_int, 2, 1024, 2048)
+
+    def op():
+        if call == "positions":
+            lib.md_system_get_positions(h, dbl(buf))
+        elif call == "set_positions":
+            lib.md_system_set_positions(h, dbl(buf))
+        elif call == "charges":
+            lib.md_system_get_charges(h, dbl(buf))
+        elif call == "rcut":
+            lib.md_system_get_rcut(h, f32.ctypes.data_as(C.POINTER(C.c_float)))
+        else:
+            lib.md_ewald_exact(h, K, 1.0, C.byref(e), 1)
+
+    op()
+    held = lib.fake_live()
+    for k in with_each_call_failing(lib, op):
+        assert lib.fake_live() == held, k
+    lib.md_system_destroy(h)
