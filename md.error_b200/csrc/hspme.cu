@@ -608,6 +608,11 @@ static bool hs_alloc(md_hspme* h, long B) {
          cudaMalloc(&h->R, sizeof(double) * B * 3 * h->N) == cudaSuccess;
 }
 
+// stencil widths 2 ceil(CC)
+#define HS_WIDTHS(X) X(2) X(4) X(6) X(8) X(10) X(12) X(14) X(16)
+
+static int hs_gather_prepare(int S);
+
 extern "C" int md_hspme_create(md_hspme** out, int natoms, const int K[3], const double L[3], double beta, double CC,
                                int nbin, int bound0, int device) {
   if (!out || natoms < 1 || !K || !L || !(beta > 0) || !(CC > 0) || nbin < 1 || nbin > HS_MAX_NBIN) {
@@ -622,6 +627,7 @@ extern "C" int md_hspme_create(md_hspme** out, int natoms, const int K[3], const
       return MD_ERR_BADARG;
     }
   MD_CUDA(cudaSetDevice(device));
+  if (int r = hs_gather_prepare(2 * half)) return r;
   md_hspme* h = new md_hspme();
   h->device = device;
   h->N = natoms;
@@ -669,9 +675,6 @@ extern "C" int md_hspme_num_coeffs(md_hspme* h, int* out) {
   return MD_OK;
 }
 
-// stencil widths 2 ceil(CC)
-#define HS_WIDTHS(X) X(2) X(4) X(6) X(8) X(10) X(12) X(14) X(16)
-
 template <int MODE>
 static int hs_spread(md_hspme* h, int nb, const double* q, const double* r, const double* c, cudaStream_t s) {
   double* re = reinterpret_cast<double*>(h->F + (long)nb * h->g.Kt);
@@ -687,20 +690,40 @@ static int hs_spread(md_hspme* h, int nb, const double* q, const double* r, cons
   return MD_OK;
 }
 
+// a block's coefficient sums
+static constexpr size_t hs_csum_bytes(int S, int ncoef) { return sizeof(double) * hs_warps(S) * HS_COPIES * ncoef; }
+
+// The gathers may take the sums of any coefficient count: the limit belongs to
+// the kernel, not to a handle, so one of fewer coefficients must not lower it
+// between another's setting and launch.
+static int hs_gather_prepare(int S) {
+  const void* f[2] = {nullptr, nullptr};
+  switch (S) {
+#define HS_CASE(W)                            \
+  case W:                                     \
+    f[0] = (const void*)k_hs_gather<W, 0>;    \
+    f[1] = (const void*)k_hs_gather<W, 2>;    \
+    break;
+    HS_WIDTHS(HS_CASE)
+#undef HS_CASE
+  }
+  for (const void* k : f) {
+    if (!k) continue;  // a support of no width has no stencil
+    MD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs_csum_bytes(S, HS_MAX_COEF)));
+  }
+  return MD_OK;
+}
+
 template <int MODE>
 static int hs_gather(md_hspme* h, int nb, const double* q, const double* r, const double* c, const double* fref,
                      const HsOut& out, cudaStream_t s) {
   const double2* f2 = h->F + (long)nb * h->g.Kt;
   switch (h->g.S) {
 #define HS_CASE(W)                                                                                               \
-  case W: {                                                                                                      \
-    const size_t dyn = out.cpart ? sizeof(double) * hs_warps(W) * HS_COPIES * h->g.ncoef : 0;                      \
-    if (dyn > 4096)                                                                                                \
-      MD_CUDA(cudaFuncSetAttribute(k_hs_gather<W, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));  \
-    k_hs_gather<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), dyn, s>>>(h->g, h->N, q, r, c, h->F, f2, h->e2,     \
-                                                                      h->w, fref, h->R, h->lpart, out);            \
-    break;                                                                                                         \
-  }
+  case W:                                                                                                        \
+    k_hs_gather<W, MODE><<<dim3(h->nab, nb), 32 * hs_warps(W), out.cpart ? hs_csum_bytes(W, h->g.ncoef) : 0, s>>>( \
+        h->g, h->N, q, r, c, h->F, f2, h->e2, h->w, fref, h->R, h->lpart, out);                                    \
+    break;
     HS_WIDTHS(HS_CASE)
 #undef HS_CASE
   }

@@ -16,7 +16,7 @@
 enum { DEVICE_MEM, POOL_MEM, PINNED_MEM };
 
 static struct { char* p; size_t bytes; int kind; } blocks[MAX_BLOCKS];
-static struct { const void* f; const char* name; int limit[DEVICES]; int lowered; } funcs[MAX_FUNCS];
+static struct { const void* f; const char* name; int limit[DEVICES], used[DEVICES], lowered; } funcs[MAX_FUNCS];
 static struct { int func, device; size_t smem; } launches[MAX_LOG];
 static int nblocks, nfuncs, nlaunches, streams, trims;
 static size_t pageable_dtoh;
@@ -80,6 +80,7 @@ static cudaError_t launch(const void* f, dim3 g, dim3 b, size_t smem) {
     return fail(cudaErrorInvalidConfiguration);
   if (smem > (size_t)funcs[k].limit[device]) return fail(cudaErrorInvalidValue);
   pthread_mutex_lock(&mutex);
+  if ((int)smem > funcs[k].used[device]) funcs[k].used[device] = (int)smem;
   if (nlaunches < MAX_LOG) {
     launches[nlaunches].func = k;
     launches[nlaunches].device = device;
@@ -109,7 +110,7 @@ long fake_pageable_dtoh(void) { return (long)pageable_dtoh; }
 int fake_trims(void) { return trims; }
 int fake_launches(void) { return nlaunches; }
 const char* fake_launch_name(int k) { return funcs[launches[k].func].name; }
-/* kernels whose shared-memory limit was lowered below one in force */
+/* a kernel whose shared-memory limit was taken below what it has been launched with */
 const char* fake_lowered(void) {
   for (int k = 0; k < nfuncs; ++k)
     if (funcs[k].lowered) return funcs[k].name;
@@ -161,8 +162,8 @@ cudaError_t cudaFuncSetAttribute(const void* f, enum cudaFuncAttribute attr, int
   if (k < 0) return fail(cudaErrorInvalidDeviceFunction);
   if (attr == cudaFuncAttributeMaxDynamicSharedMemorySize) {
     if (v > 227 * 1024) return fail(cudaErrorInvalidValue);
-    if (v < funcs[k].limit[device] && funcs[k].limit[device] > 48 * 1024) funcs[k].lowered = 1;
-    funcs[k].limit[device] = v > 48 * 1024 ? v : 48 * 1024;
+    if (v < funcs[k].used[device]) funcs[k].lowered = 1;
+    funcs[k].limit[device] = v;
   }
   return cudaSuccess;
 }

@@ -144,3 +144,25 @@ def test_failed_call_leaves_no_scratch(lib, call):
     for k in with_each_call_failing(lib, op):
         assert lib.fake_live() == held, k
     lib.md_system_destroy(h)
+
+
+def hermite(lib, nbin, CC=4.0, n=8):
+    h = C.c_void_p()
+    assert lib.md_hspme_create(C.byref(h), n, vec(C.c_int, 12, 12, 12), vec(C.c_double, 8.0, 8.0, 8.0), 1.0, CC, nbin,
+                               0, 0) == 0
+    return h
+
+
+@pytest.mark.parametrize("CC", [1.0, 4.0, 5.0])
+def test_hermite_handles_keep_their_shared_memory(lib, CC):
+    """handles of one stencil width and different coefficient counts, used in turn: neither takes
+    the kernels' shared-memory limit below what the other one launches with"""
+    big, small = hermite(lib, 64, CC), hermite(lib, 40, CC)
+    buf = np.zeros(4096)
+    p = buf.ctypes.data
+    for h in (big, small, big):
+        assert lib.md_hspme_energy(h, p, p, p, 1, p, p, p, p, p, None) == 0
+        assert lib.md_hspme_force_error(h, p, p, p, 1, p, p, p, p, p, None) == 0
+        assert lib.fake_lowered() is None
+    lib.md_hspme_destroy(big)
+    lib.md_hspme_destroy(small)
