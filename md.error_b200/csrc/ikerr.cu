@@ -358,7 +358,10 @@ extern "C" int md_ikerr_create(md_ikerr** out, const int K[3], const double L[3]
     return MD_ERR_BADARG;
   }
   h->smem = smem;
-  bool ok = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) == cudaSuccess;
+  // the kernel's own limit, not this mesh's size: it holds for every functional of the device
+  bool ok = cudaFuncSetAttribute(k_ikerr_eval, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IK_SMEM_LIMIT) ==
+                cudaSuccess &&
+            cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) == cudaSuccess;
   for (int d = 0; d < 3 && ok; ++d)
     ok = cudaMalloc(&h->hats[d], sizeof(double) * (1 + h->ncoef) * (h->kmax[d] + 1)) == cudaSuccess &&
          cudaMalloc(&h->W[d], sizeof(double) * (K[d] + 1)) == cudaSuccess;
@@ -367,8 +370,6 @@ extern "C" int md_ikerr_create(md_ikerr** out, const int K[3], const double L[3]
     delete h;
     return md_cuda_fail(cudaGetLastError(), "md_ikerr_create allocation");
   }
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_ikerr_eval, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   // hats of every basis function along each axis
   for (int d = 0; d < 3; ++d) {
     IkBasis B;

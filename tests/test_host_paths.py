@@ -166,3 +166,23 @@ def test_hermite_handles_keep_their_shared_memory(lib, CC):
         assert lib.fake_lowered() is None
     lib.md_hspme_destroy(big)
     lib.md_hspme_destroy(small)
+
+
+def functional(lib, k):
+    h = C.c_void_p()
+    assert lib.md_ikerr_create(C.byref(h), vec(C.c_int, k, k, k), vec(C.c_double, 30.0, 30.0, 30.0), 0.95, 2.0, 4, 10,
+                               0, 100, 100.0, 100.0, 0) == 0, lib.md_last_error_message()
+    return h
+
+
+def test_functionals_keep_their_shared_memory(lib):
+    """a functional of a smaller mesh made later does not take the limit that a larger one launches with"""
+    big = functional(lib, 256)
+    c, v, g = np.zeros(8), np.zeros(1), np.zeros(8)
+    assert lib.md_ikerr_evaluate(big, 1, dbl(c), dbl(v), dbl(g)) == 0
+    small = functional(lib, 224)
+    assert lib.fake_lowered() is None
+    for h in (small, big):
+        assert lib.md_ikerr_evaluate(h, 1, dbl(c), dbl(v), dbl(g)) == 0, lib.md_last_error_message()
+    lib.md_ikerr_destroy(big)
+    lib.md_ikerr_destroy(small)
