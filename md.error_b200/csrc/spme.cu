@@ -766,6 +766,7 @@ static PlaneChain plane_args(md_spme* s, int method) {
   p.partials = s->partials;
   p.with_stats = 1;
   p.merge = 0;
+  p.back = 1;
   p.energy = p.dbeta = nullptr;
   return p;
 }
@@ -846,6 +847,7 @@ static int spme_energy_grad(md_spme* s, double* energy, double* dq, double* dr, 
   if (planes) {
     // energy and dE/dbeta leave the plane pass for their device outputs
     PlaneChain p = plane_args(s, 2);
+    p.back = dq || dr;
     if (dev) {
       p.energy = energy;
       p.dbeta = dbeta;

@@ -148,14 +148,14 @@ constexpr size_t plane_smem() {
 
 // METHOD 0: C[1] = -2 pi i m_x psi Q^, C[2] = -2 pi i m_y psi Q^, C[3] = psi Q^;
 // 1: C[1] = psi Q^ / 2 (FBSpline normalisation); 2: C[1] = psi Q^; each
-// transformed back along x and y.  psi = exp(-pi^2 m^2 / beta^2) / m^2
+// transformed back along x and y (2: only with back).  psi = exp(-pi^2 m^2 / beta^2) / m^2
 // |b0|^2 |b1|^2 |b2|^2 / (pi V) (calB / calPsiFPhiF) from factors per axis, for the
 // current box.  The energy E = 1/2 sum psi |Q^|^2 with the diagonal virial
 // (METHODS 0, 1) or dE/dbeta (2) is reduced in FP64.
 template <class R, int LOGN, int METHOD>
 __global__ void __launch_bounds__(PlaneGeom<LOGN>::T)
 k_spme_plane(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, const double* __restrict__ bm, int K2,
-             double beta, DevState* st, double* partials, int with_stats, int merge, double* energy, double* dbeta) {
+             double beta, DevState* st, double* partials, int with_stats, int merge, int back, double* energy, double* dbeta) {
   typedef PlaneGeom<LOGN> P;
   typedef typename C2<R>::T T2;
   constexpr int n = P::n, T = P::T, EPT = P::EPT, NS = METHOD == 0 ? EPT : 1;
@@ -231,7 +231,7 @@ k_spme_plane(typename C2<R>::T* C, const typename C2<R>::T* __restrict__ twg, co
     }
   }
   __syncthreads();
-  if (first) {
+  if (first && (METHOD != 2 || back)) {
     plane_inverse<R, LOGN, 1>(X, tw);
     plane_inverse<R, LOGN, 0>(X, tw);
 #pragma unroll
@@ -533,11 +533,12 @@ int plane_chain(md_system* sys, const PlaneChain& p, Recorder* rec) {
   }
   {
     const Kernel k = plane_kernel(prec, p.n, p.method);
-    void* args[] = {&a.C, &a.tw_n, &a.bm, &a.K2, &a.beta, &st, &a.partials, &a.with_stats, &a.merge, &a.energy, &a.dbeta};
+    void* args[] = {&a.C, &a.tw_n, &a.bm, &a.K2, &a.beta, &st, &a.partials, &a.with_stats, &a.merge, &a.back, &a.energy, &a.dbeta};
     const int planes = p.K2 / 2 + 1;
     if (int r = rec_launch(rec, k.f, dim3(planes, ik && 2 * planes <= 148 ? 2 : 1), dim3(k.threads), k.smem, args))
       return r;
   }
+  if (!p.back) return MD_OK;
   const Kernel k = z_pass(prec, p.K2, 1, ik);
   void* args[] = {&c1, &a.G, &a.tw_z, &nlines, &st};
   return rec_launch(rec, k.f, dim3((unsigned)(nlines / k.lines)), dim3(k.threads), k.smem, args);

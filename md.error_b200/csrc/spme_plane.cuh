@@ -14,11 +14,12 @@ struct PlaneChain {
   double beta;
   double* partials;
   int with_stats, merge;
+  int back;              // 0: the adjoint ends with the k-space step (energy and dE/dbeta alone)
   double *energy, *dbeta;  // adjoint: device results (may be null)
 };
 
 // whether the chain's transforms run by planes
 bool plane_chain_ok(int prec, const int K[3]);
 int plane_prepare(int prec, const int K[3], int method);
-// z forward, plane, z backward
+// z forward, plane, z backward (with back)
 int plane_chain(md_system* sys, const PlaneChain& p, Recorder* rec);

@@ -186,3 +186,30 @@ def test_functionals_keep_their_shared_memory(lib):
         assert lib.md_ikerr_evaluate(h, 1, dbl(c), dbl(v), dbl(g)) == 0, lib.md_last_error_message()
     lib.md_ikerr_destroy(big)
     lib.md_ikerr_destroy(small)
+
+
+@pytest.mark.parametrize("K", [(16, 16, 32), (32, 16, 16)])
+@pytest.mark.parametrize("device_outputs", [False, True])
+def test_energy_alone_is_not_transformed_back(lib, K, device_outputs):
+    """an SPME energy without gradients ends with the k-space step, on meshes that run by planes too"""
+    s, sp = new_system(lib), C.c_void_p()
+    assert lib.md_spme_create(C.byref(sp), s, vec(C.c_int, *K), 4, 1.0, 0) == 0
+    out, grad = np.zeros(2), np.zeros(3 * 64)
+
+    def launched(gradient):
+        n = lib.fake_launches()
+        if device_outputs:
+            assert lib.md_spme_energy_grad_device(sp, s, out.ctypes.data, None, grad.ctypes.data if gradient else None,
+                                                  None) == 0
+        else:
+            assert lib.md_spme_energy_grad(sp, s, dbl(out), None, dbl(grad) if gradient else None, dbl(out[1:]), None) == 0
+        return [lib.fake_launch_name(k).decode() for k in range(n, lib.fake_launches())]
+
+    def back(names):
+        return [x for x in names if "gather" in x or "z_backward" in x or ("fftp" in x and "Li2E" in x)]
+
+    assert not back(launched(False))
+    with_gradient = launched(True)
+    assert any("gather" in x for x in with_gradient) and len(back(with_gradient)) >= 2
+    lib.md_spme_destroy(sp)
+    lib.md_system_destroy(s)
