@@ -707,16 +707,12 @@ k_nl_build(int N, const typename V4<R>::T* __restrict__ pos, const float* __rest
                          force_minimage, stw);
 }
 
-template <class R, int MODE>
-static const void* nl_kernel() {
-  static bool attr = false;
-  const void* f = (const void*)k_nl_build<R, MODE>;
-  if (!attr) {
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         NL_TILE_BYTES);
-    attr = true;
-  }
-  return f;
+static const void* nl_kernel(int prec, int mode) {
+  if (prec == MD_PREC_FP64)
+    return mode == MD_NL_MINIMAGE ? (const void*)k_nl_build<double, MD_NL_MINIMAGE>
+                                  : (const void*)k_nl_build<double, MD_NL_CELLSHIFT>;
+  return mode == MD_NL_MINIMAGE ? (const void*)k_nl_build<float, MD_NL_MINIMAGE>
+                                : (const void*)k_nl_build<float, MD_NL_CELLSHIFT>;
 }
 
 // cell-list criterion needs >= 4 cells per direction (DecideNumCell), else the
@@ -749,14 +745,7 @@ int nlist_build_impl(md_nlist* nl, md_system* sys, md_cell_list* cl, Recorder* r
   dim3 grid(cl->ntot), block(256);
   void* a[] = {&N, &sys->pos, &sys->rcut, &cl->start, &cl->zord, &g, &st, &rl, &skin, &cap, &nl->list,
                &nl->nnb, &nl->backup, &force_mi, &st, &gate};
-  const void* f;
-  const size_t smem = NL_TILE_BYTES;
-  if (sys->prec == MD_PREC_FP64) {
-    f = nl->mode == MD_NL_MINIMAGE ? nl_kernel<double, MD_NL_MINIMAGE>() : nl_kernel<double, MD_NL_CELLSHIFT>();
-  } else {
-    f = nl->mode == MD_NL_MINIMAGE ? nl_kernel<float, MD_NL_MINIMAGE>() : nl_kernel<float, MD_NL_CELLSHIFT>();
-  }
-  if (int r = rec_launch(rec, f, grid, block, smem, a)) return r;
+  if (int r = rec_launch(rec, nl_kernel(sys->prec, nl->mode), grid, block, NL_TILE_BYTES, a)) return r;
   if (int r = topo_exclude_launch(sys, nl, rec, gated)) return r;
   nl->built = true;
   return MD_OK;
@@ -1105,6 +1094,8 @@ extern "C" int md_nlist_create(md_nlist** out, md_system* sys, double rlist, dou
   }
   DevState hs;
   if (int r = sys->read_state(hs)) return r;
+  // with every list: the limit belongs to the kernel on the list's device
+  MD_CUDA(cudaFuncSetAttribute(nl_kernel(sys->prec, mode), cudaFuncAttributeMaxDynamicSharedMemorySize, NL_TILE_BYTES));
   md_nlist* nl = new md_nlist();
   nl->rlist = rlist;
   nl->skin = skin;

@@ -78,7 +78,7 @@ static cudaError_t launch(const void* f, dim3 g, dim3 b, size_t smem) {
   if (k < 0) return fail(cudaErrorInvalidDeviceFunction);
   if (!g.x || !g.y || !g.z || g.y > 65535 || g.z > 65535 || b.x * b.y * b.z > 1024 || !b.x || !b.y || !b.z)
     return fail(cudaErrorInvalidConfiguration);
-  if (smem > (size_t)funcs[k].limit[device]) return fail(cudaErrorInvalidValue);
+  if (smem > (size_t)(funcs[k].limit[device] ? funcs[k].limit[device] : 48 * 1024)) return fail(cudaErrorInvalidValue);
   pthread_mutex_lock(&mutex);
   if ((int)smem > funcs[k].used[device]) funcs[k].used[device] = (int)smem;
   if (nlaunches < MAX_LOG) {
@@ -116,12 +116,12 @@ const char* fake_lowered(void) {
     if (funcs[k].lowered) return funcs[k].name;
   return NULL;
 }
-/* the limit of the first kernel whose name holds `part`, on a device */
-int fake_limit(const char* part, int dev) {
-  int n = 0;
+/* a kernel launched with dynamic shared memory on a device where its limit was not set, though it was on another */
+const char* fake_unprepared(void) {
   for (int k = 0; k < nfuncs; ++k)
-    if (strstr(funcs[k].name, part) && funcs[k].limit[dev] > n) n = funcs[k].limit[dev];
-  return n;
+    for (int d = 0; d < DEVICES; ++d)
+      if (funcs[k].used[d] && !funcs[k].limit[d] && funcs[k].limit[!d]) return funcs[k].name;
+  return NULL;
 }
 
 /* ------------------------------------------------------------ the runtime */
@@ -137,7 +137,6 @@ void __cudaRegisterFunction(void** h, const char* f, char* d, const char* name, 
   if (nfuncs == MAX_FUNCS) abort();
   funcs[nfuncs].f = f;
   funcs[nfuncs].name = name;
-  for (int k = 0; k < DEVICES; ++k) funcs[nfuncs].limit[k] = 48 * 1024;
   ++nfuncs;
 }
 unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t smem, struct CUstream_st* s) {

@@ -30,10 +30,10 @@ def rt(tmp_path_factory):
     for name, (res, args) in _SIGS.items():
         getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
     for name, res in (("fake_calls", C.c_long), ("fake_live", C.c_long), ("fake_pinned", C.c_long),
-                      ("fake_pageable_dtoh", C.c_long), ("fake_launch_name", C.c_char_p), ("fake_lowered", C.c_char_p)):
+                      ("fake_pageable_dtoh", C.c_long), ("fake_launch_name", C.c_char_p), ("fake_lowered", C.c_char_p),
+                      ("fake_unprepared", C.c_char_p)):
         getattr(lib, name).restype = res
     lib.fake_fail_at.argtypes = [C.c_long]
-    lib.fake_limit.argtypes = [C.c_char_p, C.c_int]
     return lib
 
 
@@ -213,3 +213,19 @@ def test_energy_alone_is_not_transformed_back(lib, K, device_outputs):
     assert any("gather" in x for x in with_gradient) and len(back(with_gradient)) >= 2
     lib.md_spme_destroy(sp)
     lib.md_system_destroy(s)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_list_kernels_are_prepared_on_each_device(lib, precision):
+    """the list build's shared-memory limit is set on every device that has a list, not on the first one only"""
+    for device in (0, 1):
+        s, cl, nl = new_system(lib, 64, device), C.c_void_p(), C.c_void_p()
+        assert lib.md_cell_list_create(C.byref(cl), s, 2.0, 7, 1) == 0, lib.md_last_error_message()
+        for mode in (0, 1):
+            assert lib.md_nlist_create(C.byref(nl), s, 1.5, 0.3, 4.0, mode) == 0, lib.md_last_error_message()
+            assert lib.md_cell_list_rebuild(cl, s) == 0, lib.md_last_error_message()
+            assert lib.md_nlist_rebuild(nl, s, cl) == 0, lib.md_last_error_message()
+            lib.md_nlist_destroy(nl)
+        lib.md_cell_list_destroy(cl)
+        lib.md_system_destroy(s)
+    assert lib.fake_unprepared() is None
