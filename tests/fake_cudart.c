@@ -94,7 +94,7 @@ static cudaError_t launch(const void* f, dim3 g, dim3 b, size_t smem) {
 void fake_reset(void) { calls = 0; fail_at = -1; nlaunches = 0; pageable_dtoh = 0; last = cudaSuccess; device = 0; trims = 0; }
 void fake_fail_at(long k) { calls = 0; fail_at = k; }
 long fake_calls(void) { return calls; }
-long fake_live(void) {  /* bytes held, page-locked memory apart, and streams */
+long fake_live(void) {  /* bytes held, page-locked memory apart, streams and events */
   long n = streams;
   for (int k = 0; k < nblocks; ++k)
     if (blocks[k].p && blocks[k].kind != PINNED_MEM) n += (long)blocks[k].bytes;
@@ -251,6 +251,13 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) {
   return cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { (void)s; MAY_FAIL(cudaErrorUnknown); return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned f) {
+  (void)f;
+  return cudaStreamCreateWithFlags((cudaStream_t*)e, 0);
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) { return cudaStreamDestroy((cudaStream_t)e); }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { (void)e; (void)s; MAY_FAIL(cudaErrorUnknown); return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) { (void)e; MAY_FAIL(cudaErrorUnknown); return cudaSuccess; }
 cudaError_t cudaPointerGetAttributes(struct cudaPointerAttributes* a, const void* p) {
   (void)p;
   memset(a, 0, sizeof(*a));

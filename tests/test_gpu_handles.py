@@ -20,3 +20,38 @@ def test_functionals_of_two_meshes_in_turn(mdf):
     for _ in range(2):
         assert torch.equal(mdf.optibasis.ik_error_loss(c, big), want)
         assert torch.equal(mdf.optibasis.ik_error_loss(c, small), other)
+
+
+@pytest.mark.parametrize("n", [1, 21845, 21846, 87382, 3000000])
+def test_frames_come_back_whole(mdf, n):
+    """sizes around one piece of the read-back (512 KB), all of them, and above 64 MB"""
+    rng = np.random.default_rng(n)
+    pos = rng.uniform(0, 50, (n, 3))
+    sys = mdf.MDSystem(pos, (50.0,) * 3, precision=1)
+    for _ in range(2):
+        assert np.array_equal(sys.positions(), pos)
+    v = rng.normal(size=(n, 3))
+    sys.set_velocities(v)
+    assert np.array_equal(sys.velocities(), v)
+
+
+def test_two_threads_read_frames(mdf):
+    """each thread's system comes back unmixed while both read through the device's shared memory"""
+    import threading
+    rng = np.random.default_rng(5)
+    pos = [rng.uniform(0, 50, (n, 3)) for n in (150000, 70001)]
+    sys = [mdf.MDSystem(p, (50.0,) * 3, precision=1) for p in pos]
+    wrong = []
+
+    def read(s, p):
+        for _ in range(40):
+            if not np.array_equal(s.positions(), p):
+                wrong.append(len(p))
+                return
+
+    th = [threading.Thread(target=read, args=a) for a in zip(sys, pos)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not wrong

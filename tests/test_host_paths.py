@@ -229,3 +229,36 @@ def test_list_kernels_are_prepared_on_each_device(lib, precision):
         lib.md_cell_list_destroy(cl)
         lib.md_system_destroy(s)
     assert lib.fake_unprepared() is None
+
+
+@pytest.mark.parametrize("n", [1000, BIG, 3 * BIG])
+def test_frames_of_any_size_through_page_locked_memory(lib, n):
+    """frames arrive whole through a page-locked buffer of bounded size, also above what a system keeps"""
+    h = new_system(lib, n)
+    out = np.ones((n, 3))
+    before, held = lib.fake_pageable_dtoh(), lib.fake_pinned()
+    assert lib.md_system_get_positions(h, dbl(out)) == 0
+    assert lib.fake_pageable_dtoh() == before
+    assert lib.fake_pinned() - held <= 4 << 20
+    assert not out.any()
+    lib.md_system_destroy(h)
+
+
+def test_several_arrays_in_pieces(lib):
+    """arrays of no whole number of pieces, and empty ones, keep their bytes"""
+    s, a = new_system(lib, 64, 0, 120.0), C.c_void_p()
+    assert lib.md_arc_create(C.byref(a), s, 1.0, 2.5, 5.0, 0.5) == 0, lib.md_last_error_message()
+    dims = np.zeros(3, np.int32)
+    assert lib.md_arc_get_dims(a, dims.ctypes.data_as(C.POINTER(C.c_int)), None) == 0
+    n = int(dims.prod())
+    assert 8 * n > 4 * (512 << 10) and 8 * n % (512 << 10)
+    rc, idx, err = np.ones(n), np.ones(n, np.int32), np.ones(n)
+    before = lib.fake_pageable_dtoh()
+    assert lib.md_arc_get_rcut(a, dbl(rc), idx.ctypes.data_as(C.POINTER(C.c_int)), dbl(err)) == 0
+    assert lib.fake_pageable_dtoh() - before < 1 << 16  # the state alone
+    assert not rc.any() and not idx.any() and not err.any()
+    rc[:] = 1
+    assert lib.md_arc_get_rcut(a, None, None, dbl(rc)) == 0 and not rc.any()
+    assert lib.md_arc_get_rcut(a, None, None, None) == 0
+    lib.md_arc_destroy(a)
+    lib.md_system_destroy(s)
