@@ -555,8 +555,9 @@ extern "C" int md_system_destroy(md_system* s) {
   for (void* p : ptrs) if (p) cudaFree(p);
   topo_destroy(s->topo);
   if (s->h_stage) cudaFreeHost(s->h_stage);
-  // the stream is idle (synchronised above) and may be a caller's that is gone by now
-  if (s->d_stage) pool_free(s->device, s->d_stage, cudaStreamPerThread);
+  // the stream is idle (synchronised above) and may be a caller's that is gone by
+  // now; a free in order of another stream would still be pending when the pool is trimmed
+  if (s->d_stage) cudaFree(s->d_stage);
   if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
   if (s->pooled) pool_release(s->device);
   delete s;

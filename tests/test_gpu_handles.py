@@ -55,3 +55,33 @@ def test_two_threads_read_frames(mdf):
     for t in th:
         t.join()
     assert not wrong
+
+
+LAST_SYSTEM = """
+import numpy as np, torch, mdforce as mdf
+def free_after_a_frame(n):
+    sys = mdf.MDSystem(np.zeros((n, 3)), (50.0,) * 3, precision=1)
+    sys.positions()
+    del sys
+    return torch.cuda.mem_get_info()[0]
+before = free_after_a_frame(10)
+print(before - free_after_a_frame(2000000))
+"""
+
+
+def test_last_system_gives_its_staging_back(mdf):
+    """the device's pool is empty when the last system that used it is gone (a process of its own: no other system)"""
+    import os
+    import subprocess
+    import sys
+    env = dict(os.environ, PYTHONPATH=os.path.dirname(os.path.dirname(mdf.__file__)))
+    out = subprocess.run([sys.executable, "-c", LAST_SYSTEM], env=env, capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr
+    assert int(out.stdout) < 24 << 20  # of the 48 MB that a frame took
+
+
+def test_map_after_one_that_memory_does_not_hold(mdf):
+    with pytest.raises(mdf.core.MDExcptCuda):
+        mdf.ErrorEstimate_SPME_Ik((1024, 1024, 1024), (30.0,) * 3, 0.95, 6)
+    em = mdf.ErrorEstimate_SPME_Ik((16, 16, 16), (30.0,) * 3, 0.95, 6)
+    assert np.isfinite(em.rms()).all()
