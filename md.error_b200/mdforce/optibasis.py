@@ -16,7 +16,7 @@ import types
 import numpy as np
 
 from ._lib import lib
-from .core import check
+from .core import CUDA_STREAM_LEGACY, check
 
 CONVERSION = 138.93545756169981341199  # optiBasis/IkError.py:25
 
@@ -71,10 +71,13 @@ class IkErrorGPU:
         return val, g
 
     def evaluate_device(self, d_coeffs, d_values, d_grads, nc, stream=None):
-        """Raw device pointers (ints), asynchronous on `stream` (an int handle)."""
+        """Raw device pointers (ints), asynchronous on `stream` (an int handle, 0 torch's
+        default stream), or on the functional's own stream where it is None."""
+        if stream is not None and int(stream) == 0:
+            stream = CUDA_STREAM_LEGACY  # the C ABI reads 0 as the handle's own stream
         check(lib.md_ikerr_evaluate_device(self.h, int(nc), C.c_void_p(d_coeffs), C.c_void_p(d_values),
                                            C.c_void_p(d_grads) if d_grads else None,
-                                           C.c_void_p(stream) if stream else None), "md_ikerr_evaluate_device")
+                                           C.c_void_p(stream)), "md_ikerr_evaluate_device")
 
     def value(self, vv):
         return float(self.evaluate(vv, grads=False)[0][0])

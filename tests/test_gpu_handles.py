@@ -20,6 +20,19 @@ def test_functionals_of_two_meshes_in_turn(mdf):
     for _ in range(2):
         assert torch.equal(mdf.optibasis.ik_error_loss(c, big), want)
         assert torch.equal(mdf.optibasis.ik_error_loss(c, small), other)
+    assert want.item() != other.item()
+
+
+@pytest.mark.parametrize("k", [32, 200, 256])
+def test_functional_in_order_with_torch(mdf, k):
+    """a value read at once on torch's default stream is this call's, with coefficients made just before"""
+    import torch
+    f = functional(mdf, k)
+    base = mdf.optibasis.bspline_initial_basis(2.0, 4, 4)
+    for _ in range(20):
+        s = 1.0 + 0.01 * _
+        c = torch.from_numpy(base[None]).cuda() * s
+        assert mdf.optibasis.ik_error_loss(c, f).item() == f.evaluate(base * s, grads=False)[0][0]
 
 
 @pytest.mark.parametrize("n", [1, 21845, 21846, 87382, 3000000])

@@ -262,3 +262,23 @@ def test_several_arrays_in_pieces(lib):
     assert lib.md_arc_get_rcut(a, None, None, None) == 0
     lib.md_arc_destroy(a)
     lib.md_system_destroy(s)
+
+
+@pytest.mark.parametrize("given,passed", [(None, None), (0, 1), (0x7f00deadbeef, 0x7f00deadbeef)])
+def test_functional_on_the_default_stream(monkeypatch, given, passed):
+    """torch's default stream has the handle 0, which the C ABI reads as the functional's own stream:
+    its work would not be in order with torch's"""
+    import mdforce.optibasis as ob
+    seen = []
+
+    def fake(h, nc, coeffs, values, grads, stream):
+        seen.append(stream.value)
+        return 0
+
+    monkeypatch.setattr(ob.lib, "md_ikerr_evaluate_device", fake)
+
+    class Dummy:
+        h = C.c_void_p(1234)
+
+    ob.IkErrorGPU.evaluate_device(Dummy(), 16, 16, None, 1, given)
+    assert seen == [passed]
