@@ -171,7 +171,7 @@ extern "C" int md_cell_list_create(md_cell_list** out, md_system* sys, double ce
             cudaMalloc(&cl->perm, sizeof(uint32_t) * N) == cudaSuccess &&
             cudaMalloc(&cl->zord, sizeof(uint32_t) * N) == cudaSuccess &&
             cudaMalloc(&cl->busy, sizeof(uint32_t) * cl->ntot) == cudaSuccess &&
-            cudaMemset(cl->count, 0, sizeof(uint32_t) * cl->ntot) == cudaSuccess;
+            cudaMemsetAsync(cl->count, 0, sizeof(uint32_t) * cl->ntot, sys->stream) == cudaSuccess;
   if (!ok) {
     md_cuda_fail(cudaGetLastError(), "md_cell_list_create");
     md_cell_list_destroy(cl);

@@ -742,9 +742,11 @@ int lj_apply_impl(md_engine* eng, md_system* sys, md_nlist* nl, bool with_stats,
             default: break;  // kind 0: no interaction
           }
         }
-      MD_CUDA(cudaMemcpy(eng->d_tab, tf.data(), nf * sizeof(float4), cudaMemcpyHostToDevice));
-      MD_CUDA(cudaMemcpy(reinterpret_cast<char*>(eng->d_tab) + nf * sizeof(float4), td.data(),
-                         nf * sizeof(double4a), cudaMemcpyHostToDevice));
+      // in order with the kernels that read it; the wait is for the host tables
+      MD_CUDA(cudaMemcpyAsync(eng->d_tab, tf.data(), nf * sizeof(float4), cudaMemcpyHostToDevice, sys->stream));
+      MD_CUDA(cudaMemcpyAsync(reinterpret_cast<char*>(eng->d_tab) + nf * sizeof(float4), td.data(),
+                              nf * sizeof(double4a), cudaMemcpyHostToDevice, sys->stream));
+      MD_CUDA(cudaStreamSynchronize(sys->stream));
       eng->tab_dirty = false;
     }
   }

@@ -917,7 +917,7 @@ extern "C" int md_spme_create(md_spme** out, md_system* sys, const int K[3], int
             cudaMalloc(&s->G, sys->r4_size() * s->nreal) == cudaSuccess &&
             cudaMalloc(&s->psi, rs * s->nhalf) == cudaSuccess &&
             cudaMalloc(&s->d_box_tab, sizeof(double) * 3) == cudaSuccess &&
-            cudaMemset(s->d_box_tab, 0, sizeof(double) * 3) == cudaSuccess;
+            cudaMemsetAsync(s->d_box_tab, 0, sizeof(double) * 3, sys->stream) == cudaSuccess;
   if (!ok) {
     md_cuda_fail(cudaGetLastError(), "md_spme_create");
     md_spme_destroy(s);

@@ -511,8 +511,10 @@ extern "C" int md_system_create(md_system** out, int n, const double box[3], con
   memset(&hs, 0, sizeof(hs));
   box_fill(hs, box);
   for (int d = 0; d < 3; ++d) { hs.lam1[d] = hs.lam2[d] = 1.0; }
-  if (cudaMemcpy(s->st, &hs, sizeof(hs), cudaMemcpyHostToDevice) != cudaSuccess) return fail(md_cuda_fail(cudaGetLastError(), "state upload"));
-  // stage inputs through device buffers
+  // Inputs go through device buffers, by copies in order of the system's stream:
+  // a plain cudaMemcpy from pageable memory may return before its last piece has
+  // arrived, and the non-blocking stream does not wait for it.
+  cudaError_t e = cudaMemcpyAsync(s->st, &hs, sizeof(hs), cudaMemcpyHostToDevice, s->stream);
   size_t bytes = sizeof(double) * (3ull * n * 2 + 2ull * n);
   double* dbuf = nullptr;
   if (cudaMalloc(&dbuf, bytes) != cudaSuccess) return fail(md_cuda_fail(cudaGetLastError(), "stage"));
@@ -520,10 +522,11 @@ extern "C" int md_system_create(md_system** out, int n, const double box[3], con
   double* dvel = dbuf + 3ull * n;
   double* dq = dbuf + 6ull * n;
   double* dm = dbuf + 7ull * n;
-  cudaMemcpy(dpos, pos, sizeof(double) * 3 * n, cudaMemcpyHostToDevice);
-  if (vel) cudaMemcpy(dvel, vel, sizeof(double) * 3 * n, cudaMemcpyHostToDevice);
-  if (charge) cudaMemcpy(dq, charge, sizeof(double) * n, cudaMemcpyHostToDevice);
-  if (mass) cudaMemcpy(dm, mass, sizeof(double) * n, cudaMemcpyHostToDevice);
+  const struct { double* to; const double* from; size_t count; } in[] = {
+      {dpos, pos, 3ull * n}, {dvel, vel, 3ull * n}, {dq, charge, (size_t)n}, {dm, mass, (size_t)n}};
+  for (const auto& c : in)
+    if (c.from && e == cudaSuccess)
+      e = cudaMemcpyAsync(c.to, c.from, sizeof(double) * c.count, cudaMemcpyHostToDevice, s->stream);
   const double* pv = vel ? dvel : nullptr;
   const double* pq = charge ? dq : nullptr;
   const double* pm = mass ? dm : nullptr;
@@ -534,7 +537,8 @@ extern "C" int md_system_create(md_system** out, int n, const double box[3], con
     k_upload<float><<<nb, 256, 0, s->stream>>>(n, dpos, pv, pq, pm, (float4*)s->pos, (float4*)s->vel, s->id, s->image, s->force, s->rcut);
   cudaMemsetAsync(s->type_by_id, 0, (size_t)n, s->stream);
   cudaMemsetAsync(s->type, 0, (size_t)n, s->stream);
-  cudaError_t e = cudaStreamSynchronize(s->stream);
+  const cudaError_t done = cudaStreamSynchronize(s->stream);
+  if (e == cudaSuccess) e = done;
   cudaFree(dbuf);
   if (e != cudaSuccess) return fail(md_cuda_fail(e, "upload"));
   if (type)

@@ -20,6 +20,7 @@ static struct { const void* f; const char* name; int limit[DEVICES], used[DEVICE
 static struct { int func, device; size_t smem; } launches[MAX_LOG];
 static int nblocks, nfuncs, nlaunches, streams, trims;
 static size_t pageable_dtoh;
+static int unordered;
 static long calls, fail_at = -1;
 static pthread_mutex_t mutex = PTHREAD_MUTEX_INITIALIZER;
 static __thread int device;
@@ -108,6 +109,7 @@ long fake_pinned(void) {
 }
 long fake_pageable_dtoh(void) { return (long)pageable_dtoh; }
 int fake_trims(void) { return trims; }
+int fake_unordered(void) { return unordered; }  /* writes to the device that no stream of the library waits for */
 int fake_launches(void) { return nlaunches; }
 const char* fake_launch_name(int k) { return funcs[launches[k].func].name; }
 /* a kernel whose shared-memory limit was taken below what it has been launched with */
@@ -217,6 +219,7 @@ static void copied(void* d, const void* s, size_t n, enum cudaMemcpyKind k) {
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, enum cudaMemcpyKind k) {
   MAY_FAIL(cudaErrorInvalidValue);
   copied(d, s, n, k);
+  if (k == cudaMemcpyHostToDevice) ++unordered;
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, enum cudaMemcpyKind k, cudaStream_t st) {
@@ -225,7 +228,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, enum cudaMemcpyKin
   copied(d, s, n, k);
   return cudaSuccess;
 }
-cudaError_t cudaMemset(void* p, int v, size_t n) { MAY_FAIL(cudaErrorInvalidValue); memset(p, v, n); return cudaSuccess; }
+cudaError_t cudaMemset(void* p, int v, size_t n) { MAY_FAIL(cudaErrorInvalidValue); memset(p, v, n); ++unordered; return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t s) {
   (void)s;
   MAY_FAIL(cudaErrorInvalidValue);

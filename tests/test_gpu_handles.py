@@ -35,13 +35,14 @@ def test_functional_in_order_with_torch(mdf, k):
         assert mdf.optibasis.ik_error_loss(c, f).item() == f.evaluate(base * s, grads=False)[0][0]
 
 
-@pytest.mark.parametrize("n", [1, 21845, 21846, 87382, 3000000])
+@pytest.mark.parametrize("n", [1, 21845, 21846, 87382, 174763, 262145, 3000000])
 def test_frames_come_back_whole(mdf, n):
-    """sizes around one piece of the read-back (512 KB), all of them, and above 64 MB"""
+    """sizes around one piece of the read-back (512 KB), all of them, and above 64 MB; a few bytes
+    past a multiple of 2 MB, which an upload from pageable memory delivers last"""
     rng = np.random.default_rng(n)
     pos = rng.uniform(0, 50, (n, 3))
-    sys = mdf.MDSystem(pos, (50.0,) * 3, precision=1)
-    for _ in range(2):
+    for _ in range(10 if n < 1000000 else 1):
+        sys = mdf.MDSystem(pos, (50.0,) * 3, precision=1)
         assert np.array_equal(sys.positions(), pos)
     v = rng.normal(size=(n, 3))
     sys.set_velocities(v)

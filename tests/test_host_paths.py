@@ -282,3 +282,21 @@ def test_functional_on_the_default_stream(monkeypatch, given, passed):
 
     ob.IkErrorGPU.evaluate_device(Dummy(), 16, 16, None, 1, given)
     assert seen == [passed]
+
+
+def test_uploads_are_in_order_with_the_kernels(lib):
+    """no copy or fill goes around the streams that the kernels run on: what a plain cudaMemcpy has
+    not delivered when it returns, a kernel on a non-blocking stream does not wait for"""
+    before = lib.fake_unordered()
+    s, cl, nl, sp, eng = new_system(lib), C.c_void_p(), C.c_void_p(), C.c_void_p(), C.c_void_p()
+    assert lib.md_cell_list_create(C.byref(cl), s, 2.0, 7, 1) == 0
+    assert lib.md_nlist_create(C.byref(nl), s, 1.5, 0.3, 4.0, 0) == 0
+    assert lib.md_spme_create(C.byref(sp), s, vec(C.c_int, 16, 16, 16), 4, 1.0, 0) == 0
+    assert lib.md_engine_create(C.byref(eng), s) == 0
+    assert lib.md_engine_register_lj_pair(eng, 0, 0, 1.0, 1.0, 0.0) == 0, lib.md_last_error_message()
+    assert lib.md_cell_list_rebuild(cl, s) == 0 and lib.md_nlist_rebuild(nl, s, cl) == 0
+    assert lib.md_engine_apply_nonbonded(eng, s, nl, 1) == 0, lib.md_last_error_message()
+    assert lib.md_spme_apply(sp, s, 1) == 0
+    assert lib.fake_unordered() == before
+    for destroy, h in (("spme", sp), ("nlist", nl), ("cell_list", cl), ("engine", eng), ("system", s)):
+        getattr(lib, f"md_{destroy}_destroy")(h)
