@@ -14,7 +14,10 @@
 
 namespace {
 
-// K is a power of two: the product with 1/K rounds as the quotient
+// K is a power of two: the product with 1/K rounds as the quotient, and the mask
+// takes b = K to 0.  It also keeps every base inside the mesh: a binary64 NaN
+// (a coordinate that is none) becomes the lowest int, from which the extent of a
+// staged region would come out negative and its reads outside the block's memory.
 template <class R>
 __device__ __forceinline__ void grid_coord(R x, R Linv, int K, int& base, R& frac) {
   const R kinv = sizeof(R) == 4 ? (R)__int_as_float((127 - (31 - __clz(K))) << 23)
@@ -23,8 +26,7 @@ __device__ __forceinline__ void grid_coord(R x, R Linv, int K, int& base, R& fra
   u -= floor_r(u * kinv) * R(K);
   R b = floor_r(u);
   frac = u - b;
-  base = (int)b;
-  if (base >= K) { base -= K; }
+  base = (int)b & (K - 1);
 }
 
 // M_n(f + j), j = 0..n-1, and derivatives (D) by the recursion
