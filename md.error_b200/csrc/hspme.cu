@@ -40,7 +40,7 @@
 // Candidates go through in batches of up to four, one launch per step.  All
 // meshes are real, so the FP64 grid transforms (dft.cu) carry two fields of a
 // candidate each where it has two, as the real and imaginary parts: (E_0, E_1)
-// and (E_2, phi_pot) back, (B_0, B_1) forward -- 9 complex transforms per
+// and (E_2, kap phi_pot) back, (B_0, B_1) forward -- 9 complex transforms per
 // candidate for both functionals where one per mesh takes 14 -- and read and write
 // real grids where it has one.  Two candidates
 // never share a transform: the rounding of one (or its infinities) would reach
@@ -78,6 +78,7 @@ struct HsGeom {
   int K[3];
   double L[3];
   double beta, CC, h;
+  double kap;  // of E_2 + i kap phi (k_hs_kspace_fwd), a power of two
   int nbin, nk, ncoef, S, half;  // half = ceil(CC)
   long Kt;
 };
@@ -291,15 +292,20 @@ __device__ __forceinline__ double2 hs_second(double2 z, double2 y) { return make
 
 // k space of the forward pass, a point per thread, nb candidates: with
 // g = G Qh, F[c] = transform of E_0 + i E_1 = (i k_0 - k_1) g; energy pass
-// (loss = 0) F[nb + c] = E_2 + i phi = i (k_2 + 1) g; force error (loss = 1)
+// (loss = 0) F[nb + c] = E_2 + i kap phi = i (k_2 + kap) g; force error (loss = 1)
 // F[nb + c] = E_2 = i k_2 g.  w[c] = G |Qh|^2 (or null).
+// A transform rounds to its larger part, and a field is a potential over a
+// length: kap, near sqrt(2 pi beta / L) (the ratio of the two in a disordered
+// system, whose modes reach from 2 pi / L to about beta), keeps the parts alike
+// in any unit of length.  With kap = 1 the forces along z of a box 10^4 times as
+// long were off by 3e-12, and dE/dq of one 10^4 times as short by 1e-12.
 __global__ void __launch_bounds__(256)
 k_hs_kspace_fwd(HsGeom g, int nb, int loss, const double2* __restrict__ Z, const double* __restrict__ bfac, int Kmax,
                 double2* __restrict__ F, double* __restrict__ w) {
   const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (p >= g.Kt) return;
   const HsPoint h = hs_point(g, p);
-  const double k2 = loss ? h.k[2] : h.k[2] + 1.0;
+  const double k2 = loss ? h.k[2] : h.k[2] + g.kap;
   for (int c = 0; c < nb; ++c) {
     const double2 Q = Z[c * g.Kt + p];
     const double G = hs_factor2(h, bfac + (long)c * 3 * Kmax, Kmax);
@@ -357,7 +363,7 @@ struct HsOut {
 };
 
 // Gather, a candidate per blockIdx.y, a warp per atom.
-//   MODE 0 (energy): f1 = (E_0, E_1), f2 = (E_2, phi): F_i, dE/dq_i, dE/dr_i and
+//   MODE 0 (energy): f1 = (E_0, E_1), f2 = (E_2, kap phi): F_i, dE/dq_i, dE/dr_i and
 //     the coefficient partials of the scalar phi
 //   MODE 1 (loss): E_2 from the real grid e2: F_i, the residual R_i = 2 (F_i - Fref_i) / N
 //     and the block's part of the loss
@@ -393,6 +399,7 @@ k_hs_gather(HsGeom g, int N, const double* __restrict__ q, const double* __restr
   const double2* e01 = f1 + (long)cand * g.Kt;
   const double2* e2p = f2 + (long)cand * g.Kt;
   const double *e2r = e2 + (long)cand * g.Kt, *lm = lam + (long)cand * g.Kt;
+  const double kinv = 1.0 / g.kap;  // exact
   double loss = 0.0;
   for (int n = 0; n < HS_ATOMS; ++n) {
     const int i = (blockIdx.x * W + warp) * HS_ATOMS + n;
@@ -426,8 +433,9 @@ k_hs_gather(HsGeom g, int N, const double* __restrict__ q, const double* __restr
           Ef[1] += wxy * a.y;
           Ef[2] += wxy * b.x;
           if (MODE == 0) {
-            ss[warp][row * LD + z] = b.y;
-            t2 += wxy * b.y;
+            const double s = b.y * kinv;
+            ss[warp][row * LD + z] = s;
+            t2 += wxy * s;
           }
         }
       }
@@ -642,6 +650,7 @@ extern "C" int md_hspme_create(md_hspme** out, int natoms, const int K[3], const
   g.half = half;
   g.S = 2 * half;
   g.Kt = (long)K[0] * K[1] * K[2];
+  g.kap = exp2(rint(0.5 * log2(2.0 * M_PI * beta / cbrt(L[0] * L[1] * L[2]))));
   h->Kmax = std::max(K[0], std::max(K[1], K[2]));
   const int per = HS_ATOMS * hs_warps(g.S);
   h->nab = (natoms + per - 1) / per;
