@@ -62,7 +62,8 @@ k_ew_sk(int i0, int nc, const double4a* __restrict__ pos, const float4* __restri
         const double2* __restrict__ tab, int per, int accumulate, double* __restrict__ part) {
   __shared__ double2 A[EW_A][EW_T], B[EW_A][EW_T];
   const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
-  const int r0 = blockIdx.x * EW_T, c0 = blockIdx.y * EW_T;
+  const int ct = (g.ncol + EW_T - 1) / EW_T;  // tiles along blockIdx.x, the one index that reaches any count
+  const int r0 = (int)(blockIdx.x / ct) * EW_T, c0 = (int)(blockIdx.x % ct) * EW_T;
   const int a0 = blockIdx.z * per, a1 = min(nc, a0 + per);
   const double2* e0 = tab;
   const double2* e1 = e0 + (size_t)(g.M[0] + 1) * nc;
@@ -264,8 +265,7 @@ extern "C" int md_ewald_exact(md_system* sys, const int K[3], double beta, doubl
   for (int i0 = 0; i0 < N; i0 += EW_CHUNK) {
     const int nc = std::min(EW_CHUNK, N - i0);
     tables(i0, nc);
-    k_ew_sk<<<dim3(ceil_div(g.nrow, EW_T), ceil_div(g.ncol, EW_T), ns), 64, 0, s>>>(i0, nc, pos, posf, g, tab, per,
-                                                                                    i0 > 0, part);
+    k_ew_sk<<<dim3(tiles, 1, ns), 64, 0, s>>>(i0, nc, pos, posf, g, tab, per, i0 > 0, part);
   }
   k_ew_coef<<<nbc, 256, 0, s>>>(g, beta, ns, part, sys->st, coef, red, e);
   MD_CHECK_LAUNCH("ewald sk");

@@ -300,3 +300,11 @@ def test_uploads_are_in_order_with_the_kernels(lib):
     assert lib.fake_unordered() == before
     for destroy, h in (("spme", sp), ("nlist", nl), ("cell_list", cl), ("engine", eng), ("system", s)):
         getattr(lib, f"md_{destroy}_destroy")(h)
+
+
+def test_exact_sum_over_a_long_axis(lib):
+    """mode boxes of more columns than a grid has rows of blocks"""
+    s, e = new_system(lib, 2), C.c_double()
+    for K in ((1, 1, 2200000), (1, 2200000, 1), (2200000, 1, 1)):
+        assert lib.md_ewald_exact(s, vec(C.c_int, *K), 1.0, C.byref(e), 1) == 0, lib.md_last_error_message()
+    lib.md_system_destroy(s)
