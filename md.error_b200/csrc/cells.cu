@@ -159,6 +159,7 @@ extern "C" int md_cell_list_create(md_cell_list** out, md_system* sys, double ce
     if (nc < 1) nc = 1;
     if (on) nc *= divide;
     cl->ncell[d] = nc;
+    cl->h[d] = hs.L[d] / nc;
   }
   cl->ntot = cl->ncell[0] * cl->ncell[1] * cl->ncell[2];
   int N = sys->N;

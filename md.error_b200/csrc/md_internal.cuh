@@ -143,6 +143,7 @@ struct md_cell_list {
   int ncell[3] = {1, 1, 1};
   int ntot = 1;
   double cell_size = 0;
+  double h[3] = {1, 1, 1};         // cell edges in the box at creation
   int bdir = 7, divide = 1;
   uint32_t* cell_of = nullptr;     // cell of slot k (after sort: sorted order)
   uint32_t* t_cell = nullptr;      // cell of slot k before the sort
@@ -173,6 +174,8 @@ struct md_nlist {
   int mode = MD_NL_MINIMAGE;
   int cap = 0;
   int N = 0;
+  int sms = 0;            // of the device
+  const void* prepared = nullptr;  // build whose shared-memory limit is set
   int* list = nullptr;    // [N][cap] row-major (slot indices)
   int* nnb = nullptr;     // [N]
   void* backup = nullptr; // Real4 positions at the last build

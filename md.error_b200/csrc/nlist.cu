@@ -4,7 +4,8 @@
 // NeighborList::mallocDeviceNeighborList (UNI/src/NeighborList_interface.cu:187-208),
 // Displacement_max (ENG/src/Displacement_interface.cu:80-126).
 //
-// One block per home cell of NL_LIGHT atoms or more, one warp per lighter cell.
+// One block per home cell, one warp per cell of fewer than NL_LIGHT atoms where
+// there are many cells (nl_light_cells).
 // The candidate cells of the home cell (every cell
 // whose box comes within the largest list radius of the home-cell box, or the
 // reference's c +- 1 stencil in cell-shift mode) are enumerated as (x, y)
@@ -12,8 +13,9 @@
 // cell-sorted arrays -- and staged into a shared-memory tile.  Each warp then
 // takes one home atom i at a time; its 32 lanes test 2 x 32 tile entries at once,
 // skipping runs whose box lies beyond rlist_i, and a ballot compacts the
-// accepted ones into row i of the list.  When the tile would not fit, the same
-// loop reads the runs from global memory.
+// accepted ones into row i of the list.  When the tile would not fit, or the
+// stencil spans the box or is the reference's, a second loop takes the stored
+// positions one chunk at a time, from the tile or from global memory.
 // A pair within rounding of the radius is decided by the reference's binary32
 // (or binary64) operations without FMA contraction, every other by a binary32
 // distance with a proven error bound, so the neighbour SETS are bit-identical to
@@ -40,9 +42,37 @@ struct NlGeom {
 // stencil (2,270 atoms at density 0.78 and cells of 2.86; 2,600 at 0.8 and
 // 2.96) fit with four blocks on an SM
 #define NL_TILE_BYTES 44032
+// Builds of at most NL_SMALL blocks per SM take the registers and the memory of
+// two blocks an SM: no spills, and stencils that span the box (2,816 binary64
+// positions, 5,632 packed) staged whole.  Binary64, 2,000 atoms in 27 cells 241 us
+// with it, 327 with four blocks' share; 1,000 95 and 111.
+#define NL_WIDE 4
+#define NL_SMALL 2
+#define NL_TILE_SMALL 98304
+// Binary64 minimum-image builds whose stencil spans the box along an axis: three
+// blocks an SM (slab of 4,096 atoms in 550 cells 138 us, 203 with four)
+#define NL_MID 3
+#define NL_TILE_MID 71680
+// Stencils of more atoms than a tile holds read global memory, and the tile's share
+// serves as L1 (binary32, 65,536 atoms at 8.0: 1,155 us, 1,351 with the tile's)
+#define NL_TILE_NONE 16384
 #define NL_MAX_RUNS 160
+// the periodic shifts of the runs that a warp walks (32 of them), kept at the
+// end of the tile's memory where the packed tile is not used
+template <class R> constexpr int nl_shift_bytes() { return 8 * 32 * (int)sizeof(typename V4<R>::T); }
 #define NL_RUN_MAXZ 7   // z cells of a run with per-atom z windows (longer runs are scanned whole)
-#define NL_LIGHT 4      // home cells below this many atoms are built warp per cell
+#define NL_LIGHT 4      // home cells below this many atoms are built warp per cell (nl_light_cells)
+// By themselves above two waves of blocks: below, a warp's chain of loads over its
+// atoms outlasts the blocks (us by warp / by block: 500 atoms in 216 cells 48 / 36,
+// 2,000 in 343 60 / 39; 16,000 in 15,625 131 / 270, 65,536 of a slab in 9,295 205 / 220).
+// Up to NL_LIGHT_OWN cells they have blocks of their own, after a quarter of the
+// others (8,000 atoms in 1,331 cells 60, 73 by the block of every eighth cell before
+// its own; 16,000 in 2,744 85 / 97; last in the grid 2,400 cells 97, first 87, so 86); above,
+// those blocks take longer than the chains (500,000 in 130,000 1,437 / 1,400).
+#define NL_LIGHT_CELLS 1184
+#define NL_LIGHT_OWN 5000
+__host__ __device__ __forceinline__ bool nl_light_cells(int ntot) { return ntot > NL_LIGHT_CELLS; }
+__device__ __forceinline__ int nl_light_at(int ntot) { return ntot / 4; }
 
 // Runs of a home cell, one array per field (the 32 lanes of a warp read the
 // fields of 32 different runs at once, which a struct per run would turn
@@ -65,6 +95,13 @@ template <class R> __device__ __forceinline__ R img_shift(int code, int d, R L) 
   return b == 1u ? R(0) : b == 2u ? L : -L;
 }
 #define NL_SLOT_MASK 0x03FFFFFF
+// the slot index carried in the w component of a staged position (bit copy)
+template <class R> __device__ __forceinline__ R slot_as_w(int j);
+template <> __device__ __forceinline__ float slot_as_w<float>(int j) { return __int_as_float(j); }
+template <> __device__ __forceinline__ double slot_as_w<double>(int j) { return __longlong_as_double((long long)j); }
+template <class R> __device__ __forceinline__ int slot_of_w(R w);
+template <> __device__ __forceinline__ int slot_of_w<float>(float w) { return __float_as_int(w); }
+template <> __device__ __forceinline__ int slot_of_w<double>(double w) { return (int)__double_as_longlong(w); }
 
 // cells along one axis whose box comes within rle of home cell hc's box
 __device__ __forceinline__ void nl_stencil_axis(double L, int nc, int hc, double rle, double& h, int& lo, int& hi,
@@ -224,14 +261,18 @@ __device__ __forceinline__ bool nl_light_cell(int c, int i0, int i1, bool per_at
 // The lists of the atoms of home cell c, by one block of 8 warps.  Every
 // exit is uniform over the block; the shared state is first written after a
 // block barrier, so a block may run this for one cell after another.
-template <class R, int MODE>
+// SCREEN: binary64 stencils that are neither packed nor staged whole are staged in
+// binary32.  The minimum-image build at four blocks an SM leaves it out: the
+// stencils that need it span the box and go to three or two, and its registers
+// cost the packed ones 2 to 7 % (65,536 atoms at density 0.1 278 us, 266 without).
+template <class R, int MODE, bool SCREEN>
 __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __restrict__ pos,
                                               const float* __restrict__ rcut, const uint32_t* __restrict__ start,
                                               const uint32_t* __restrict__ zord, NlGeom g,
                                               const DevState* __restrict__ st, double rlist_uniform, double skin,
                                               int cap, int* __restrict__ list, int* __restrict__ nnb,
                                               typename V4<R>::T* __restrict__ backup, int force_minimage,
-                                              DevState* stw) {
+                                              DevState* stw, int tile_bytes) {
   typedef typename V4<R>::T T4;
   extern __shared__ __align__(16) unsigned char nl_smem[];
   // one image per run: home frame, w carries the list entry (slot and image);
@@ -246,16 +287,21 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
   const bool minimg = (MODE == MD_NL_MINIMAGE) || force_minimage;
   const int hc[3] = {c / (g.nc[2] * g.nc[1]), (c / g.nc[2]) % g.nc[1], c % g.nc[2]};
 
-  // largest list radius among the home atoms, from it the stencil of the home
-  // cell (cells per axis whose box comes within that radius), and from that
-  // the runs of candidate cells: warp 0, its lanes first taking an axis each,
-  // then an (x, y) column each of at most 3 z segments, whose slots and tile
-  // offsets come from warp scans in column order.  (All 8 warps with block
-  // scans took five barriers a cell for work that 25 lanes do.)
-  __shared__ double s_h[3];
-  __shared__ int s_nr, s_atoms, s_flags;  // runs, their atoms; 1: box spanned per axis excluded (shift per run), 2: too many runs
-  const bool per_atom = MODE == MD_NL_MINIMAGE;
+  // Largest list radius among the home atoms, from it the stencil of the home cell
+  // (cells per axis whose box comes within that radius), warp 0, its lanes an axis
+  // each; and from that the runs of candidate cells, a lane per (x, y) column of
+  // at most 3 z segments, whose slots and tile offsets come from scans in column
+  // order.  Up to 32 columns are warp 0's work as well (all 8 warps with their
+  // scans across the block took five barriers a cell), more of them are dealt to
+  // all warps (49 to 81 columns, 1,000 to 32,768 cells: a build took 10 to 17 % longer
+  // by one).
+  __shared__ double s_h[3], s_rle;
+  __shared__ int s_lo[3], s_hi[3], s_full[3];
+  __shared__ int s_nr, s_atoms, scan_r[8], scan_a[8];
+  auto columns = [&]() -> int { return (s_hi[0] - s_lo[0] + 1) * (s_hi[1] - s_lo[1] + 1); };
+  bool wide = false;
   if (warp == 0) {
+    const bool per_atom = MODE == MD_NL_MINIMAGE;
     float m = per_atom ? 0.f : (float)rlist_uniform;
     if (per_atom) {
       for (int i = i0 + lane; i < i1; i += 32) m = fmaxf(m, __fadd_rn(rcut[i], (float)skin));
@@ -263,13 +309,11 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
       for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     }
     const double rle = nl_stencil_radius(m);
-    double h[3], hd;
-    int lo[3], hi[3], a, b, f;
-    bool full[3];
-    {
-      const int d = lane < 3 ? lane : 0;
-      const int ncd = d == 0 ? g.nc[0] : d == 1 ? g.nc[1] : g.nc[2];
+    if (lane < 3) {
+      const int d = lane, ncd = d == 0 ? g.nc[0] : d == 1 ? g.nc[1] : g.nc[2];
       const int hcd = d == 0 ? hc[0] : d == 1 ? hc[1] : hc[2];
+      double hd;
+      int a, b, f;
       if (!minimg) {
         hd = st->L[d] / ncd;
         const int reach = (hd >= rlist_uniform) ? 1 : (int)ceil(rlist_uniform / hd);
@@ -277,129 +321,153 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
       } else {
         nl_stencil_axis(st->L[d], ncd, hcd, rle, hd, a, b, f);
       }
-      if (lane < 3) s_h[d] = hd;
+      s_h[d] = hd;
+      s_lo[d] = a;
+      s_hi[d] = b;
+      s_full[d] = f;
+      s_rle = rle;
     }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      h[d] = __shfl_sync(0xffffffffu, hd, d);
-      lo[d] = __shfl_sync(0xffffffffu, a, d);
-      hi[d] = __shfl_sync(0xffffffffu, b, d);
-      full[d] = __shfl_sync(0xffffffffu, f, d) != 0;
-    }
-    const int ncy = hi[1] - lo[1] + 1;
-    const int ncols = (hi[0] - lo[0] + 1) * ncy;
-    // When the stencil spans less than the box along every axis, each cell
-    // appears in exactly one run, at that run's periodic image k_run, and
-    // 2 rlist < L.  For any pair within rlist the reference's image
-    // floor((r_j - r_i)/L + 1/2) is then k_run (it can differ only where
-    // |d| is within rounding of L/2 > rlist, where both reject), so
-    // d = (r_j - r_i) - k_run L repeats the reference's binary32 operations and
-    // the image code is the run's.
-    const bool runshift = minimg && !full[0] && !full[1] && !full[2];
-    // columns are then cut to the cells within the largest radius of the home
-    // cell: at 4.0 with cells of 2.86, 81 cells of 125 remain
-    const bool trim = runshift && nl_runs_bounded(ncols);
-    int base_r = 0, base_a = 0;
-    bool over = false;
-    for (int col0 = 0; col0 < ncols; col0 += 32) {
-      const int col = col0 + lane;
-      int jb_s[3], cnt_s[3], rs[3], rz0[3], len_s[3], ra_s[3], nseg = 0;
-      int ix = 0, iy = 0, sx = 0, sy = 0, colbase = 0;
-      if (col < ncols) {
-        ix = lo[0] + col / ncy;
-        iy = lo[1] + col % ncy;
-        int cx = ix, cy = iy;
-        if (cx < 0) { cx += g.nc[0]; sx = 1; } else if (cx >= g.nc[0]) { cx -= g.nc[0]; sx = -1; }
-        if (cy < 0) { cy += g.nc[1]; sy = 1; } else if (cy >= g.nc[1]) { cy -= g.nc[1]; sy = -1; }
-        colbase = g.nc[2] * (cy + g.nc[1] * cx);
-        int ra[3], rb[3], ns = 0;
-        if (full[2]) { ra[0] = 0; rb[0] = g.nc[2] - 1; rs[0] = 0; rz0[0] = 0; ns = 1; }
-        else {
-          int zlo = lo[2], zhi = hi[2];
-          if (trim) {
-            const float gx = (float)h[0] * (float)max(0, max(ix - hc[0], hc[0] - ix) - 1);
-            const float gy = (float)h[1] * (float)max(0, max(iy - hc[1], hc[1] - iy) - 1);
-            const float rf = (float)rle, w2 = rf * rf - (gx * gx + gy * gy);
-            const float zc = sqrtf(fmaxf(w2, 0.f)) / (float)h[2];  // reach along z in cells
-            zlo = max(zlo, hc[2] - (int)ceilf(zc));
-            zhi = w2 < 0.f ? zlo - 1 : min(zhi, hc[2] + 1 + (int)floorf(zc));
-          }
-          if (zlo <= zhi) {
-            if (zlo < 0) {
-              ra[ns] = zlo + g.nc[2]; rb[ns] = min(zhi, -1) + g.nc[2]; rs[ns] = 1; rz0[ns] = zlo; ++ns;
-            }
-            const int za = max(zlo, 0), zb = min(zhi, g.nc[2] - 1);
-            if (za <= zb) { ra[ns] = za; rb[ns] = zb; rs[ns] = 0; rz0[ns] = za; ++ns; }
-            if (zhi >= g.nc[2]) {
-              const int z0 = max(zlo, g.nc[2]);
-              ra[ns] = z0 - g.nc[2]; rb[ns] = zhi - g.nc[2]; rs[ns] = -1; rz0[ns] = z0; ++ns;
-            }
-          }
-        }
-        for (int s = 0; s < ns; ++s) {
-          const int jb = (int)start[colbase + ra[s]], je = (int)start[colbase + rb[s] + 1];
-          if (je == jb) continue;
-          jb_s[nseg] = jb; cnt_s[nseg] = je - jb; len_s[nseg] = rb[s] - ra[s];
-          rs[nseg] = rs[s]; rz0[nseg] = rz0[s]; ra_s[nseg] = ra[s];
-          ++nseg;
-        }
-      }
-      int atoms = 0;
-      for (int s = 0; s < nseg; ++s) atoms += cnt_s[s];
-      int ir = nseg, ia = atoms;  // inclusive scans
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int vr = __shfl_up_sync(0xffffffffu, ir, o), va = __shfl_up_sync(0xffffffffu, ia, o);
-        if (lane >= o) { ir += vr; ia += va; }
-      }
-      int r_off = base_r + ir - nseg, a_off = base_a + ia - atoms;
-      for (int s = 0; s < nseg; ++s) {
-        if (r_off >= NL_MAX_RUNS) { over = true; break; }
-        const int q = r_off;
-        rt.jb[q] = jb_s[s]; rt.cnt[q] = cnt_s[s]; rt.off[q] = a_off;
-        rt.code[q] = img_code(sx, sy, rs[s]);
-        const int zc0 = rz0[s], zc1 = rz0[s] + len_s[s];
-        rt.b0[0][q] = full[0] ? -1e30f : (float)(ix * h[0]); rt.b1[0][q] = full[0] ? 1e30f : (float)((ix + 1) * h[0]);
-        rt.b0[1][q] = full[1] ? -1e30f : (float)(iy * h[1]); rt.b1[1][q] = full[1] ? 1e30f : (float)((iy + 1) * h[1]);
-        rt.b0[2][q] = full[2] ? -1e30f : (float)(zc0 * h[2]); rt.b1[2][q] = full[2] ? 1e30f : (float)((zc1 + 1) * h[2]);
-        // per-cell offsets for the per-atom z window (runs that do not wrap the
-        // whole z axis and have at most NL_RUN_MAXZ cells)
-        rt.zc0[q] = zc0;
-        const int nzq = (!full[2] && len_s[s] + 1 <= NL_RUN_MAXZ && cnt_s[s] <= 65535) ? len_s[s] + 1 : 0;
-        rt.nz[q] = nzq;
-        for (int k = 0; k < nzq; ++k)
-          rt.zoff[k][q] = (unsigned short)((int)start[colbase + ra_s[s] + k] - jb_s[s]);
-        if (nzq) rt.zoff[nzq][q] = (unsigned short)cnt_s[s];
-        ++r_off;
-        a_off += cnt_s[s];
-      }
-      base_r += __shfl_sync(0xffffffffu, ir, 31);
-      base_a += __shfl_sync(0xffffffffu, ia, 31);
-    }
-    over = __any_sync(0xffffffffu, over);
-    if (lane == 0) {
-      s_nr = min(base_r, NL_MAX_RUNS);
-      s_atoms = base_a;
-      s_flags = (runshift ? 1 : 0) | (over ? 2 : 0);
-      if (over) atomicOr(&stw->flags, FLAG_NL_OVERFLOW);
-    }
+    __syncwarp();
+    wide = columns() > 32;
   }
-  __syncthreads();
-  const double h[3] = {s_h[0], s_h[1], s_h[2]};
-  const int nr = s_nr, tile_n = s_atoms;
-  const bool runshift = s_flags & 1;
+  double h[3];
+  // warp 0 by itself, or, when it finds more columns than lanes, all warps after the barrier
+  for (bool all = false;; all = true) {
+    if (all || (warp == 0 && !wide)) {
+      const int lo[3] = {s_lo[0], s_lo[1], s_lo[2]}, hi[3] = {s_hi[0], s_hi[1], s_hi[2]};
+      const bool full[3] = {s_full[0] != 0, s_full[1] != 0, s_full[2] != 0};
+#pragma unroll
+      for (int d = 0; d < 3; ++d) h[d] = s_h[d];
+      const int ncy = hi[1] - lo[1] + 1, ncols = columns();
+      // columns are cut to the cells within the largest radius of the home
+      // cell: at 4.0 with cells of 2.86, 81 cells of 125 remain
+      const bool trim = minimg && !full[0] && !full[1] && !full[2] && nl_runs_bounded(ncols);
+      int base_r = 0, base_a = 0;
+      for (int col0 = 0; col0 < ncols; col0 += all ? (int)blockDim.x : 32) {
+        const int col = col0 + threadIdx.x;
+        int jb_s[3], cnt_s[3], rs[3], rz0[3], len_s[3], ra_s[3], nseg = 0;
+        int ix = 0, iy = 0, sx = 0, sy = 0, colbase = 0;
+        if (col < ncols) {
+          ix = lo[0] + col / ncy;
+          iy = lo[1] + col % ncy;
+          int cx = ix, cy = iy;
+          if (cx < 0) { cx += g.nc[0]; sx = 1; } else if (cx >= g.nc[0]) { cx -= g.nc[0]; sx = -1; }
+          if (cy < 0) { cy += g.nc[1]; sy = 1; } else if (cy >= g.nc[1]) { cy -= g.nc[1]; sy = -1; }
+          colbase = g.nc[2] * (cy + g.nc[1] * cx);
+          int ra[3], rb[3], ns = 0;
+          if (full[2]) { ra[0] = 0; rb[0] = g.nc[2] - 1; rs[0] = 0; rz0[0] = 0; ns = 1; }
+          else {
+            int zlo = lo[2], zhi = hi[2];
+            if (trim) {
+              const float gx = (float)h[0] * (float)max(0, max(ix - hc[0], hc[0] - ix) - 1);
+              const float gy = (float)h[1] * (float)max(0, max(iy - hc[1], hc[1] - iy) - 1);
+              const float rf = (float)s_rle, w2 = rf * rf - (gx * gx + gy * gy);
+              const float zc = sqrtf(fmaxf(w2, 0.f)) / (float)h[2];  // reach along z in cells
+              zlo = max(zlo, hc[2] - (int)ceilf(zc));
+              zhi = w2 < 0.f ? zlo - 1 : min(zhi, hc[2] + 1 + (int)floorf(zc));
+            }
+            if (zlo <= zhi) {
+              if (zlo < 0) {
+                ra[ns] = zlo + g.nc[2]; rb[ns] = min(zhi, -1) + g.nc[2]; rs[ns] = 1; rz0[ns] = zlo; ++ns;
+              }
+              const int za = max(zlo, 0), zb = min(zhi, g.nc[2] - 1);
+              if (za <= zb) { ra[ns] = za; rb[ns] = zb; rs[ns] = 0; rz0[ns] = za; ++ns; }
+              if (zhi >= g.nc[2]) {
+                const int z0 = max(zlo, g.nc[2]);
+                ra[ns] = z0 - g.nc[2]; rb[ns] = zhi - g.nc[2]; rs[ns] = -1; rz0[ns] = z0; ++ns;
+              }
+            }
+          }
+          for (int s = 0; s < ns; ++s) {
+            const int jb = (int)start[colbase + ra[s]], je = (int)start[colbase + rb[s] + 1];
+            if (je == jb) continue;
+            jb_s[nseg] = jb; cnt_s[nseg] = je - jb; len_s[nseg] = rb[s] - ra[s];
+            rs[nseg] = rs[s]; rz0[nseg] = rz0[s]; ra_s[nseg] = ra[s];
+            ++nseg;
+          }
+        }
+        int atoms = 0;
+        for (int s = 0; s < nseg; ++s) atoms += cnt_s[s];
+        int ir = nseg, ia = atoms;  // inclusive scans
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int vr = __shfl_up_sync(0xffffffffu, ir, o), va = __shfl_up_sync(0xffffffffu, ia, o);
+          if (lane >= o) { ir += vr; ia += va; }
+        }
+        int r_off = base_r + ir - nseg, a_off = base_a + ia - atoms;
+        if (all) {
+          if (lane == 31) { scan_r[warp] = ir; scan_a[warp] = ia; }
+          __syncthreads();
+          for (int w = 0; w < nwarp; ++w) {
+            const int vr = scan_r[w], va = scan_a[w];
+            if (w < warp) { r_off += vr; a_off += va; }
+            base_r += vr;
+            base_a += va;
+          }
+        } else {
+          base_r += __shfl_sync(0xffffffffu, ir, 31);
+          base_a += __shfl_sync(0xffffffffu, ia, 31);
+        }
+        for (int s = 0; s < nseg; ++s) {
+          if (r_off >= NL_MAX_RUNS) break;
+          const int q = r_off;
+          rt.jb[q] = jb_s[s]; rt.cnt[q] = cnt_s[s]; rt.off[q] = a_off;
+          rt.code[q] = img_code(sx, sy, rs[s]);
+          const int zc0 = rz0[s], zc1 = rz0[s] + len_s[s];
+          rt.b0[0][q] = full[0] ? -1e30f : (float)(ix * h[0]); rt.b1[0][q] = full[0] ? 1e30f : (float)((ix + 1) * h[0]);
+          rt.b0[1][q] = full[1] ? -1e30f : (float)(iy * h[1]); rt.b1[1][q] = full[1] ? 1e30f : (float)((iy + 1) * h[1]);
+          rt.b0[2][q] = full[2] ? -1e30f : (float)(zc0 * h[2]); rt.b1[2][q] = full[2] ? 1e30f : (float)((zc1 + 1) * h[2]);
+          // per-cell offsets for the per-atom z window (runs that do not wrap the
+          // whole z axis and have at most NL_RUN_MAXZ cells)
+          rt.zc0[q] = zc0;
+          const int nzq = (!full[2] && len_s[s] + 1 <= NL_RUN_MAXZ && cnt_s[s] <= 65535) ? len_s[s] + 1 : 0;
+          rt.nz[q] = nzq;
+          for (int k = 0; k < nzq; ++k)
+            rt.zoff[k][q] = (unsigned short)((int)start[colbase + ra_s[s] + k] - jb_s[s]);
+          if (nzq) rt.zoff[nzq][q] = (unsigned short)cnt_s[s];
+          ++r_off;
+          a_off += cnt_s[s];
+        }
+        if (all && col0 + (int)blockDim.x < ncols) __syncthreads();  // the scans have been read
+      }
+      if (threadIdx.x == 0) {
+        s_nr = base_r;
+        s_atoms = base_a;
+        if (base_r > NL_MAX_RUNS) atomicOr(&stw->flags, FLAG_NL_OVERFLOW);
+      }
+    }
+    __syncthreads();
+    if (all || columns() <= 32) break;
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) h[d] = s_h[d];
+  // When the stencil spans less than the box along every axis, each cell
+  // appears in exactly one run, at that run's periodic image k_run, and
+  // 2 rlist < L.  For any pair within rlist the reference's image
+  // floor((r_j - r_i)/L + 1/2) is then k_run (it can differ only where
+  // |d| is within rounding of L/2 > rlist, where both reject), so
+  // d = (r_j - r_i) - k_run L repeats the reference's binary32 operations and
+  // the image code is the run's.
+  const bool runshift = minimg && !s_full[0] && !s_full[1] && !s_full[2];
+  const int nr = min(s_nr, NL_MAX_RUNS), tile_n = s_atoms;
   // stage the runs into the tile; a home cell with fewer than NL_LIGHT atoms
   // reads its candidates from L2 instead (staging would cost more than the
   // few reads it saves).  A run's cells are staged in their z order (zord),
   // so each cell of the run is a z-sorted slice of the tile.
-  const bool stage = tile_n <= NL_TILE_BYTES / (int)sizeof(float4) && !(s_flags & 2) && (i1 - i0) >= NL_LIGHT;
+  const int room = tile_bytes - (runshift ? 0 : nl_shift_bytes<R>());
+  const int entry = runshift || SCREEN ? (int)sizeof(float4) : (int)sizeof(T4);
+  const bool stage = tile_n <= room / entry && s_nr <= NL_MAX_RUNS && (i1 - i0) >= NL_LIGHT;
   const bool fast = stage && runshift;
+  // binary64 without one image per run: the stored positions where they fit, so
+  // that a candidate within the radius is not read from L2 again
+  const bool whole = stage && !runshift && tile_n <= room / (int)sizeof(T4);
+  T4* const wtile = reinterpret_cast<T4*>(nl_smem);
   // frame of the packed tile: the box (binary32), or the home cell's corner,
   // so that binary64 positions lose nothing but their last binary32 digit
   R corner[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) corner[d] = (fast && sizeof(R) == 8) ? (R)(hc[d] * h[d]) : R(0);
-  if (stage) {
+  if (fast) {
     // a warp takes four runs at a time, so that four of the two dependent
     // loads of an entry (its slot, then the position) are in flight per lane
     constexpr int U = 4;
@@ -423,16 +491,26 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
         for (int u = 0; u < U; ++u)
           if (jj[u] >= 0) v[u] = pos[jj[u]];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (jj[u] < 0) continue;
-          if (runshift) {
+        for (int u = 0; u < U; ++u)
+          if (jj[u] >= 0)
             ftile[off[u] + t] = make_float4((float)(v[u].x - img_shift<R>(code[u], 0, L[0]) - corner[0]),
                                             (float)(v[u].y - img_shift<R>(code[u], 1, L[1]) - corner[1]),
                                             (float)(v[u].z - img_shift<R>(code[u], 2, L[2]) - corner[2]),
                                             __int_as_float(jj[u] | code[u]));
-          } else {
-            ftile[off[u] + t] = make_float4((float)v[u].x, (float)v[u].y, (float)v[u].z, __int_as_float(jj[u]));
-          }
+      }
+    }
+  } else if (stage) {
+    // whole stencils without a radius to cut them: long runs, a warp each
+    for (int r = warp; r < nr; r += nwarp) {
+      const int cnt = rt.cnt[r], off = rt.off[r], jb = rt.jb[r];
+      for (int t = lane; t < cnt; t += 32) {
+        const int j = (int)zord[jb + t];
+        T4 v = pos[j];
+        if (sizeof(R) == 4 || whole) {
+          v.w = slot_as_w<R>(j);
+          wtile[off + t] = v;
+        } else {
+          ftile[off + t] = make_float4((float)v.x, (float)v.y, (float)v.z, __int_as_float(j));
         }
       }
     }
@@ -443,13 +521,13 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
   const unsigned lemask = (2u << lane) - 1u;  // lanes 0..lane (all 32 for lane 31)
   // per-warp table of the current run group's non-empty runs (rank order)
   __shared__ int wdelta[8][32];
-  __shared__ int wcode[8][32];
+  T4* const wshift = reinterpret_cast<T4*>(nl_smem + tile_bytes - nl_shift_bytes<R>()) + 32 * warp;
   const float hz = (float)h[2], hzi = 1.0f / hz;
   const float Lzf = (float)st->L[2], cz = (float)corner[2];
   // z of entry t of a run (z order) in the frame of the run: the stored,
   // wrapped one, or the packed tile's
   auto zat = [&](int roff, int rjb, int t) -> float {
-    return glob ? (float)pos[zord[rjb + t]].z : ftile[roff + t].z;
+    return glob ? (float)pos[zord[rjb + t]].z : sizeof(R) == 8 && whole ? (float)wtile[roff + t].z : ftile[roff + t].z;
   };
   // Bound on the difference between the packed tile's squared distance and
   // the reference's (coordinates and differences rounded to binary32, each
@@ -553,7 +631,11 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
         const int r = rb + lane;
         const int k = __popc(nem & ltmask);
         wdelta[warp][k] = (glob ? rt.jb[r] : rt.off[r]) + tbl - excl;
-        wcode[warp][k] = rt.code[r];
+        if (!fast) {
+          const int code = rt.code[r];
+          wshift[k] = T4{img_shift<R>(code, 0, L[0]), img_shift<R>(code, 1, L[1]), img_shift<R>(code, 2, L[2]),
+                         slot_as_w<R>(code)};
+        }
       }
       __syncwarp();
       const int first = ne ? excl : 0x7fffffff;  // where the lane's range starts
@@ -594,75 +676,105 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
         }
         continue;
       }
-      for (int t0 = 0; t0 < total; t0 += 32) {
-        const int cidx = t0 + lane;
+      // the candidates of one chunk in the order of the runs; k: which run's
+      auto chunk = [&](int t0) -> int {
         const unsigned rel = (unsigned)(first - t0);
         const unsigned smask = __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
         const int k = before + __popc(smask & lemask);
         before += __popc(smask);
-        bool ok = false, test = cidx < total;
-        int j = 0, code = 0;
-        T4 pj = pi;
-        if (test) {
-          const int x = cidx + wdelta[warp][k];
-          code = wcode[warp][k];
-          if (glob) {
-            j = (int)zord[x];
-            pj = pos[j];
+        return k;
+      };
+      // the reference's operations on a stored position; the image in code
+      auto exact = [&](const T4& pj, const T4& sh, int& code) -> bool {
+        R dx, dy, dz, d2;
+        if (runshift) {
+          dz = sub_rn(sub_rn(pj.z, pi.z), sh.z);
+          if constexpr (std::is_same<R, float>::value) {
+            // x and y as one packed binary32 pair: the same roundings
+            const F2 dxy = f2_sub(f2_sub(f2(pj.x, pj.y), f2(pi.x, pi.y)), f2(sh.x, sh.y));
+            float sx, sy;
+            f2_split(f2_mul(dxy, dxy), sx, sy);
+            d2 = __fadd_rn(__fadd_rn(sx, sy), __fmul_rn(dz, dz));
           } else {
-            const float4 q = ftile[x];
-            j = __float_as_int(q.w);
-            if constexpr (sizeof(R) == 4) {
-              pj = T4{q.x, q.y, q.z, q.w};
-            } else {
-              // binary64: a binary32 distance (nearest image, or the run's in
-              // cell-shift mode) first; what is within its error bound of the
-              // radius, or nearer, is read and tested as stored
-              float dx = q.x - ri.x, dy = q.y - ri.y, dz = q.z - ri.z;
-              if (minimg) {
-                dx -= Lf[0] * rintf(dx * Lif[0]);
-                dy -= Lf[1] * rintf(dy * Lif[1]);
-                dz -= Lf[2] * rintf(dz * Lif[2]);
-              } else {
-                dx -= img_shift<float>(code, 0, Lf[0]);
-                dy -= img_shift<float>(code, 1, Lf[1]);
-                dz -= img_shift<float>(code, 2, Lf[2]);
-              }
-              test = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < out2;
-              if (test) pj = pos[j];
-            }
-          }
-        }
-        if (test) {
-          R d2;
-          if (runshift) {
-            d2 = nl_exact_d2<R>(pj, pi, code, L);
-          } else {
-            const R rx = sub_rn(pj.x, pi.x), ry = sub_rn(pj.y, pi.y), rz = sub_rn(pj.z, pi.z);
-            const R kx = floor_r(add_rn(mul_rn(rx, Li[0]), R(0.5)));
-            const R ky = floor_r(add_rn(mul_rn(ry, Li[1]), R(0.5)));
-            const R kz = floor_r(add_rn(mul_rn(rz, Li[2]), R(0.5)));
-            R dx, dy, dz;
-            if (minimg) {
-              dx = sub_rn(rx, mul_rn(kx, L[0]));
-              dy = sub_rn(ry, mul_rn(ky, L[1]));
-              dz = sub_rn(rz, mul_rn(kz, L[2]));
-            } else {
-              dx = sub_rn(sub_rn(pj.x, img_shift<R>(code, 0, L[0])), pi.x);
-              dy = sub_rn(sub_rn(pj.y, img_shift<R>(code, 1, L[1])), pi.y);
-              dz = sub_rn(sub_rn(pj.z, img_shift<R>(code, 2, L[2])), pi.z);
-            }
-            code = img_code((int)kx, (int)ky, (int)kz);
+            dx = sub_rn(sub_rn(pj.x, pi.x), sh.x);
+            dy = sub_rn(sub_rn(pj.y, pi.y), sh.y);
             d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
           }
-          ok = (d2 < rl2) && (j != i);
+          code = slot_of_w<R>(sh.w);
+        } else {
+          const R rx = sub_rn(pj.x, pi.x), ry = sub_rn(pj.y, pi.y), rz = sub_rn(pj.z, pi.z);
+          const R kx = floor_r(add_rn(mul_rn(rx, Li[0]), R(0.5)));
+          const R ky = floor_r(add_rn(mul_rn(ry, Li[1]), R(0.5)));
+          const R kz = floor_r(add_rn(mul_rn(rz, Li[2]), R(0.5)));
+          if (minimg) {
+            dx = sub_rn(rx, mul_rn(kx, L[0]));
+            dy = sub_rn(ry, mul_rn(ky, L[1]));
+            dz = sub_rn(rz, mul_rn(kz, L[2]));
+          } else {
+            dx = sub_rn(sub_rn(pj.x, sh.x), pi.x);
+            dy = sub_rn(sub_rn(pj.y, sh.y), pi.y);
+            dz = sub_rn(sub_rn(pj.z, sh.z), pi.z);
+          }
+          code = img_code((int)kx, (int)ky, (int)kz);
+          d2 = add_rn(add_rn(mul_rn(dx, dx), mul_rn(dy, dy)), mul_rn(dz, dz));
         }
+        return d2 < rl2;
+      };
+      auto keep_entry = [&](bool ok, int j, int code) {
         const unsigned m = __ballot_sync(0xffffffffu, ok);
         if (ok) {
           const int p = n + __popc(m & ltmask);
           if (p < cap) rowp[nl_slot(p)] = j | code;
         }
         n += __popc(m);
+      };
+      if constexpr (sizeof(R) == 8 && SCREEN) {
+        if (!glob && !whole) {
+          // binary64: a binary32 distance (nearest image, or the run's in
+          // cell-shift mode) first; what is within its error bound of the
+          // radius, or nearer, is read and tested as stored
+          for (int t0 = 0; t0 < total; t0 += 32) {
+            const int k = chunk(t0), cidx = t0 + lane;
+            bool ok = false;
+            int j = 0, code = 0;
+            if (cidx < total) {
+              const float4 q = ftile[cidx + wdelta[warp][k]];
+              const T4 sh = wshift[k];
+              j = __float_as_int(q.w);
+              float dx = q.x - ri.x, dy = q.y - ri.y, dz = q.z - ri.z;
+              if (minimg) {
+                dx -= Lf[0] * rintf(dx * Lif[0]);
+                dy -= Lf[1] * rintf(dy * Lif[1]);
+                dz -= Lf[2] * rintf(dz * Lif[2]);
+              } else {
+                dx -= (float)sh.x;
+                dy -= (float)sh.y;
+                dz -= (float)sh.z;
+              }
+              if (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < out2) ok = exact(pos[j], sh, code) && j != i;
+            }
+            keep_entry(ok, j, code);
+          }
+          continue;
+        }
+      }
+      for (int t0 = 0; t0 < total; t0 += 32) {
+        const int k = chunk(t0), cidx = t0 + lane;
+        bool ok = false;
+        int j = 0, code = 0;
+        if (cidx < total) {
+          const int x = cidx + wdelta[warp][k];
+          T4 pj;
+          if (glob) {
+            j = (int)zord[x];
+            pj = pos[j];
+          } else {
+            pj = wtile[x];
+            j = slot_of_w<R>(pj.w);
+          }
+          ok = exact(pj, wshift[k], code) && j != i;
+        }
+        keep_entry(ok, j, code);
       }
     }
     nmax = max(nmax, n);
@@ -679,40 +791,61 @@ __device__ __forceinline__ void nl_build_cell(int c, const typename V4<R>::T* __
   }
 }
 
-template <class R, int MODE>
-__global__ void __launch_bounds__(256, 4)
+template <class R, int MODE, int MINB>
+__global__ void __launch_bounds__(256, MINB)
 k_nl_build(int N, const typename V4<R>::T* __restrict__ pos, const float* __restrict__ rcut,
            const uint32_t* __restrict__ start, const uint32_t* __restrict__ zord, NlGeom g,
            const DevState* __restrict__ st, double rlist_uniform, double skin, int cap, int* __restrict__ list,
            int* __restrict__ nnb, typename V4<R>::T* __restrict__ backup, int force_minimage, DevState* stw,
-           int gate) {
+           int gate, int light_blocks, int tile_bytes) {
   if (gate && !(st->flags & FLAG_REBUILD)) return;
-  const bool minimg = (MODE == MD_NL_MINIMAGE) || force_minimage;
-  const int c = blockIdx.x;
-  if (minimg) {
-    // the light cells among 8 neighbouring ones, a warp each
-    const int ntot = g.nc[0] * g.nc[1] * g.nc[2], cw = c + (int)(threadIdx.x >> 5);
-    if ((c & 7) == 0 && cw < ntot) {
+  int c = (int)blockIdx.x;
+  if (light_blocks >= 0) {
+    // light cells a warp each, 8 neighbouring cells a block: by light_blocks blocks of
+    // their own, or (0) by the block of the first of them before its own cell
+    const int ntot = g.nc[0] * g.nc[1] * g.nc[2], warp = (int)(threadIdx.x >> 5), l = c - nl_light_at(ntot);
+    const bool own = l >= 0 && l < light_blocks;
+    if (light_blocks > 0 && l >= light_blocks) c -= light_blocks;
+    const int cw = own ? 8 * l + warp : c + warp;
+    if ((own || (light_blocks == 0 && (c & 7) == 0)) && cw < ntot) {
       const int a = (int)start[cw], n = (int)start[cw + 1] - a;
       if (n > 0 && n < NL_LIGHT)
         nl_light_cell<R>(cw, a, a + n, MODE == MD_NL_MINIMAGE, pos, rcut, start, zord, g, st, rlist_uniform, skin, cap,
                          false, list, nnb, backup, stw);
     }
+    if (own) return;
     const int a = (int)start[c], n = (int)start[c + 1] - a;
     if (n < NL_LIGHT && (n == 0 || nl_light_cell<R>(c, a, a + n, MODE == MD_NL_MINIMAGE, pos, rcut, start, zord, g, st,
                                                     rlist_uniform, skin, cap, true, list, nnb, backup, stw)))
       return;
   }
-  nl_build_cell<R, MODE>(c, pos, rcut, start, zord, g, st, rlist_uniform, skin, cap, list, nnb, backup,
-                         force_minimage, stw);
+  constexpr bool SCREEN = MODE != MD_NL_MINIMAGE || MINB != NL_WIDE;
+  nl_build_cell<R, MODE, SCREEN>(c, pos, rcut, start, zord, g, st, rlist_uniform, skin, cap, list, nnb, backup,
+                                 force_minimage, stw, tile_bytes);
 }
 
-static const void* nl_kernel(int prec, int mode) {
+template <int MINB>
+static const void* nl_pick(int prec, int mode) {
   if (prec == MD_PREC_FP64)
-    return mode == MD_NL_MINIMAGE ? (const void*)k_nl_build<double, MD_NL_MINIMAGE>
-                                  : (const void*)k_nl_build<double, MD_NL_CELLSHIFT>;
-  return mode == MD_NL_MINIMAGE ? (const void*)k_nl_build<float, MD_NL_MINIMAGE>
-                                : (const void*)k_nl_build<float, MD_NL_CELLSHIFT>;
+    return mode == MD_NL_MINIMAGE ? (const void*)k_nl_build<double, MD_NL_MINIMAGE, MINB>
+                                  : (const void*)k_nl_build<double, MD_NL_CELLSHIFT, MINB>;
+  return mode == MD_NL_MINIMAGE ? (const void*)k_nl_build<float, MD_NL_MINIMAGE, MINB>
+                                : (const void*)k_nl_build<float, MD_NL_CELLSHIFT, MINB>;
+}
+
+// the kernel of a build, its tile and the largest tile it is launched with
+struct NlPlan {
+  const void* f;
+  int tile_bytes, limit;
+};
+
+// stencil: atoms of a stencil at the mean density; spans: a minimum-image stencil
+// spans the box along an axis
+static NlPlan nl_plan(int prec, int mode, int ntot, int sms, double stencil, bool spans) {
+  if (ntot <= NL_SMALL * sms) return {nl_pick<NL_SMALL>(prec, mode), NL_TILE_SMALL, NL_TILE_SMALL};
+  if (prec == MD_PREC_FP64 && spans) return {nl_pick<NL_MID>(prec, mode), NL_TILE_MID, NL_TILE_MID};
+  const bool none = stencil > 1.25 * NL_TILE_BYTES / sizeof(float4);
+  return {nl_pick<NL_WIDE>(prec, mode), none ? NL_TILE_NONE : NL_TILE_BYTES, NL_TILE_BYTES};
 }
 
 // cell-list criterion needs >= 4 cells per direction (DecideNumCell), else the
@@ -742,10 +875,28 @@ int nlist_build_impl(md_nlist* nl, md_system* sys, md_cell_list* cl, Recorder* r
   double rl = nl->rlist, skin = nl->skin;
   DevState* st = sys->st;
   int cap = nl->cap;
-  dim3 grid(cl->ntot), block(256);
+  const bool minimg = nl->mode == MD_NL_MINIMAGE || force_mi;
+  int light_blocks = !minimg || !nl_light_cells(cl->ntot) ? -1 : cl->ntot <= NL_LIGHT_OWN ? ceil_div(cl->ntot, 8) : 0;
+  // (cells keep their number when the box breathes: their size at creation serves)
+  double cells = 1.0;
+  bool spans = false;
+  for (int d = 0; d < 3; ++d) {
+    const double across = 2.0 * std::ceil(nl->rlist / cl->h[d]) + 1.0;
+    spans = spans || across >= cl->ncell[d];
+    cells *= std::min(across, (double)cl->ncell[d]);
+  }
+  // of a stencil cut to the sphere about two thirds remain
+  const double stencil = cells * (minimg && !spans ? 0.65 : 1.0) * N / cl->ntot;
+  NlPlan plan = nl_plan(sys->prec, nl->mode, cl->ntot, nl->sms, stencil, spans && minimg);
+  // the limit belongs to the kernel on the list's device: with every list, for the builds that it takes
+  if (nl->prepared != plan.f) {
+    MD_CUDA(cudaFuncSetAttribute(plan.f, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.limit));
+    nl->prepared = plan.f;
+  }
+  dim3 grid(cl->ntot + std::max(light_blocks, 0)), block(256);
   void* a[] = {&N, &sys->pos, &sys->rcut, &cl->start, &cl->zord, &g, &st, &rl, &skin, &cap, &nl->list,
-               &nl->nnb, &nl->backup, &force_mi, &st, &gate};
-  if (int r = rec_launch(rec, nl_kernel(sys->prec, nl->mode), grid, block, NL_TILE_BYTES, a)) return r;
+               &nl->nnb, &nl->backup, &force_mi, &st, &gate, &light_blocks, &plan.tile_bytes};
+  if (int r = rec_launch(rec, plan.f, grid, block, plan.tile_bytes, a)) return r;
   if (int r = topo_exclude_launch(sys, nl, rec, gated)) return r;
   nl->built = true;
   return MD_OK;
@@ -778,7 +929,7 @@ struct RebuildArgs {
   uint8_t* type;
   DevState* st;
   double rlist, skin;
-  int cap, force_mi;
+  int cap, force_mi, tile_bytes;
   int *list, *nnb;
   T4* backup;
 };
@@ -786,8 +937,6 @@ struct RebuildArgs {
 // Resident blocks per SM the kernels are built for: four, which is what the list
 // tile leaves room for, at 64 registers and some spills; or two, without spills,
 // where a launch has no more than two blocks per SM (rebuild_kernel)
-#define REBUILD_WIDE 4
-#define REBUILD_SMALL 2
 
 // the atoms of this block in the per-atom phases: a contiguous share of
 // ceil(N / blocks), so that every block (and every SM) takes part
@@ -855,8 +1004,8 @@ __device__ __forceinline__ void rebuild_phases(const RebuildArgs<R>& a) {
   // change any list), the light ones eight at a time, a warp each; the next
   // share is fetched while this one is built
   const int nfull = (int)__ldcg(&st->ncell_busy), nlight = (int)__ldcg(&st->ncell_light);
-  const int nbusy = nfull + (nlight + 7) / 8;
-  const bool minimg = (MODE == MD_NL_MINIMAGE) || a.force_mi;
+  const bool by_warp = (MODE == MD_NL_MINIMAGE) || a.force_mi;
+  const int share = by_warp ? 8 : 1, nbusy = nfull + (nlight + share - 1) / share;
   __shared__ int s_work;
   __shared__ unsigned s_left;  // light cells of a share that need the whole block
   if (threadIdx.x == 0) s_work = (int)atomicAdd(&st->red_counter[RED_NLWORK], 1u);
@@ -866,13 +1015,13 @@ __device__ __forceinline__ void rebuild_phases(const RebuildArgs<R>& a) {
     int nxt = 0;
     if (threadIdx.x == 0) { nxt = (int)atomicAdd(&st->red_counter[RED_NLWORK], 1u); s_left = 0u; }
     unsigned left = 1u;  // cells of this share for the whole block
-    const int l0 = 8 * (w - nfull);
-    if (w >= nfull) {
+    const int l0 = share * (w - nfull);
+    if (w >= nfull && by_warp) {
       __syncthreads();
       const int l = l0 + (int)(threadIdx.x >> 5);
       if (l < nlight) {
         const int c = (int)__ldcg(&a.busy[a.ntot - 1 - l]), i0 = (int)a.start[c], i1 = (int)a.start[c + 1];
-        const bool done = minimg && nl_light_cell<R>(c, i0, i1, MODE == MD_NL_MINIMAGE, a.pos, a.rcut, a.start, a.zord,
+        const bool done = nl_light_cell<R>(c, i0, i1, MODE == MD_NL_MINIMAGE, a.pos, a.rcut, a.start, a.zord,
                                                      a.ng, st, a.rlist, a.skin, a.cap, false, a.list, a.nnb, a.backup,
                                                      st);
         if (!done && lane == 0) atomicOr(&s_left, 1u << (threadIdx.x >> 5));
@@ -882,8 +1031,8 @@ __device__ __forceinline__ void rebuild_phases(const RebuildArgs<R>& a) {
     }
     for (; left; left &= left - 1u) {
       const int b = w < nfull ? w : a.ntot - 1 - (l0 + __ffs((int)left) - 1);
-      nl_build_cell<R, MODE>((int)__ldcg(&a.busy[b]), a.pos, a.rcut, a.start, a.zord, a.ng, st, a.rlist, a.skin, a.cap,
-                             a.list, a.nnb, a.backup, a.force_mi, st);
+      nl_build_cell<R, MODE, true>((int)__ldcg(&a.busy[b]), a.pos, a.rcut, a.start, a.zord, a.ng, st, a.rlist, a.skin, a.cap,
+                             a.list, a.nnb, a.backup, a.force_mi, st, a.tile_bytes);
       __syncthreads();
     }
     __syncthreads();
@@ -946,9 +1095,9 @@ static const void* rebuild_pick(int prec, int mode, bool with_lv) {
 
 static const void* rebuild_kernel(int prec, int mode, size_t* smem, int* blocks, bool with_lv = false,
                                   int* sms = nullptr, bool small = false) {
-  const void* f = small ? rebuild_pick<REBUILD_SMALL>(prec, mode, with_lv)
-                        : rebuild_pick<REBUILD_WIDE>(prec, mode, with_lv);
-  *smem = NL_TILE_BYTES;
+  const void* f = small ? rebuild_pick<NL_SMALL>(prec, mode, with_lv)
+                        : rebuild_pick<NL_WIDE>(prec, mode, with_lv);
+  *smem = small ? NL_TILE_SMALL : NL_TILE_BYTES;
   *blocks = 0;
   int dev = 0, coop = 0, nsm = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
@@ -1012,11 +1161,13 @@ static int rebuild_fused_t(md_cell_list* cl, md_nlist* nl, md_system* sys, Recor
   // 12,000 63 and 4.6, 68 and 4.7; binary64 4,000 55 and 4.7, 60 and 4.9, and 33
   // against 37 a whole step from a cold L2).  More blocks want the registers: the
   // 65,536-atom slab in binary64 348 with four blocks an SM, 427 with two
-  if (want <= REBUILD_SMALL * sms && blocks >= want) {
+  if (want <= NL_SMALL * sms && blocks >= want) {
     int fit = 0;
-    const void* g = rebuild_kernel(sys->prec, nl->mode, &smem, &fit, with_lv, nullptr, true);
-    if (fit >= want) { f = g; blocks = fit; }
+    size_t mem = 0;
+    const void* g = rebuild_kernel(sys->prec, nl->mode, &mem, &fit, with_lv, nullptr, true);
+    if (fit >= want) { f = g; blocks = fit; smem = mem; }
   }
+  a.tile_bytes = (int)smem;
   blocks = std::min(blocks, want);
   if (!with_lv) {
     void* args[] = {&a};
@@ -1094,14 +1245,16 @@ extern "C" int md_nlist_create(md_nlist** out, md_system* sys, double rlist, dou
   }
   DevState hs;
   if (int r = sys->read_state(hs)) return r;
-  // with every list: the limit belongs to the kernel on the list's device
-  MD_CUDA(cudaFuncSetAttribute(nl_kernel(sys->prec, mode), cudaFuncAttributeMaxDynamicSharedMemorySize, NL_TILE_BYTES));
+  int device = 0, sms = 0;
+  MD_CUDA(cudaGetDevice(&device));
+  MD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   md_nlist* nl = new md_nlist();
   nl->rlist = rlist;
   nl->skin = skin;
   nl->expansion = expansion;
   nl->mode = mode;
   nl->N = sys->N;
+  nl->sms = sms;
   // mallocDeviceNeighborList: 4/3 pi rlist^3 rho * expansion, at least 30
   double rho = sys->N / (hs.L[0] * hs.L[1] * hs.L[2]);
   double expect = 4.0 / 3.0 * M_PI * rlist * rlist * rlist * rho;
