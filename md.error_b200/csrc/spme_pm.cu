@@ -309,7 +309,10 @@ k_spme_spread_direct(int N, const typename V4<R>::T* __restrict__ pos, int K0, i
 // reads where neighbouring atoms share little (ik, 65,536 charges on
 // 128 x 128 x 512: 62 us for 270 MB of sectors), else latency.  Against staging
 // each block's mesh region in shared memory (us): 20,736 charges on 64^3 14.6
-// from 22.4 (ik), 11.6 from 25.1 (analytic); in binary64 15.5 from 37.7.
+// from 22.4 (ik), 11.6 from 25.1 (analytic); in binary64 15.5 from 37.7.  Orders 11
+// to 14 put two rows to an instruction and go plane by plane (whole forces,
+// 1,000,000 charges on 128^3 at order 14: 5.3 ms analytic and 6.3 ik, 8.1 and 8.2 with
+// every row's weights read anew, 6.5 and 14.3 by staged regions).
 //   MODE 0: ik, the three convolved meshes interleaved, one Real4 per point
 //   MODE 1: analytic differentiation of the single convolved mesh
 // store: force is a separate buffer that receives every atom's reciprocal
@@ -361,25 +364,60 @@ k_spme_gather_t(int N, const typename V4<R>::T* __restrict__ pos, int K0, int K1
       if (((charged >> at) & 1u) && in) {
         const int b0 = sb[warp][0][at], b1 = sb[warp][1][at], gz = (sb[warp][2][at] - c) & (K2 - 1);
         const R wz = sw[warp][2][at][c][0];
-#pragma unroll 8
-        for (int j = 0; j < NI; ++j) {
-          const int row = j * RP + k;
-          if (row < NR) {
-            const int a = row / NO, b = row - a * NO;
-            const size_t at_mesh = ((size_t)((b0 - a) & (K0 - 1)) * K1 + ((b1 - b) & (K1 - 1))) * K2 + gz;
-            const R wa = sw[warp][0][at][a][0], wb = sw[warp][1][at][b][0];
+        if constexpr (RP == 2) {
+          // orders 11 to 14, two rows an instruction: the rows of a plane share its weights
+#pragma unroll 1
+          for (int a = 0; a < NO; ++a) {
+            const size_t plane = (size_t)((b0 - a) & (K0 - 1)) * K1;
+            R t0 = R(0), t1 = R(0), t2 = R(0);  // over the plane's rows: m w_b each, or m w_b and m w'_b
+#pragma unroll
+            for (int b = 0; b < NO; b += 2) {
+              if (NO % 2 && b + k >= NO) break;
+              const size_t at_mesh = (plane + ((b1 - b - k) & (K1 - 1))) * K2 + gz;
+              const R wb = sw[warp][1][at][b + k][0];
+              if constexpr (MODE == 0) {
+                const R4 m = reinterpret_cast<const R4*>(Gv)[at_mesh];
+                t0 += m.x * wb;
+                t1 += m.y * wb;
+                t2 += m.z * wb;
+              } else {
+                const R m = reinterpret_cast<const R*>(Gv)[at_mesh];
+                t0 += m * wb;
+                t1 += m * sw[warp][1][at][b + k][ND - 1];
+              }
+            }
+            const R wa = sw[warp][0][at][a][0];
             if constexpr (MODE == 0) {
-              const R4 m = reinterpret_cast<const R4*>(Gv)[at_mesh];
-              const R w = wa * wb;
-              s0 += m.x * w;
-              s1 += m.y * w;
-              s2 += m.z * w;
+              s0 += wa * t0;
+              s1 += wa * t1;
+              s2 += wa * t2;
             } else {
-              const R m = reinterpret_cast<const R*>(Gv)[at_mesh];
-              const R da = sw[warp][0][at][a][ND - 1], db = sw[warp][1][at][b][ND - 1];
-              s0 += m * (da * wb);
-              s1 += m * (wa * db);
-              s2 += m * (wa * wb);
+              s0 += sw[warp][0][at][a][ND - 1] * t0;
+              s1 += wa * t1;
+              s2 += wa * t0;
+            }
+          }
+        } else {
+#pragma unroll 8
+          for (int j = 0; j < NI; ++j) {
+            const int row = j * RP + k;
+            if (row < NR) {
+              const int a = row / NO, b = row - a * NO;
+              const size_t at_mesh = ((size_t)((b0 - a) & (K0 - 1)) * K1 + ((b1 - b) & (K1 - 1))) * K2 + gz;
+              const R wa = sw[warp][0][at][a][0], wb = sw[warp][1][at][b][0];
+              if constexpr (MODE == 0) {
+                const R4 m = reinterpret_cast<const R4*>(Gv)[at_mesh];
+                const R w = wa * wb;
+                s0 += m.x * w;
+                s1 += m.y * w;
+                s2 += m.z * w;
+              } else {
+                const R m = reinterpret_cast<const R*>(Gv)[at_mesh];
+                const R da = sw[warp][0][at][a][ND - 1], db = sw[warp][1][at][b][ND - 1];
+                s0 += m * (da * wb);
+                s1 += m * (wa * db);
+                s2 += m * (wa * wb);
+              }
             }
           }
         }
