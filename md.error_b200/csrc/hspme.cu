@@ -591,29 +591,37 @@ struct md_hspme {
   double* cpart = nullptr;   // [B][nab][ncoef]
   double* lpart = nullptr;   // [B][nab]
   double* R = nullptr;       // [B][N][3] residual weights
+  void* slab = nullptr;      // the memory of all of these
 };
 
 static void hs_free(md_hspme* h) {
-  void* p[] = {h->Z, h->F, h->Y, h->e2, h->w, h->bfac, h->dbfac, h->marg, h->cpart, h->lpart, h->R};
-  for (void* x : p) if (x) cudaFree(x);
-  h->Z = h->F = h->Y = nullptr;
-  h->e2 = h->w = h->bfac = h->dbfac = h->marg = h->cpart = h->lpart = h->R = nullptr;
+  if (h->slab) cudaFree(h->slab);
+  h->slab = nullptr;
 }
 
-// workspace for batches of B candidates
+// Workspace for batches of B candidates, from one allocation: an object per mesh
+// and box is made in a loop over them, and eleven of them were most of its cost.
 static bool hs_alloc(md_hspme* h, long B) {
-  const long Kt = h->g.Kt, nco = std::max(h->g.ncoef, 1);
-  return cudaMalloc(&h->Z, sizeof(double2) * B * Kt) == cudaSuccess &&
-         cudaMalloc(&h->F, sizeof(double2) * 2 * B * Kt) == cudaSuccess &&
-         cudaMalloc(&h->Y, sizeof(double2) * 2 * B * Kt) == cudaSuccess &&
-         cudaMalloc(&h->e2, sizeof(double) * B * Kt) == cudaSuccess &&
-         cudaMalloc(&h->w, sizeof(double) * B * Kt) == cudaSuccess &&
-         cudaMalloc(&h->bfac, sizeof(double) * B * 3 * h->Kmax) == cudaSuccess &&
-         cudaMalloc(&h->dbfac, sizeof(double) * B * 3 * nco * h->Kmax) == cudaSuccess &&
-         cudaMalloc(&h->marg, sizeof(double) * B * 3 * h->Kmax) == cudaSuccess &&
-         cudaMalloc(&h->cpart, sizeof(double) * B * h->nab * nco) == cudaSuccess &&
-         cudaMalloc(&h->lpart, sizeof(double) * B * h->nab) == cudaSuccess &&
-         cudaMalloc(&h->R, sizeof(double) * B * 3 * h->N) == cudaSuccess;
+  const size_t Kt = h->g.Kt, nco = std::max(h->g.ncoef, 1), b = B;
+  const struct { void** p; size_t doubles; } part[] = {
+      {(void**)&h->Z, 2 * b * Kt},          {(void**)&h->F, 4 * b * Kt},
+      {(void**)&h->Y, 4 * b * Kt},          {(void**)&h->e2, b * Kt},
+      {(void**)&h->w, b * Kt},              {(void**)&h->bfac, b * 3 * h->Kmax},
+      {(void**)&h->dbfac, b * 3 * nco * h->Kmax}, {(void**)&h->marg, b * 3 * h->Kmax},
+      {(void**)&h->cpart, b * h->nab * nco}, {(void**)&h->lpart, b * h->nab},
+      {(void**)&h->R, b * 3 * h->N}};
+  size_t bytes = 0;
+  for (const auto& q : part) bytes += (q.doubles * sizeof(double) + 255) & ~(size_t)255;
+  if (cudaMalloc(&h->slab, bytes) != cudaSuccess) {
+    h->slab = nullptr;
+    return false;
+  }
+  char* at = (char*)h->slab;
+  for (const auto& q : part) {
+    *q.p = at;
+    at += (q.doubles * sizeof(double) + 255) & ~(size_t)255;
+  }
+  return true;
 }
 
 // stencil widths 2 ceil(CC)

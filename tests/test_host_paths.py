@@ -308,3 +308,18 @@ def test_exact_sum_over_a_long_axis(lib):
     for K in ((1, 1, 2200000), (1, 2200000, 1), (2200000, 1, 1)):
         assert lib.md_ewald_exact(s, vec(C.c_int, *K), 1.0, C.byref(e), 1) == 0, lib.md_last_error_message()
     lib.md_system_destroy(s)
+
+
+def test_hermite_workspace_falls_back_to_smaller_batches(lib):
+    """one allocation; where memory does not hold a batch of four, two, and calls of more candidates go through"""
+    h = hermite(lib, 8)
+    full, calls = lib.fake_live(), lib.fake_calls()
+    lib.md_hspme_destroy(h)
+    lib.fake_fail_at(calls - 1)  # the last call of the creation: the workspace
+    h = hermite(lib, 8)
+    lib.fake_fail_at(NO_FAILURE)
+    assert abs(lib.fake_live() - full // 2) <= full // 8
+    buf = np.zeros(1 << 14)
+    p = buf.ctypes.data
+    assert lib.md_hspme_energy(h, p, p, p, 5, p, p, p, p, p, None) == 0
+    lib.md_hspme_destroy(h)
