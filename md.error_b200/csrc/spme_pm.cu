@@ -656,12 +656,15 @@ const void* gather_fn(int order, int mode) {
   return nullptr;
 }
 
-// The tile pays where many charges share its margins: binary32, 200,000
-// charges and more on at most 16 mesh points per charge (us, direct / tile of
-// 32 charges: 1,048,576 charges on 8 points each 300 / 232, 300,000 on 7 80 /
-// 73, 60,000 on 35 21 / 29, 20,736 on 13 9.4 / 11.9).  16 KB hold the stencils of
-// 32 charges in cell order at these densities.
-constexpr int SPREAD_TILE_MIN = 200000, SPREAD_TILE_PPC = 16, SPREAD_TILE_BYTES = 16 * 1024;
+// The tile pays where many charges share its margins: binary32, 200,000 charges and
+// more on at most 10 mesh points per charge (forces by analytic differentiation, us,
+// direct / tile of 32 charges at order 6 and 8: 1,000,000 charges on 8.4 points each
+// 709 / 669 and 1,177 / 1,027, on 16.8 994 / 1,073 and 1,459 / 1,463; 400,000 on 5.2 290 /
+// 272 and 486 / 394, on 10.5 309 / 307 and 500 / 474, on 21 360 / 421 and 554 / 553; 200,000 on
+// 5.2 171 / 164 and 274 / 228, on 10.5 175 / 180 and 275 / 265; at order 4 the two are within
+// 4 % of each other there).  16 KB hold the stencils of 32 charges in cell order at
+// these densities.
+constexpr int SPREAD_TILE_MIN = 200000, SPREAD_TILE_PPC = 10, SPREAD_TILE_BYTES = 16 * 1024;
 bool spread_by_tile(int prec, int N, const int K[3]) {
   return prec == MD_PREC_MIXED && N >= SPREAD_TILE_MIN && (double)K[0] * K[1] * K[2] / N <= SPREAD_TILE_PPC;
 }
