@@ -534,6 +534,9 @@ int plane_chain(md_system* sys, const PlaneChain& p, Recorder* rec) {
   {
     const Kernel k = plane_kernel(prec, p.n, p.method);
     void* args[] = {&a.C, &a.tw_n, &a.bm, &a.K2, &a.beta, &st, &a.partials, &a.with_stats, &a.merge, &a.back, &a.energy, &a.dbeta};
+    // two blocks a plane while all of them fit one an SM (whole forces, one / two blocks:
+    // 128 x 128 x 128, 65 planes, 81 / 66 us, x 256, 129 planes, 118 / 128; binary64 64 x 64 x 128
+    // 52 / 46, x 256 66 / 70)
     const int planes = p.K2 / 2 + 1;
     if (int r = rec_launch(rec, k.f, dim3(planes, ik && 2 * planes <= 148 ? 2 : 1), dim3(k.threads), k.smem, args))
       return r;
