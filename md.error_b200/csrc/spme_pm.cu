@@ -66,7 +66,8 @@ __device__ __forceinline__ void bsp_t(R f, R (&w)[NO], R (&dw)[NO]) {
 // are distinct, with plain loads and stores.  (Shared atomics run as a retry
 // loop; 64 charges per block of 256 threads with them took 415 us for
 // 1,048,576 charges on 128 x 128 x 512 at order 6, bound by the shared-memory
-// pipe at 76 wavefronts per charge; this takes 232 us.)  Weights are read for
+// pipe at 76 wavefronts per charge; this takes 232 us,
+// that pipe at 95 %.)  Weights are read for
 // four charges at once (they lie along the charges), and the tile's row
 // stride is +-n modulo the banks, so that the 32 / n rows of an instruction
 // fall on consecutive banks.  The tile is then added to the mesh with one
@@ -494,7 +495,7 @@ k_spme_gather_t(int N, const typename V4<R>::T* __restrict__ pos, int K0, int K1
 // that is one shared load and two FMA (the four products per point it
 // replaces needed 864 conversions an atom).  The weights are worked out once
 // per (atom, axis).  1,048,576 charges, order 6: 887 -> 334 us, now bound by
-// shared-memory wavefronts (73 %) and the staging latency; 20,736 in binary64:
+// shared-memory wavefronts (76 %) and the staging latency; 20,736 in binary64:
 // 31 -> 15 us.  A block whose region does not fit reads the mesh.
 __host__ __device__ constexpr int gather_lanes(int order) { return order <= 4 ? 4 : (order <= 8 ? 8 : 16); }
 constexpr int ADJ_ATOMS = 32;
